@@ -162,7 +162,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (b200_elect()) {
       unsigned int slot = 0, phase = 0;
       bool live = true;
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
@@ -217,7 +217,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (the leader CTA of a pair)
-    if (lane == 0 && cta_rank == 0u) {
+    if (cta_rank == 0u && b200_elect()) {
       unsigned int slot = 0, phase = 0, acc = 0, acc_phase = 0;
       bool live = true;
       // operand descriptors of ring slot 0.  k-major: rows of 128 bytes, 8-row groups 1024 bytes

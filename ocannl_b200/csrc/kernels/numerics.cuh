@@ -145,6 +145,12 @@ __device__ __forceinline__ float b200_tanh_fast(float x) {
   return y;
 }
 
+// the nearest tf32 value (the low 13 bits of the result are zero)
+__device__ __forceinline__ float b200_tf32(float f) {
+  b200_u32 u;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(f));
+  return __uint_as_float(u & 0xFFFFE000u);
+}
 __device__ __forceinline__ b200_u32 b200_bits32(float f) { return __float_as_uint(f); }
 __device__ __forceinline__ b200_u32 b200_bits32(b200_u32 u) { return u; }
 __device__ __forceinline__ b200_u32 b200_bits32(int i) { return (b200_u32)i; }

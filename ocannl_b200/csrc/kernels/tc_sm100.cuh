@@ -63,6 +63,18 @@ __device__ __forceinline__ bool b200_wait(unsigned int bar, unsigned int parity,
   }
 }
 
+// One thread of a converged warp, chosen by the hardware.  The roles that issue tcgen05.mma and TMA
+// copies enter through this instead of `lane == 0`: the compiler then knows that exactly one thread
+// runs the region and keeps descriptors and addresses in uniform registers.  Behind a comparison of
+// the lane index it moves every operand of every instruction there first; a 128 x 16 x 16 MMA was
+// issued every 67 cycles that way, every 44 behind the election (128 x 128: 65 either way, 128 x 256:
+// 130, the tensor pipe's own rate).
+__device__ __forceinline__ bool b200_elect() {
+  unsigned int p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0u;
+}
+
 // B200_CTA_PAIR: two CTAs of a cluster (one TPC) work on one 256 x BN tile.  Each stages its own
 // 128 rows of A and half of the BN columns of B; the even CTA (the leader) issues the
 // cta_group::2 MMAs, which read both CTAs' shared memory and write each CTA's 128 accumulator rows
