@@ -202,8 +202,26 @@ bool accum_form(const Stmt& st, int sid, int tn, std::string* op) {
 
 }  // namespace
 
+int64_t PackOp::rows() const {
+  int64_t r = kmajor ? 1 : seg * (split ? 3 : 1);
+  if (kmajor)
+    for (auto& a : mn) r *= a.extent;
+  for (auto& a : batch) r *= a.extent;
+  return r;
+}
+int64_t PackOp::bytes() const { return rows() * ld * prec_bytes(prec); }
+std::string PackOp::key() const {
+  std::ostringstream o;
+  o << tn << ":" << off << ":" << kmajor << ":" << ld << ":" << seg << ":" << split;
+  for (auto* v : {&batch, &mn, &k}) {
+    o << ";";
+    for (auto& a : *v) o << a.extent << "," << a.stride << " ";
+  }
+  return o.str();
+}
+
 double GemmPlan::flops() const {
-  double f = 2.0 * (double)m.extent * (double)n.extent * (double)k.extent;
+  double f = 2.0 * (double)m.extent * (double)n.extent * (double)k.extent / k_segments;
   for (auto& b : batch) f *= (double)b.extent;
   return f;
 }
@@ -1937,6 +1955,167 @@ struct Builder {
     return off;
   }
 
+  // Operands of a contraction that have to be gathered first (PackOp): one kernel fills the slots of both.
+  // A thread owns 16 bytes of a packed row: it takes the row apart into the operand's loops once and
+  // reads its 8 (4) elements one by one, so neither the alignment nor the layout of the node matters;
+  // neighbouring threads read neighbouring elements wherever the node has a contiguous axis.
+  // Contents are shared by the contractions of a routine (the three projections of an attention layer
+  // read one input) until some stage writes the node.
+  std::map<std::string, std::pair<int, size_t>> packed;   // key -> (slot, index of the stage that filled it)
+  void pack_stage(Stage& g) {
+    std::vector<const PackOp*> todo;
+    std::vector<int> slots;
+    for (auto& op : g.gemm.packs) {
+      const std::string key = op.key();
+      int slot = -1;
+      auto it = packed.find(key);
+      if (it != packed.end()) {
+        slot = it->second.first;
+        for (size_t i = it->second.second; i < code.stages.size() && slot >= 0; ++i) {
+          const Stage& st = code.stages[i];
+          if (std::count(st.writes.begin(), st.writes.end(), op.tn)) slot = -1;
+        }
+      }
+      if (slot < 0) {
+        slot = (int)code.pack_bytes.size();
+        code.pack_bytes.push_back((size_t)op.bytes());
+        packed[key] = {slot, code.stages.size()};
+        todo.push_back(&op);
+        slots.push_back(slot);
+      }
+      (&op == &g.gemm.packs[0] && g.gemm.pack_a ? g.gemm.a_slot : g.gemm.b_slot) = slot;
+    }
+    if (todo.empty()) return;
+    Stage st;
+    st.kind = Stage::Generic;
+    st.kernel = kernel_name();
+    st.block = 256;
+    std::ostringstream params, body;
+    std::set<int> nodes;
+    for (auto* op : todo) nodes.insert(op->tn);
+    for (auto& t : code.prog.tnodes)
+      if (nodes.count(t.id)) {
+        params << (params.tellp() > 0 ? ", " : "") << "const " << Emitter::ctype(t.prec) << "* __restrict__ " << t.ident;
+        st.args.push_back({KArg::Node, t.id});
+      }
+    int64_t total = 0;
+    std::string what;
+    for (size_t i = 0; i < todo.size(); ++i) {
+      const PackOp& op = *todo[i];
+      const std::string dst = "b200_pack" + std::to_string(slots[i]);
+      params << ", uint4* __restrict__ " << dst;
+      st.args.push_back({KArg::Pack, slots[i]});
+      st.pack_writes.push_back(slots[i]);
+      const int64_t first = total;
+      total += op.rows() * op.ld * prec_bytes(op.prec) / 16;
+      body << "    " << (i ? "else " : "") << "if (b200_g < " << total << "ull) {\n" << pack_body(op, dst, first) << "    }\n";
+      what += (i ? ", " : "") + code.prog.tn(op.tn).ident;
+    }
+    st.total = total;
+    st.note = "gathers operands of the next contraction into padded rows" + std::string(g.gemm.k_segments > 1 ? " (tf32 pairs)" : "") + ": " + what;
+    src << "extern \"C\" __global__ void __launch_bounds__(256) " << st.kernel << "(" << params.str() << ") {\n" << kGridEntry
+        << "  for (unsigned long long b200_g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_g < " << total
+        << "ull; b200_g += (unsigned long long)gridDim.x * blockDim.x) {\n" << body.str() << "  }\n}\n\n";
+    code.stages.push_back(st);
+  }
+  std::string pack_body(const PackOp& op, const std::string& dst, int64_t first) {
+    const std::string src_name = code.prog.tn(op.tn).ident;
+    const int eb = prec_bytes(op.prec), V = 16 / eb;
+    const int64_t groups = op.ld / V;
+    std::ostringstream o;
+    // 32-bit arithmetic throughout where the packed copy has fewer than 2^31 groups and the node fewer elements
+    const bool narrow = first + op.rows() * groups < (1ll << 31) && code.prog.tn(op.tn).num_elems() < (1ll << 31);
+    const std::string IT = narrow ? "unsigned int" : "unsigned long long", S = narrow ? "u" : "ull";
+    auto num = [&](int64_t v) { return std::to_string(v) + S; };
+    o << "      const " << IT << " i = (" << IT << ")(b200_g - " << first << "ull);\n"
+      << "      const " << IT << " grp = i % " << num(groups) << ", row = i / " << num(groups) << ";\n";
+    // `at`: adds the position `var` along the axes to the variable `acc`
+    int tmp = 0;
+    auto at = [&](const std::vector<PackOp::Axis>& axes, std::string var, const std::string& acc, const std::string& pad) {
+      std::string t;
+      for (size_t a = axes.size(); a-- > 0;) {
+        if (a == 0) {
+          t += pad + acc + " += (" + var + ") * " + num(axes[a].stride) + ";\n";
+        } else {
+          const std::string q = "q" + std::to_string(tmp++);
+          t += pad + acc + " += ((" + var + ") % " + num(axes[a].extent) + ") * " + num(axes[a].stride) + ";\n" + pad + "const " + IT + " " + q + " = (" + var +
+               ") / " + num(axes[a].extent) + ";\n";
+          var = q;
+        }
+      }
+      return t;
+    };
+    auto extent = [](const std::vector<PackOp::Axis>& axes) {
+      int64_t e = 1;
+      for (auto& a : axes) e *= a.extent;
+      return e;
+    };
+    const int64_t K = extent(op.k), MN = extent(op.mn);
+    const std::vector<PackOp::Axis>& inner = op.kmajor ? op.k : op.mn;
+    const int64_t outer_rows = op.kmajor ? MN : op.seg * (op.split ? 3 : 1);
+    o << "      " << IT << " base = " << num(op.off) << ";\n";
+    if (!op.batch.empty()) o << "      const " << IT << " bt = row / " << num(outer_rows) << ", rr = row % " << num(outer_rows) << ";\n" << at(op.batch, "bt", "base", "      ");
+    else o << "      const " << IT << " rr = row;\n";
+    const int64_t inner_real = op.kmajor ? K : MN;
+    std::string seg_of, in0;
+    if (op.kmajor) {
+      o << at(op.mn, "rr", "base", "      ");
+      if (op.split) {
+        o << "      const " << IT << " sg = (grp * " << V << S << ") / " << num(op.seg) << ", j0 = grp * " << V << S << " - sg * " << num(op.seg) << ";\n";
+      } else {
+        o << "      const " << IT << " j0 = grp * " << V << S << ";\n";
+      }
+      o << "      const bool row_ok = true;\n";
+    } else {
+      if (op.split) o << "      const " << IT << " sg = rr / " << num(op.seg) << ", kk = rr % " << num(op.seg) << ";\n";
+      else o << "      const " << IT << " kk = rr;\n";
+      o << "      const bool row_ok = kk < " << num(K) << ";\n" << at(op.k, "kk", "base", "      ") << "      const " << IT << " j0 = grp * " << V << S << ";\n";
+    }
+    const std::string T = Emitter::ctype(op.prec);
+    o << "      " << T << " v[" << V << "];\n#pragma unroll\n      for (unsigned int e = 0; e < " << V << "u; ++e) {\n"
+      << "        const " << IT << " j = j0 + e;\n        " << IT << " p = base;\n" << at(inner, "j", "p", "        ")
+      << "        v[e] = row_ok && j < " << num(inner_real) << " ? " << src_name << "[p] : (" << T << ")0;\n      }\n";
+    if (op.split) {
+      const std::string lo_seg = op.split == 1 ? "2" : "1";
+      o << "      b200_u32 w[4];\n#pragma unroll\n      for (int e = 0; e < 4; ++e) {\n        const float hi = b200_tf32(v[e]);\n"
+        << "        w[e] = __float_as_uint(sg == " << lo_seg << S << " ? b200_tf32(v[e] - hi) : hi);\n      }\n"
+        << "      " << dst << "[i] = make_uint4(w[0], w[1], w[2], w[3]);\n";
+    } else if (eb == 4) {
+      o << "      " << dst << "[i] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));\n";
+    } else {
+      o << "      " << dst << "[i] = make_uint4((b200_u32)v[0] | ((b200_u32)v[1] << 16), (b200_u32)v[2] | ((b200_u32)v[3] << 16), "
+        << "(b200_u32)v[4] | ((b200_u32)v[5] << 16), (b200_u32)v[6] | ((b200_u32)v[7] << 16));\n";
+    }
+    return o.str();
+  }
+  // Places the slots in the routine's scratch: a slot lives from the stage that fills it to the last
+  // contraction that reads it, and takes the lowest place no slot alive at the same time occupies (what
+  // was just read is then overwritten while it is still in L2).
+  void place_packs() {
+    const size_t n = code.pack_bytes.size();
+    std::vector<size_t> from(n, 0), to(n, 0);
+    for (size_t i = 0; i < code.stages.size(); ++i) {
+      for (int s : code.stages[i].pack_writes) from[(size_t)s] = to[(size_t)s] = i;
+      for (int s : {code.stages[i].gemm.a_slot, code.stages[i].gemm.b_slot})
+        if (s >= 0) to[(size_t)s] = i;
+    }
+    code.pack_offsets.assign(n, 0);
+    for (size_t s = 0; s < n; ++s) {
+      const size_t bytes = (code.pack_bytes[s] + 255) & ~(size_t)255;
+      std::vector<std::pair<size_t, size_t>> taken;
+      for (size_t q = 0; q < s; ++q)
+        if (from[q] <= to[s] && from[s] <= to[q]) taken.push_back({code.pack_offsets[q], code.pack_offsets[q] + ((code.pack_bytes[q] + 255) & ~(size_t)255)});
+      std::sort(taken.begin(), taken.end());
+      size_t off = 0;
+      for (auto& t : taken) {
+        if (off + bytes <= t.first) break;
+        off = std::max(off, t.second);
+      }
+      code.pack_offsets[s] = off;
+      code.pack_scratch_bytes = std::max(code.pack_scratch_bytes, off + bytes);
+    }
+  }
+
   // an epilogue that ends in a grid-wide sum keeps its per-warp partials and its ticket in the
   // routine's reduction scratch (zeroed at link; the kernel resets its ticket itself)
   void assign_epilogue_scratch(Stage& g) {
@@ -2145,6 +2324,7 @@ struct Builder {
           if (body->kind == Stmt::Set && body->tn == s->tn &&
               match_gemm(code.prog, nest, *body, true, opt, followers_after(flat, i + 2), &n_fused, &g)) {
             if (g.gemm.split_k > 1) memset_stage(s->tn);   // partial tiles are added to the zeroed node
+            pack_stage(g);
             assign_epilogue_scratch(g);
             g.kernel = kernel_name();
             g.gemm_source = gemm_translation_unit(code.prog, g, g.kernel, opt);
@@ -2216,6 +2396,7 @@ struct Builder {
           for (int f = 0; f < n_fused; ++f) zeroed.erase(fol[(size_t)f].set->tn);
           // beta = 0 over the whole node: the zero_out before it has no reader left
           if (was_zero && !g.gemm.accumulate && g.gemm.split_k == 1 && covers_node(*body, nest)) drop_zero_out(body->tn);
+          pack_stage(g);
           assign_epilogue_scratch(g);
           g.kernel = kernel_name();
           g.gemm_source = gemm_translation_unit(code.prog, g, g.kernel, opt);
@@ -2234,6 +2415,7 @@ struct Builder {
         for (size_t o = first; o <= i; ++o) code.stages[k].origins.push_back((int)o);
     }
     emit_kernels();
+    place_packs();
     code.source = src.str();
     if (opt.bounds) apply_bounds();
     // routine-local nodes that some stage touches get scratch (a node whose every use was fused

@@ -20,8 +20,8 @@ struct LoopDim {
 // One kernel argument: a tensor node pointer (in-context node, or a routine-local node that
 // lives in the routine's scratch slab), the static-index table, or the merge buffer.
 struct KArg {
-  enum Kind { Node, Statics, Merge, Scratch, Status } kind;   // Status: the device status word (range-checked builds)
-  int tn = -1;  // node id; for Scratch: byte offset into the routine's reduction scratch
+  enum Kind { Node, Statics, Merge, Scratch, Status, Pack } kind;   // Status: the device status word (range-checked builds)
+  int tn = -1;  // node id; for Scratch: byte offset into the routine's reduction scratch; for Pack: slot of a packed operand
 };
 
 // A dense contraction recognised in the loop nest, in GEMM terms:
@@ -30,6 +30,28 @@ struct KArg {
 struct GemmDim {
   int64_t extent = 1;
   int64_t sa = 0, sb = 0, sd = 0;  // element strides in A, B and the output
+};
+// An operand the tensor maps cannot describe where it lies (rows that are no multiple of 16 bytes, a
+// convolution's patches, an axis made of loops whose strides do not compose): a kernel ahead of the
+// contraction gathers it into the routine's scratch as rows padded to 16 bytes,
+//   k-major   [batch][m or n][k padded]      or      m/n-major   [batch][k][m or n padded],
+// whichever keeps the node's own contiguous axis.  Single-precision operands are stored as two
+// tf32 values, x = hi + lo, in three segments along k -- (hi, hi, lo) for A, (hi, lo, hi) for B -- so
+// that one pass of the tensor cores sums hi hi + hi lo + lo hi: the products keep 21 bits, where the
+// exact path they would otherwise take keeps 24.
+struct PackOp {
+  struct Axis { int64_t extent, stride; };
+  int tn = -1;
+  int64_t off = 0;                     // element offset of the operand's first element in its node
+  std::vector<Axis> batch, mn, k;      // outer to inner, strides in elements
+  bool kmajor = true;
+  int64_t ld = 0;                      // elements per packed row
+  int64_t seg = 0;                     // k positions per segment (k's extent, padded when split and k-major)
+  int split = 0;                       // 0: as stored; 1: hi, hi, lo; 2: hi, lo, hi
+  Prec prec = Prec::Bfloat16;
+  int64_t rows() const;                // packed rows
+  int64_t bytes() const;
+  std::string key() const;             // equal keys: equal contents
 };
 struct GemmPlan {
   int a_tn = -1, b_tn = -1, d_tn = -1;  // d_tn: the node the epilogue's Set writes
@@ -42,6 +64,10 @@ struct GemmPlan {
   bool may_split = false;            // an fp32 accumulation whose K may be cut into work units (see split_k)
   int split_k = 1;                   // >1: that many work units per tile, each over a slice of K, added with vector reds
   std::string epilogue;              // generated device code, see codegen
+  std::vector<PackOp> packs;         // operands to gather first (A before B)
+  bool pack_a = false, pack_b = false;
+  int a_slot = -1, b_slot = -1;      // scratch slots of the packed operands
+  int k_segments = 1;                // 3 when single-precision operands are split into tf32 pairs: k.extent counts all segments
   double flops() const;
 };
 
@@ -108,6 +134,7 @@ struct Stage {
   std::string note;              // human-readable classification, for debug info
   std::vector<int> origins;      // indices of the routine's top-level statements this stage runs
   std::vector<int> writes;       // nodes the stage writes
+  std::vector<int> pack_writes;  // slots of packed operands the stage fills
 };
 
 // A loop nest that follows a contraction and may be folded into its epilogue.
@@ -122,6 +149,10 @@ struct Code {
   std::string source;            // one translation unit holding every generic kernel
   std::vector<int> local_nodes;  // routine-local nodes that need scratch
   size_t reduce_scratch_bytes = 0;  // partial results of grid-wide reductions
+  // packed operands: size and place of every slot in their part of the routine's scratch.  Slots whose
+  // stages do not overlap share memory.
+  std::vector<size_t> pack_bytes, pack_offsets;
+  size_t pack_scratch_bytes = 0;
   std::string describe() const;  // JSON-ish summary for b200_code_info
 };
 

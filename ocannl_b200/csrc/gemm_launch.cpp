@@ -80,7 +80,8 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
     return it->second;
   };
   const int eb = prec_bytes(g.in_prec);
-  CUdeviceptr a = ptr(g.a_tn) + (CUdeviceptr)(g.a_off * eb), b = ptr(g.b_tn) + (CUdeviceptr)(g.b_off * eb);
+  CUdeviceptr a = (g.pack_a ? r->pack_address(g.a_slot) : ptr(g.a_tn)) + (CUdeviceptr)(g.a_off * eb);
+  CUdeviceptr b = (g.pack_b ? r->pack_address(g.b_slot) : ptr(g.b_tn)) + (CUdeviceptr)(g.b_off * eb);
   if ((a & 15) || (b & 15))
     throw Error(B200_E_INVALID, "link: internal error: a contraction stage was kept for operands that are not 16-byte aligned");
   auto* L = new GemmLaunch();

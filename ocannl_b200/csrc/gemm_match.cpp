@@ -45,7 +45,13 @@ bool strides_of(const Tnode& t, const Indices& idcs, std::map<std::string, int64
     const Index& ix = idcs[a];
     if (ix.kind == Index::Iter) stride[ix.sym] += s;
     else if (ix.kind == Index::Fixed) const_off += ix.fixed * s;
-    else return false;
+    else if (ix.kind == Index::Affine) {   // c1 * i + c2 * j + fixed: still linear in every symbol
+      for (auto& term : ix.terms) {
+        if (term.first < 0) return false;
+        stride[term.second] += term.first * s;
+      }
+      const_off += ix.fixed * s;
+    } else return false;
     s *= t.dims[a];
   }
   return true;
@@ -302,42 +308,150 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (s.extent == 1) continue;
     gk.push_back(Dim{{{s.sym, s.extent}}, s.extent, s.sa, s.sb, 0});
   }
+  const std::vector<Dim> all_m = gm, all_n = gn, all_k = gk, all_b = gb;
   merge(gm); merge(gn); merge(gk); merge(gb);
   // leftover outer M / N dims become batch axes along which one operand is broadcast
   while (gm.size() > 1) { gb.push_back(gm.front()); gm.erase(gm.begin()); }
   while (gn.size() > 1) { gb.push_back(gn.front()); gn.erase(gn.begin()); }
-  if (gm.size() != 1 || gn.size() != 1 || gk.size() != 1 || gb.size() > 2) return false;
-  const Dim &dm = gm[0], &dn = gn[0], &dk = gk[0];
 
   GemmPlan g;
   g.a_tn = x->tn;
   g.b_tn = y->tn;
   g.d_tn = set.tn;
-  g.m = {dm.extent, dm.sa, 0, dm.sd};
-  g.n = {dn.extent, 0, dn.sb, dn.sd};
-  g.k = {dk.extent, dk.sa, dk.sb, 0};
-  for (auto& d : gb) g.batch.push_back({d.extent, d.sa, d.sb, d.sd});
   g.a_off = offx;
   g.b_off = offy;
   g.in_prec = A.prec;
   g.accumulate = form_b && !zeroed_before;
-  if (g.k.sa == 1) g.a_kmajor = true;
-  else if (g.m.sa == 1) g.a_kmajor = false;
-  else return false;
-  if (g.k.sb == 1) g.b_kmajor = true;
-  else if (g.n.sb == 1) g.b_kmajor = false;
-  else return false;
-
-  // ---- what the tensor maps can express: 16-byte aligned bases and strides, 32-bit extents
   const int eb = prec_bytes(A.prec);
   auto ok16 = [&](int64_t elems) { return (elems * eb) % 16 == 0; };
-  if (!ok16(g.a_off) || !ok16(g.b_off)) return false;
-  if (!ok16(g.a_kmajor ? g.m.sa : g.k.sa) || !ok16(g.b_kmajor ? g.n.sb : g.k.sb)) return false;
-  for (auto& b : g.batch)
-    if ((b.sa && !ok16(b.sa)) || (b.sb && !ok16(b.sb))) return false;
+
+  // ---- what the tensor maps can express: 16-byte aligned bases and strides, 32-bit extents, one axis
+  // each for m, n and k, unit stride along k or along m / n
+  auto as_it_lies = [&] {
+    if (gm.size() != 1 || gn.size() != 1 || gk.size() != 1 || gb.size() > 2) return false;
+    g.m = {gm[0].extent, gm[0].sa, 0, gm[0].sd};
+    g.n = {gn[0].extent, 0, gn[0].sb, gn[0].sd};
+    g.k = {gk[0].extent, gk[0].sa, gk[0].sb, 0};
+    g.batch.clear();
+    for (auto& d : gb) g.batch.push_back({d.extent, d.sa, d.sb, d.sd});
+    if (g.k.sa == 1) g.a_kmajor = true;
+    else if (g.m.sa == 1) g.a_kmajor = false;
+    else return false;
+    if (g.k.sb == 1) g.b_kmajor = true;
+    else if (g.n.sb == 1) g.b_kmajor = false;
+    else return false;
+    if (!ok16(g.a_off) || !ok16(g.b_off)) return false;
+    if (!ok16(g.a_kmajor ? g.m.sa : g.k.sa) || !ok16(g.b_kmajor ? g.n.sb : g.k.sb)) return false;
+    for (auto& b : g.batch)
+      if ((b.sa && !ok16(b.sa)) || (b.sb && !ok16(b.sb))) return false;
+    // neighbouring convolution patches overlap; only a gathered copy has them one after the other
+    return true;
+  };
+  auto product = [](const std::vector<Dim>& v) {
+    int64_t p = 1;
+    for (auto& d : v) p *= d.extent;
+    return p;
+  };
+  auto worth = [&](int64_t m, int64_t n, int64_t k, int64_t batch) {
+    return m >= 32 && n >= 8 && k >= 16 && 2.0 * (double)m * (double)n * (double)k * (double)batch >= 4.0e6;
+  };
+  if (as_it_lies()) {
+    if (!worth(g.m.extent, g.n.extent, g.k.extent, product(gb))) return false;
+  } else {
+    // ---- gather what the maps cannot express.  m, n, k and the batch become one axis each, the
+    // loops concatenated outer to inner; an operand that already lies that way stays where it is.
+    if (!worth(product(all_m), product(all_n), product(all_k), product(all_b))) return false;
+    if (all_m.empty() || all_n.empty() || all_k.empty()) return false;
+    auto concat = [&](const std::vector<Dim>& v) {
+      Dim d;
+      for (auto& e : v) {
+        d.syms.insert(d.syms.end(), e.syms.begin(), e.syms.end());
+        d.extent *= e.extent;
+      }
+      return d;
+    };
+    // do the strides of one operand compose to a single one along the axis?
+    auto composes = [](const std::vector<Dim>& v, bool of_a, int64_t* stride) {
+      *stride = v.empty() ? 0 : (of_a ? v.back().sa : v.back().sb);
+      for (size_t i = 0; i + 1 < v.size(); ++i)
+        if ((of_a ? v[i].sa : v[i].sb) != (of_a ? v[i + 1].sa : v[i + 1].sb) * v[i + 1].extent) return false;
+      return true;
+    };
+    gm = {concat(all_m)};
+    gn = {concat(all_n)};
+    gk = {concat(all_k)};
+    gb.clear();
+    if (!all_b.empty()) gb = {concat(all_b)};
+    g.m = {gm[0].extent, 0, 0, 0};
+    g.n = {gn[0].extent, 0, 0, 0};
+    g.k = {gk[0].extent, 0, 0, 0};
+    g.batch.clear();
+    if (!gb.empty()) g.batch = {{gb[0].extent, 0, 0, 0}};
+    const bool split = A.prec == Prec::Single;   // both operands as tf32 pairs
+    for (int side = 0; side < 2; ++side) {
+      const bool of_a = side == 0;
+      const std::vector<Dim>& mn = of_a ? all_m : all_n;
+      int64_t s_mn, s_k, s_b;
+      const int64_t off = of_a ? g.a_off : g.b_off;
+      bool lies = composes(mn, of_a, &s_mn);
+      lies = composes(all_k, of_a, &s_k) && lies;
+      lies = composes(all_b, of_a, &s_b) && lies;
+      lies = lies && !split && (s_k == 1 || s_mn == 1) && ok16(off) && ok16(s_k == 1 ? s_mn : s_k) && ok16(s_b);
+      bool kmajor = s_k == 1;
+      if (!lies) {
+        PackOp op;
+        op.tn = of_a ? g.a_tn : g.b_tn;
+        op.off = off;
+        op.prec = A.prec;
+        auto axes = [&](const std::vector<Dim>& v, std::vector<PackOp::Axis>* out) {
+          for (auto& d : v) {
+            const int64_t st = of_a ? d.sa : d.sb;
+            if (!out->empty() && out->back().stride == st * d.extent) out->back() = {out->back().extent * d.extent, st};
+            else out->push_back({d.extent, st});
+          }
+        };
+        axes(all_b, &op.batch);
+        axes(mn, &op.mn);
+        axes(all_k, &op.k);
+        op.kmajor = op.k.back().stride == 1 || op.mn.back().stride != 1;
+        kmajor = op.kmajor;
+        op.split = split ? (of_a ? 1 : 2) : 0;
+        op.seg = g.k.extent;
+        const int64_t unit = 16 / eb;
+        const int64_t inner = kmajor ? g.k.extent : (of_a ? g.m.extent : g.n.extent);
+        const int64_t padded = (inner + unit - 1) / unit * unit;
+        op.ld = kmajor ? padded * (split ? 3 : 1) : padded;
+        if (op.bytes() > (2ll << 30)) return false;   // the copy would cost more memory than it is worth
+        const int64_t rows = kmajor ? (of_a ? g.m.extent : g.n.extent) : g.k.extent * (split ? 3 : 1);
+        s_mn = kmajor ? op.ld : 1;
+        s_k = kmajor ? 1 : op.ld;
+        s_b = rows * op.ld;
+        (of_a ? g.pack_a : g.pack_b) = true;
+        (of_a ? g.a_off : g.b_off) = 0;
+        g.packs.push_back(op);
+      }
+      if (of_a) { g.m.sa = s_mn; g.k.sa = s_k; g.a_kmajor = kmajor; }
+      else { g.n.sb = s_mn; g.k.sb = s_k; g.b_kmajor = kmajor; }
+      if (!g.batch.empty()) (of_a ? g.batch[0].sa : g.batch[0].sb) = s_b;
+    }
+    if (split) {
+      // the segments of a k-major operand start at padded positions: both operands use the same ones
+      const bool any_kmajor = g.a_kmajor || g.b_kmajor;
+      const int64_t seg = any_kmajor ? (g.k.extent + 3) / 4 * 4 : g.k.extent;
+      g.k_segments = 3;
+      for (auto& op : g.packs) {
+        op.seg = seg;
+        if (!op.kmajor) {
+          // rows of the m/n-major form: one per position of every segment
+          const int64_t s_b = 3 * seg * op.ld;
+          if (!g.batch.empty()) (&op == &g.packs[0] ? g.batch[0].sa : g.batch[0].sb) = s_b;
+        }
+      }
+      g.k.extent = 3 * seg;
+    }
+  }
   if (g.m.extent >= (1ll << 31) || g.n.extent >= (1ll << 31) || g.k.extent >= (1ll << 31)) return false;
-  // ---- worth a tensor-core launch?
-  if (g.m.extent < 32 || g.n.extent < 8 || g.k.extent < 16 || g.flops() < 4.0e6) return false;
+  const Dim &dm = gm[0], &dn = gn[0];
   (void)B;
   (void)opt;
 
@@ -404,7 +518,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // pair mode: b200_j counts PAIRS of columns; tiles hold one pair per entry.  Neighbouring columns
   // differ only in the innermost n symbol as long as its loop has an even length.
   // (a materialised accumulate that reads its output back stays in the one-column form)
-  if (pair && ((form_b && g.accumulate) || n_sym.empty() || g.n.extent % 2 != 0 || dn.syms.back().second % 2 != 0)) return false;
+  // an odd row length is fine when n is one loop: the pair across its end is clipped like every column
+  // beyond N, as long as nothing of it is read from memory by itself (checked below)
+  const bool odd_n = g.n.extent % 2 != 0;
+  if (pair && ((form_b && g.accumulate) || n_sym.empty() || (n_syms == 1 ? false : (odd_n || dn.syms.back().second % 2 != 0)))) return false;
   em.pair = pair;
   em.pair_sym = n_sym;
   bool pair_fail = false;
@@ -973,7 +1090,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   }
   fused += row_fused;
   *n_fused = fused;
-  if (pair_fail) return false;
+  if (pair_fail || (pair && odd_n && em.direct_reads > 0)) return false;
 
   // ---- outputs as TMA stores.  A chunk (32 rows of the warp x the chunk's columns) that sits in the
   // staging tile leaves with one copy instruction when the node is a regular [batch.., m, n] array
@@ -1163,7 +1280,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // the accumulator chunk is consumed: start fetching the next one while this one is stored
   // ... or, after the tile's last chunk, the operand tiles of the first chunk of this warp's NEXT
   // tile: their latency then hides behind this chunk's stores and the wait for the next accumulator
-  fn << "  B200_TRE(13);\n  if (b200_has_next) {\n    b200_tmem_ld_chunk(b200_next_taddr, b200_r);\n"
+  fn << "  B200_TRE(13);\n  if (b200_has_next) {\n#if !B200_FLUSH\n    b200_tmem_ld_chunk(b200_next_taddr, b200_r);\n#endif\n"
      << "    b200_epilogue_load(b200_t, b200_b0, b200_b1, b200_m, b200_row_ok, b200_n0 + B200_EPI_CHUNK, b200_N, b200_es" << args << ");\n"
      << "  } else if (b200_nx_ok) {\n"
      << "    b200_epilogue_load(b200_t, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_row_ok, b200_nx_n0, b200_N, b200_es" << args << ");\n  }\n  B200_TRE(10);\n";
@@ -1255,20 +1372,33 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
                     : "        if (dst) *(uint4*)(dst + (unsigned long long)b200_n0 * ")
            << ebytes << (reds ? "ull + 16ull * c, q);\n      }\n" : "ull + 16ull * c) = q;\n      }\n")
            << "      B200_TRE(12);\n      __syncwarp();\n      B200_TRE(11);\n"
-           << "    } else if (b200_row_ok) {\n";
+           // Rows that are no multiple of 16 bytes long (odd row lengths), or a chunk that ends beyond N:
+           // the chunk goes through the same staging tile, then the lanes take neighbouring elements of
+           // one row, so that a store instruction covers one stretch of it instead of 32 rows.
+           << "    } else {\n      uint4* b200_tile = b200_stage;\n"
+           << sts_code(o)
+           << "      __syncwarp();\n      constexpr unsigned int V = " << V << "u, R = 32u / B200_EPI_CHUNK;   // elements per group, rows per step\n"
+           << "      const unsigned int b200_c = b200_lane % B200_EPI_CHUNK;\n"
+           << "#pragma unroll 8\n      for (unsigned int it = 0; it < 32u / R; ++it) {\n"
+           << "        const unsigned int r = it * R + b200_lane / B200_EPI_CHUNK;\n"
+           << "        " << T << "* const b200_q = (" << T << "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, r);\n"
+           << "        const " << T << " b200_v = ((const " << T << "*)(b200_stage + r * G + ((b200_c / V) ^ B200_STAGE_KEY(r, G))))[b200_c % V];\n"
+           << "        if (b200_q && b200_n0 + b200_c < b200_N) "
+           << (reds ? "atomicAdd(&b200_q[b200_c], b200_v);\n" : "b200_q[b200_c] = b200_v;\n")
+           << "      }\n      __syncwarp();\n";
       } else {
         fn << "    if (b200_row_ok) {\n";
+        fn << "#pragma unroll\n      for (int b200_j = 0; b200_j < B200_EPI_CHUNK; ++b200_j)\n";
+        if (reds)
+          fn << "        if (b200_n0 + (unsigned int)b200_j < b200_N) atomicAdd(&b200_p[b200_j], "
+             << (pair ? "((b200_j & 1) ? " + o.arr + "[b200_j >> 1].y : " + o.arr + "[b200_j >> 1].x)" : o.arr + "[b200_j]") << ");\n";
+        else
+          fn << "        if (b200_n0 + (unsigned int)b200_j < b200_N) b200_p[b200_j] = "
+             << (!pair ? Emitter::store_wrap(t.prec, o.arr + "[b200_j]")
+                       : ebytes == 4 ? "((b200_j & 1) ? " + o.arr + "[b200_j >> 1].y : " + o.arr + "[b200_j >> 1].x)"
+                                     : "(unsigned short)(" + o.arr + "[b200_j >> 1] >> (16 * (b200_j & 1)))")
+             << ";\n";
       }
-      fn << "#pragma unroll\n      for (int b200_j = 0; b200_j < B200_EPI_CHUNK; ++b200_j)\n";
-      if (reds)
-        fn << "        if (b200_n0 + (unsigned int)b200_j < b200_N) atomicAdd(&b200_p[b200_j], "
-           << (pair ? "((b200_j & 1) ? " + o.arr + "[b200_j >> 1].y : " + o.arr + "[b200_j >> 1].x)" : o.arr + "[b200_j]") << ");\n";
-      else
-        fn << "        if (b200_n0 + (unsigned int)b200_j < b200_N) b200_p[b200_j] = "
-           << (!pair ? Emitter::store_wrap(t.prec, o.arr + "[b200_j]")
-                     : ebytes == 4 ? "((b200_j & 1) ? " + o.arr + "[b200_j >> 1].y : " + o.arr + "[b200_j >> 1].x)"
-                                   : "(unsigned short)(" + o.arr + "[b200_j >> 1] >> (16 * (b200_j & 1)))")
-           << ";\n";
       fn << "    }\n" << (vec ? "    }\n" : "") << "  }\n";
     } else {
       // general position: recompute the offset per column
@@ -1329,9 +1459,15 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
   double best = 1e300;
   int best_bn = bn0;
   bool best_pair = false;
-  for (int pair = 1; pair >= 0; --pair) {
-    for (int bn = bn0; bn >= 16; bn = (bn > 64 ? bn / 2 : 0)) {
-      if (bn != bn0 && (bn % 64 != 0 || (!g.b_kmajor && bn % row_elems != 0))) continue;
+  const bool flush = g.k_segments > 1;   // running sums in registers: at most 64 columns per epilogue thread
+  std::vector<int> widths = {bn0};
+  // (an output row of up to 32 columns stays in one tile: assignments over whole rows may follow it)
+  if (bn0 > 32) for (int w : {128, 64, 32, 16})
+    if (w != bn0 && (w < bn0 || (flush && bn0 > 64 && w == 128))) widths.push_back(w);
+  for (int pair = flush ? 0 : 1; pair >= 0; --pair) {
+    for (int bn : widths) {
+      if (flush && bn != 16 && bn != 32 && bn != 64 && bn != 128) continue;
+      if (bn != bn0 && !g.b_kmajor && bn % row_elems != 0) continue;
       // two CTAs per 256 x bn tile need a full pair tile of rows; each CTA stages half of B
       if (pair && !(g.m.extent >= 256 && bn >= 64 && bn % 32 == 0 && (g.b_kmajor || (bn / 2) % row_elems == 0))) continue;
       const long long bm = pair ? 256 : 128, workers = pair ? 74 : 148;
@@ -1421,7 +1557,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
     << "\n#define B200_STAGES " << stages << "\n#define B200_EPI_WARPS " << epi_warps << "\n#define B200_A_KMAJOR "
     << (g.a_kmajor ? 1 : 0) << "\n#define B200_B_KMAJOR " << (g.b_kmajor ? 1 : 0) << "\n#define B200_IDESC " << idesc
     << "u\n#define B200_TMEM_COLS " << tmem_cols << "\n#define B200_RASTER " << raster << "\n#define B200_CTA_PAIR "
-    << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n";
+    << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n#define B200_FLUSH " << (g.k_segments > 1 ? 2 : 0) << "\n";
   o << "#define B200_EPI_CHUNK " << chunk << "\n#define B200_STAGING_BYTES " << staging << "\n#define B200_STAGING_TILES " << staging_tiles << "\n#define B200_LOAD_TILE_BYTES " << load_tile << "\n";
   o << "#define B200_EPI_PROLOGUE " << [&] { std::string p = st.epi_prologue; for (auto& c : p) if (c == '\n') c = ' '; return p; }() << "\n";
   o << kTcSource << "\n" << g.epilogue << "\n";
@@ -1431,7 +1567,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   o << "#define B200_EPILOGUE_ROW b200_epilogue_row(b200_r, b200_b0, b200_b1, b200_m, b200_m < shape.M, b200_n0, shape.N, b200_stage, b200_has_next, b200_next_taddr, b200_tiles, b200_slot, b200_nslots, b200_nx_ok, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_m < shape.M, b200_nx_n0, b200_es" << args << ");\n";
   o << kGemmSource << "\n";
   std::ostringstream note;
-  note << "tcgen05 " << (g.in_prec == Prec::Single ? "tf32 " : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages
+  note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.k_segments > 1 ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages
        << " epi_warps=" << epi_warps << (g.split_k > 1 ? " split_k=" + std::to_string(g.split_k) : std::string())
        << (g.accumulate ? " beta=1" : "")
        << (st.row_followers ? " + " + std::to_string(st.row_followers) + " whole-row assignments in the epilogue" +

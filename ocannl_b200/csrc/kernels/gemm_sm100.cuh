@@ -88,6 +88,14 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 #ifndef B200_SPLITK
 #define B200_SPLITK 1
 #endif
+// B200_FLUSH > 0: the accumulator leaves tensor memory every B200_FLUSH k blocks and is summed in the
+// epilogue threads' registers.  The tensor cores cut every addition into the accumulator off instead of
+// rounding it, which after n MMAs has moved a sum by about n 2^-25 of itself towards zero: too much for
+// operands that travel as tf32 pairs and are meant to keep single precision (3e-6 at K = 131, growing
+// with K).  Short runs that are added up with rounding stay within what a chain of fp32 additions does.
+#ifndef B200_FLUSH
+#define B200_FLUSH 0
+#endif
 
 extern "C" __global__ void __launch_bounds__(B200_THREADS, 1)
 B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ b200_tmap map_b,
@@ -237,30 +245,35 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
         const unsigned int split = unit / total_tiles;
         const unsigned int kb0 = split * k_blocks / B200_SPLITK, kb1 = (split + 1u) * k_blocks / B200_SPLITK;
-        if (!b200_wait(bar_acc_empty + 8u * acc, acc_phase ^ 1u, abort_flag, status, 2u)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned int d_tmem = tmem_base + acc * B200_BN;
-        for (unsigned int kb = kb0; kb < kb1; ++kb) {
-          if (!b200_wait(bar_full + 8u * slot, phase, abort_flag, status, 3u)) { live = false; break; }
+        for (unsigned int kbf = kb0; live && kbf < kb1;) {
+          // one run of k blocks into one accumulator buffer: the whole unit, or B200_FLUSH blocks of it
+          const unsigned int kbe = B200_FLUSH ? min(kbf + (unsigned int)B200_FLUSH, kb1) : kb1;
+          if (!b200_wait(bar_acc_empty + 8u * acc, acc_phase ^ 1u, abort_flag, status, 2u)) { live = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (unit == worker && kb == kb0) B200_TR(5);   // first operands landed
-          // descriptors of this slot: the start-address field (bits 0-13, address >> 4) moves, the rest is fixed
-          const unsigned long long da0 = desc_a0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
-          const unsigned long long db0 = desc_b0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
+          const unsigned int d_tmem = tmem_base + acc * B200_BN;
+          for (unsigned int kb = kbf; kb < kbe; ++kb) {
+            if (!b200_wait(bar_full + 8u * slot, phase, abort_flag, status, 3u)) { live = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (unit == worker && kb == kb0) B200_TR(5);   // first operands landed
+            // descriptors of this slot: the start-address field (bits 0-13, address >> 4) moves, the rest is fixed
+            const unsigned long long da0 = desc_a0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
+            const unsigned long long db0 = desc_b0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
 #pragma unroll
-          for (unsigned int ks = 0; ks < B200_BK / B200_UMMA_K; ++ks) {
-            // a k step moves UMMA_K elements along a k-major row, or UMMA_K rows of 128 bytes in the m/n-major form
-            const unsigned long long da = da0 + (unsigned long long)((ks * (B200_A_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
-            const unsigned long long db = db0 + (unsigned long long)((ks * (B200_B_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
-            b200_umma(d_tmem, da, db, (unsigned int)B200_IDESC, (kb != kb0 || ks != 0u) ? 1u : 0u);
+            for (unsigned int ks = 0; ks < B200_BK / B200_UMMA_K; ++ks) {
+              // a k step moves UMMA_K elements along a k-major row, or UMMA_K rows of 128 bytes in the m/n-major form
+              const unsigned long long da = da0 + (unsigned long long)((ks * (B200_A_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
+              const unsigned long long db = db0 + (unsigned long long)((ks * (B200_B_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
+              b200_umma(d_tmem, da, db, (unsigned int)B200_IDESC, (kb != kbf || ks != 0u) ? 1u : 0u);
+            }
+            b200_umma_commit(bar_empty + 8u * slot);  // frees the slot once these MMAs retire
+            if (++slot == B200_STAGES) { slot = 0; phase ^= 1u; }
           }
-          b200_umma_commit(bar_empty + 8u * slot);  // frees the slot once these MMAs retire
-          if (++slot == B200_STAGES) { slot = 0; phase ^= 1u; }
+          if (live) b200_umma_commit(bar_acc_full + 8u * acc);
+          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+          kbf = kbe;
         }
-        if (live) b200_umma_commit(bar_acc_full + 8u * acc);
         if (unit == worker) B200_TR(6);                  // tile 0 MMAs issued
         else if (unit == worker + n_workers) B200_TR(7); // tile 1 MMAs issued
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
     }
   } else {
@@ -324,6 +337,48 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
         if (b200_pn0 < shape.N) { B200_EPILOGUE_LOAD }
       }
       b200_prefetched = b200_nx_ok && (nt * B200_BN + col_half * cols_per_warp < shape.N);
+#if B200_FLUSH
+      constexpr int kCols = (B200_BN / (B200_EPI_WARPS / 4) + B200_EPI_CHUNK - 1) / B200_EPI_CHUNK * B200_EPI_CHUNK;
+      const unsigned int col0 = col_half * cols_per_warp;
+      float b200_sum[kCols];
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) b200_sum[j] = 0.0f;
+      {
+        const unsigned int split = unit / total_tiles;
+        const unsigned int kb0 = split * k_blocks / B200_SPLITK, kb1 = (split + 1u) * k_blocks / B200_SPLITK;
+        bool got = true;
+        for (unsigned int kbf = kb0; kbf < kb1; kbf += B200_FLUSH) {
+          got = b200_wait(bar_acc_full + 8u * acc, acc_phase, abort_flag, status, 4u);
+          if (!got) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const unsigned int taddr = tmem_base + acc * B200_BN + ((quarter * 32u) << 16) + col0;
+#pragma unroll
+          for (int c = 0; c < kCols; c += B200_EPI_CHUNK) {
+            unsigned int part[B200_EPI_CHUNK];
+            b200_tmem_ld_chunk(taddr + c, part);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < B200_EPI_CHUNK; ++j) b200_sum[c + j] += __uint_as_float(part[j]);
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) b200_mbar_arrive_relaxed(bar_acc_empty + 8u * acc);
+          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        }
+        if (!got) break;
+      }
+#pragma unroll
+      for (int c = 0; c < kCols; c += B200_EPI_CHUNK) {
+        const unsigned int b200_n0 = nt * B200_BN + col0 + c;
+        if (b200_n0 >= shape.N) break;  // warp-uniform
+        unsigned int b200_r[B200_EPI_CHUNK];
+#pragma unroll
+        for (int j = 0; j < B200_EPI_CHUNK; ++j) b200_r[j] = __float_as_uint(b200_sum[c + j]);
+        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < shape.N);
+        const unsigned int b200_next_taddr = tmem_base;   // (a load that nothing reads)
+        B200_EPILOGUE_ROW
+      }
+#else
       if (!b200_wait(bar_acc_full + 8u * acc, acc_phase, abort_flag, status, 4u)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (warp == 2 && lane == 0) { if (unit == worker) B200_TR(8); else if (unit == worker + n_workers) B200_TR(10); }
@@ -360,6 +415,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
 #endif
       if (warp == 2 && lane == 0) { if (unit == worker) B200_TR(9); else if (unit == worker + n_workers) B200_TR(11); }
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+#endif
 #ifdef B200_TRACE
       B200_TRE(5);   // release of the accumulator buffer
 #endif

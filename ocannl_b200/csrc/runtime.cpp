@@ -81,7 +81,8 @@ static bool misaligned_stages(const b200_code* c, const std::map<int, CUdevicept
       const int eb = prec_bytes(st.gemm.in_prec);
       const CUdeviceptr a = at(st.gemm.a_tn) + (CUdeviceptr)(st.gemm.a_off * eb), b = at(st.gemm.b_tn) + (CUdeviceptr)(st.gemm.b_off * eb);
       (void)P;
-      if ((a & 15) || (b & 15))
+      // (a packed operand lies in the routine's own scratch)
+      if ((!st.gemm.pack_a && (a & 15)) || (!st.gemm.pack_b && (b & 15)))
         for (int o : st.origins) any |= no_gemm_at->insert(o).second;
     } else if (st.kind == Stage::Attn) {
       // tensor maps over the queries, keys and values; 16-byte row stores into every node it writes
@@ -145,6 +146,9 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
   }
   const size_t reduce_off = off;
   off += c->code.reduce_scratch_bytes;
+  off = (off + 255) & ~(size_t)255;
+  pack_base = off;
+  off += c->code.pack_scratch_bytes;
   scratch_bytes = off;
   if (scratch_bytes) {
     cu_check(cu().cuMemAlloc_(&scratch, scratch_bytes), "cuMemAlloc(scratch)");
@@ -193,6 +197,8 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
         arg_values[i].push_back(statics_dev);
       } else if (a.kind == KArg::Scratch) {
         arg_values[i].push_back(scratch + reduce_off + (size_t)a.tn);
+      } else if (a.kind == KArg::Pack) {
+        arg_values[i].push_back(pack_address(a.tn));
       } else {
         arg_values[i].push_back(0);  // merge buffer: resolved at launch (pool 0 may be re-allocated)
         reads_merge = true;

@@ -130,6 +130,8 @@ struct b200_routine {
   std::map<int, CUdeviceptr> node_ptr;
   CUdeviceptr scratch = 0;                         // routine-local nodes
   size_t scratch_bytes = 0;
+  size_t pack_base = 0;                            // packed operands of contractions lie behind this offset of the scratch slab
+  CUdeviceptr pack_address(int slot) const { return scratch + pack_base + code->code.pack_offsets.at((size_t)slot); }
   std::vector<std::pair<size_t, size_t>> scratch_zero;  // (offset, bytes) cleared every run
   CUdeviceptr statics_dev = 0;
   unsigned int* statics_ring = nullptr;            // page-locked staging

@@ -1,0 +1,72 @@
+"""Contractions whose operands the tensor maps cannot describe where they lie: they are gathered into
+padded rows first and run on the tensor-core path.  Sizes at the edges of that copy: odd row lengths
+in either layout, one element short of and past a 16-byte group, axes made of several loops, affine
+positions, odd output rows.  16-bit operands: the tolerance of bf16 contractions; single-precision
+operands travel as tf32 pairs and keep the tolerance of single precision."""
+import numpy as np
+import pytest
+
+from ocannl_b200 import workloads as W
+from ocannl_b200.low_level import Affine, Routine, Seq, Set, loops, un
+from tests.parity import compare, run_device, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _mm(b, m, n, k, prec, a_mmajor, b_nmajor, act):
+    r = Routine("packed_%d_%d_%d_%d" % (b, m, n, k))
+    x = r.tn("x", prec, [b, k, m] if a_mmajor else [b, m, k], read_only=True)
+    w = r.tn("w", prec, [b, k, n] if b_nmajor else [b, n, k], read_only=True)
+    bias = r.tn("bias", "single", [n], read_only=True)
+    y = r.tn("y", prec, [b, m, n])
+    ib, i, j, kk = r.syms(4)
+    acc = W.reduce_scope(r, "acc", "single", [(kk, k)], lambda: (x[ib, kk, i] if a_mmajor else x[ib, i, kk],
+                                                                 w[ib, kk, j] if b_nmajor else w[ib, j, kk]), orig=(ib, i, j))
+    v = acc + bias[j]
+    r.body = Seq([loops([(ib, b), (i, m), (j, n)], Set(y, (ib, i, j), un("relu", v) if act else v))])
+    return r
+
+
+def _inputs(ir, k, seed=5):
+    g = np.random.default_rng(seed)
+    return {t.ident: W.store(t.prec, (g.standard_normal(t.dims) / (np.sqrt(k) if t.ident in ("w", "kernel") else 1.0)).astype(np.float32))
+            for t in ir.params() if t.read_only}
+
+
+@pytest.mark.parametrize("shape", [(1, 333, 77, 131), (3, 129, 255, 33), (2, 64, 65, 519), (1, 300, 9, 1001)])
+@pytest.mark.parametrize("a_mmajor,b_nmajor", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("prec", ["bfloat16", "half", "single"])
+def test_odd_rows(device, shape, a_mmajor, b_nmajor, prec):
+    ir = _mm(*shape, prec, a_mmajor, b_nmajor, act=a_mmajor == b_nmajor)
+    inputs = _inputs(ir, shape[3])
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    kinds = [s["kind"] for s in info["stages"]]
+    assert kinds[-1] == "gemm" and "gathers operands" in info["stages"][0]["note"], info
+    tol = dict(rtol=1e-5, atol=2e-6) if prec == "single" else dict(rtol=2e-2, atol=2e-3)
+    compare(ir, got, want, only=["y"], **tol)
+
+
+@pytest.mark.parametrize("cin,cout,kernel,stride", [(3, 40, 3, 1), (8, 17, 5, 2), (16, 32, 3, 1)])
+@pytest.mark.parametrize("prec", ["bfloat16", "single"])
+def test_convolution_patches(device, cin, cout, kernel, stride, prec):
+    """Patches of an image (positions `stride * o + k`) against a kernel: m is (image, row, column),
+    k is (kernel row, kernel column, channel)."""
+    batch, size = 3, 21
+    out = (size - kernel) // stride + 1
+    r = Routine("patches_%d_%d_%d_%d" % (cin, cout, kernel, stride))
+    x = r.tn("x", prec, [batch, size, size, cin], read_only=True)
+    w = r.tn("kernel", prec, [cout, kernel, kernel, cin], read_only=True)
+    y = r.tn("y", prec, [batch, out, out, cout])
+    ib, oh, ow, co, kh, kw, ci = r.syms(7)
+    at = lambda: x[ib, Affine(((stride, oh), (1, kh))), Affine(((stride, ow), (1, kw))), ci]
+    acc = W.reduce_scope(r, "acc", "single", [(kh, kernel), (kw, kernel), (ci, cin)], lambda: (w[co, kh, kw, ci], at()), orig=(ib, oh, ow, co))
+    r.body = Seq([loops([(ib, batch), (oh, out), (ow, out), (co, cout)], Set(y, (ib, oh, ow, co), un("relu", acc)))])
+    if 2 * batch * out * out * cout * kernel * kernel * cin < 4e6:      # below the size the tensor cores are used from
+        pytest.skip("small")
+    inputs = _inputs(r, kernel * kernel * cin)
+    want = run_oracle(r, inputs)
+    got, info = run_device(device, r, inputs)
+    assert [s["kind"] for s in info["stages"]][-1] == "gemm", info
+    tol = dict(rtol=1e-5, atol=2e-6) if prec == "single" else dict(rtol=2e-2, atol=2e-3)
+    compare(r, got, want, only=["y"], **tol)
