@@ -203,7 +203,7 @@ bool accum_form(const Stmt& st, int sid, int tn, std::string* op) {
 }  // namespace
 
 int64_t PackOp::rows() const {
-  int64_t r = kmajor ? 1 : seg * (split ? 3 : 1);
+  int64_t r = kmajor ? 1 : seg * (split ? 2 : 1);
   if (kmajor)
     for (auto& a : mn) r *= a.extent;
   for (auto& a : batch) r *= a.extent;
@@ -221,7 +221,7 @@ std::string PackOp::key() const {
 }
 
 double GemmPlan::flops() const {
-  double f = 2.0 * (double)m.extent * (double)n.extent * (double)k.extent / k_segments;
+  double f = 2.0 * (double)m.extent * (double)n.extent * (double)k.extent;
   for (auto& b : batch) f *= (double)b.extent;
   return f;
 }
@@ -2012,7 +2012,7 @@ struct Builder {
       what += (i ? ", " : "") + code.prog.tn(op.tn).ident;
     }
     st.total = total;
-    st.note = "gathers operands of the next contraction into padded rows" + std::string(g.gemm.k_segments > 1 ? " (tf32 pairs)" : "") + ": " + what;
+    st.note = "gathers operands of the next contraction into padded rows" + std::string(g.gemm.tf32_pairs ? " (tf32 pairs)" : "") + ": " + what;
     src << "extern \"C\" __global__ void __launch_bounds__(256) " << st.kernel << "(" << params.str() << ") {\n" << kGridEntry
         << "  for (unsigned long long b200_g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_g < " << total
         << "ull; b200_g += (unsigned long long)gridDim.x * blockDim.x) {\n" << body.str() << "  }\n}\n\n";
@@ -2052,7 +2052,7 @@ struct Builder {
     };
     const int64_t K = extent(op.k), MN = extent(op.mn);
     const std::vector<PackOp::Axis>& inner = op.kmajor ? op.k : op.mn;
-    const int64_t outer_rows = op.kmajor ? MN : op.seg * (op.split ? 3 : 1);
+    const int64_t outer_rows = op.kmajor ? MN : op.seg * (op.split ? 2 : 1);
     o << "      " << IT << " base = " << num(op.off) << ";\n";
     if (!op.batch.empty()) o << "      const " << IT << " bt = row / " << num(outer_rows) << ", rr = row % " << num(outer_rows) << ";\n" << at(op.batch, "bt", "base", "      ");
     else o << "      const " << IT << " rr = row;\n";
@@ -2076,9 +2076,8 @@ struct Builder {
       << "        const " << IT << " j = j0 + e;\n        " << IT << " p = base;\n" << at(inner, "j", "p", "        ")
       << "        v[e] = row_ok && j < " << num(inner_real) << " ? " << src_name << "[p] : (" << T << ")0;\n      }\n";
     if (op.split) {
-      const std::string lo_seg = op.split == 1 ? "2" : "1";
       o << "      b200_u32 w[4];\n#pragma unroll\n      for (int e = 0; e < 4; ++e) {\n        const float hi = b200_tf32(v[e]);\n"
-        << "        w[e] = __float_as_uint(sg == " << lo_seg << S << " ? b200_tf32(v[e] - hi) : hi);\n      }\n"
+        << "        w[e] = __float_as_uint(sg == 1" << S << " ? b200_tf32(v[e] - hi) : hi);\n      }\n"
         << "      " << dst << "[i] = make_uint4(w[0], w[1], w[2], w[3]);\n";
     } else if (eb == 4) {
       o << "      " << dst << "[i] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));\n";

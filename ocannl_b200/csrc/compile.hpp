@@ -36,9 +36,9 @@ struct GemmDim {
 // contraction gathers it into the routine's scratch as rows padded to 16 bytes,
 //   k-major   [batch][m or n][k padded]      or      m/n-major   [batch][k][m or n padded],
 // whichever keeps the node's own contiguous axis.  Single-precision operands are stored as two
-// tf32 values, x = hi + lo, in three segments along k -- (hi, hi, lo) for A, (hi, lo, hi) for B -- so
-// that one pass of the tensor cores sums hi hi + hi lo + lo hi: the products keep 21 bits, where the
-// exact path they would otherwise take keeps 24.
+// tf32 values, x = hi + lo, in two segments along k (each padded to whole k blocks); the contraction sums
+// hi lo + lo hi + hi hi: each value is kept to 2^-24 of itself and what is left out of a product, lo lo,
+// lies below 2^-24 of it -- single-precision products.
 struct PackOp {
   struct Axis { int64_t extent, stride; };
   int tn = -1;
@@ -46,8 +46,8 @@ struct PackOp {
   std::vector<Axis> batch, mn, k;      // outer to inner, strides in elements
   bool kmajor = true;
   int64_t ld = 0;                      // elements per packed row
-  int64_t seg = 0;                     // k positions per segment (k's extent, padded when split and k-major)
-  int split = 0;                       // 0: as stored; 1: hi, hi, lo; 2: hi, lo, hi
+  int64_t seg = 0;                     // k positions per segment (k's extent, padded to whole k blocks when split)
+  bool split = false;                  // two segments along k, the tf32 parts of the values
   Prec prec = Prec::Bfloat16;
   int64_t rows() const;                // packed rows
   int64_t bytes() const;
@@ -67,7 +67,7 @@ struct GemmPlan {
   std::vector<PackOp> packs;         // operands to gather first (A before B)
   bool pack_a = false, pack_b = false;
   int a_slot = -1, b_slot = -1;      // scratch slots of the packed operands
-  int k_segments = 1;                // 3 when single-precision operands are split into tf32 pairs: k.extent counts all segments
+  bool tf32_pairs = false;           // single-precision operands packed as tf32 pairs
   double flops() const;
 };
 

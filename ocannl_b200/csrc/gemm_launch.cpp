@@ -88,8 +88,10 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
   try {
     std::vector<int64_t> sa, sb;
     for (auto& d : g.batch) { sa.push_back(d.sa); sb.push_back(d.sb); }
-    encode_operand(&L->map_a, a, g.in_prec, g.a_kmajor, g.m, g.m.sa, g.k, g.k.sa, g.batch, sa, st.box_m, st.tile_k);
-    encode_operand(&L->map_b, b, g.in_prec, g.b_kmajor, g.n, g.n.sb, g.k, g.k.sb, g.batch, sb, st.box_n, st.tile_k);
+    GemmDim k = g.k;
+    if (g.tf32_pairs) k.extent = 2 * g.packs[0].seg;   // both segments of the packed operands
+    encode_operand(&L->map_a, a, g.in_prec, g.a_kmajor, g.m, g.m.sa, k, g.k.sa, g.batch, sa, st.box_m, st.tile_k);
+    encode_operand(&L->map_b, b, g.in_prec, g.b_kmajor, g.n, g.n.sb, k, g.k.sb, g.batch, sb, st.box_n, st.tile_k);
   } catch (...) {
     delete L;
     throw;

@@ -15,6 +15,7 @@
 // is not fp32 (the cc backend would round every step, arrayjit/lib/cc_backend.ml:169-186),
 // strides the tensor maps cannot express — is left to the generic loop-nest kernels.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <functional>
 #include <set>
@@ -415,17 +416,15 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
         axes(all_k, &op.k);
         op.kmajor = op.k.back().stride == 1 || op.mn.back().stride != 1;
         kmajor = op.kmajor;
-        op.split = split ? (of_a ? 1 : 2) : 0;
-        op.seg = g.k.extent;
-        const int64_t unit = 16 / eb;
-        const int64_t inner = kmajor ? g.k.extent : (of_a ? g.m.extent : g.n.extent);
-        const int64_t padded = (inner + unit - 1) / unit * unit;
-        op.ld = kmajor ? padded * (split ? 3 : 1) : padded;
+        op.split = split;
+        op.seg = split ? (g.k.extent + 31) / 32 * 32 : g.k.extent;
+        const int64_t unit = 16 / eb, parts = split ? 2 : 1;
+        const int64_t mn_extent = of_a ? g.m.extent : g.n.extent;
+        op.ld = kmajor ? (op.seg * parts + unit - 1) / unit * unit : (mn_extent + unit - 1) / unit * unit;
         if (op.bytes() > (2ll << 30)) return false;   // the copy would cost more memory than it is worth
-        const int64_t rows = kmajor ? (of_a ? g.m.extent : g.n.extent) : g.k.extent * (split ? 3 : 1);
         s_mn = kmajor ? op.ld : 1;
         s_k = kmajor ? 1 : op.ld;
-        s_b = rows * op.ld;
+        s_b = (kmajor ? mn_extent : op.seg * parts) * op.ld;
         (of_a ? g.pack_a : g.pack_b) = true;
         (of_a ? g.a_off : g.b_off) = 0;
         g.packs.push_back(op);
@@ -434,21 +433,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
       else { g.n.sb = s_mn; g.k.sb = s_k; g.b_kmajor = kmajor; }
       if (!g.batch.empty()) (of_a ? g.batch[0].sa : g.batch[0].sb) = s_b;
     }
-    if (split) {
-      // the segments of a k-major operand start at padded positions: both operands use the same ones
-      const bool any_kmajor = g.a_kmajor || g.b_kmajor;
-      const int64_t seg = any_kmajor ? (g.k.extent + 3) / 4 * 4 : g.k.extent;
-      g.k_segments = 3;
-      for (auto& op : g.packs) {
-        op.seg = seg;
-        if (!op.kmajor) {
-          // rows of the m/n-major form: one per position of every segment
-          const int64_t s_b = 3 * seg * op.ld;
-          if (!g.batch.empty()) (&op == &g.packs[0] ? g.batch[0].sa : g.batch[0].sb) = s_b;
-        }
-      }
-      g.k.extent = 3 * seg;
-    }
+    g.tf32_pairs = split;
   }
   if (g.m.extent >= (1ll << 31) || g.n.extent >= (1ll << 31) || g.k.extent >= (1ll << 31)) return false;
   const Dim &dm = gm[0], &dn = gn[0];
@@ -487,6 +472,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     bool unit_n = false;   // the node's last axis is the n symbol: a chunk is contiguous
     std::string row_off;   // element offset of column n = 0 of this row
     int tma = -1;          // index of the tensor map that stores this node's chunks (-1: none)
+    int64_t m_stride = 0;  // > 0: neighbouring rows of this contraction lie that many elements apart
   };
   std::vector<Out> outs;
   // The n axis may be several merged loop symbols (the (head, d) of an attention projection).  A
@@ -524,30 +510,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   if (pair && ((form_b && g.accumulate) || n_sym.empty() || (n_syms == 1 ? false : (odd_n || dn.syms.back().second % 2 != 0)))) return false;
   em.pair = pair;
   em.pair_sym = n_sym;
-  bool pair_fail = false;
-  auto add_out = [&](int tn, const Indices& idcs) {
-    Out o;
-    o.tn = tn;
-    o.idcs = idcs;
-    o.arr = "b200_o" + std::to_string(tn);
-    const Tnode& t = P.tn(tn);
-    {
-      Indices row;
-      if (along_n(idcs, t.dims, &row)) {
-        o.unit_n = true;
-        o.row_off = em.offset(row, t.dims);
-      }
-    }
-    if (pair && (!o.unit_n || !Emitter::pair_prec(t.prec))) pair_fail = true;
-    em.set_redirect[tn] = {idcs, o.arr + "[b200_j]"};
-    em.used_nodes.insert(tn);
-    outs.push_back(o);
-  };
-
   // A node as a regular [batch.., m, n] array for this contraction, for the TMA unit: the m symbols
   // (and each batch group's) compose to one stride, n is contiguous, everything 16-byte aligned,
   // and no other symbol moves the address.
-  auto make_map = [&](int tn, const Indices& idcs, OutMap* m) {
+  auto regular = [&](int tn, const Indices& idcs, OutMap* m) {
     const Tnode& t = P.tn(tn);
     const int ebytes = prec_bytes(t.prec);
     std::map<std::string, int64_t> st_;
@@ -570,8 +536,6 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (!group_stride(dm, &m->m_stride) || !group_stride(dn, &n_stride) || n_stride != 1) return false;
     if (gb.size() == 2) { if (!group_stride(gb[0], &m->b0_stride) || !group_stride(gb[1], &m->b1_stride)) return false; }
     else if (gb.size() == 1) { if (!group_stride(gb[0], &m->b1_stride)) return false; }
-    for (int64_t v : {m->off, m->m_stride, m->b0_stride, m->b1_stride})
-      if ((v * ebytes) % 16 != 0) return false;
     for (auto& kv : st_) {
       bool known_sym = false;
       for (auto* d : {&dm, &dn}) for (auto& sy : d->syms) known_sym |= sy.first == kv.first;
@@ -581,6 +545,34 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     m->elem_bytes = ebytes;
     return true;
   };
+  auto make_map = [&](int tn, const Indices& idcs, OutMap* m) {
+    if (!regular(tn, idcs, m)) return false;
+    for (int64_t v : {m->off, m->m_stride, m->b0_stride, m->b1_stride})
+      if ((v * m->elem_bytes) % 16 != 0) return false;
+    return true;
+  };
+  bool pair_fail = false;
+  auto add_out = [&](int tn, const Indices& idcs) {
+    Out o;
+    o.tn = tn;
+    o.idcs = idcs;
+    o.arr = "b200_o" + std::to_string(tn);
+    const Tnode& t = P.tn(tn);
+    {
+      Indices row;
+      if (along_n(idcs, t.dims, &row)) {
+        o.unit_n = true;
+        o.row_off = em.offset(row, t.dims);
+        OutMap rows;
+        if (regular(tn, idcs, &rows)) o.m_stride = rows.m_stride;
+      }
+    }
+    if (pair && (!o.unit_n || !Emitter::pair_prec(t.prec))) pair_fail = true;
+    em.set_redirect[tn] = {idcs, o.arr + "[b200_j]"};
+    em.used_nodes.insert(tn);
+    outs.push_back(o);
+  };
+
   std::vector<OutMap> in_maps;       // row operands of the epilogue that arrive by TMA (at most one)
   std::string tma_in_wait;           // code at the top of the epilogue step that takes the operand's chunk out of its tile
 
@@ -1379,13 +1371,22 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
            << sts_code(o)
            << "      __syncwarp();\n      constexpr unsigned int V = " << V << "u, R = 32u / B200_EPI_CHUNK;   // elements per group, rows per step\n"
            << "      const unsigned int b200_c = b200_lane % B200_EPI_CHUNK;\n"
-           << "#pragma unroll 8\n      for (unsigned int it = 0; it < 32u / R; ++it) {\n"
-           << "        const unsigned int r = it * R + b200_lane / B200_EPI_CHUNK;\n"
-           << "        " << T << "* const b200_q = (" << T << "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, r);\n"
-           << "        const " << T << " b200_v = ((const " << T << "*)(b200_stage + r * G + ((b200_c / V) ^ B200_STAGE_KEY(r, G))))[b200_c % V];\n"
-           << "        if (b200_q && b200_n0 + b200_c < b200_N) "
-           << (reds ? "atomicAdd(&b200_q[b200_c], b200_v);\n" : "b200_q[b200_c] = b200_v;\n")
-           << "      }\n      __syncwarp();\n";
+           << "      const bool b200_in = b200_n0 + b200_c < b200_N;\n";
+        if (o.m_stride > 0)
+          fn << "      const unsigned int b200_live = __popc(__ballot_sync(0xffffffffu, b200_row_ok));\n"
+             << "      " << T << "* const b200_q0 = (" << T << "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, 0) + b200_c;\n";
+        // (eight values at a time: the compiler cannot move the reads of the staging tile over the stores)
+        fn << "#pragma unroll\n      for (unsigned int i0 = 0; i0 < 32u / R; i0 += 8u) {\n        " << T << " b200_v[8];\n"
+           << "#pragma unroll\n        for (unsigned int i = 0; i < 8u; ++i) {\n          const unsigned int r = (i0 + i) * R + b200_lane / B200_EPI_CHUNK;\n"
+           << "          b200_v[i] = ((const " << T << "*)(b200_stage + r * G + ((b200_c / V) ^ B200_STAGE_KEY(r, G))))[b200_c % V];\n        }\n"
+           << "#pragma unroll\n        for (unsigned int i = 0; i < 8u; ++i) {\n          const unsigned int r = (i0 + i) * R + b200_lane / B200_EPI_CHUNK;\n";
+        if (o.m_stride > 0)
+          fn << "          " << T << "* const b200_q = b200_q0 + (unsigned long long)r * " << o.m_stride << "ull;\n          if (b200_in && r < b200_live) ";
+        else
+          fn << "          " << T << "* const b200_q = (" << T << "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, r) + b200_c;\n"
+             << "          const bool b200_on = __shfl_sync(0xffffffffu, b200_row_ok ? 1 : 0, r) != 0;\n          if (b200_in && b200_on) ";
+        fn << (reds ? "atomicAdd(b200_q, b200_v[i]);\n" : "*b200_q = b200_v[i];\n")
+           << "        }\n      }\n      __syncwarp();\n";
       } else {
         fn << "    if (b200_row_ok) {\n";
         fn << "#pragma unroll\n      for (int b200_j = 0; b200_j < B200_EPI_CHUNK; ++b200_j)\n";
@@ -1436,15 +1437,33 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   return true;
 }
 
+// Microseconds per k block (128 bytes of k) of one tile, by its columns, measured back to back on a full
+// machine.  Narrow tiles are bound by the issue of their MMAs (44 to 50 cycles each up to 64 columns),
+// wide ones by the delivery of the operands into shared memory (about 64 bytes per clock and SM), which is
+// why a CTA pair, each CTA staging half of B, is faster per tile at the same width.
+static double gemm_kb_us(int bn, bool pair, bool tf32_pairs) {
+  static const double single[][2] = {{16, 0.15}, {32, 0.152}, {64, 0.158}, {128, 0.205}, {256, 0.315}};
+  static const double paired[][2] = {{64, 0.17}, {128, 0.193}, {256, 0.29}};
+  const double(*t)[2] = pair ? paired : single;
+  const int n = pair ? 3 : 5;
+  double v = t[n - 1][1];
+  for (int i = 0; i < n; ++i)
+    if (bn <= t[i][0]) {
+      v = i == 0 ? t[0][1] : t[i - 1][1] + (t[i][1] - t[i - 1][1]) * (bn - t[i - 1][0]) / (t[i][0] - t[i - 1][0]);
+      break;
+    }
+  return tf32_pairs ? 2.5 * v : v;   // three products per k block, twice the operand bytes
+}
+
 // Tile shape of a contraction: columns per tile, and whether two CTAs share a 256-row tile.
 //
-// One tcgen05.mma of K = 16 takes about 128 cycles whether the tile is 16 or 256 columns wide (the
-// A operand's 128 rows come out of shared memory at 32 bytes per clock), so a k block costs the
-// same ~0.26 us for every shape and wide tiles do more work in it: large problems want the widest
-// tile.  A problem of few tiles is different: its time is one tile's main loop plus one tile's
-// epilogue, and the epilogue shrinks with the tile (about 3.7 us for 128 rows x 256 columns).  The
-// choice minimises  waves x k blocks x 0.26 us + 3.7 us x columns / 256  over the shapes the
-// operands allow; 148 SMs are assumed (compilation knows no device).
+// Measured times follow   2.3 us + e + l + (waves - 1) max(l, e)   within 10 %, with l the main loop of one
+// tile (k blocks x gemm_kb_us) and e its epilogue, 0.25 us + 3.4 us x columns / 256: the last tile's
+// epilogue is exposed, the others hide behind the next tile's main loop or the other way round; a CTA
+// pair pays 0.5 us more set-up (cluster barrier, paired tensor-memory allocation).  Large problems
+// therefore take the widest pairs; one of few tiles takes the shape that spreads it over the SMs
+// (1024^3: 64 columns 5.9 us, 256 columns 10.2 us; 500 x 1024 x 256: 32 columns 3.4 us, 128 columns
+// 4.9 us).  148 SMs are assumed (compilation knows no device).
 static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
   const int eb = prec_bytes(g.in_prec);
   const int row_elems = 128 / eb;
@@ -1459,7 +1478,7 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
   double best = 1e300;
   int best_bn = bn0;
   bool best_pair = false;
-  const bool flush = g.k_segments > 1;   // running sums in registers: at most 64 columns per epilogue thread
+  const bool flush = g.tf32_pairs;   // running sums in registers: at most 64 columns per epilogue thread
   std::vector<int> widths = {bn0};
   // (an output row of up to 32 columns stays in one tile: assignments over whole rows may follow it)
   if (bn0 > 32) for (int w : {128, 64, 32, 16})
@@ -1476,12 +1495,9 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
       long long split = 1;
       if (g.may_split && tiles * 2 <= workers) split = std::max<long long>(1, std::min<long long>({workers / tiles, (long long)k_blocks / 8, 32ll}));
       const double waves = (double)((tiles * split + workers - 1) / workers);
-      // per k block: the MMA floor, or the delivery of the CTA's operand bytes into shared memory
-      // (sustained about 64 bytes per clock per SM: single CTAs on 128 x 256 tiles reach 54 % of the
-      // tensor peak, CTA pairs, which stage half of B each, 88 %); a CTA pair pays ~0.4 us more
-      // set-up (cluster barrier, paired tensor-memory allocation)
-      const double kb_us = std::max(0.26, (128.0 + (pair ? bn / 2 : bn)) * 128.0 / 64.0 / 1900.0);
-      const double t = waves * (k_blocks / (double)split) * kb_us + 3.7 * bn / 256.0 + (pair ? 0.4 : 0.0);
+      const double loop = std::ceil(k_blocks / (double)split) * gemm_kb_us(bn, pair, g.tf32_pairs);
+      const double epi = 0.25 + 3.4 * bn / 256.0;
+      const double t = 2.3 + (pair ? 0.5 : 0.0) + epi + loop + (waves - 1.0) * std::max(loop, epi);
       if (t < best - 1e-9) {
         best = t;
         best_bn = bn;
@@ -1520,7 +1536,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   gemm_tile_shape(g, &bn, &pair);
   const int bm = pair ? 256 : 128, bk = row_elems;
   const int umma_k = 32 / eb;
-  const int stage_bytes = (128 + (pair ? bn / 2 : bn)) * bk * eb;   // per CTA
+  const int stage_bytes = (128 + (pair ? bn / 2 : bn)) * bk * eb * (g.tf32_pairs ? 2 : 1);   // per CTA
   // Epilogue width: the epilogue is a chain of dependent instructions per warp, so it is bound
   // by latency, not issue rate; light epilogues (few register tiles) get 16 warps, which fits
   // the register file at <= 112 registers per thread.
@@ -1530,7 +1546,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   int chunk = bn >= 32 ? 32 : 16;
   if (st.row_followers > 0) chunk = bn;   // the whole row in one chunk
   const bool light = false;  // 16 warps measured slower: the register cap (96) makes the epilogue spill
-  int epi_warps = light ? 16 : (bn >= 128 ? 8 : 4);
+  int epi_warps = light ? 16 : (bn >= 64 && bn % 64 == 0 ? 8 : 4);
   const int staging = 32 * chunk * st.epi_out_bytes;   // one staging tile
   const int load_tile = st.in_maps.empty() ? 0 : 32 * chunk * st.in_maps[0].elem_bytes;   // a row operand's chunk, per warp
   // outputs that leave as TMA stores alternate between two tiles per warp (the copy engine reads one
@@ -1557,7 +1573,8 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
     << "\n#define B200_STAGES " << stages << "\n#define B200_EPI_WARPS " << epi_warps << "\n#define B200_A_KMAJOR "
     << (g.a_kmajor ? 1 : 0) << "\n#define B200_B_KMAJOR " << (g.b_kmajor ? 1 : 0) << "\n#define B200_IDESC " << idesc
     << "u\n#define B200_TMEM_COLS " << tmem_cols << "\n#define B200_RASTER " << raster << "\n#define B200_CTA_PAIR "
-    << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n#define B200_FLUSH " << (g.k_segments > 1 ? 2 : 0) << "\n";
+    << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n#define B200_FLUSH " << (g.tf32_pairs ? 1 : 0) << "\n";
+  if (g.tf32_pairs) o << "#define B200_PAIRS 1\n#define B200_SEG " << g.packs[0].seg << "\n";
   o << "#define B200_EPI_CHUNK " << chunk << "\n#define B200_STAGING_BYTES " << staging << "\n#define B200_STAGING_TILES " << staging_tiles << "\n#define B200_LOAD_TILE_BYTES " << load_tile << "\n";
   o << "#define B200_EPI_PROLOGUE " << [&] { std::string p = st.epi_prologue; for (auto& c : p) if (c == '\n') c = ' '; return p; }() << "\n";
   o << kTcSource << "\n" << g.epilogue << "\n";
@@ -1567,7 +1584,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   o << "#define B200_EPILOGUE_ROW b200_epilogue_row(b200_r, b200_b0, b200_b1, b200_m, b200_m < shape.M, b200_n0, shape.N, b200_stage, b200_has_next, b200_next_taddr, b200_tiles, b200_slot, b200_nslots, b200_nx_ok, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_m < shape.M, b200_nx_n0, b200_es" << args << ");\n";
   o << kGemmSource << "\n";
   std::ostringstream note;
-  note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.k_segments > 1 ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages
+  note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.tf32_pairs ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages
        << " epi_warps=" << epi_warps << (g.split_k > 1 ? " split_k=" + std::to_string(g.split_k) : std::string())
        << (g.accumulate ? " beta=1" : "")
        << (st.row_followers ? " + " + std::to_string(st.row_followers) + " whole-row assignments in the epilogue" +

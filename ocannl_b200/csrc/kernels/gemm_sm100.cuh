@@ -69,7 +69,17 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 #define B200_CTA_N (B200_BN / (1 + B200_CTA_PAIR))
 #define B200_A_TILE_BYTES (B200_CTA_M * B200_BK * B200_ELEM_BYTES)
 #define B200_B_TILE_BYTES (B200_CTA_N * B200_BK * B200_ELEM_BYTES)
-#define B200_STAGE_BYTES (B200_A_TILE_BYTES + B200_B_TILE_BYTES)
+// B200_PAIRS: single-precision operands as tf32 pairs, x = hi + lo, stored by the gathering kernel as two
+// segments of B200_SEG positions along k.  A ring slot then holds both parts of both operands, and each
+// is used twice: hi lo + lo hi + hi hi.  (Three passes over segments of 3 k positions, as if k were
+// three times as long, moved half as many bytes again into shared memory per product and were bound by
+// that: 665 cycles per k block of a 128 x 128 tile.)
+#ifndef B200_PAIRS
+#define B200_PAIRS 0
+#define B200_SEG 0
+#endif
+#define B200_STAGE_BYTES ((B200_A_TILE_BYTES + B200_B_TILE_BYTES) * (1 + B200_PAIRS))
+#define B200_B_AT (B200_A_TILE_BYTES * (1 + B200_PAIRS))   // where a slot's B tile (or pair of tiles) begins
 #define B200_THREADS (64 + 32 * B200_EPI_WARPS)
 // elements of the contiguous axis covered by one 128-byte swizzle row
 #define B200_ROW_ELEMS (128 / B200_ELEM_BYTES)
@@ -199,24 +209,28 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           const unsigned int full = b200_map_to_cta(bar_full + 8u * slot, 0u);   // (the barrier itself when not paired)
           if (cta_rank == 0u) b200_mbar_expect_tx(bar_full + 8u * slot, B200_STAGE_BYTES * (1 + B200_CTA_PAIR));
           const unsigned int sa = tiles_at + slot * B200_STAGE_BYTES;
-          const unsigned int sb = sa + B200_A_TILE_BYTES;
-          const int k0 = (int)(kb * B200_BK);
+          const unsigned int sb = sa + B200_B_AT;
+#pragma unroll
+          for (int part = 0; part < 1 + B200_PAIRS; ++part) {
+          const int k0 = (int)(kb * B200_BK) + part * B200_SEG;
+          const unsigned int pa = sa + part * B200_A_TILE_BYTES, pb = sb + part * B200_B_TILE_BYTES;
 #if B200_A_KMAJOR
-          b200_tma_load_4d(sa, &map_a, full, k0, m0, (int)(b1 * shape.a_b1), (int)(b0 * shape.a_b0));
+          b200_tma_load_4d(pa, &map_a, full, k0, m0, (int)(b1 * shape.a_b1), (int)(b0 * shape.a_b0));
 #else
 #pragma unroll
           for (int c = 0; c < B200_CTA_M / B200_ROW_ELEMS; ++c)
-            b200_tma_load_4d(sa + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_a, full, m0 + c * B200_ROW_ELEMS, k0,
+            b200_tma_load_4d(pa + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_a, full, m0 + c * B200_ROW_ELEMS, k0,
                              (int)(b1 * shape.a_b1), (int)(b0 * shape.a_b0));
 #endif
 #if B200_B_KMAJOR
-          b200_tma_load_4d(sb, &map_b, full, k0, n0, (int)(b1 * shape.b_b1), (int)(b0 * shape.b_b0));
+          b200_tma_load_4d(pb, &map_b, full, k0, n0, (int)(b1 * shape.b_b1), (int)(b0 * shape.b_b0));
 #else
 #pragma unroll
           for (int c = 0; c < B200_CTA_N / B200_ROW_ELEMS; ++c)
-            b200_tma_load_4d(sb + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_b, full, n0 + c * B200_ROW_ELEMS, k0,
+            b200_tma_load_4d(pb + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_b, full, n0 + c * B200_ROW_ELEMS, k0,
                              (int)(b1 * shape.b_b1), (int)(b0 * shape.b_b0));
 #endif
+          }
           if (unit == worker && kb == kb0) B200_TR(3);   // first loads issued
           if (++slot == B200_STAGES) { slot = 0; phase ^= 1u; }
         }
@@ -237,10 +251,10 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       const unsigned long long desc_a0 = b200_smem_desc(tiles_at, B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES, B200_MN_GROUP_BYTES, B200_MN_SWIZZLE);
 #endif
 #if B200_B_KMAJOR
-      const unsigned long long desc_b0 = b200_smem_desc(tiles_at + B200_A_TILE_BYTES, 16u, 1024u);
+      const unsigned long long desc_b0 = b200_smem_desc(tiles_at + B200_B_AT, 16u, 1024u);
 #else
       const unsigned long long desc_b0 =
-          b200_smem_desc(tiles_at + B200_A_TILE_BYTES, B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES, B200_MN_GROUP_BYTES, B200_MN_SWIZZLE);
+          b200_smem_desc(tiles_at + B200_B_AT, B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES, B200_MN_GROUP_BYTES, B200_MN_SWIZZLE);
 #endif
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
         const unsigned int split = unit / total_tiles;
@@ -259,11 +273,17 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
             const unsigned long long da0 = desc_a0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
             const unsigned long long db0 = desc_b0 + (unsigned long long)((slot * B200_STAGE_BYTES) >> 4);
 #pragma unroll
-            for (unsigned int ks = 0; ks < B200_BK / B200_UMMA_K; ++ks) {
-              // a k step moves UMMA_K elements along a k-major row, or UMMA_K rows of 128 bytes in the m/n-major form
-              const unsigned long long da = da0 + (unsigned long long)((ks * (B200_A_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
-              const unsigned long long db = db0 + (unsigned long long)((ks * (B200_B_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
-              b200_umma(d_tmem, da, db, (unsigned int)B200_IDESC, (kb != kbf || ks != 0u) ? 1u : 0u);
+            for (unsigned int p = 0; p < 1 + 2 * B200_PAIRS; ++p) {
+              // the parts multiplied: both as stored, or (A hi, B lo), (A lo, B hi), (A hi, B hi)
+              const unsigned long long dap = da0 + (unsigned long long)((p == 1u ? B200_A_TILE_BYTES : 0u) >> 4);
+              const unsigned long long dbp = db0 + (unsigned long long)((B200_PAIRS && p == 0u ? B200_B_TILE_BYTES : 0u) >> 4);
+#pragma unroll
+              for (unsigned int ks = 0; ks < B200_BK / B200_UMMA_K; ++ks) {
+                // a k step moves UMMA_K elements along a k-major row, or UMMA_K rows of 128 bytes in the m/n-major form
+                const unsigned long long da = dap + (unsigned long long)((ks * (B200_A_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
+                const unsigned long long db = dbp + (unsigned long long)((ks * (B200_B_KMAJOR ? B200_UMMA_K * B200_ELEM_BYTES : B200_UMMA_K * 128u)) >> 4);
+                b200_umma(d_tmem, da, db, (unsigned int)B200_IDESC, (kb != kbf || ks != 0u || p != 0u) ? 1u : 0u);
+              }
             }
             b200_umma_commit(bar_empty + 8u * slot);  // frees the slot once these MMAs retire
             if (++slot == B200_STAGES) { slot = 0; phase ^= 1u; }
@@ -352,14 +372,12 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           if (!got) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const unsigned int taddr = tmem_base + acc * B200_BN + ((quarter * 32u) << 16) + col0;
+          unsigned int part[kCols];
 #pragma unroll
-          for (int c = 0; c < kCols; c += B200_EPI_CHUNK) {
-            unsigned int part[B200_EPI_CHUNK];
-            b200_tmem_ld_chunk(taddr + c, part);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int c = 0; c < kCols; c += B200_EPI_CHUNK) b200_tmem_ld_chunk(taddr + c, part + c);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < B200_EPI_CHUNK; ++j) b200_sum[c + j] += __uint_as_float(part[j]);
-          }
+          for (int j = 0; j < kCols; ++j) b200_sum[j] += __uint_as_float(part[j]);
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) b200_mbar_arrive_relaxed(bar_acc_empty + 8u * acc);
