@@ -144,6 +144,27 @@ bool accumulates_into_self(const Stmt& set) {
   return false;
 }
 
+// Innermost iterations one execution of a statement takes (loops and reductions inside it multiplied out).
+double iterations(const Stmt& s);
+double iterations(const Scalar& e) {
+  double n = e.kind == Scalar::LocalScope ? iterations(*e.body) : 0.0;
+  for (auto& a : e.args) n += iterations(*a.s);
+  return n;
+}
+double iterations(const Stmt& s) {
+  switch (s.kind) {
+    case Stmt::Seq: {
+      double n = 0;
+      for (auto& x : s.items) n += iterations(*x);
+      return n;
+    }
+    case Stmt::For: return (double)std::max<int64_t>(0, s.to - s.from + 1) * iterations(*s.body);
+    case Stmt::Set:
+    case Stmt::SetLocal: return 1.0 + iterations(*s.value);
+    default: return 0.0;
+  }
+}
+
 bool body_has_set(const Stmt& s) {
   bool any = false;
   walk_stmt(s, [](const Scalar&) {}, [&](const Stmt& st) {
@@ -525,9 +546,10 @@ struct Builder {
 
   // Accumulation whose reduced loops are OUTSIDE the output loops (back-propagation keeps the
   // forward loop order: `for b { for o { g[o] := g[o] + dz[b, o] } }`, or the fma form with two
-  // factors).  A 32x32 block owns 32 consecutive outputs (threadIdx.x, coalesced) and splits the
-  // flattened serial loop space over threadIdx.y; partial sums meet in shared memory and the
-  // y == 0 row adds them to the node in a fixed order.
+  // factors).  A block owns up to 128 neighbouring outputs (or pairs) and splits the flattened serial
+  // loop space over its other threads; partial sums meet through shuffles and shared memory.
+  // dW of a 10-class output layer over 8192 rows and 1024 inputs: 33 us with one pair per thread, whose ten
+  // factors were then loaded for two products each.
   bool ser_split_stage(Stage st, const Stmt& set) {
     if (set.kind != Stmt::Set) return false;
     const Tnode& t = code.prog.tn(set.tn);
@@ -618,87 +640,109 @@ struct Builder {
     const bool tiled = !term && st.par.size() >= 2 && st.par[0].extent() <= 16;
     const int64_t e0 = tiled ? st.par[0].extent() : 1;
     const size_t first_par = tiled ? 1 : 0;
-    const int64_t outputs = st.total / e0 / (pairs ? 2 : 1);   // output elements (or pairs) spread over threadIdx.x
+    const int64_t outputs = st.total / e0 / (pairs ? 2 : 1);   // output elements (or pairs) spread over the columns
+    // A block is 32 lanes x BY rows of threads.  CW lanes take neighbouring outputs, Q of them each, CW
+    // apart (what does not depend on the output -- the other factor of every tiled value -- is then loaded
+    // once for Q outputs); the 32 / CW lane groups and the BY rows share out the serial loop space.  Few
+    // outputs (the 24 channels of a convolution's bias) thus keep whole warps busy.
+    int64_t CW = 1;
+    while (CW < 32 && CW < outputs) CW *= 2;
+    // (at most 80 accumulator registers per thread)
+    const int64_t q_max = std::max<int64_t>(1, 80 / (e0 * (pairs ? 2 : 1)));
+    const int64_t Q = outputs >= 4 * CW && q_max >= 4 ? 4 : (outputs >= 2 * CW && q_max >= 2 ? 2 : 1);
+    const int64_t XR = 32 / CW, BY = tiled ? 16 : 32, SUBS = BY * XR;
     std::string decomp, sdecomp;
     {
       std::string rem = "b200_g";
       for (size_t i = st.par.size(); i-- > first_par;) {
         const LoopDim& d = st.par[i];
         const bool pair_dim = pairs && i + 1 == st.par.size();
-        std::string ext = std::to_string(pair_dim ? d.extent() / 2 : d.extent()) + "ull";
-        decomp += "      const unsigned int " + d.sym + " = " + (pair_dim ? "2u * " : "") + "(unsigned int)" +
+        std::string ext = std::to_string(pair_dim ? d.extent() / 2 : d.extent()) + "u";
+        decomp += "          const unsigned int " + d.sym + " = " + (pair_dim ? "2u * " : "") +
                   (i == first_par ? rem : "(" + rem + " % " + ext + ")") + ";\n";
         if (i != first_par) {
-          decomp += "      const unsigned long long b200_r" + std::to_string(i) + " = " + rem + " / " + ext + ";\n";
+          decomp += "          const unsigned int b200_r" + std::to_string(i) + " = " + rem + " / " + ext + ";\n";
           rem = "b200_r" + std::to_string(i);
         }
       }
       rem = "b200_l";
       for (size_t i = st.ser.size(); i-- > 0;) {
         const LoopDim& d = st.ser[i];
-        std::string ext = std::to_string(d.extent()) + "ull";
-        sdecomp += "        const unsigned int " + d.sym + " = (unsigned int)" + (i == 0 ? rem : "(" + rem + " % " + ext + ")") + ";\n";
+        std::string ext = std::to_string(d.extent()) + "u";
+        sdecomp += "        const unsigned int " + d.sym + " = " + (i == 0 ? rem : "(" + rem + " % " + ext + ")") + ";\n";
         if (i != 0) {
-          sdecomp += "        const unsigned long long b200_q" + std::to_string(i) + " = " + rem + " / " + ext + ";\n";
+          sdecomp += "        const unsigned int b200_q" + std::to_string(i) + " = " + rem + " / " + ext + ";\n";
           rem = "b200_q" + std::to_string(i);
         }
       }
     }
+    if (st.total >= (1ll << 31) || ser_total >= (1ll << 31)) return false;   // (positions are counted in 32 bits)
     const std::string off = em.offset(set.idcs, t.dims);
     std::string text = decomp + sdecomp + step + off;
     std::string statics = static_prologue(text, em, 2);
     // Few output groups leave most SMs idle: the serial loop space is then also cut into Z slices,
     // one block per (group, slice), and the slices meet in the output through atomic adds (their
     // order is not fixed; the node is fp32 or fp64 and already holds the value being added to).
-    const int64_t groups = (outputs + 31) / 32;
+    const int64_t groups = (outputs + CW * Q - 1) / (CW * Q);
     int64_t Z = 1;
-    if (groups < 2 * 148) Z = std::max<int64_t>(1, std::min<int64_t>((4 * 148 + groups - 1) / groups, ser_total / 256));
+    if (groups < 2 * 148) Z = std::max<int64_t>(1, std::min<int64_t>(((tiled ? 148 : 2 * 148) + groups - 1) / groups, ser_total / std::max<int64_t>(2 * SUBS, 128)));
     st.block = 32;
-    st.block_y = 32;
-    st.coop = 32;  // 32 threads per output element
+    st.block_y = (int)BY;
+    st.coop = 32;  // several threads per output element
     st.grid_override = (int)std::min<int64_t>(groups * Z, 148 * 8);
     std::set<int> written = {set.tn};
     const std::string o_sym = tiled ? st.par[0].sym : std::string();
-    const std::string E0 = std::to_string(e0);
+    const std::string E0 = std::to_string(e0), QS = std::to_string(Q), CWS = std::to_string(CW);
+    auto sum_of = [&](const std::string& a, const std::string& b) {
+      return pairs ? "b200_f2{" + a + ".x + " + b + ".x, " + a + ".y + " + b + ".y}" : a + " + " + b;
+    };
     std::ostringstream k;
-    k << "extern \"C\" __global__ void __launch_bounds__(1024) " << st.kernel << "(";
+    k << "extern \"C\" __global__ void __launch_bounds__(" << 32 * BY << ") " << st.kernel << "(";
     emit_params(k, st, em, written);
-    k << ") {\n" << kGridEntry << statics << "  __shared__ " << T << " b200_part[32][33];\n"
-      << "  for (unsigned long long b200_u = blockIdx.x; b200_u < " << groups * Z << "ull; b200_u += gridDim.x) {\n"
-      << "    const unsigned long long b200_g = (b200_u % " << groups << "ull) * 32ull + threadIdx.x, b200_z = b200_u / " << groups << "ull;\n"
-      << "    const unsigned long long b200_l0 = b200_z * " << ser_total << "ull / " << Z << "ull, b200_l1 = (b200_z + 1ull) * "
-      << ser_total << "ull / " << Z << "ull;\n"
-      << "    const bool b200_ok = b200_g < " << outputs << "ull;\n";
-    if (tiled) k << "    " << T << " b200_accs[" << E0 << "];\n#pragma unroll\n    for (int b200_o = 0; b200_o < " << E0 << "; ++b200_o) b200_accs[b200_o] = " << zero << ";\n";
-    else k << "    " << T << " b200_acc = " << zero << ";\n";
-    k << "    if (b200_ok) {\n" << decomp
-      << "#pragma unroll 4\n      for (unsigned long long b200_l = b200_l0 + threadIdx.y; b200_l < b200_l1; b200_l += 32ull) {\n" << sdecomp;
-    if (tiled)
-      k << "#pragma unroll\n        for (unsigned int " << o_sym << " = 0; " << o_sym << " < " << E0 << "u; ++" << o_sym << ") {\n"
-        << "          " << T << " b200_acc = b200_accs[" << o_sym << "];\n          " << step << "\n          b200_accs[" << o_sym
-        << "] = b200_acc;\n        }\n";
-    else
-      k << "        " << step << "\n";
-    k << "      }\n    }\n";
-    // combine the 32 slices of threadIdx.y, one output value (of the tiled loop) at a time
-    if (tiled) k << "#pragma unroll\n    for (unsigned int " << o_sym << " = 0; " << o_sym << " < " << E0 << "u; ++" << o_sym << ") {\n      const "
-                 << T << " b200_acc = b200_accs[" << o_sym << "];\n";
-    else k << "    {\n";
-    k << "      b200_part[threadIdx.y][threadIdx.x] = b200_acc;\n      __syncthreads();\n"
-      << "      if (threadIdx.y == 0 && b200_ok) {\n" << decomp << "        " << T << " b200_s = " << zero << ";\n";
+    k << ") {\n" << kGridEntry << statics << "  __shared__ " << T << " b200_part[" << BY << "][" << Q * CW + 1 << "];\n"
+      << "  const unsigned int b200_c = threadIdx.x % " << CWS << "u, b200_sub = threadIdx.y * " << XR << "u + threadIdx.x / " << CWS << "u;\n"
+      << "  for (unsigned int b200_u = blockIdx.x; b200_u < " << groups * Z << "u; b200_u += gridDim.x) {\n"
+      << "    const unsigned int b200_g0 = (b200_u % " << groups << "u) * " << Q * CW << "u, b200_z = b200_u / " << groups << "u;\n"
+      << "    const unsigned int b200_l0 = (unsigned int)(b200_z * " << ser_total << "ull / " << Z << "ull), b200_l1 = (unsigned int)((b200_z + 1ull) * "
+      << ser_total << "ull / " << Z << "ull);\n"
+      << "    " << T << " b200_accs[" << QS << "][" << E0 << "];\n#pragma unroll\n    for (int b200_q = 0; b200_q < " << QS
+      << "; ++b200_q)\n#pragma unroll\n      for (int b200_o = 0; b200_o < " << E0 << "; ++b200_o) b200_accs[b200_q][b200_o] = " << zero << ";\n"
+      << "#pragma unroll " << (Q * e0 <= 8 ? 4 : (Q * e0 <= 16 ? 2 : 1)) << "\n      for (unsigned int b200_l = b200_l0 + b200_sub; b200_l < b200_l1; b200_l += " << SUBS << "u) {\n" << sdecomp
+      << "#pragma unroll\n        for (unsigned int b200_q = 0; b200_q < " << QS << "u; ++b200_q) {\n"
+      // (columns past the end repeat the last one; nothing of them is added to the output)
+      << "          const unsigned int b200_g = min(b200_g0 + b200_q * " << CWS << "u + b200_c, " << outputs - 1 << "u);\n" << decomp
+      << "#pragma unroll\n          for (unsigned int " << (tiled ? o_sym : std::string("b200_one")) << " = 0; " << (tiled ? o_sym : std::string("b200_one")) << " < " << E0 << "u; ++"
+      << (tiled ? o_sym : std::string("b200_one")) << ") {\n"
+      << "            " << T << " b200_acc = b200_accs[b200_q][" << (tiled ? o_sym : std::string("0")) << "];\n            " << step << "\n            b200_accs[b200_q]["
+      << (tiled ? o_sym : std::string("0")) << "] = b200_acc;\n          }\n        }\n      }\n";
+    // combine: lane groups by shuffles, then the BY rows through shared memory, one tiled value at a time
+    k << "#pragma unroll\n    for (unsigned int " << (tiled ? o_sym : std::string("b200_one")) << " = 0; " << (tiled ? o_sym : std::string("b200_one")) << " < " << E0 << "u; ++"
+      << (tiled ? o_sym : std::string("b200_one")) << ") {\n#pragma unroll\n      for (int b200_q = 0; b200_q < " << QS << "; ++b200_q) {\n        " << T
+      << " b200_acc = b200_accs[b200_q][" << (tiled ? o_sym : std::string("0")) << "];\n";
+    if (XR > 1) {
+      k << "#pragma unroll\n        for (unsigned int b200_s = " << CWS << "u; b200_s < 32u; b200_s <<= 1) {\n";
+      if (pairs)
+        k << "          const " << T << " b200_w = {__shfl_xor_sync(0xffffffffu, b200_acc.x, b200_s), __shfl_xor_sync(0xffffffffu, b200_acc.y, b200_s)};\n";
+      else
+        k << "          const " << T << " b200_w = __shfl_xor_sync(0xffffffffu, b200_acc, b200_s);\n";
+      k << "          b200_acc = " << sum_of("b200_acc", "b200_w") << ";\n        }\n";
+    }
+    k << "        if (threadIdx.x < " << CWS << "u) b200_part[threadIdx.y][b200_q * " << CWS << " + b200_c] = b200_acc;\n      }\n      __syncthreads();\n"
+      << "      for (unsigned int b200_i = threadIdx.y * 32u + threadIdx.x; b200_i < " << Q * CW << "u; b200_i += " << 32 * BY << "u) {\n"
+      << "        const unsigned int b200_g = b200_g0 + b200_i;\n        if (b200_g < " << outputs << "u) {\n" << decomp
+      << "          " << T << " b200_s = b200_part[0][b200_i];\n#pragma unroll\n          for (int b200_y = 1; b200_y < " << BY << "; ++b200_y) b200_s = "
+      << sum_of("b200_s", "b200_part[b200_y][b200_i]") << ";\n";
     if (pairs) {
-      k << "        for (int b200_y = 0; b200_y < 32; ++b200_y) { b200_s.x += b200_part[b200_y][threadIdx.x].x; b200_s.y += b200_part[b200_y][threadIdx.x].y; }\n";
-      if (Z > 1) k << "        atomicAdd(&" << t.ident << "[" << off << "], b200_s.x);\n        atomicAdd(&" << t.ident << "[(" << off << ") + 1], b200_s.y);\n";
-      else k << "        " << t.ident << "[" << off << "] = " << t.ident << "[" << off << "] + b200_s.x;\n        " << t.ident << "[(" << off
+      if (Z > 1) k << "          b200_red2(" << t.ident << " + (" << off << "), b200_s.x, b200_s.y);\n";
+      else k << "          " << t.ident << "[" << off << "] = " << t.ident << "[" << off << "] + b200_s.x;\n          " << t.ident << "[(" << off
              << ") + 1] = " << t.ident << "[(" << off << ") + 1] + b200_s.y;\n";
     } else {
-      k << "        for (int b200_y = 0; b200_y < 32; ++b200_y) b200_s += b200_part[b200_y][threadIdx.x];\n";
-      if (Z > 1) k << "        atomicAdd(&" << t.ident << "[" << off << "], b200_s);\n";
-      else k << "        " << t.ident << "[" << off << "] = " << t.ident << "[" << off << "] + b200_s;\n";
+      if (Z > 1) k << "          atomicAdd(&" << t.ident << "[" << off << "], b200_s);\n";
+      else k << "          " << t.ident << "[" << off << "] = " << t.ident << "[" << off << "] + b200_s;\n";
     }
-    k << "      }\n      __syncthreads();\n    }\n  }\n}\n\n";
+    k << "        }\n      }\n      __syncthreads();\n    }\n  }\n}\n\n";
     src << k.str();
-    st.note = "par=" + std::to_string(st.par.size()) + " ser=" + std::to_string(st.ser.size()) + " serial loops split over a 32x32 block" +
+    st.note = "par=" + std::to_string(st.par.size()) + " ser=" + std::to_string(st.ser.size()) + " serial loops split over a 32x" + std::to_string(BY) + " block" +
               (Z > 1 ? ", " + std::to_string(Z) + " slices per output group (atomic adds)" : std::string()) +
               (tiled ? ", outer loop of " + E0 + " kept in registers" : std::string()) + (pairs ? ", pairs" : std::string());
     st.writes = {set.tn};
@@ -986,6 +1030,17 @@ struct Builder {
     pc.fusable = opt.enable_fuse && st.total > 0 && (st.coop == 0 || st.coop == 32) &&
                  st.total * std::max(1, st.coop) <= 16384 && ser_work <= 4096;
     if (scatter) pc.fusable = false;
+    {
+      // A stage shares the single block of small stages only while that block gets through it in less
+      // than what leaving it out costs: its own launch, and a second one for the block's other half (8 us,
+      // 16000 cycles, with the stage's own time on many SMs).  Each of a thread's iterations takes the
+      // latency of its loads or, with many warps, their issue, about six instructions per warp and
+      // scheduler.  (The 37 x 10 logits over 1024 hidden units took 25 us of one block.)
+      const double threads = (double)st.total * std::max(1, st.coop);
+      const double rounds = std::ceil(threads / 1024.0), warps = std::ceil(std::min(threads, 1024.0) / 32.0);
+      const double iters = rounds * (double)ser_work * iterations(*body) / std::max(1, st.coop);
+      if (iters * std::max(30.0, 6.0 * warps / 4.0) > 16000.0) pc.fusable = false;
+    }
     if (opt.enable_fuse && !scatter && st.coop == 0 && st.total > 0 && !st.par.empty() && st.par[0].from == 0 && !(pairs && st.par.size() == 1)) {
       pc.body = body;
       pc.row_sym = st.par[0].sym;
@@ -2072,9 +2127,29 @@ struct Builder {
       o << "      const bool row_ok = kk < " << num(K) << ";\n" << at(op.k, "kk", "base", "      ") << "      const " << IT << " j0 = grp * " << V << S << ";\n";
     }
     const std::string T = Emitter::ctype(op.prec);
-    o << "      " << T << " v[" << V << "];\n#pragma unroll\n      for (unsigned int e = 0; e < " << V << "u; ++e) {\n"
-      << "        const " << IT << " j = j0 + e;\n        " << IT << " p = base;\n" << at(inner, "j", "p", "        ")
-      << "        v[e] = row_ok && j < " << num(inner_real) << " ? " << src_name << "[p] : (" << T << ")0;\n      }\n";
+    // the group's elements: the first position is taken apart with divisions, the others by counting on
+    o << "      " << T << " v[" << V << "];\n      " << IT << " p = base;\n";
+    std::string rest = "j0";
+    for (size_t a = inner.size(); a-- > 0;) {
+      const std::string c = "c" + std::to_string(a);
+      if (a == 0) {
+        o << "      p += (" << rest << ") * " << num(inner[a].stride) << ";\n";
+      } else {
+        o << "      " << IT << " " << c << " = (" << rest << ") % " << num(inner[a].extent) << ";\n      p += " << c << " * " << num(inner[a].stride) << ";\n"
+          << "      const " << IT << " r" << a << " = (" << rest << ") / " << num(inner[a].extent) << ";\n";
+        rest = "r" + std::to_string(a);
+      }
+    }
+    o << "#pragma unroll\n      for (unsigned int e = 0; e < " << V << "u; ++e) {\n"
+      << "        v[e] = row_ok && j0 + e < " << num(inner_real) << " ? " << src_name << "[p] : (" << T << ")0;\n        p += " << num(inner.back().stride) << ";\n";
+    for (size_t a = inner.size(); a-- > 1;) {
+      const std::string c = "c" + std::to_string(a);
+      // carry: this axis starts over, the one outside moves on (strides are unsigned and wrap around)
+      o << "        if (++" << c << " == " << num(inner[a].extent) << ") {\n        " << c << " = 0;\n        p += " << num(inner[a - 1].stride) << " - "
+        << num(inner[a].extent * inner[a].stride) << ";\n";
+    }
+    for (size_t a = 1; a < inner.size(); ++a) o << "        }\n";
+    o << "      }\n";
     if (op.split) {
       o << "      b200_u32 w[4];\n#pragma unroll\n      for (int e = 0; e < 4; ++e) {\n        const float hi = b200_tf32(v[e]);\n"
         << "        w[e] = __float_as_uint(sg == 1" << S << " ? b200_tf32(v[e] - hi) : hi);\n      }\n"
@@ -2114,6 +2189,187 @@ struct Builder {
       code.pack_scratch_bytes = std::max(code.pack_scratch_bytes, off + bytes);
     }
   }
+
+  // A scatter accumulation that is a contraction per written window: the input gradient of a convolution,
+  //   for b, oh, ow, co, kh, kw, ci:  gx[b, s oh + kh, s ow + kw, ci] += w[co, kh, kw, ci] * dz[b, oh, ow, co].
+  // The products summed over the loops that do not move the position (co) form a dense contraction
+  // [b oh ow] x [kh kw ci] on the tensor cores, into scratch; a second kernel gives every element of the
+  // node a thread that gathers the windows covering it.  One atomic add per product sum became one read
+  // (48 x 48 x 5 images, 5 x 5 kernels, 37 of them: 171 us of atomic adds).
+  bool scatter_contraction(const std::vector<LoopDim>& nest, const StmtP& body, bool was_zero) {
+    const Stmt& set = *body;
+    if (set.kind != Stmt::Set || set.vec_len > 0 || !accumulates_into_self(set) || !opt.enable_coop) return false;
+    const Scalar& v = *set.value;
+    if (v.kind != Scalar::Tern || v.op != "fma") return false;
+    if (code.prog.tn(set.tn).prec != Prec::Single) return false;
+    const Scalar &x = *v.args[0].s, &y = *v.args[1].s;
+    if (x.kind != Scalar::Get || y.kind != Scalar::Get) return false;
+    std::map<std::string, int64_t> extent;
+    for (auto& d : nest) {
+      if (d.from != 0 || d.extent() <= 0) return false;
+      extent[d.sym] = d.extent();
+    }
+    // written position: loops by themselves, or c1 * i + c2 * j (+ fixed) with both coefficients positive
+    bool any_affine = false;
+    std::map<std::string, int> seen;
+    for (auto& ix : set.idcs) {
+      if (ix.kind == Index::Fixed) continue;
+      if (ix.kind == Index::Iter) { if (++seen[ix.sym] > 1 || !extent.count(ix.sym)) return false; continue; }
+      if (ix.kind != Index::Affine || ix.terms.empty() || ix.terms.size() > 2) return false;
+      for (auto& t : ix.terms)
+        if (t.first <= 0 || !extent.count(t.second) || ++seen[t.second] > 1) return false;
+      any_affine = any_affine || ix.terms.size() == 2;
+    }
+    if (!any_affine) return false;
+    auto uses = [](const Indices& idcs, const std::string& sy) {
+      for (auto& ix : idcs)
+        if (ix.uses(sy)) return true;
+      return false;
+    };
+    // loops of the scratch node: those of one factor, then those of the other (which holds the last axis)
+    std::vector<LoopDim> first, second, red;
+    const Index& last = set.idcs.back();
+    const std::string last_sym = last.kind == Index::Iter ? last.sym : (last.kind == Index::Affine ? last.terms.back().second : std::string());
+    const bool last_in_x = uses(x.idcs, last_sym);
+    int64_t elems = 1;
+    for (auto& d : nest) {
+      const bool ix = uses(x.idcs, d.sym), iy = uses(y.idcs, d.sym);
+      if (!seen.count(d.sym)) {
+        if (!ix || !iy) return false;
+        red.push_back(d);
+        continue;
+      }
+      if (ix == iy) return false;
+      (ix == last_in_x ? second : first).push_back(d);
+      elems *= d.extent();
+    }
+    if (first.empty() || second.empty() || red.empty() || elems * 4 > (1ll << 30) || elems >= (1ll << 31)) return false;
+    const std::string t_ident = code.prog.tn(set.tn).ident;
+    const std::vector<int64_t> t_dims = code.prog.tn(set.tn).dims;
+    const int64_t t_elems = code.prog.tn(set.tn).num_elems();
+    if (t_elems >= (1ll << 31)) return false;
+    // the contraction as a statement of its own:  P[first.., second..] := sum over red of x * y
+    int next_id = 0;
+    for (auto& t : code.prog.tnodes) next_id = std::max(next_id, t.id + 1);
+    Tnode acc, P;
+    acc.id = next_id;
+    acc.ident = "b200_acc" + std::to_string(acc.id);
+    acc.dims = {1};
+    acc.mode = Mode::Virtual;
+    P.id = next_id + 1;
+    P.ident = "b200_windows" + std::to_string(P.id);
+    P.mode = Mode::Local;
+    std::vector<LoopDim> free_loops = first;
+    free_loops.insert(free_loops.end(), second.begin(), second.end());
+    Indices at;
+    for (auto& d : free_loops) {
+      P.dims.push_back(d.extent());
+      Index ix;
+      ix.kind = Index::Iter;
+      ix.sym = d.sym;
+      at.push_back(ix);
+    }
+    auto stmt = [](Stmt::Kind k) { auto p = std::make_shared<Stmt>(); p->kind = k; return p; };
+    auto scal = [](Scalar::Kind k) { auto p = std::make_shared<Scalar>(); p->kind = k; return p; };
+    const int sid = -1000 - acc.id;
+    auto zero = scal(Scalar::Const);
+    auto init = stmt(Stmt::SetLocal);
+    init->scope_id = sid; init->tn = acc.id; init->value = zero;
+    auto get = scal(Scalar::GetLocal);
+    get->scope_id = sid; get->tn = acc.id;
+    auto mac = scal(Scalar::Tern);
+    mac->op = "fma";
+    mac->args = {v.args[0], v.args[1], {get, Prec::Single}};
+    StmtP loop = stmt(Stmt::SetLocal);
+    loop->scope_id = sid; loop->tn = acc.id; loop->value = mac;
+    for (size_t i = red.size(); i-- > 0;) {
+      auto f = stmt(Stmt::For);
+      f->index = red[i].sym; f->from = 0; f->to = red[i].to; f->body = loop;
+      loop = f;
+    }
+    auto seq = stmt(Stmt::Seq);
+    seq->items = {init, loop};
+    auto scope = scal(Scalar::LocalScope);
+    scope->scope_id = sid; scope->tn = acc.id; scope->body = seq; scope->idcs = at;
+    auto product = stmt(Stmt::Set);
+    product->tn = P.id; product->idcs = at; product->value = scope;
+    const size_t had = code.prog.tnodes.size();
+    for (auto* t : {&acc, &P}) {
+      code.prog.tn_index[t->id] = code.prog.tnodes.size();
+      code.prog.tnodes.push_back(*t);
+    }
+    Stage g;
+    int n_fused = 0;
+    CompileOptions exact = opt;
+    exact.exact_single = true;    // single-precision products were exact here, and stay so
+    if (!match_gemm(code.prog, free_loops, *product, false, exact, {}, &n_fused, &g)) {
+      code.prog.tn_index.erase(acc.id);
+      code.prog.tn_index.erase(P.id);
+      code.prog.tnodes.resize(had);
+      return false;
+    }
+    kept_stmts.push_back(product);
+    pack_stage(g);
+    g.kernel = kernel_name();
+    g.gemm_source = gemm_translation_unit(code.prog, g, g.kernel, opt);
+    code.stages.push_back(g);
+    // the gathering kernel: one thread per element of the node
+    Stage st;
+    st.kind = Stage::Generic;
+    st.kernel = kernel_name();
+    st.block = 256;
+    st.total = t_elems;
+    st.args = {{KArg::Node, set.tn}, {KArg::Node, P.id}};
+    st.writes = {set.tn};
+    std::ostringstream b;
+    std::string rem = "b200_g";
+    std::vector<std::string> pos(t_dims.size());
+    for (size_t a = t_dims.size(); a-- > 0;) {
+      pos[a] = "p" + std::to_string(a);
+      b << "    const unsigned int " << pos[a] << " = " << (a == 0 ? rem : rem + " % " + std::to_string(t_dims[a]) + "u") << ";\n";
+      if (a) {
+        b << "    const unsigned int r" << a << " = " << rem << " / " << t_dims[a] << "u;\n";
+        rem = "r" + std::to_string(a);
+      }
+    }
+    b << "    float sum = 0.0f;\n";
+    std::string pad = "    ", close;
+    for (size_t a = 0; a < set.idcs.size(); ++a) {
+      const Index& ix = set.idcs[a];
+      if (ix.kind == Index::Fixed) {
+        b << pad << "if (" << pos[a] << " == " << ix.fixed << "u) {\n";
+      } else if (ix.kind == Index::Iter) {
+        b << pad << "const unsigned int " << ix.sym << " = " << pos[a] << ";\n" << pad << "if (" << ix.sym << " < " << extent[ix.sym] << "u) {\n";
+      } else {
+        // the inner loop (the kernel position) runs, the outer one follows from what is left
+        const auto& o = ix.terms.size() == 2 ? (extent[ix.terms[0].second] >= extent[ix.terms[1].second] ? ix.terms[0] : ix.terms[1]) : ix.terms[0];
+        if (ix.terms.size() == 2) {
+          const auto& k = &o == &ix.terms[0] ? ix.terms[1] : ix.terms[0];
+          b << "#pragma unroll\n" << pad << "for (unsigned int " << k.second << " = 0; " << k.second << " < " << extent[k.second] << "u; ++" << k.second << ") {\n";
+          pad += "  ";
+          close = pad.substr(2) + "}\n" + close;
+          b << pad << "const unsigned int d" << a << " = " << pos[a] << " - " << ix.fixed << "u - " << k.second << " * " << k.first << "u;\n";
+        } else {
+          b << pad << "const unsigned int d" << a << " = " << pos[a] << " - " << ix.fixed << "u;\n";
+        }
+        // (a difference below zero wraps around and fails the comparison)
+        b << pad << "const unsigned int " << o.second << " = d" << a << (o.first > 1 ? " / " + std::to_string(o.first) + "u" : std::string()) << ";\n"
+          << pad << "if (" << o.second << " < " << extent[o.second] << "u" << (o.first > 1 ? " && d" + std::to_string(a) + " % " + std::to_string(o.first) + "u == 0u" : std::string()) << ") {\n";
+      }
+      close = pad + "}\n" + close;
+      pad += "  ";
+    }
+    Emitter em(code.prog);
+    b << pad << "sum += " << P.ident << "[" << em.offset(at, P.dims) << "];\n" << close
+      << "    " << t_ident << "[b200_g] = " << (was_zero ? "sum" : t_ident + "[b200_g] + sum") << ";\n";
+    src << "extern \"C\" __global__ void __launch_bounds__(256) " << st.kernel << "(float* " << t_ident << ", const float* __restrict__ " << P.ident << ") {\n" << kGridEntry
+        << "  for (unsigned int b200_g = blockIdx.x * 256u + threadIdx.x; b200_g < " << t_elems << "u; b200_g += gridDim.x * 256u) {\n"
+        << b.str() << "  }\n}\n\n";
+    st.note = "gathers the windows that cover an element (accumulation with moving positions)";
+    code.stages.push_back(st);
+    return true;
+  }
+  std::vector<StmtP> kept_stmts;   // statements made here whose indices stages may refer to
 
   // an epilogue that ends in a grid-wide sum keeps its per-warp partials and its ticket in the
   // routine's reduction scratch (zeroed at link; the kernel resets its ticket itself)
@@ -2403,6 +2659,10 @@ struct Builder {
           i += (size_t)n_fused;
           return;
         }
+      }
+      if (gemm_at(i) && scatter_contraction(nest, body, was_zero)) {
+        if (was_zero) drop_zero_out(body->tn);   // every element of the node is stored
+        return;
       }
       if (generic_stage(nest, body, was_zero)) drop_zero_out(body->tn);
     };

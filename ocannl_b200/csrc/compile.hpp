@@ -164,6 +164,7 @@ struct CompileOptions {
   bool enable_pairs = true;  // contraction epilogues over pairs of columns with packed 16-bit arithmetic
   bool enable_attn = true;   // the attention chain as one fused kernel
   bool enable_tf32 = true;   // single-precision operands of a contraction go through the tensor cores as tf32
+  bool exact_single = false; // (planner only) single-precision operands keep their precision: as tf32 pairs
   bool large_models = false;
   // Range-checked build: every access a generated kernel makes to a node is checked against the node's
   // size; an access outside it is skipped and reported through the device status word.  Implies the

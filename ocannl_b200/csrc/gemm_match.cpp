@@ -309,6 +309,9 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (s.extent == 1) continue;
     gk.push_back(Dim{{{s.sym, s.extent}}, s.extent, s.sa, s.sb, 0});
   }
+  // (one row, one class: the axis exists all the same)
+  if (gm.empty()) gm.push_back(Dim{});
+  if (gn.empty()) gn.push_back(Dim{});
   const std::vector<Dim> all_m = gm, all_n = gn, all_k = gk, all_b = gb;
   merge(gm); merge(gn); merge(gk); merge(gb);
   // leftover outer M / N dims become batch axes along which one operand is broadcast
@@ -326,9 +329,18 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   const int eb = prec_bytes(A.prec);
   auto ok16 = [&](int64_t elems) { return (elems * eb) % 16 == 0; };
 
+  auto product = [](const std::vector<Dim>& v) {
+    int64_t p = 1;
+    for (auto& d : v) p *= d.extent;
+    return p;
+  };
   // ---- what the tensor maps can express: 16-byte aligned bases and strides, 32-bit extents, one axis
   // each for m, n and k, unit stride along k or along m / n
+  // Single-precision operands of the shapes the tensor cores are also used for, but which are small or
+  // narrow in some direction, keep their precision (tf32 pairs); so do those that have to be gathered.
+  const bool pairs_of_tf32 = A.prec == Prec::Single && (opt.exact_single || product(all_m) < 32 || product(all_n) < 8 || product(all_k) < 16);
   auto as_it_lies = [&] {
+    if (pairs_of_tf32) return false;
     if (gm.size() != 1 || gn.size() != 1 || gk.size() != 1 || gb.size() > 2) return false;
     g.m = {gm[0].extent, gm[0].sa, 0, gm[0].sd};
     g.n = {gn[0].extent, 0, gn[0].sb, gn[0].sd};
@@ -348,13 +360,17 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     // neighbouring convolution patches overlap; only a gathered copy has them one after the other
     return true;
   };
-  auto product = [](const std::vector<Dim>& v) {
-    int64_t p = 1;
-    for (auto& d : v) p *= d.extent;
-    return p;
-  };
+  // Worth a tensor-core launch?  From a few million operations on, whatever the shape: a tile that is mostly
+  // padding (a handful of rows, two classes, a contraction over ten) still costs the epilogue of its real
+  // outputs plus about 3 us, where the loop-nest kernels take a warp or a serial loop per output
+  // (303 x 5 x 1608: 21 us).  Accumulations into few rows stay with the kernel that keeps them in registers,
+  // unless an operand has to be looked up element by element (a convolution's patches).
+  bool affine_operand = false;
+  for (auto* op : {x, y})
+    for (auto& ix : op->idcs) affine_operand = affine_operand || ix.kind == Index::Affine;
   auto worth = [&](int64_t m, int64_t n, int64_t k, int64_t batch) {
-    return m >= 32 && n >= 8 && k >= 16 && 2.0 * (double)m * (double)n * (double)k * (double)batch >= 4.0e6;
+    if (form_b ? ((m <= 16 && !affine_operand) || n < 8 || k < 4) : k < 8) return false;
+    return 2.0 * (double)m * (double)n * (double)k * (double)batch >= 4.0e6;
   };
   if (as_it_lies()) {
     if (!worth(g.m.extent, g.n.extent, g.k.extent, product(gb))) return false;
@@ -482,23 +498,29 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   const size_t n_syms = dn.syms.size();
   const std::string n_sym = n_syms >= 1 ? dn.syms.back().first : std::string();   // innermost: neighbours differ in it
   auto along_n = [&](const Indices& idcs, const std::vector<int64_t>& dims, Indices* row) {
-    if (n_syms == 0 || idcs.size() < n_syms || idcs.size() != dims.size()) return false;
-    const size_t first = idcs.size() - n_syms;
-    for (size_t q = 0; q < n_syms; ++q) {
-      const Index& ix = idcs[first + q];
-      if (ix.kind != Index::Iter || ix.sym != dn.syms[q].first) return false;
-      if (q > 0 && dims[first + q] != dn.syms[q].second) return false;
-    }
-    for (size_t a = 0; a < first; ++a)
-      for (auto& sy : dn.syms)
-        if (idcs[a].uses(sy.first)) return false;
+    if (n_syms == 0 || idcs.size() != dims.size()) return false;
     *row = idcs;
-    for (size_t q = 0; q < n_syms; ++q) {
-      Index& ix = (*row)[first + q];
-      ix.kind = Index::Fixed;
-      ix.fixed = 0;
-      ix.sym.clear();
+    size_t q = n_syms;
+    size_t a = idcs.size();
+    while (q > 0) {
+      if (a == 0) return false;
+      --a;
+      const Index& ix = idcs[a];
+      if (dims[a] == 1) {   // an axis of one position moves nothing
+        for (auto& sy : dn.syms)
+          if (ix.uses(sy.first)) return false;
+        continue;
+      }
+      --q;
+      if (ix.kind != Index::Iter || ix.sym != dn.syms[q].first) return false;
+      if (q > 0 && dims[a] != dn.syms[q].second) return false;
+      (*row)[a].kind = Index::Fixed;
+      (*row)[a].fixed = 0;
+      (*row)[a].sym.clear();
     }
+    for (size_t b = 0; b < a; ++b)
+      for (auto& sy : dn.syms)
+        if (idcs[b].uses(sy.first)) return false;
     return true;
   };
   // pair mode: b200_j counts PAIRS of columns; tiles hold one pair per entry.  Neighbouring columns
@@ -582,13 +604,27 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   std::string load_code, tile_decls;
   int n_in_tiles = 0;
   std::set<int> not_loadable = {set.tn};
-  auto collect_loads = [&](const Scalar& root, const std::map<std::string, std::string>* ren) {
+  // `col_syms`: symbols of a whole-row assignment that run over the columns; a read along one of them takes
+  // the tile's entry of that column
+  auto collect_loads = [&](const Scalar& root, const std::map<std::string, std::string>* ren, const std::set<std::string>* col_syms = nullptr) {
     std::function<void(const Scalar&)> go = [&](const Scalar& e) {
-      if (e.kind == Scalar::LocalScope) return;
+      if (e.kind == Scalar::LocalScope) {
+        if (col_syms) walk_stmt_simple(*e.body, [&](const Scalar& x) { if (x.kind == Scalar::Get) go(x); });
+        return;
+      }
       if (e.kind == Scalar::Get && !not_loadable.count(e.tn) && !n_sym.empty() && !e.idcs.empty()) {
         const Tnode& t = P.tn(e.tn);
         Indices canon = e.idcs;
-        bool ok = t.mode != Mode::Virtual && (t.prec == Prec::Single || prec_bytes(t.prec) == 2) && t.prec != Prec::Uint16;
+        std::string entry = "b200_j";
+        if (col_syms) {
+          entry.clear();
+          for (auto& ix : canon)
+            if (ix.kind == Index::Iter && col_syms->count(ix.sym)) {
+              entry = ix.sym;
+              ix.sym = n_sym;
+            }
+        }
+        bool ok = !entry.empty() && t.mode != Mode::Virtual && (t.prec == Prec::Single || prec_bytes(t.prec) == 2) && t.prec != Prec::Uint16;
         for (auto& ix : canon) {
           if (ix.kind == Index::Iter) {
             if (ren) {
@@ -671,7 +707,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
             lc << "      }\n    }\n  }\n";
             }
             load_code += lc.str();
-            em.load_tiles.push_back({e.tn, e.idcs, arr + "[b200_j]"});
+            em.load_tiles.push_back({e.tn, e.idcs, arr + "[" + entry + "]"});
             em.used_nodes.insert(e.tn);
           }
         }
@@ -807,7 +843,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     bool from_main;     // the main output's tile (already stored by the column loop's store path)
   };
   std::vector<RowNode> rownodes;
-  std::string row_code, row_decls, row_stores, final_code;
+  std::string row_code, row_decls, row_stores, final_sum, final_code;
   std::set<int> row_written;   // nodes the row followers write
   int row_fused = 0;
   size_t scratch_bytes = 0;
@@ -938,15 +974,20 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
         em.row_forwards.clear();
         for (auto& r : rownodes) em.row_forwards.push_back({r.tn, r.canon, r.n_axis, r.name, ""});
         em.unroll_loops = true;
-        std::string code = "  {\n    float b200_part = 0.0f;\n    if (b200_row_ok) {\n";
+        for (int tn : row_produced) not_loadable.insert(tn);
+        not_loadable.insert(fo.set->tn);
+        collect_loads(*fo.set->value, &ren, &col_syms);
+        std::string code = "  if (b200_row_ok) {\n";
         for (size_t i = 0; i < row_loops.size(); ++i)
           if (gloops[i].sym != row_loops[i].sym)
             code += "      const unsigned int " + gloops[i].sym + " = " + row_loops[i].sym + ";\n";
         em.scope_subst[gscope->scope_id] = "b200_part";
         code += "#pragma unroll\n      for (unsigned int " + gloops.back().sym + " = 0; " + gloops.back().sym + " < " + std::to_string(N) + "u; ++" +
-                gloops.back().sym + ") {\n" + em.stmt(*gstep, 8) + "      }\n    }\n";
+                gloops.back().sym + ") {\n" + em.stmt(*gstep, 8) + "      }\n  }\n";
+        final_sum = code;
+        row_decls += "  float b200_part = 0.0f;\n";
         // per-warp partial, ticket, ordered combine by the last warp
-        code += "    b200_part = b200_warp_sum(b200_part);\n"
+        code = "  {\n    b200_part = b200_warp_sum(b200_part);\n"
                 "    float* b200_slots = (float*)b200_partials;\n"
                 "    unsigned int* b200_ticket = (unsigned int*)(b200_partials + 4ull * b200_nslots);\n"
                 "    unsigned int b200_last = 0u;\n"
@@ -1040,6 +1081,9 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
       em.row_forwards.clear();
       for (auto& r : rownodes) em.row_forwards.push_back({r.tn, r.canon, r.n_axis, r.name, ""});
       em.unroll_loops = true;
+      for (int tn : row_produced) not_loadable.insert(tn);
+      not_loadable.insert(fo.set->tn);
+      collect_loads(*fo.set->value, &ren, &col_syms);
       const auto saved_redirect = em.set_redirect;
       em.set_redirect[fo.set->tn] = {fo.set->idcs, na >= 0 ? name + "[" + col_loop + "]" : name};
       std::string code = "    {\n";
@@ -1269,6 +1313,11 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   }
   recover(dn, "b200_n");
   fn << ep.str() << body << "    }\n  }\n";
+  // row followers: assignments over whole rows, from the register tiles -- before the operand tiles are
+  // refilled for the next tile (their rows are stored further down)
+  fn << row_decls;
+  if (!row_code.empty()) fn << "  if (b200_row_ok) {\n" << row_code << "  }\n";
+  fn << final_sum;
   // the accumulator chunk is consumed: start fetching the next one while this one is stored
   // ... or, after the tile's last chunk, the operand tiles of the first chunk of this warp's NEXT
   // tile: their latency then hides behind this chunk's stores and the wait for the next accumulator
@@ -1410,9 +1459,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
       fn << ep.str() << "      " << t.ident << "[" << em.offset(o.idcs, t.dims) << "] = " << Emitter::store_wrap(t.prec, o.arr + "[b200_j]") << ";\n    }\n  }\n";
     }
   }
-  // row followers: assignments over whole rows, from the register tiles; then the rows' stores
-  fn << row_decls;
-  if (!row_code.empty()) fn << "  if (b200_row_ok) {\n" << row_code << row_stores << "  }\n";
+  if (!row_stores.empty()) fn << "  if (b200_row_ok) {\n" << row_stores << "  }\n";
   fn << final_code;
   fn << "  B200_TRE(15);\n}\n";
 
@@ -1493,7 +1540,7 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
       const long long tiles = batch * ((g.m.extent + bm - 1) / bm) * ((g.n.extent + bn - 1) / bn);
       // few tiles over a long K: several work units per tile, each over a slice of K (gemm_split_k)
       long long split = 1;
-      if (g.may_split && tiles * 2 <= workers) split = std::max<long long>(1, std::min<long long>({workers / tiles, (long long)k_blocks / 8, 32ll}));
+      if (g.may_split && tiles * 2 <= workers) split = std::max<long long>(1, std::min<long long>(workers / tiles, (long long)k_blocks / 8));
       const double waves = (double)((tiles * split + workers - 1) / workers);
       const double loop = std::ceil(k_blocks / (double)split) * gemm_kb_us(bn, pair, g.tf32_pairs);
       const double epi = 0.25 + 3.4 * bn / 256.0;
@@ -1523,8 +1570,7 @@ static int gemm_split_k(const GemmPlan& g) {
   const long long workers = pair ? 74 : 148;
   const long long k_blocks = (g.k.extent + (128 / prec_bytes(g.in_prec)) - 1) / (128 / prec_bytes(g.in_prec));
   if (tiles * 2 > workers) return 1;
-  long long s = std::min<long long>(workers / tiles, k_blocks / 8);
-  return (int)std::max<long long>(1, std::min<long long>(s, 32));
+  return (int)std::max<long long>(1, std::min<long long>(workers / tiles, k_blocks / 8));
 }
 
 std::string gemm_translation_unit(const Program& P, Stage& st, const std::string& kernel_name, const CompileOptions&) {

@@ -100,6 +100,10 @@ __device__ __forceinline__ b200_u32 b200_pack_hf(float lo, float hi) {
 struct __align__(8) b200_f2 {
   float x, y;
 };
+// two neighbouring floats (8-byte aligned) added to memory by one instruction
+__device__ __forceinline__ void b200_red2(float* p, float x, float y) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
+}
 __device__ __forceinline__ float b200_bf2_lo(b200_u32 v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float b200_bf2_hi(b200_u32 v) { return __uint_as_float(v & 0xFFFF0000u); }
 __device__ __forceinline__ float b200_hf2_lo(b200_u32 v) { return b200_h2f((unsigned short)(v & 0xFFFFu)); }

@@ -70,3 +70,20 @@ def test_convolution_patches(device, cin, cout, kernel, stride, prec):
     assert [s["kind"] for s in info["stages"]][-1] == "gemm", info
     tol = dict(rtol=1e-5, atol=2e-6) if prec == "single" else dict(rtol=2e-2, atol=2e-3)
     compare(r, got, want, only=["y"], **tol)
+
+
+@pytest.mark.parametrize("cfg", [dict(batch=8, size=16, cin=8, cout=16), dict(batch=5, size=23, cin=3, cout=33, kernel=5),
+                                 dict(batch=40, size=17, cin=8, cout=20, stride=2)])
+@pytest.mark.parametrize("prec", ["bfloat16", "single"])
+def test_convolution_gradients_by_windows(device, cfg, prec):
+    """The input gradient as a contraction per window and a gathering kernel, the kernel gradient as a
+    contraction over all positions; strides of one and two, odd images."""
+    ir = W.conv2d_update(prec=prec, **cfg)
+    inputs = W.conv2d_inputs(prec=prec, **cfg)
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert any("gathers the windows" in s["note"] for s in info["stages"]), [s["note"] for s in info["stages"]]
+    for name in ("y", "loss", "z_grad", "bias_grad", "kernel_grad", "x_padded_grad"):
+        w, g = (W.load(prec, a[name]) if a[name].dtype == np.uint16 else a[name] for a in (want, got))
+        scale = float(np.abs(w).max())
+        np.testing.assert_allclose(g, w, rtol=2e-2 if prec != "single" else 1e-4, atol=(2e-2 if prec != "single" else 1e-5) * scale, err_msg=name)
