@@ -25,7 +25,8 @@ HOST_SOURCES = ["ir.cpp", "emit.cpp", "compile.cpp", "gemm_match.cpp", "attn_mat
                 "gemm_launch.cpp", "api.cpp"]
 CUDA_SOURCES = ["sum_static.cu"]
 EMBED = {"kNumericsSource": "kernels/numerics.cuh", "kTcSource": "kernels/tc_sm100.cuh",
-         "kGemmSource": "kernels/gemm_sm100.cuh", "kAttnSource": "kernels/attn_sm100.cuh"}
+         "kGemmSource": "kernels/gemm_sm100.cuh", "kAttnSource": "kernels/attn_sm100.cuh",
+         "kAttnRowsSource": "kernels/attn_rows.cuh"}
 
 
 def _embed() -> str:

@@ -9,8 +9,9 @@
 //   4. sum[b, s, h, 0]    := E4( v { v := 0; for t { v := v + exp[b, s, h, t] } } )
 //   5. w[b, s, h, t]      := E5( exp[b, s, h, t], sum[b, s, h, 0] )
 //   6. out[b, s, h, e]    := E6( v { v := 0; for t { v := fma(w[b, s, h, t], val[b, t, h, e], v) } } )
-// with at most two batch symbols (b, h), 16-bit q / k / val / w of one format, a head dimension of
-// 64 and 64, 128 or 256 keys.  E1 .. E6 are arbitrary expressions of the routine (a scale, a
+// with at most two batch symbols (b, h), 16-bit q / k / val / w of one format, and a head dimension of
+// 64 with 64, 128 or 256 keys (kernels/attn_sm100.cuh), or any other multiple of 16 up to 128 with any number
+// of keys up to 256 (kernels/attn_rows.cuh).  E1 .. E6 are arbitrary expressions of the routine (a scale, a
 // `where` on a mask, ...): they are emitted with the rules of every other kernel.  Operands of E1
 // that run along t and vary with s (the mask) are loaded a 32 x 32 chunk at a time with whole-row
 // accesses.  A node of the chain that is routine-local and not read after statement 6 is never
@@ -278,7 +279,11 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     return -1;
   };
   const int64_t S = extent_of(n[0], s_sym), T = extent_of(n[0], t_sym), E = r1.loop.extent();
-  if (E != 64 || !(T == 64 || T == 128 || T == 256) || S < 64) return false;
+  // Tiles of 128 queries on the tensor cores for whole tiles of keys; every other number of keys up to 256
+  // (and every head dimension that is a multiple of 16, and short sequences) goes to the kernel that keeps
+  // score rows in registers.
+  const bool rows_kernel = !(E == 64 && (T == 64 || T == 128 || T == 256) && S >= 64);
+  if (rows_kernel && (T > 256 || E % 16 != 0 || E > 128)) return false;
   if (SC.dims.back() != T) return false;
   Ren ren1;
   ren1[s_sym] = kS;
@@ -317,7 +322,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     Ren r = ren1;
     r[e_sym1] = kE;
     if (!operand(*x, r, kS, kE, &oq) || !operand(*y, r, kT, kE, &ok_)) return false;
-    if (P.tn(x->tn).dims.back() != 64 || P.tn(y->tn).dims.back() != 64) return false;
+    if (P.tn(x->tn).dims.back() != E || P.tn(y->tn).dims.back() != E) return false;
   }
 
   // ---- the row statements: each is mapped to the canonical symbols through its read of the node before it
@@ -437,14 +442,14 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
       if (!e_sym6.empty()) return false;
       e_sym6 = d.sym;
     }
-  if (e_sym6.empty() || extent_of(n[5], e_sym6) != 64) return false;
+  if (e_sym6.empty() || extent_of(n[5], e_sym6) != E) return false;
   ren6[e_sym6] = kE;
   if (!nest_matches(n[5], ren6, false, kE)) return false;
-  if (!operand(*vy, ren6, kT, kE, &ov) || V.dims.back() != 64) return false;
+  if (!operand(*vy, ren6, kT, kE, &ov) || V.dims.back() != E) return false;
   Indices out_idcs = s6.idcs;
   rename_idcs(out_idcs, ren6);
   if (out_idcs.size() != O.dims.size() || out_idcs.empty() || out_idcs.back().kind != Index::Iter || out_idcs.back().sym != kE ||
-      O.dims.back() != 64 || !plain_indices(out_idcs) || !uses(out_idcs, kS))
+      O.dims.back() != E || !plain_indices(out_idcs) || !uses(out_idcs, kS))
     return false;
   for (size_t a = 0; a + 1 < out_idcs.size(); ++a)
     if (out_idcs[a].uses(kE) || out_idcs[a].uses(kT)) return false;
@@ -529,11 +534,20 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
       written.insert(tn);
       em.used_nodes.insert(tn);   // stays a parameter: link checks its binding and alignment through it
     }
-  ptr_line("p_max", s2.tn, max_idcs, kT);
-  ptr_line("p_sum", s4.tn, sum_idcs, kT);
-  ptr_line("p_out", s6.tn, out_idcs, kE);
+  if (rows_kernel) {
+    ptr_line("p.scores", s1.tn, scores_idcs, kT);
+    ptr_line("p.mx", s2.tn, max_idcs, kT);
+    ptr_line("p.exps", s3.tn, exp_idcs, kT);
+    ptr_line("p.sum", s4.tn, sum_idcs, kT);
+    ptr_line("p.w", s5.tn, w_idcs, kT);
+    ptr_line("p.out", s6.tn, out_idcs, kE);
+  } else {
+    ptr_line("p_max", s2.tn, max_idcs, kT);
+    ptr_line("p_sum", s4.tn, sum_idcs, kT);
+    ptr_line("p_out", s6.tn, out_idcs, kE);
+  }
   // the transposing stores write 16 bytes at a time
-  {
+  if (!rows_kernel) {
     auto row16 = [&](const Tnode& t, const Indices& idcs) {
       std::map<std::string, int64_t> st;
       int64_t off = 0;
@@ -549,6 +563,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   // E1: the score of one column.  Operands that run along t and vary with s come from register
   // tiles; those that are only ever the condition of a `where` (masks) come as one bit per element.
   std::string score_loads, score_decls, cond_rows;
+  bool masked = false;
   int n_cond = 0, n_tiles_used = 0;
   std::vector<int> cond_tns;
   {
@@ -578,29 +593,33 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
       bool aligned = (off * eb) % 16 == 0;
       for (auto& kv : st)
         if (kv.first != kT && (kv.second * eb) % 16 != 0) aligned = false;
-      if (!aligned) continue;
+      if (!aligned && !rows_kernel) continue;
       bool have = false;
       for (auto& lt : em.load_tiles) have = have || (lt.tn == e.tn && same_idcs(lt.idcs, e.idcs));
       if (have) continue;
       // a mask: only ever a `where` condition.  It reaches the kernel packed to one bit per element (a
       // stage of its own makes the bits); a row's bits must start on a word boundary
-      bool cond_only = n_cond < 2 && st[kT] == 1 && off % 32 == 0;
+      // (the bits of every row of the node start on a word of their own)
+      bool cond_only = n_cond < 2 && st[kT] == 1 && t.dims.back() == T && off % T == 0;
       for (auto& kv : st)
-        if (kv.first != kT && kv.second % 32 != 0) cond_only = false;
+        if (kv.first != kT && kv.second % T != 0) cond_only = false;
       for (auto& o : reads)
         if (o.get->tn == e.tn && same_idcs(o.get->idcs, e.idcs) && !o.cond) cond_only = false;
       if (cond_only) {
         // (the tile expression stands for the node's storage bits: one and zero in its format)
         const std::string one = t.prec == Prec::Single ? "1.0f : 0.0f" : t.prec == Prec::Bfloat16 ? "(unsigned short)0x3F80 : (unsigned short)0"
                                                                                                    : "(unsigned short)0x3C00 : (unsigned short)0";
-        em.load_tiles.push_back({e.tn, e.idcs, "(((cw[" + std::to_string(n_cond) + "] >> b200_j) & 1u) ? " + one + ")"});
-        // the row's first bit, as a byte address
-        cond_rows += "  p[" + std::to_string(n_cond) + "] = row.ok ? (unsigned long long)b200_bits" + std::to_string(n_cond) + " + ((unsigned long long)(" +
-                     em.offset(zero_t(e.idcs, kT), t.dims) + ") >> 3) : 0ull;\n";
+        em.load_tiles.push_back({e.tn, e.idcs, rows_kernel ? "(cb" + std::to_string(n_cond) + " ? " + one + ")"
+                                                           : "(((cw[" + std::to_string(n_cond) + "] >> b200_j) & 1u) ? " + one + ")"});
+        // the row's first word
+        const std::string first_word = "b200_bits" + std::to_string(n_cond) + " + (unsigned long long)(" + em.offset(zero_t(e.idcs, kT), t.dims) + ") / " +
+                                       std::to_string(T) + "ull * " + std::to_string((T + 31) / 32 * 4) + "ull";
+        cond_rows += "  p[" + std::to_string(n_cond) + "] = row.ok ? " + (rows_kernel ? "(const unsigned int*)(" : "(unsigned long long)(") + first_word + ") : 0;\n";
         cond_tns.push_back(e.tn);
         ++n_cond;
         continue;
       }
+      if (rows_kernel) continue;   // read element by element where the expression needs it
       const std::string arr = "b200_op" + std::to_string(n_tiles++);
       em.load_tiles.push_back({e.tn, e.idcs, arr + "[b200_j]"});
       const int words = 32 * eb / 4;
@@ -619,6 +638,20 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     // rows beyond the last query compute on whatever the registers hold (nothing of it is stored)
     // unless the expression reads memory itself: no branch per element
     const std::string guard1 = em.direct_reads > reads_before ? "row.ok ? (float)(" + r.expr + ") : 0.f" : "(float)(" + r.expr + ")";
+    if (rows_kernel) {
+      // where(mask, score, constant): the score of a masked position is known without its product
+      std::string masked_value = "0.0f";
+      if (v1->kind == Scalar::Tern && v1->op == "where" && n_cond == 1 && v1->args[0].s->kind == Scalar::Get && v1->args[0].s->tn == cond_tns[0] &&
+          v1->args[2].s->kind == Scalar::Const) {
+        masked = true;
+        masked_value = em.constant(v1->args[2].s->cval, Prec::Single);
+      }
+      fn << "__device__ __forceinline__ float b200_ar_score(const b200_attn_row& row, unsigned int b200_t, float b200_acc, unsigned int cb0, unsigned int cb1 B200_ATTN_PARAMS) {\n"
+         << syms << "  return " << guard1 << ";\n}\n"
+         << "__device__ __forceinline__ float b200_ar_masked_score() { return " << masked_value << "; }\n"
+         << "__device__ __forceinline__ void b200_ar_cond_rows(const b200_attn_row& row, const unsigned int** p B200_ATTN_PARAMS) {\n"
+         << syms << cond_rows << "}\n";
+    } else {
     fn << "__device__ __forceinline__ void b200_attn_score_chunk(const b200_attn_row& row, unsigned int t0, const unsigned int* acc, float* x, "
           "const unsigned int* cw B200_ATTN_PARAMS) {\n"
        << syms << score_decls << score_loads
@@ -627,6 +660,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
        << "    x[b200_j] = " << guard1 << ";\n  }\n}\n";
     fn << "__device__ __forceinline__ void b200_attn_cond_rows(const b200_attn_row& row, unsigned long long* p B200_ATTN_PARAMS) {\n"
        << syms << cond_rows << "}\n";
+    }
     em.scope_subst.clear();
     em.load_tiles.clear();
   }
@@ -636,27 +670,32 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     em.scope_subst[r2.scope_id] = "reduced";
     Emitter::Res r = em.scalar(Prec::Single, *v2);
     if (!r.defs.empty()) return false;
-    fn << "__device__ __forceinline__ float b200_attn_max_init() { return " << em.constant(r2.init, Prec::Single) << "; }\n"
-       << "__device__ __forceinline__ float b200_attn_row_max(const b200_attn_row& row, float reduced B200_ATTN_PARAMS) {\n"
+    const std::string pre = rows_kernel ? "b200_ar_" : "b200_attn_";
+    fn << "__device__ __forceinline__ float " << pre << "max_init() { return " << em.constant(r2.init, Prec::Single) << "; }\n"
+       << "__device__ __forceinline__ float " << pre << "row_max(const b200_attn_row& row, float reduced B200_ATTN_PARAMS) {\n"
        << syms << "  return row.ok ? (float)(" << r.expr << ") : 0.f;\n}\n";
     em.scope_subst.clear();
     ScalarP v4 = rename_scalar(s4.value, ren4);
     em.scope_subst[r4.scope_id] = "reduced";
     Emitter::Res q = em.scalar(Prec::Single, *v4);
     if (!q.defs.empty()) return false;
-    fn << "__device__ __forceinline__ float b200_attn_row_sum(const b200_attn_row& row, float reduced B200_ATTN_PARAMS) {\n"
+    fn << "__device__ __forceinline__ float " << pre << "row_sum(const b200_attn_row& row, float reduced B200_ATTN_PARAMS) {\n"
        << syms << "  return row.ok ? (float)(" << q.expr << ") : 1.f;\n}\n";
     em.scope_subst.clear();
   }
   // E3
   {
     ScalarP v3 = rename_scalar(s3.value, ren3);
-    em.forwarded[s1.tn] = {scores_idcs, "x[b200_j]"};
+    em.forwarded[s1.tn] = {scores_idcs, rows_kernel ? "x" : "x[b200_j]"};
     em.forwarded[s2.tn] = {max_idcs, "mx"};
     const int reads_before = em.direct_reads;
     Emitter::Res r = em.scalar(Prec::Single, *v3);
     if (!r.defs.empty()) return false;
     const std::string guard3 = em.direct_reads > reads_before ? "row.ok ? (float)(" + r.expr + ") : 0.f" : "(float)(" + r.expr + ")";
+    if (rows_kernel)
+      fn << "__device__ __forceinline__ float b200_ar_exp(const b200_attn_row& row, unsigned int b200_t, float x, float mx B200_ATTN_PARAMS) {\n"
+         << syms << "  return " << guard3 << ";\n}\n";
+    else
     fn << "__device__ __forceinline__ void b200_attn_exp_chunk(const b200_attn_row& row, unsigned int t0, float* x, float mx B200_ATTN_PARAMS) {\n"
        << syms
        << "#pragma unroll\n  for (int b200_j = 0; b200_j < 32; ++b200_j) {\n    const unsigned int b200_t = t0 + (unsigned int)b200_j; (void)b200_t;\n"
@@ -667,11 +706,11 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   // value that is the same for the whole row (the sum), the divisor is prepared once per row.
   {
     ScalarP v5 = rename_scalar(s5.value, ren5);
-    em.forwarded[s3.tn] = {exp_idcs, "e[b200_j]"};
+    em.forwarded[s3.tn] = {exp_idcs, rows_kernel ? "e" : "e[b200_j]"};
     em.forwarded[s4.tn] = {sum_idcs, "sum"};
     // the expression twice when it divides by a row-invariant value: with the prepared divisor's
     // short sequence, and with the plain division for divisors outside its range (one test per chunk)
-    std::string divisor_def, fast_expr;
+    std::string divisor_def, fast_expr, divisor_expr = "1.0f";
     const int reads_before = em.direct_reads;
     if (v5->kind == Scalar::Bin && v5->op == "div" && (W.prec == Prec::Bfloat16 || W.prec == Prec::Half)) {
       bool row_invariant = true;
@@ -684,6 +723,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
       if (row_invariant && d.defs.empty() && d.expr.find("b200_j") == std::string::npos && d.expr.find("b200_t") == std::string::npos) {
         em.divisor_vars[d.expr] = "b200_dv";
         divisor_def = "  const b200_divisor b200_dv = b200_divisor_of(" + d.expr + ");\n";
+        divisor_expr = d.expr;
         Emitter::Res f = em.scalar(W.prec, *v5);
         if (!f.defs.empty()) return false;
         fast_expr = f.expr;
@@ -698,11 +738,20 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
              "    b200_a[b200_j] = " + (guarded ? "row.ok ? (float)(" + expr + ") : 0.f" : "(float)(" + expr + ")") + ";\n  }\n";
     };
     const char* pack = W.prec == Prec::Bfloat16 ? "b200_pack_bf" : "b200_pack_hf";
+    if (rows_kernel) {
+      auto guarded_expr = [&](const std::string& e) { return guarded ? "row.ok ? (float)(" + e + ") : 0.f" : "(float)(" + e + ")"; };
+      fn << "__device__ __forceinline__ float b200_ar_divisor(const b200_attn_row& row, float sum B200_ATTN_PARAMS) {\n" << syms << "  return "
+         << (divisor_expr == "1.0f" ? divisor_expr : "row.ok ? (float)(" + divisor_expr + ") : 1.0f") << ";\n}\n"
+         << "template <bool FAST>\n__device__ __forceinline__ float b200_ar_weight(const b200_attn_row& row, unsigned int b200_t, float e, float sum, const b200_divisor& b200_dv B200_ATTN_PARAMS) {\n"
+         << syms << (fast_expr.empty() ? std::string() : "  if (FAST) return " + guarded_expr(fast_expr) + ";\n") << "  return " << guarded_expr(r.expr) << ";\n}\n";
+    } else
     fn << "__device__ __forceinline__ void b200_attn_weight_chunk(const b200_attn_row& row, unsigned int t0, const float* e, float sum, unsigned int* w B200_ATTN_PARAMS) {\n"
        << syms << divisor_def << "  float b200_a[32];\n";
+    if (!rows_kernel) {
     if (!fast_expr.empty()) fn << "  if (b200_dv.fast) {\n" << loop(fast_expr) << "  } else {\n" << loop(r.expr) << "  }\n";
     else fn << loop(r.expr);
     fn << "#pragma unroll\n  for (int b200_j = 0; b200_j < 16; ++b200_j) w[b200_j] = " << pack << "(b200_a[2 * b200_j], b200_a[2 * b200_j + 1]);\n}\n";
+    }
     em.forwarded.clear();
     em.divisor_vars.clear();
   }
@@ -712,6 +761,10 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     em.scope_subst[r6.scope_id] = "b200_acc";
     Emitter::Res r = em.scalar(O.prec, *v6);
     if (!r.defs.empty()) return false;
+    if (rows_kernel) {
+      fn << "__device__ __forceinline__ " << Emitter::ctype(O.prec) << " b200_ar_out(const b200_attn_row& row, unsigned int b200_e, float b200_acc B200_ATTN_PARAMS) {\n"
+         << syms << "  return " << Emitter::store_wrap(O.prec, "(row.ok ? (" + r.expr + ") : 0.f)") << ";\n}\n";
+    } else {
     fn << "__device__ __forceinline__ void b200_attn_out_chunk(const b200_attn_row& row, unsigned int e0, const unsigned int* acc, unsigned int* w B200_ATTN_PARAMS) {\n"
        << syms << "  float b200_a[32];\n"
        << "#pragma unroll\n  for (int b200_j = 0; b200_j < 32; ++b200_j) {\n    const unsigned int b200_e = e0 + (unsigned int)b200_j; (void)b200_e;\n"
@@ -722,8 +775,12 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     else
       fn << "#pragma unroll\n  for (int b200_j = 0; b200_j < 16; ++b200_j) w[b200_j] = "
          << (O.prec == Prec::Bfloat16 ? "b200_pack_bf" : "b200_pack_hf") << "(b200_a[2 * b200_j], b200_a[2 * b200_j + 1]);\n}\n";
+    }
     em.scope_subst.clear();
   }
+  if (rows_kernel)
+    fn << "__device__ __forceinline__ void b200_ar_rows(const b200_attn_row& row, b200_ar_ptrs& p B200_ATTN_PARAMS) {\n" << syms << rows_body << "}\n";
+  else
   fn << "__device__ __forceinline__ void b200_attn_rows(const b200_attn_row& row, unsigned long long& p_max, unsigned long long& p_sum, "
         "unsigned long long& p_out B200_ATTN_PARAMS) {\n"
      << syms << rows_body << "}\n";
@@ -750,9 +807,14 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   st.args = kargs;
   st.epi_params = params;
   st.epi_args = args;
-  st.block = 256;
-  st.min_align = 16;
   AttnPlan& a = st.attn;
+  a.rows_kernel = rows_kernel;
+  a.masked = masked;
+  a.out_type = Emitter::ctype(O.prec);
+  // (sequences of a few positions: no idle warps)
+  a.warps = (int)std::min<int64_t>(4, (S + 15) / 16);
+  st.block = rows_kernel ? 32 * a.warps : 256;
+  st.min_align = rows_kernel ? 0 : 16;
   a.q_tn = oq.tn; a.k_tn = ok_.tn; a.v_tn = ov.tn;
   a.q_off = oq.off; a.k_off = ok_.off; a.v_off = ov.off;
   a.S = S; a.T = T; a.E = E; a.B0 = B0; a.B1 = B1;
@@ -788,6 +850,9 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   for (int c : {s1.tn, s3.tn, s5.tn}) kept_rows += written.count(c) > 0;
   st.note = "fused attention: scores, softmax and weights . values in one tcgen05 kernel (" + std::to_string(T) + " keys, " +
             std::to_string(kept_rows) + " of the 3 row nodes written)";
+  if (rows_kernel)
+    st.note = "fused attention, rows in registers: " + std::to_string(T) + " keys, head dimension " + std::to_string(E) + ", " + std::to_string(kept_rows) +
+              " of the 3 row nodes written";
   *out = st;
   *n_absorbed = 6;
   return true;
@@ -795,6 +860,16 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
 
 std::string attn_translation_unit(const Program&, Stage& st, const std::string& kernel_name) {
   const AttnPlan& a = st.attn;
+  if (a.rows_kernel) {
+    std::ostringstream o;
+    o << kNumericsSource << "\n#define B200_AR_NAME " << kernel_name << "\n#define B200_T " << a.T << "\n#define B200_E " << a.E << "\n#define B200_HALF "
+      << (a.in_prec == Prec::Half ? 1 : 0) << "\n#define B200_WARPS " << a.warps << "\n#define B200_OUT_T " << a.out_type << "\n#define B200_NCOND " << a.n_cond
+      << "\n#define B200_MASKED " << (a.masked ? 1 : 0) << "\n#define B200_KEEP_SCORES " << (a.scores.keep ? 1 : 0) << "\n#define B200_KEEP_EXP "
+      << (a.exps.keep ? 1 : 0) << "\n#define B200_KEEP_W " << (a.weights.keep ? 1 : 0) << "\n#define B200_ATTN_PARAMS " << st.epi_params
+      << "\n#define B200_ATTN_ARGS " << st.epi_args << "\n" << kAttnRowsSource << "\n" << a.code << "\n";
+    st.smem_bytes = (int)(2 * ((a.T + 15) / 16 * 16) * (a.E + 8) * 2);
+    return o.str();
+  }
   const unsigned int fmt = a.in_prec == Prec::Bfloat16 ? 1u : 0u;
   // instruction descriptors: fp32 accumulate, operand formats, majors (bit 16: B is n-major), N >> 3, M >> 4
   const unsigned int idesc1 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((unsigned int)(a.T >> 3) << 17) | ((128u >> 4) << 24);

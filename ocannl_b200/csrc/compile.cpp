@@ -253,7 +253,7 @@ std::string Code::describe() const {
   for (size_t i = 0; i < stages.size(); ++i) {
     const Stage& s = stages[i];
     if (i) o << ",";
-    o << "{\"kind\":\"" << (s.kind == Stage::Memset ? "memset" : s.kind == Stage::Gemm ? "gemm" : s.kind == Stage::Attn ? "attention" : "generic") << "\"";
+    o << "{\"kind\":\"" << (s.kind == Stage::Memset ? "memset" : s.kind == Stage::Gemm ? "gemm" : s.kind == Stage::Attn ? (s.attn.rows_kernel ? "row attention" : "attention") : "generic") << "\"";
     o << ",\"kernel\":\"" << s.kernel << "\",\"total\":" << s.total << ",\"coop\":" << s.coop;
     if (s.kind == Stage::Gemm) {
       o << ",\"m\":" << s.gemm.m.extent << ",\"n\":" << s.gemm.n.extent << ",\"k\":" << s.gemm.k.extent;
@@ -1977,7 +1977,7 @@ struct Builder {
   }
 
   // A node that a later stage only tests against zero (the mask of an attention stage), packed to
-  // one bit per element in element order: bit (i % 32) of word (i / 32) = (node[i] != 0).  The bits
+  // one bit per element: bit (i % 32) of word (i / 32) of its row's words = (element i != 0).  The bits
   // live in the routine's scratch; for a read-only node they are made once per run and shared by
   // every stage that asks for them.  Returns the byte offset in the reduction scratch.
   std::map<int, size_t> packed_bits;
@@ -1987,7 +1987,8 @@ struct Builder {
       auto it = packed_bits.find(tn);
       if (it != packed_bits.end()) return it->second;
     }
-    const long long words = (t.num_elems() + 31) / 32;
+    // the bits of every row (last axis) start on a word of their own
+    const long long len = t.dims.back(), row_words = (len + 31) / 32, words = t.num_elems() / len * row_words;
     const size_t off = code.reduce_scratch_bytes;
     code.reduce_scratch_bytes = (code.reduce_scratch_bytes + (size_t)words * 4 + 255) & ~(size_t)255;
     Stage st;
@@ -2002,7 +2003,9 @@ struct Builder {
         << "  unsigned int* b200_words = (unsigned int*)b200_bits;\n"
         << "  for (unsigned long long b200_i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_i < " << words * 32
         << "ull; b200_i += (unsigned long long)gridDim.x * blockDim.x) {\n"
-        << "    const bool b200_nz = b200_i < " << t.num_elems() << "ull && " << Emitter::load_wrap(t.prec, t.ident + "[b200_i]") << " != 0;\n"
+        << "    const unsigned long long b200_row = b200_i / " << row_words * 32 << "ull, b200_col = b200_i % " << row_words * 32 << "ull;\n"
+        << "    const unsigned long long b200_at = b200_row * " << len << "ull + b200_col;\n"
+        << "    const bool b200_nz = b200_col < " << len << "ull && " << Emitter::load_wrap(t.prec, t.ident + "[b200_at]") << " != 0;\n"
         << "    const unsigned int b200_w = __ballot_sync(0xffffffffu, b200_nz);\n"
         << "    if ((threadIdx.x & 31u) == 0u) b200_words[b200_i >> 5] = b200_w;\n  }\n}\n\n";
     code.stages.push_back(st);

@@ -211,6 +211,12 @@ struct AttnLaunch {
   AttnShape shape;
   unsigned int grid = 1;
   CUdeviceptr status = 0;
+  // short rows (kernels/attn_rows.cuh): plain pointers and strides
+  CUdeviceptr q = 0, k = 0, v = 0;
+  struct RowsShape {   // must match b200_ar_shape
+    unsigned int S, B0, B1, tiles;
+    long long q_row, q_b0, q_b1, k_row, k_b0, k_b1, v_row, v_b0, v_b1;
+  } rows;
 };
 
 AttnLaunch* attn_prepare(b200_routine* r, int si) {
@@ -228,6 +234,16 @@ AttnLaunch* attn_prepare(b200_routine* r, int si) {
   if ((q | k | v) & 15)
     throw Error(B200_E_INVALID, "link: internal error: an attention stage was kept for operands that are not 16-byte aligned");
   auto* L = new AttnLaunch();
+  if (a.rows_kernel) {
+    L->q = q; L->k = k; L->v = v;
+    L->rows = {(unsigned)a.S, (unsigned)a.B0, (unsigned)a.B1, (unsigned)((a.S + 16 * a.warps - 1) / (16 * a.warps)), a.q_row, a.q_b0, a.q_b1,
+               a.k_row, a.k_b0, a.k_b1, a.v_row, a.v_b0, a.v_b1};
+    L->grid = L->rows.tiles * L->rows.B0 * L->rows.B1;
+    const CUresult e = cu().cuFuncSetAttribute_(r->fns[si], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, st.smem_bytes);
+    if (e != CUDA_SUCCESS) delete L;
+    cu_check(e, "cuFuncSetAttribute(max dynamic shared memory)");
+    return L;
+  }
   try {
     // in the terms of encode_operand: the head dimension is "k" of the first contraction (unit stride);
     // the values are the n-major B operand of the second one (n = head dimension, k = key position)
@@ -282,6 +298,12 @@ void attn_enqueue(b200_routine* r, int si) {
   const Stage& st = r->code->code.stages[si];
   AttnLaunch* L = r->attn[si];
   std::vector<void*> args;
+  if (st.attn.rows_kernel) {
+    args = {&L->q, &L->k, &L->v, &L->rows};
+    for (auto& v : r->arg_values[si]) args.push_back(&v);
+    launch_kernel(r->dev, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(row attention)", 1u);
+    return;
+  }
   args.push_back(&L->map_q);
   args.push_back(&L->map_k);
   args.push_back(&L->map_v);

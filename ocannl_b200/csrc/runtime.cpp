@@ -87,8 +87,9 @@ static bool misaligned_stages(const b200_code* c, const std::map<int, CUdevicept
     } else if (st.kind == Stage::Attn) {
       // tensor maps over the queries, keys and values; 16-byte row stores into every node it writes
       bool bad = ((at(st.attn.q_tn) | at(st.attn.k_tn) | at(st.attn.v_tn)) & 15) != 0;
-      for (auto& a : st.args)
-        if (a.kind == KArg::Node && (at(a.tn) & 15) != 0) bad = true;
+      if (!st.attn.rows_kernel)   // (whose row nodes and output are written element by element)
+        for (auto& a : st.args)
+          if (a.kind == KArg::Node && (at(a.tn) & 15) != 0) bad = true;
       if (bad)
         for (int o : st.origins) any |= no_gemm_at->insert(o).second;
     }

@@ -1,0 +1,26 @@
+"""The attention chain with short or odd rows in one kernel (score rows in registers): key counts at the
+edges of its tiles of 8 and 16, head dimensions of one to eight k steps, fewer queries than a warp takes,
+with and without a mask, a row masked throughout, nodes kept or routine-local."""
+import numpy as np
+import pytest
+
+from ocannl_b200 import workloads as W
+from tests.parity import compare, run_device, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("b,h,s,t,e", [(2, 3, 5, 7, 16), (2, 2, 16, 8, 32), (1, 2, 33, 100, 64), (3, 1, 65, 129, 48),
+                                       (1, 1, 200, 255, 32), (2, 1, 30, 256, 128), (1, 4, 17, 31, 112)])
+@pytest.mark.parametrize("mode,mask,prec", [("ctx", True, "bfloat16"), ("local", True, "half"), ("ctx", False, "half"), ("local", False, "bfloat16")])
+def test_row_attention(device, b, h, s, t, e, mode, mask, prec):
+    ir = W.attention(b, h, s, t, prec=prec, mask=mask, row_mode=mode, d_head=e)
+    inputs = W.attention_inputs(b, h, s, t, prec=prec, d_head=e)
+    if mask:
+        inputs["mask"][s // 2] = 0.0        # every key masked: equal weights
+    else:
+        del inputs["mask"]
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert any(st["kind"] == "row attention" for st in info["stages"]), info
+    compare(ir, got, want, rtol=2e-2, atol=2e-2 if prec == "bfloat16" else 4e-3)
