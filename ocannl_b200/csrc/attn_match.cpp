@@ -812,7 +812,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   a.masked = masked;
   a.out_type = Emitter::ctype(O.prec);
   // (sequences of a few positions: no idle warps)
-  a.warps = (int)std::min<int64_t>(4, (S + 15) / 16);
+  a.warps = (int)std::min<int64_t>(8, (S + 15) / 16);
   st.block = rows_kernel ? 32 * a.warps : 256;
   st.min_align = rows_kernel ? 0 : 16;
   a.q_tn = oq.tn; a.k_tn = ok_.tn; a.v_tn = ov.tn;

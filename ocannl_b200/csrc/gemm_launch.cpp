@@ -8,7 +8,7 @@ using namespace b200;
 
 // must match b200_gemm_shape in kernels/gemm_sm100.cuh
 struct GemmShape {
-  unsigned int M, N, K, B0, B1, a_b0, a_b1, b_b0, b_b1, tiles_m, tiles_n, tma_out;
+  unsigned int tma_out;
 };
 
 struct GemmLaunch {
@@ -98,21 +98,7 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
   }
   GemmShape& s = L->shape;
   memset(&s, 0, sizeof s);
-  s.M = (unsigned)g.m.extent;
-  s.N = (unsigned)g.n.extent;
-  s.K = (unsigned)g.k.extent;
-  s.B0 = s.B1 = 1;
-  s.a_b0 = s.a_b1 = s.b_b0 = s.b_b1 = 0;
   const int nb = (int)g.batch.size();
-  if (nb == 2) {
-    s.B0 = (unsigned)g.batch[0].extent;
-    s.B1 = (unsigned)g.batch[1].extent;
-    s.a_b0 = g.batch[0].sa != 0; s.b_b0 = g.batch[0].sb != 0;
-    s.a_b1 = g.batch[1].sa != 0; s.b_b1 = g.batch[1].sb != 0;
-  } else if (nb == 1) {
-    s.B1 = (unsigned)g.batch[0].extent;
-    s.a_b1 = g.batch[0].sa != 0; s.b_b1 = g.batch[0].sb != 0;
-  }
   // The outputs as TMA store destinations: [n, m, inner batch, outer batch], a box of 32 rows x one
   // epilogue chunk, swizzled like the staging tile (128 / 64 / 32 bytes per row).  If any of them
   // cannot be described (an address that is not 16-byte aligned), the kernel keeps to plain stores.
@@ -151,9 +137,9 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
   } else {
     L->in_maps.assign(st.in_maps.size(), L->map_a);
   }
-  s.tiles_m = (s.M + st.tile_m - 1) / st.tile_m;
-  s.tiles_n = (s.N + st.tile_n - 1) / st.tile_n;
-  unsigned long long tiles = (unsigned long long)s.tiles_m * s.tiles_n * s.B0 * s.B1 * (unsigned long long)(g.split_k > 0 ? g.split_k : 1);
+  unsigned long long tiles = (unsigned long long)((g.m.extent + st.tile_m - 1) / st.tile_m) * (unsigned long long)((g.n.extent + st.tile_n - 1) / st.tile_n) *
+                             (unsigned long long)(g.split_k > 0 ? g.split_k : 1);
+  for (auto& d : g.batch) tiles *= (unsigned long long)d.extent;
   cu_check(cu().cuFuncSetAttribute_(r->fns[si], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, st.smem_bytes),
            "cuFuncSetAttribute(max dynamic shared memory)");
   if (st.cta_pair) {

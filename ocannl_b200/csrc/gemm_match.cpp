@@ -369,6 +369,9 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   for (auto* op : {x, y})
     for (auto& ix : op->idcs) affine_operand = affine_operand || ix.kind == Index::Affine;
   auto worth = [&](int64_t m, int64_t n, int64_t k, int64_t batch) {
+    // (products of single rows or columns, one per batch index, are reductions: a layer norm's sum of squares)
+    if (batch > 1 && (m < 16 || n < 8)) return false;
+    if (m == 1 && n == 1) return false;
     if (form_b ? ((m <= 16 && !affine_operand) || n < 8 || k < 4) : k < 8) return false;
     return 2.0 * (double)m * (double)n * (double)k * (double)batch >= 4.0e6;
   };
@@ -1621,13 +1624,25 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
     << "u\n#define B200_TMEM_COLS " << tmem_cols << "\n#define B200_RASTER " << raster << "\n#define B200_CTA_PAIR "
     << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n#define B200_FLUSH " << (g.tf32_pairs ? 1 : 0) << "\n";
   if (g.tf32_pairs) o << "#define B200_PAIRS 1\n#define B200_SEG " << g.packs[0].seg << "\n";
+  {
+    int64_t b0 = 1, b1 = 1;
+    const GemmDim *d0 = nullptr, *d1 = nullptr;
+    if (g.batch.size() == 2) { d0 = &g.batch[0]; d1 = &g.batch[1]; }
+    else if (g.batch.size() == 1) d1 = &g.batch[0];
+    if (d0) b0 = d0->extent;
+    if (d1) b1 = d1->extent;
+    o << "#define B200_M " << g.m.extent << "u\n#define B200_N " << g.n.extent << "u\n#define B200_K " << g.k.extent << "u\n#define B200_B0 " << b0
+      << "u\n#define B200_B1 " << b1 << "u\n#define B200_A_B0 " << (d0 && d0->sa != 0) << "u\n#define B200_A_B1 " << (d1 && d1->sa != 0)
+      << "u\n#define B200_B_B0 " << (d0 && d0->sb != 0) << "u\n#define B200_B_B1 " << (d1 && d1->sb != 0) << "u\n#define B200_TILES_M "
+      << (g.m.extent + bm - 1) / bm << "u\n#define B200_TILES_N " << (g.n.extent + bn - 1) / bn << "u\n";
+  }
   o << "#define B200_EPI_CHUNK " << chunk << "\n#define B200_STAGING_BYTES " << staging << "\n#define B200_STAGING_TILES " << staging_tiles << "\n#define B200_LOAD_TILE_BYTES " << load_tile << "\n";
   o << "#define B200_EPI_PROLOGUE " << [&] { std::string p = st.epi_prologue; for (auto& c : p) if (c == '\n') c = ' '; return p; }() << "\n";
   o << kTcSource << "\n" << g.epilogue << "\n";
   o << "#define B200_EPI_PARAMS " << params << "\n";
-  o << "#define B200_EPILOGUE_ROWS b200_epilogue_rows(b200_tiles, b200_b0, b200_b1, b200_m, b200_m < shape.M" << args << ");\n";
-  o << "#define B200_EPILOGUE_LOAD b200_epilogue_load(b200_tiles, b200_b0, b200_b1, b200_m, b200_m < shape.M, b200_pn0, shape.N, b200_es" << args << ");\n";
-  o << "#define B200_EPILOGUE_ROW b200_epilogue_row(b200_r, b200_b0, b200_b1, b200_m, b200_m < shape.M, b200_n0, shape.N, b200_stage, b200_has_next, b200_next_taddr, b200_tiles, b200_slot, b200_nslots, b200_nx_ok, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_m < shape.M, b200_nx_n0, b200_es" << args << ");\n";
+  o << "#define B200_EPILOGUE_ROWS b200_epilogue_rows(b200_tiles, b200_b0, b200_b1, b200_m, b200_m < B200_M" << args << ");\n";
+  o << "#define B200_EPILOGUE_LOAD b200_epilogue_load(b200_tiles, b200_b0, b200_b1, b200_m, b200_m < B200_M, b200_pn0, B200_N, b200_es" << args << ");\n";
+  o << "#define B200_EPILOGUE_ROW b200_epilogue_row(b200_r, b200_b0, b200_b1, b200_m, b200_m < B200_M, b200_n0, B200_N, b200_stage, b200_has_next, b200_next_taddr, b200_tiles, b200_slot, b200_nslots, b200_nx_ok, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_m < B200_M, b200_nx_n0, b200_es" << args << ");\n";
   o << kGemmSource << "\n";
   std::ostringstream note;
   note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.tf32_pairs ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages

@@ -35,12 +35,11 @@
 #ifndef B200_TC_SM100_CUH
 #include "tc_sm100.cuh"
 #endif
+// The shape is part of what is compiled: B200_M / _N / _K, batch extents B200_B0 (outer) and B200_B1 (inner),
+// B200_A_B0 .. B200_B_B1 (1 when the operand varies along that batch axis), B200_TILES_M / _N.  Tile coordinates
+// are quotients by these; as kernel arguments they cost the producer seven chained divisions, about 0.3 us,
+// before its first copy.
 struct b200_gemm_shape {
-  unsigned int M, N, K;
-  unsigned int B0, B1;          // batch extents, outer and inner (1 when absent)
-  unsigned int a_b0, a_b1;      // 1 when the operand varies along that batch axis
-  unsigned int b_b0, b_b1;
-  unsigned int tiles_m, tiles_n;
   unsigned int tma_out;         // != 0: the epilogue's row-contiguous outputs leave as TMA stores (their maps are valid)
 };
 
@@ -173,10 +172,10 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
   const unsigned int worker = blockIdx.x / (1 + B200_CTA_PAIR), n_workers = gridDim.x / (1 + B200_CTA_PAIR);
   if (threadIdx.x == 0) B200_TR(2);   // set-up done
 
-  const unsigned int tiles_per_batch = shape.tiles_m * shape.tiles_n;
-  const unsigned int total_tiles = tiles_per_batch * shape.B0 * shape.B1;
-  const unsigned int k_blocks = (shape.K + B200_BK - 1) / B200_BK;
-  const unsigned int total_units = total_tiles * B200_SPLITK;
+  constexpr unsigned int tiles_per_batch = B200_TILES_M * B200_TILES_N;
+  constexpr unsigned int total_tiles = tiles_per_batch * B200_B0 * B200_B1;
+  constexpr unsigned int k_blocks = (B200_K + B200_BK - 1) / B200_BK;
+  constexpr unsigned int total_units = total_tiles * B200_SPLITK;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -189,13 +188,13 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
         const unsigned int bidx = tile / tiles_per_batch;
         const unsigned int t = tile - bidx * tiles_per_batch;
         // consecutive tiles walk down m first so that a wave of CTAs shares few B tiles
-        const unsigned int group = t / (B200_RASTER * shape.tiles_n);
+        const unsigned int group = t / (B200_RASTER * B200_TILES_N);
         const unsigned int first_m = group * B200_RASTER;
-        const unsigned int rows = min((unsigned int)B200_RASTER, shape.tiles_m - first_m);
-        const unsigned int r = t - group * B200_RASTER * shape.tiles_n;
+        const unsigned int rows = min((unsigned int)B200_RASTER, B200_TILES_M - first_m);
+        const unsigned int r = t - group * B200_RASTER * B200_TILES_N;
         const unsigned int mt = first_m + r % rows;
         const unsigned int nt = r / rows;
-        const unsigned int b0 = bidx / shape.B1, b1 = bidx - b0 * shape.B1;
+        const unsigned int b0 = bidx / B200_B1, b1 = bidx - b0 * B200_B1;
         // this CTA's rows of A and its share of the tile's B columns
         const int m0 = (int)(mt * B200_BM + cta_rank * B200_CTA_M), n0 = (int)(nt * B200_BN + cta_rank * B200_CTA_N);
         for (unsigned int kb = kb0; kb < kb1; ++kb) {
@@ -215,20 +214,20 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           const int k0 = (int)(kb * B200_BK) + part * B200_SEG;
           const unsigned int pa = sa + part * B200_A_TILE_BYTES, pb = sb + part * B200_B_TILE_BYTES;
 #if B200_A_KMAJOR
-          b200_tma_load_4d(pa, &map_a, full, k0, m0, (int)(b1 * shape.a_b1), (int)(b0 * shape.a_b0));
+          b200_tma_load_4d(pa, &map_a, full, k0, m0, (int)(b1 * B200_A_B1), (int)(b0 * B200_A_B0));
 #else
 #pragma unroll
           for (int c = 0; c < B200_CTA_M / B200_ROW_ELEMS; ++c)
             b200_tma_load_4d(pa + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_a, full, m0 + c * B200_ROW_ELEMS, k0,
-                             (int)(b1 * shape.a_b1), (int)(b0 * shape.a_b0));
+                             (int)(b1 * B200_A_B1), (int)(b0 * B200_A_B0));
 #endif
 #if B200_B_KMAJOR
-          b200_tma_load_4d(pb, &map_b, full, k0, n0, (int)(b1 * shape.b_b1), (int)(b0 * shape.b_b0));
+          b200_tma_load_4d(pb, &map_b, full, k0, n0, (int)(b1 * B200_B_B1), (int)(b0 * B200_B_B0));
 #else
 #pragma unroll
           for (int c = 0; c < B200_CTA_N / B200_ROW_ELEMS; ++c)
             b200_tma_load_4d(pb + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_b, full, n0 + c * B200_ROW_ELEMS, k0,
-                             (int)(b1 * shape.b_b1), (int)(b0 * shape.b_b0));
+                             (int)(b1 * B200_B_B1), (int)(b0 * B200_B_B0));
 #endif
           }
           if (unit == worker && kb == kb0) B200_TR(3);   // first loads issued
@@ -321,14 +320,14 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       tile = u % total_tiles;
       const unsigned int bidx = tile / tiles_per_batch;
       const unsigned int t = tile - bidx * tiles_per_batch;
-      const unsigned int group = t / (B200_RASTER * shape.tiles_n);
+      const unsigned int group = t / (B200_RASTER * B200_TILES_N);
       const unsigned int first_m = group * B200_RASTER;
-      const unsigned int rows = min((unsigned int)B200_RASTER, shape.tiles_m - first_m);
-      const unsigned int r = t - group * B200_RASTER * shape.tiles_n;
+      const unsigned int rows = min((unsigned int)B200_RASTER, B200_TILES_M - first_m);
+      const unsigned int r = t - group * B200_RASTER * B200_TILES_N;
       mt = first_m + r % rows;
       nt = r / rows;
-      b0 = bidx / shape.B1;
-      b1 = bidx - b0 * shape.B1;
+      b0 = bidx / B200_B1;
+      b1 = bidx - b0 * B200_B1;
     };
     // operand tiles of the epilogue (bias, mask, residual rows ...): loaded for a tile's first chunk
     // before its accumulator is waited for -- by the previous tile's last chunk when there was one
@@ -349,14 +348,14 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
         b200_coords(unit + n_workers, ntile, b200_nx_b0, b200_nx_b1, nmt, nnt);
         b200_nx_m = nmt * B200_BM + cta_rank * B200_CTA_M + quarter * 32u + lane;
         b200_nx_n0 = nnt * B200_BN + col_half * cols_per_warp;
-        b200_nx_ok = b200_nx_n0 < shape.N;
+        b200_nx_ok = b200_nx_n0 < B200_N;
       }
       B200_EPILOGUE_ROWS
       if (!b200_prefetched) {
         const unsigned int b200_pn0 = nt * B200_BN + col_half * cols_per_warp;
-        if (b200_pn0 < shape.N) { B200_EPILOGUE_LOAD }
+        if (b200_pn0 < B200_N) { B200_EPILOGUE_LOAD }
       }
-      b200_prefetched = b200_nx_ok && (nt * B200_BN + col_half * cols_per_warp < shape.N);
+      b200_prefetched = b200_nx_ok && (nt * B200_BN + col_half * cols_per_warp < B200_N);
 #if B200_FLUSH
       constexpr int kCols = (B200_BN / (B200_EPI_WARPS / 4) + B200_EPI_CHUNK - 1) / B200_EPI_CHUNK * B200_EPI_CHUNK;
       const unsigned int col0 = col_half * cols_per_warp;
@@ -388,11 +387,11 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
 #pragma unroll
       for (int c = 0; c < kCols; c += B200_EPI_CHUNK) {
         const unsigned int b200_n0 = nt * B200_BN + col0 + c;
-        if (b200_n0 >= shape.N) break;  // warp-uniform
+        if (b200_n0 >= B200_N) break;  // warp-uniform
         unsigned int b200_r[B200_EPI_CHUNK];
 #pragma unroll
         for (int j = 0; j < B200_EPI_CHUNK; ++j) b200_r[j] = __float_as_uint(b200_sum[c + j]);
-        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < shape.N);
+        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < B200_N);
         const unsigned int b200_next_taddr = tmem_base;   // (a load that nothing reads)
         B200_EPILOGUE_ROW
       }
@@ -409,17 +408,17 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       // deliberately not unrolled: the generated epilogue can be thousands of instructions.)
       unsigned int b200_r[B200_EPI_CHUNK];
       const unsigned int col0 = col_half * cols_per_warp;
-      if (nt * B200_BN + col0 < shape.N) b200_tmem_ld_chunk(taddr + col0, b200_r);
+      if (nt * B200_BN + col0 < B200_N) b200_tmem_ld_chunk(taddr + col0, b200_r);
 #pragma unroll 1
       for (unsigned int c = 0; c < cols_per_warp; c += B200_EPI_CHUNK) {
         const unsigned int col = col0 + c;
         const unsigned int b200_n0 = nt * B200_BN + col;
-        if (b200_n0 >= shape.N) break;  // warp-uniform
+        if (b200_n0 >= B200_N) break;  // warp-uniform
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #ifdef B200_TRACE
         B200_TRE(4);
 #endif
-        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < shape.N);
+        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < B200_N);
         const unsigned int b200_next_taddr = taddr + col + B200_EPI_CHUNK;
         // every lane takes part: rows beyond M compute nothing but help move the chunk
         B200_EPILOGUE_ROW
