@@ -178,7 +178,7 @@ void gemm_enqueue(b200_routine* r, int si) {
   for (size_t a = 0; a < vals.size(); ++a) args.push_back(&vals[a]);
   for (auto& m : L->in_maps) args.push_back(&m);
   for (auto& m : L->out_maps) args.push_back(&m);
-  launch_kernel(r->dev, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(contraction)",
+  launch_kernel(r, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(contraction)",
                 st.cta_pair ? 2u : 1u);
 }
 
@@ -287,7 +287,7 @@ void attn_enqueue(b200_routine* r, int si) {
   if (st.attn.rows_kernel) {
     args = {&L->q, &L->k, &L->v, &L->rows};
     for (auto& v : r->arg_values[si]) args.push_back(&v);
-    launch_kernel(r->dev, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(row attention)", 1u);
+    launch_kernel(r, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(row attention)", 1u);
     return;
   }
   args.push_back(&L->map_q);
@@ -300,7 +300,7 @@ void attn_enqueue(b200_routine* r, int si) {
   args.push_back(&L->status);
   std::vector<CUdeviceptr>& vals = r->arg_values[si];
   for (size_t a = 0; a < vals.size(); ++a) args.push_back(&vals[a]);
-  launch_kernel(r->dev, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(attention)", 1u);
+  launch_kernel(r, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(attention)", 1u);
 }
 
 void attn_release(AttnLaunch* a) { delete a; }

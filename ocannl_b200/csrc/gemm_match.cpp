@@ -1507,8 +1507,8 @@ static double gemm_kb_us(int bn, bool pair, bool tf32_pairs) {
 
 // Tile shape of a contraction: columns per tile, and whether two CTAs share a 256-row tile.
 //
-// Measured times follow   2.3 us + e + l + (waves - 1) max(l, e)   within 10 %, with l the main loop of one
-// tile (k blocks x gemm_kb_us) and e its epilogue, 0.25 us + 3.4 us x columns / 256: the last tile's
+// Measured times follow   2.3 us + e + l + (waves - 1) (max(l, e) + 0.25 us)   within 10 %, with l the main
+// loop of one tile (k blocks x gemm_kb_us) and e its epilogue, 0.25 us + 3.4 us (3.2 in pairs) x columns / 256: the last tile's
 // epilogue is exposed, the others hide behind the next tile's main loop or the other way round; a CTA
 // pair pays 0.5 us more set-up (cluster barrier, paired tensor-memory allocation).  Large problems
 // therefore take the widest pairs; one of few tiles takes the shape that spreads it over the SMs
@@ -1546,8 +1546,8 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
       if (g.may_split && tiles * 2 <= workers) split = std::max<long long>(1, std::min<long long>(workers / tiles, (long long)k_blocks / 8));
       const double waves = (double)((tiles * split + workers - 1) / workers);
       const double loop = std::ceil(k_blocks / (double)split) * gemm_kb_us(bn, pair, g.tf32_pairs);
-      const double epi = 0.25 + 3.4 * bn / 256.0;
-      const double t = 2.3 + (pair ? 0.5 : 0.0) + epi + loop + (waves - 1.0) * std::max(loop, epi);
+      const double epi = 0.25 + (pair ? 3.2 : 3.4) * bn / 256.0;
+      const double t = 2.3 + (pair ? 0.5 : 0.0) + epi + loop + (waves - 1.0) * (std::max(loop, epi) + 0.25);
       if (t < best - 1e-9) {
         best = t;
         best_bn = bn;

@@ -146,6 +146,7 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
     scratch_zero.swap(merged);
   }
   const size_t reduce_off = off;
+  reduce_base = off;
   off += c->code.reduce_scratch_bytes;
   off = (off + 255) & ~(size_t)255;
   pack_base = off;
@@ -220,7 +221,7 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
 // the grids before it (griddepcontrol) ahead of its first access to memory, so a launch may be
 // marked for programmatic stream serialisation: the next kernel's blocks are placed, and run their
 // set-up, while the tail of the previous kernel drains.  B200_PDL=0 turns the marking off.
-void launch_kernel(b200_dev* dev, CUfunction fn, unsigned grid, unsigned bx, unsigned by, unsigned smem, void** args,
+void launch_kernel(b200_routine* r, CUfunction fn, unsigned grid, unsigned bx, unsigned by, unsigned smem, void** args,
                    const char* what, unsigned cluster) {
   static const bool pdl = [] {
     const char* e = getenv("B200_PDL");
@@ -231,7 +232,7 @@ void launch_kernel(b200_dev* dev, CUfunction fn, unsigned grid, unsigned bx, uns
   cfg.gridDimX = grid; cfg.gridDimY = 1; cfg.gridDimZ = 1;
   cfg.blockDimX = bx; cfg.blockDimY = by; cfg.blockDimZ = 1;
   cfg.sharedMemBytes = smem;
-  cfg.hStream = dev->stream;
+  cfg.hStream = r->on;
   CUlaunchAttribute attr[2];
   memset(attr, 0, sizeof attr);
   unsigned n = 0;
@@ -240,7 +241,7 @@ void launch_kernel(b200_dev* dev, CUfunction fn, unsigned grid, unsigned bx, uns
     attr[n].value.clusterDim.x = cluster; attr[n].value.clusterDim.y = 1; attr[n].value.clusterDim.z = 1;
     ++n;
   }
-  if (pdl) {
+  if (pdl && r->pdl) {
     attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
     attr[n].value.programmaticStreamSerializationAllowed = 1;
     ++n;
@@ -269,10 +270,128 @@ void b200_routine::enqueue_bucket(OverlapBucket& b) {
   cu_check(cu().cuEventRecord_(b.done, c->stream), "cuEventRecord(bucket done)");
 }
 
-void b200_routine::enqueue_stages() {
+// Which stages of a captured graph may run beside one another.  Two stages are ordered when one writes
+// memory the other touches; everything else is independent -- the three projections of an attention layer, a
+// layer's weight, bias and input gradients, the updates of different parameters -- and small kernels leave
+// most of the machine idle.  A stage continues the branch of the latest stage it depends on if nothing has
+// continued it yet (a chain stays in one stream, where a launch overlaps the end of the one before it);
+// otherwise it goes to a branch whose last stage it depends on anyway, or to a free one, and waits for its
+// dependencies there.  At most kBranches; the last one takes what finds no place.
+static const int kBranches = 4;
+std::vector<b200_routine::Placed> b200_routine::branches() const {
   const Program& P = code->code.prog;
+  const auto& stages = code->code.stages;
+  const size_t n = stages.size();
+  struct Range { CUdeviceptr lo, hi; bool write; };
+  std::vector<std::vector<Range>> touched(n);
+  for (size_t i = 0; i < n; ++i) {
+    const Stage& st = stages[i];
+    auto node = [&](int tn, bool write) {
+      auto it = node_ptr.find(tn);
+      if (it != node_ptr.end()) touched[i].push_back({it->second, it->second + (CUdeviceptr)P.tn(tn).bytes(), write});
+    };
+    auto slot = [&](int s, bool write) {
+      if (s >= 0) touched[i].push_back({pack_address(s), pack_address(s) + (CUdeviceptr)code->code.pack_bytes[(size_t)s], write});
+    };
+    for (int tn : st.writes) node(tn, true);
+    if (st.kind == Stage::Memset) node(st.memset_tn, true);
+    for (auto& a : st.args) {
+      if (a.kind == KArg::Node && !std::count(st.writes.begin(), st.writes.end(), a.tn)) node(a.tn, false);
+      // a piece of the reduction scratch (partials with their ticket, packed masks): known by its first byte
+      if (a.kind == KArg::Scratch) {
+        const CUdeviceptr p = scratch + (CUdeviceptr)reduce_base + (CUdeviceptr)a.tn;
+        touched[i].push_back({p, p + 1, true});
+      }
+    }
+    for (int s : st.pack_writes) slot(s, true);
+    if (st.kind == Stage::Gemm) {
+      if (st.gemm.pack_a) slot(st.gemm.a_slot, false); else node(st.gemm.a_tn, false);
+      if (st.gemm.pack_b) slot(st.gemm.b_slot, false); else node(st.gemm.b_tn, false);
+    }
+    if (st.kind == Stage::Attn)
+      for (int tn : {st.attn.q_tn, st.attn.k_tn, st.attn.v_tn}) node(tn, false);
+  }
+  std::vector<std::vector<char>> before(n, std::vector<char>(n, 0));   // before[i][j]: stage j has to be complete when i starts
+  std::vector<Placed> out(n);
+  std::vector<int> last(kBranches, -1);
+  for (size_t i = 0; i < n; ++i) {
+    std::vector<int> deps;   // latest first, without those implied by a later one
+    for (size_t j = i; j-- > 0;) {
+      if (before[i][j]) continue;
+      bool ordered = false;
+      for (auto& a : touched[i])
+        for (auto& b : touched[j])
+          if ((a.write || b.write) && a.lo < b.hi && b.lo < a.hi) ordered = true;
+      if (!ordered) continue;
+      deps.push_back((int)j);
+      before[i][j] = 1;
+      for (size_t k = 0; k < j; ++k) before[i][k] |= before[j][k];
+    }
+    int br = -1;
+    for (int d : deps)
+      if (last[(size_t)out[(size_t)d].branch] == d) { br = out[(size_t)d].branch; break; }
+    for (int b = 0; b < kBranches && br < 0; ++b)
+      if (last[(size_t)b] >= 0 && before[i][(size_t)last[(size_t)b]]) br = b;
+    for (int b = 0; b < kBranches && br < 0; ++b)
+      if (last[(size_t)b] < 0) br = b;
+    if (br < 0) br = kBranches - 1;
+    out[i].branch = br;
+    // what the branch's own order already implies
+    const int prev = last[(size_t)br];
+    if (prev >= 0) {
+      before[i][(size_t)prev] = 1;
+      for (int k = 0; k < prev; ++k) before[i][(size_t)k] |= before[(size_t)prev][(size_t)k];
+    }
+    for (int d : deps)
+      if (out[(size_t)d].branch != br && !(prev >= 0 && before[(size_t)prev][(size_t)d])) {
+        out[i].waits.push_back(d);
+        out[(size_t)d].awaited = true;
+      }
+    last[(size_t)br] = (int)i;
+  }
+  for (int b = 1; b < kBranches; ++b)
+    if (last[(size_t)b] >= 0) out[(size_t)last[(size_t)b]].awaited = true;   // joined at the end
+  return out;
+}
+
+void b200_routine::enqueue_stages(bool capturing) {
+  const Program& P = code->code.prog;
+  on = dev->stream;
+  pdl = true;
+  // branches of the graph: streams and events that only exist while it is captured
+  std::vector<Placed> placed;
+  if (capturing && buckets.empty() && !profiling && code->code.stages.size() > 1) placed = branches();
+  std::map<int, CUevent> done;
+  std::vector<CUstream>& streams = fork_streams;   // (released once the capture has ended)
+  auto mark = [&](int key, CUstream s) {
+    CUevent e = nullptr;
+    cu_check(cu().cuEventCreate_(&e, CU_EVENT_DISABLE_TIMING), "cuEventCreate(branch)");
+    fork_events.push_back(e);
+    done[key] = e;
+    cu_check(cu().cuEventRecord_(e, s), "cuEventRecord(branch)");
+  };
   for (auto& z : scratch_zero)
     cu_check(cu().cuMemsetD8Async_(scratch + z.first, 0, z.second, dev->stream), "cuMemsetD8Async(scratch)");
+  if (!placed.empty()) {
+    streams.assign(kBranches, nullptr);
+    streams[0] = dev->stream;
+    bool any = false;
+    for (auto& p : placed) any = any || p.branch > 0;
+    if (any) mark(-1, dev->stream);
+  }
+  // puts stage i on its branch and makes it wait for its dependencies on other branches
+  auto place = [&](size_t i) {
+    if (placed.empty()) return;
+    const Placed& p = placed[i];
+    pdl = p.waits.empty();
+    if (!streams[(size_t)p.branch]) {
+      cu_check(cu().cuStreamCreate_(&streams[(size_t)p.branch], CU_STREAM_NON_BLOCKING), "cuStreamCreate(branch)");
+      cu_check(cu().cuStreamWaitEvent_(streams[(size_t)p.branch], done[-1], 0), "cuStreamWaitEvent(branch)");
+      pdl = false;
+    }
+    on = streams[(size_t)p.branch];
+    for (int d : p.waits) cu_check(cu().cuStreamWaitEvent_(on, done.at(d), 0), "cuStreamWaitEvent(branch)");
+  };
   if (profiling && stage_events.size() != code->code.stages.size()) stage_events.assign(code->code.stages.size(), {});
   struct Timer {
     b200_routine* r;
@@ -296,6 +415,7 @@ void b200_routine::enqueue_stages() {
   // queues stage i (a clear may take the clears that follow along, advancing i)
   auto queue_stage = [&](size_t& i) {
     const Stage& st = code->code.stages[i];
+    place(i);
     Timer timer(this, i);
     if (st.kind == Stage::Memset) {
       // zero_outs of nodes that lie back to back in memory (parameter gradients allocated as one
@@ -307,7 +427,7 @@ void b200_routine::enqueue_stages() {
           if (b.after_stage == (int)k) return true;
         return false;
       };
-      while (!profiling && !fires_after(i) && i + 1 < code->code.stages.size() && code->code.stages[i + 1].kind == Stage::Memset) {
+      while (!profiling && placed.empty() && !fires_after(i) && i + 1 < code->code.stages.size() && code->code.stages[i + 1].kind == Stage::Memset) {
         const int next_tn = code->code.stages[i + 1].memset_tn;
         const CUdeviceptr next_at = node_ptr[next_tn];
         const size_t next_bytes = (size_t)P.tn(next_tn).bytes();
@@ -316,7 +436,7 @@ void b200_routine::enqueue_stages() {
         else break;
         ++i;
       }
-      cu_check(cu().cuMemsetD8Async_(at, 0, bytes, dev->stream), "cuMemsetD8Async");
+      cu_check(cu().cuMemsetD8Async_(at, 0, bytes, on), "cuMemsetD8Async");
       return;
     }
     if (st.kind == Stage::Generic && st.total <= 0) return;
@@ -338,14 +458,24 @@ void b200_routine::enqueue_stages() {
     if (blocks < 1) blocks = 1;
     if (st.block_y > 1) blocks = std::min<long long>(cap, (st.total + st.block - 1) / st.block);
     if (st.grid_override > 0) blocks = st.grid_override;
-    launch_kernel(dev, fns[i], (unsigned)blocks, (unsigned)st.block, (unsigned)st.block_y, 0, args.data(), "cuLaunchKernelEx");
+    launch_kernel(this, fns[i], (unsigned)blocks, (unsigned)st.block, (unsigned)st.block_y, 0, args.data(), "cuLaunchKernelEx");
     dev->n_launches++;
   };
   for (size_t i = 0; i < code->code.stages.size(); ++i) {
     queue_stage(i);
+    if (!placed.empty() && placed[i].awaited) mark((int)i, on);
     for (auto& b : buckets)
       if (b.after_stage == (int)i) enqueue_bucket(b);
   }
+  // every branch ends in the device's stream
+  if (!placed.empty()) {
+    std::vector<int> tail(kBranches, -1);
+    for (size_t i = 0; i < placed.size(); ++i) tail[(size_t)placed[i].branch] = (int)i;
+    for (int b = 1; b < kBranches; ++b)
+      if (tail[(size_t)b] >= 0) cu_check(cu().cuStreamWaitEvent_(dev->stream, done.at(tail[(size_t)b]), 0), "cuStreamWaitEvent(join)");
+  }
+  on = dev->stream;
+  pdl = true;
   // whatever follows the routine on the compute stream (the optimizer step) sees the reduced ranges
   for (auto& b : buckets) cu_check(cu().cuStreamWaitEvent_(dev->stream, b.done, 0), "cuStreamWaitEvent(bucket done)");
 }
@@ -395,14 +525,24 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       graph_merge_epoch = dev->merge_epoch;
       CUgraph g = nullptr;
       cu_check(cu().cuStreamBeginCapture_(dev->stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL), "cuStreamBeginCapture");
+      auto release_branches = [&] {
+        for (auto e : fork_events) cu().cuEventDestroy_(e);
+        for (size_t b = 1; b < fork_streams.size(); ++b)
+          if (fork_streams[b]) cu().cuStreamDestroy_(fork_streams[b]);
+        fork_events.clear();
+        fork_streams.clear();
+      };
       try {
-        enqueue_stages();
+        enqueue_stages(/*capturing=*/true);
       } catch (...) {
         cu().cuStreamEndCapture_(dev->stream, &g);
         if (g) cu().cuGraphDestroy_(g);
+        release_branches();
         throw;
       }
-      cu_check(cu().cuStreamEndCapture_(dev->stream, &g), "cuStreamEndCapture");
+      const CUresult ended = cu().cuStreamEndCapture_(dev->stream, &g);
+      release_branches();
+      cu_check(ended, "cuStreamEndCapture");
       CUresult r = cu().cuGraphInstantiateWithFlags_(&graph, g, 0);
       cu().cuGraphDestroy_(g);
       cu_check(r, "cuGraphInstantiate");

@@ -130,6 +130,7 @@ struct b200_routine {
   std::map<int, CUdeviceptr> node_ptr;
   CUdeviceptr scratch = 0;                         // routine-local nodes
   size_t scratch_bytes = 0;
+  size_t reduce_base = 0;                          // ... partial results of reductions behind this one
   size_t pack_base = 0;                            // packed operands of contractions lie behind this offset of the scratch slab
   CUdeviceptr pack_address(int slot) const { return scratch + pack_base + code->code.pack_offsets.at((size_t)slot); }
   std::vector<std::pair<size_t, size_t>> scratch_zero;  // (offset, bytes) cleared every run
@@ -149,11 +150,24 @@ struct b200_routine {
   std::vector<OverlapBucket> buckets;
   bool overlap_warm = false;      // the attached collectives have run once outside a capture
   void enqueue_bucket(OverlapBucket& b);
+  // Where the next stage is queued: the device's stream, or -- while a graph is being captured -- the branch
+  // the stage belongs to; and whether its launch may start before the one ahead of it in that stream ends.
+  CUstream on = nullptr;
+  bool pdl = true;
+  // The stages of a captured graph as branches (see branches() in runtime.cpp).
+  struct Placed {
+    int branch = 0;
+    std::vector<int> waits;   // stages on other branches this one has to wait for
+    bool awaited = false;     // some stage on another branch, or the end of the routine, waits for this one
+  };
+  std::vector<Placed> branches() const;
+  std::vector<CUstream> fork_streams;   // of the capture under way
+  std::vector<CUevent> fork_events;
   std::set<int> pools_used;   // pools of the bound nodes (what a launch has to wait for, uploads-wise)
   b200_code* requested = nullptr;  // the code `link` was given; `code` may be a variant of it
   void link(b200_dev* d, b200_code* c, const b200_binding* b, int n);
   void launch(const int64_t* static_idx, int n_static);
-  void enqueue_stages();
+  void enqueue_stages(bool capturing = false);
   void set_graph(bool on);
   void stage_time(int stage, float* total_ms, int* runs);
   void destroy();
@@ -170,5 +184,5 @@ void attn_release(AttnLaunch* a);
 
 // One kernel launch on the device's stream, marked for programmatic stream serialisation
 // (runtime.cpp).
-void launch_kernel(b200_dev* dev, CUfunction fn, unsigned grid, unsigned bx, unsigned by, unsigned smem, void** args,
+void launch_kernel(b200_routine* r, CUfunction fn, unsigned grid, unsigned bx, unsigned by, unsigned smem, void** args,
                    const char* what, unsigned cluster = 1);
