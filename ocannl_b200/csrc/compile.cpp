@@ -310,6 +310,11 @@ struct Piece {
   bool pairs = false;
   int64_t ser_work = 1;
   std::vector<int> staged;   // small read-only nodes the kernel first copies into shared memory
+  // a sum kept in `b200_self` over the serial loops (`t[p] := t[p] + term`): its parts, so that several
+  // lanes may share one sum
+  bool sum = false;
+  std::string self_type, self_init, zero, inner, after;
+  std::vector<LoopDim> ser;
 };
 
 struct Builder {
@@ -856,7 +861,7 @@ struct Builder {
     // Accumulator promotion: `t[p] := f(t[p], ...)` under serial loops that do not move p keeps
     // t[p] in a register across those loops (one load, or none when the node is known to be zero,
     // and one store) instead of a read-modify-write of memory per iteration.
-    std::string before, after;
+    std::string before, after, self_type, self_init;
     if (scatter) {
       const Stmt& set = *body;
       const Tnode& t = code.prog.tn(set.tn);
@@ -891,12 +896,14 @@ struct Builder {
         if (pairs) {
           const std::string PT = Emitter::pair_type(t.prec);
           const std::string at = "(" + t.ident + " + " + off + ")";
-          before = "    " + PT + " b200_self = " +
-                   (lhs_zero ? (t.prec == Prec::Single ? std::string("b200_f2{0.0f, 0.0f}") : std::string("0u")) : "*(const " + PT + "*)" + at) + ";\n";
+          self_type = PT;
+          self_init = lhs_zero ? (t.prec == Prec::Single ? std::string("b200_f2{0.0f, 0.0f}") : std::string("0u")) : "*(const " + PT + "*)" + at;
+          before = "    " + PT + " b200_self = " + self_init + ";\n";
           after = "    *(" + PT + "*)" + at + " = b200_self;\n";
         } else {
-          before = std::string("    ") + Emitter::rtype(t.prec) + " b200_self = " +
-                   (lhs_zero ? em.constant(0.0, t.prec) : Emitter::load_wrap(t.prec, lv)) + ";\n";
+          self_type = Emitter::rtype(t.prec);
+          self_init = lhs_zero ? em.constant(0.0, t.prec) : Emitter::load_wrap(t.prec, lv);
+          before = "    " + self_type + " b200_self = " + self_init + ";\n";
           after = "    " + lv + " = " + Emitter::store_wrap(t.prec, "b200_self") + ";\n";
         }
         em.forwarded[set.tn] = {set.idcs, "b200_self"};
@@ -1048,6 +1055,16 @@ struct Builder {
       pc.per_row = st.total / pc.rows * ser_work;
     }
     if (!scatter) pc.any_body = body;
+    if (!self_type.empty() && ser_work > 1 && (code.prog.tn(body->tn).prec == Prec::Single || code.prog.tn(body->tn).prec == Prec::Double) &&
+        accumulates_into_self(*body)) {
+      pc.sum = true;
+      pc.self_type = self_type;
+      pc.self_init = self_init;
+      pc.zero = pairs ? "b200_f2{0.0f, 0.0f}" : "0";
+      pc.inner = inner;
+      pc.after = after;
+      pc.ser = st.ser;
+    }
     if (!staged.empty()) {      // keeps a kernel of its own
       pc.staged = staged;
       pc.fusable = false;
@@ -1121,6 +1138,31 @@ struct Builder {
     f.writes.assign(w.begin(), w.end());
   }
 
+  // Nodes small enough live in shared memory for the length of the block: read once at its start, written
+  // back at its end, and routine-local ones that no other stage touches never reach memory at all.  A stage
+  // then waits some 30 cycles for what the one before it wrote instead of some 300.  The barrier
+  // between two stages is left out when neither writes what the other touches; a sum with few outputs
+  // (a gradient over the batch) is shared by as many lanes of a warp as there are.  (The 25 stages of the
+  // 2-16-16-1 training step: 11.6 us through memory.)
+  std::map<int, std::set<size_t>> node_stages;   // node -> stages that touch it, by index into code.stages
+  void note_node_stages() {
+    node_stages.clear();
+    for (size_t i = 0; i < code.stages.size(); ++i) {
+      const Stage& st = code.stages[i];
+      if (st.kind == Stage::Memset) node_stages[st.memset_tn].insert(i);
+      auto it = pieces.find(i);
+      if (it != pieces.end())
+        for (int n : it->second.used) node_stages[n].insert(i);
+      for (auto& a : st.args)
+        if (a.kind == KArg::Node) node_stages[a.tn].insert(i);
+      if (st.kind == Stage::Gemm)
+        for (int n : {st.gemm.a_tn, st.gemm.b_tn, st.gemm.d_tn}) node_stages[n].insert(i);
+      if (st.kind == Stage::Attn)
+        for (int n : {st.attn.q_tn, st.attn.k_tn, st.attn.v_tn}) node_stages[n].insert(i);
+      for (int n : st.writes) node_stages[n].insert(i);
+    }
+  }
+
   Stage emit_fused(const std::vector<size_t>& idx) {
     Stage f;
     merge_origins(f, idx);
@@ -1132,42 +1174,158 @@ struct Builder {
     Emitter em(code.prog);
     std::set<int> written;
     std::string text;
+    std::set<int> fresh_w, fresh_r;   // written / read since the last barrier
+    auto barrier_for = [&](const std::set<int>& used, const std::set<int>& writes) {
+      bool need = false;
+      for (int n : used) need = need || fresh_w.count(n);
+      for (int n : writes) need = need || fresh_r.count(n);
+      if (need) {
+        text += "  __syncthreads();\n";
+        fresh_w.clear();
+        fresh_r.clear();
+      } else if (!text.empty()) {
+        text += "  // __syncthreads() left out: neither stage writes what the other touches\n";
+      }
+      fresh_r.insert(used.begin(), used.end());
+      fresh_w.insert(writes.begin(), writes.end());
+    };
+    std::set<int> first_cleared;   // nodes whose first use here overwrites them
+    std::set<int> moving;          // nodes read at a static index: a slice of something larger
+    std::set<std::string> statics_syms;
+    for (auto& sy : code.prog.statics) statics_syms.insert(sy.sym);
     for (size_t i : idx) {
       const Stage& st = code.stages[i];
       if (st.kind == Stage::Memset) {
         const Tnode& t = code.prog.tn(st.memset_tn);
+        if (!em.used_nodes.count(t.id)) first_cleared.insert(t.id);
+        barrier_for({t.id}, {t.id});
         em.used_nodes.insert(t.id);
         written.insert(t.id);
         text += "  for (unsigned int b200_z = threadIdx.x; b200_z < " + std::to_string(t.num_elems()) +
                 "u; b200_z += blockDim.x) " + t.ident + "[b200_z] = " + em.storage_zero(t.prec) + ";\n";
       } else {
         const Piece& pc = pieces[i];
+        barrier_for(pc.used, pc.written);
+        if (pc.any_body && pc.any_body->kind == Stmt::Set && !em.used_nodes.count(pc.any_body->tn) && !pc.sum && covers_node(*pc.any_body, pc.par)) {
+          bool reads = false;
+          walk_scalar(*pc.any_body->value, [&](const Scalar& e) {
+            if ((e.kind == Scalar::Get || e.kind == Scalar::GetDyn) && e.tn == pc.any_body->tn) reads = true;
+          }, [](const Stmt&) {});
+          if (!reads) first_cleared.insert(pc.any_body->tn);   // written in full before anything reads it
+        }
         f.min_align = std::max(f.min_align, st.min_align);
         em.used_nodes.insert(pc.used.begin(), pc.used.end());
         written.insert(pc.written.begin(), pc.written.end());
         em.uses_merge |= pc.uses_merge;
-        text += "  {\n";
-        if (st.coop) {
-          text += "  const unsigned int b200_t = threadIdx.x & 31u;\n";
-          text += "  for (unsigned long long b200_g = threadIdx.x >> 5; b200_g < " + std::to_string(st.total) +
-                  "ull; b200_g += blockDim.x >> 5) {\n";
+        if (pc.any_body)
+          walk_stmt(*pc.any_body, [&](const Scalar& e) {
+            if (e.kind == Scalar::Get || e.kind == Scalar::GetDyn)
+              for (auto& ix : e.idcs)
+                for (auto& sy : statics_syms)
+                  if (ix.uses(sy)) moving.insert(e.tn);
+          }, [&](const Stmt& w) {
+            if (w.kind == Stmt::Set)
+              for (auto& ix : w.idcs)
+                for (auto& sy : statics_syms)
+                  if (ix.uses(sy)) moving.insert(w.tn);
+          });
+        int64_t ser_total = 1;
+        for (auto& d : pc.ser) ser_total *= d.extent();
+        int64_t share = 1;   // lanes per sum
+        if (pc.sum)
+          while (share < 32 && share * 2 * st.total <= 1024 && share * 4 <= ser_total) share *= 2;
+        if (share > 1) {
+          const std::string S = std::to_string(share) + "u";
+          text += "  {\n  const unsigned int b200_s = threadIdx.x % " + S + ", b200_gq = threadIdx.x / " + S + ";\n  const bool b200_on = b200_gq < " +
+                  std::to_string(st.total) + "u;\n  const unsigned int b200_g = b200_on ? b200_gq : 0u;\n" + pc.decomp + "    " + pc.self_type + " b200_self = " +
+                  pc.zero + ";\n    if (b200_on) {\n      if (b200_s == 0u) b200_self = " + pc.self_init + ";\n      for (unsigned int b200_l = b200_s; b200_l < " +
+                  std::to_string(ser_total) + "u; b200_l += " + S + ") {\n";
+          std::string rem = "b200_l";
+          for (size_t q = pc.ser.size(); q-- > 0;) {
+            const LoopDim& d = pc.ser[q];
+            const std::string ext = std::to_string(d.extent()) + "u";
+            text += "        const unsigned int " + d.sym + " = " + (q == 0 ? rem : rem + " % " + ext) + (d.from ? " + " + std::to_string(d.from) + "u" : std::string()) + ";\n";
+            if (q) {
+              text += "        const unsigned int b200_lq" + std::to_string(q) + " = " + rem + " / " + ext + ";\n";
+              rem = "b200_lq" + std::to_string(q);
+            }
+          }
+          text += pc.inner + "      }\n    }\n#pragma unroll\n    for (unsigned int b200_o = 1u; b200_o < " + S + "; b200_o <<= 1) ";
+          if (pc.pairs)
+            text += "{\n      const b200_f2 b200_w = {__shfl_xor_sync(0xffffffffu, b200_self.x, b200_o), __shfl_xor_sync(0xffffffffu, b200_self.y, b200_o)};\n"
+                    "      b200_self = b200_f2{b200_self.x + b200_w.x, b200_self.y + b200_w.y};\n    }\n";
+          else
+            text += "b200_self = b200_self + __shfl_xor_sync(0xffffffffu, b200_self, b200_o);\n";
+          text += "    if (b200_on && b200_s == 0u) {\n" + pc.after + "    }\n  }\n";
         } else {
-          text += "  for (unsigned long long b200_g = threadIdx.x; b200_g < " + std::to_string(st.total) +
-                  "ull; b200_g += blockDim.x) {\n";
+          text += "  {\n";
+          if (st.coop) {
+            text += "  const unsigned int b200_t = threadIdx.x & 31u;\n";
+            text += "  for (unsigned int b200_g = threadIdx.x >> 5; b200_g < " + std::to_string(st.total) + "u; b200_g += blockDim.x >> 5) {\n";
+          } else {
+            text += "  for (unsigned int b200_g = threadIdx.x; b200_g < " + std::to_string(st.total) + "u; b200_g += blockDim.x) {\n";
+          }
+          text += pc.decomp + pc.body_text + "  }\n  }\n";
         }
-        text += pc.decomp + pc.body_text + "  }\n  }\n";
       }
-      text += "  __syncthreads();\n";
+    }
+    // which nodes move into shared memory: the smallest first
+    std::vector<int> small;
+    if (!opt.bounds)
+      for (int n : em.used_nodes) {
+        const Tnode& t = code.prog.tn(n);
+        if (t.mode != Mode::Virtual && t.prec != Prec::Uint4x32 && t.bytes() <= 12288 && !moving.count(n)) small.push_back(n);
+      }
+    std::sort(small.begin(), small.end(), [&](int a, int b) { return code.prog.tn(a).bytes() < code.prog.tn(b).bytes() || (code.prog.tn(a).bytes() == code.prog.tn(b).bytes() && a < b); });
+    std::string decls, load, land, store;
+    size_t bytes = 0;
+    for (int n : small) {
+      const Tnode& t = code.prog.tn(n);
+      const size_t sz = ((size_t)t.bytes() + 15) & ~(size_t)15;
+      if (bytes + sz > 45056) break;
+      const std::string T = Emitter::ctype(t.prec), count = std::to_string(t.num_elems()) + "u";
+      bool mine = t.mode == Mode::Local;   // a routine-local node no other stage touches
+      for (size_t i : node_stages[n]) mine = mine && std::count(idx.begin(), idx.end(), i);
+      decls += "  __shared__ __align__(16) " + T + " b200_sm_" + t.ident + "[" + std::to_string(t.num_elems()) + "];\n";
+      const std::string each = "  for (unsigned int b200_z = threadIdx.x; b200_z < " + count + "; b200_z += 1024u) ";
+      if (mine) {
+        if (t.zero_init && !first_cleared.count(n)) load += each + "b200_sm_" + t.ident + "[b200_z] = " + em.storage_zero(t.prec) + ";\n";
+        em.used_nodes.erase(n);
+      } else {
+        // (all of the block's loads are in flight before the first of them is stored)
+        if (!first_cleared.count(n))
+          for (int64_t q = 0; q * 1024 < t.num_elems(); ++q) {
+            const std::string v = "b200_in" + std::to_string(n) + "_" + std::to_string(q), at = "threadIdx.x + " + std::to_string(q * 1024) + "u";
+            const std::string in = at + " < " + count;
+            load += "  " + T + " " + v + " = 0;\n  if (" + in + ") " + v + " = " + t.ident + "__g[" + at + "];\n";
+            land += "  if (" + in + ") b200_sm_" + t.ident + "[" + at + "] = " + v + ";\n";
+          }
+        if (written.count(n)) store += each + t.ident + "__g[b200_z] = b200_sm_" + t.ident + "[b200_z];\n";
+      }
+      decls += "  " + T + "* const " + t.ident + " = b200_sm_" + t.ident + ";\n";
+      bytes += sz;
+      moved_to_shared.insert(n);
     }
     std::string statics = static_prologue(text, em, 2);
-    std::ostringstream k_src;
-    k_src << "extern \"C\" __global__ void __launch_bounds__(1024) " << f.kernel << "(";
-    emit_params(k_src, f, em, written);
-    k_src << ") {\n" << kGridEntry << statics << text << "}\n\n";
+    std::ostringstream params, k_src;
+    emit_params(params, f, em, written);
+    // parameters of the nodes that moved get another name; the node's own name is its copy
+    std::string ps = params.str();
+    for (int n : moved_to_shared) {
+      const std::string& id = code.prog.tn(n).ident;
+      for (size_t q = 0; (q = ps.find(id, q)) != std::string::npos; q += id.size()) {
+        const bool l = q > 0 && ps[q - 1] == ' ', r = q + id.size() == ps.size() || ps[q + id.size()] == ',';
+        if (l && r) ps.insert(q + id.size(), "__g");
+      }
+    }
+    moved_to_shared.clear();
+    k_src << "extern \"C\" __global__ void __launch_bounds__(1024) " << f.kernel << "(" << ps << ") {\n" << kGridEntry << decls << statics << load << land
+          << (load.empty() ? "" : "  __syncthreads();\n") << text << (store.empty() ? "" : "  __syncthreads();\n") << store << "}\n\n";
     src << k_src.str();
     f.note = "fused " + std::to_string(idx.size()) + " small stages in one block";
     return f;
   }
+  std::set<int> moved_to_shared;
 
   // Warp-per-row fusion.  A run of stages that share their L outermost parallel loops ("the
   // row": (batch, position, head) of an attention softmax), some of which reduce over the rest of
@@ -1813,6 +1971,7 @@ struct Builder {
       code.stages.swap(kept);
       pieces.swap(moved);
     }
+    note_node_stages();
     std::vector<Stage> out;
     auto fusable = [&](size_t i) {
       const Stage& st = code.stages[i];
@@ -1878,7 +2037,10 @@ struct Builder {
           continue;
         }
       }
-      if (opt.enable_fuse && !fusable(i) && pointwise_member(i, nullptr)) {
+      // (a long chain over thousands of elements -- the momentum update of a 300 x 100 layer -- is a kernel of
+      // its own even where one block could take it: that block spent 30 us on four passes over it)
+      const bool long_chain = code.stages[i].kind == Stage::Generic && code.stages[i].total >= 4096;
+      if (opt.enable_fuse && (!fusable(i) || long_chain) && pointwise_member(i, nullptr)) {
         const Piece& first = pieces[i];
         std::vector<size_t> run = {i};
         size_t j = i + 1;
@@ -1887,7 +2049,7 @@ struct Builder {
           if (!rows_independent_prefix(run, first.par.size())) { run.pop_back(); break; }
           ++j;
         }
-        if (run.size() >= 2) {
+        if (run.size() >= (fusable(i) ? 3u : 2u)) {
           out.push_back(emit_pointwise_chain(run));
           i = run.back() + 1;
           continue;
@@ -2384,6 +2546,23 @@ struct Builder {
     code.reduce_scratch_bytes = (code.reduce_scratch_bytes + 255) & ~(size_t)255;
   }
 
+  // A routine of one kernel takes its static indices as a kernel argument instead of through the device
+  // table: such a routine is always launched directly (see b200_routine::launch), where the table would cost a
+  // copy ahead of the kernel every time an index moves -- the next minibatch of a training step.
+  void statics_by_value() {
+    if (code.stages.size() != 1 || code.stages[0].kind != Stage::Generic || opt.bounds) return;
+    for (auto& a : code.stages[0].args)
+      if (a.kind == KArg::Statics) a.kind = KArg::StaticValues;
+      else continue;
+    const std::string was = "const unsigned int* __restrict__ b200_statics";
+    const size_t at = code.source.find(was);
+    if (at == std::string::npos) return;
+    code.source.replace(at, was.size(), "const b200_static_values b200_statics");
+    const size_t k = code.source.rfind("extern \"C\" __global__", at);
+    code.source.insert(k, "struct b200_static_values {\n  unsigned int v[" + std::to_string(code.prog.statics.size()) +
+                              "];\n  __device__ __forceinline__ unsigned int operator[](int i) const { return v[i]; }\n};\n");
+  }
+
   // Range-checked build.  Every generic kernel's node pointers are renamed and shadowed by a
   // b200_checked proxy of the node's size (kernels/numerics.cuh), so that each `node[offset]` the
   // emitters wrote is compared with the number of elements the node has; the kernels get the device
@@ -2679,6 +2858,7 @@ struct Builder {
     emit_kernels();
     place_packs();
     code.source = src.str();
+    statics_by_value();
     if (opt.bounds) apply_bounds();
     // routine-local nodes that some stage touches get scratch (a node whose every use was fused
     // away, such as the score matrix of a fused attention stage, needs none)

@@ -20,7 +20,7 @@ struct LoopDim {
 // One kernel argument: a tensor node pointer (in-context node, or a routine-local node that
 // lives in the routine's scratch slab), the static-index table, or the merge buffer.
 struct KArg {
-  enum Kind { Node, Statics, Merge, Scratch, Status, Pack } kind;   // Status: the device status word (range-checked builds)
+  enum Kind { Node, Statics, StaticValues, Merge, Scratch, Status, Pack } kind;   // Status: the device status word (range-checked builds)
   int tn = -1;  // node id; for Scratch: byte offset into the routine's reduction scratch; for Pack: slot of a packed operand
 };
 

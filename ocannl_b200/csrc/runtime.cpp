@@ -164,7 +164,14 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
     else if (param_ptr.count(t.id)) node_ptr[t.id] = param_ptr[t.id];
   }
 
-  if (!P.statics.empty()) {
+  for (auto& st : c->code.stages)
+    for (auto& a : st.args) statics_by_value |= a.kind == KArg::StaticValues;
+  if (statics_by_value) static_values.assign(P.statics.size(), 0u);
+  // One kernel and nothing else: launched on its own even when graphs are on.  A graph of one node adds about
+  // 1.5 us between two runs (and waits for the previous one at a granularity of 2 us); from two kernels on
+  // it saves as much in launch calls.
+  direct = c->code.stages.size() == 1 && c->code.stages[0].kind != Stage::Memset && scratch_zero.empty();
+  if (!P.statics.empty() && !statics_by_value) {
     cu_check(cu().cuMemAlloc_(&statics_dev, 256 + 4 * P.statics.size()), "cuMemAlloc(statics)");
     void* hp = nullptr;
     cu_check(cu().cuMemHostAlloc_(&hp, kRing * 4 * P.statics.size(), 0), "cuMemHostAlloc(statics)");
@@ -199,6 +206,8 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
         arg_values[i].push_back(statics_dev);
       } else if (a.kind == KArg::Scratch) {
         arg_values[i].push_back(scratch + reduce_off + (size_t)a.tn);
+      } else if (a.kind == KArg::StaticValues) {
+        arg_values[i].push_back(0);   // (the launch passes static_values)
       } else if (a.kind == KArg::Pack) {
         arg_values[i].push_back(pack_address(a.tn));
       } else {
@@ -449,8 +458,9 @@ void b200_routine::enqueue_stages(bool capturing) {
     std::vector<CUdeviceptr>& vals = arg_values[i];
     for (size_t a = 0; a < st.args.size(); ++a)
       if (st.args[a].kind == KArg::Merge) vals[a] = dev->address(0, 0, (size_t)P.tn(P.merge_node).bytes());
-    std::vector<void*> args(vals.size());
-    for (size_t a = 0; a < vals.size(); ++a) args[a] = &vals[a];
+    std::vector<void*>& args = launch_args;
+    args.resize(vals.size());
+    for (size_t a = 0; a < vals.size(); ++a) args[a] = st.args[a].kind == KArg::StaticValues ? (void*)static_values.data() : (void*)&vals[a];
     long long threads = st.coop ? st.total * st.coop : st.total;
     long long blocks = (threads + st.block - 1) / st.block;
     long long cap = (long long)dev->sm_count * 16;
@@ -497,6 +507,9 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       if (!statics_valid || last_statics[i] != v) changed = true;
     }
     if (changed) {
+      if (statics_by_value) {
+        for (int i = 0; i < n_static; ++i) static_values[(size_t)i] = (unsigned int)static_idx[i];
+      } else {
       if (ring_pos == kRing) {  // staging slots may still be in flight: drain before reuse
         cu_check(cu().cuStreamSynchronize_(dev->stream), "cuStreamSynchronize");
         ring_pos = 0;
@@ -507,6 +520,7 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       for (int i = 0; i < n_static; ++i) slot[i] = (unsigned int)static_idx[i];
       cu_check(cu().cuMemcpyHtoDAsync_(statics_dev, slot, 4 * (size_t)n_static, dev->stream), "cuMemcpyHtoDAsync(statics)");
       statics_valid = true;
+      }
     }
   }
   // The first run with collectives attached is queued directly: NCCL sets up the connections a
@@ -514,7 +528,7 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
   // not happen inside a stream capture.  Later runs capture and replay.
   const bool capture_ok = buckets.empty() || overlap_warm;
   if (!buckets.empty()) overlap_warm = true;
-  if (want_graph && !profiling && capture_ok) {
+  if (want_graph && !direct && !profiling && capture_ok) {
     if (graph && reads_merge && graph_merge_epoch != dev->merge_epoch) {
       // the merge buffer moved since the capture (`b200_merge_copy` grew pool 0): the graph holds
       // the old address

@@ -138,6 +138,9 @@ struct b200_routine {
   unsigned int* statics_ring = nullptr;            // page-locked staging
   size_t ring_pos = 0;
   std::vector<long long> last_statics;
+  std::vector<unsigned int> static_values;         // ... as an argument of a routine's only kernel (then there is no table)
+  bool statics_by_value = false;
+  bool direct = false;                            // so few launches that a graph would only add its own
   bool statics_valid = false;
   bool want_graph = false;
   bool profiling = false;
@@ -161,6 +164,7 @@ struct b200_routine {
     bool awaited = false;     // some stage on another branch, or the end of the routine, waits for this one
   };
   std::vector<Placed> branches() const;
+  std::vector<void*> launch_args;       // (kept between launches: no allocation on the way)
   std::vector<CUstream> fork_streams;   // of the capture under way
   std::vector<CUevent> fork_events;
   std::set<int> pools_used;   // pools of the bound nodes (what a launch has to wait for, uploads-wise)
