@@ -373,7 +373,8 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (batch > 1 && (m < 16 || n < 8)) return false;
     if (m == 1 && n == 1) return false;
     if (form_b ? ((m <= 16 && !affine_operand) || n < 8 || k < 4) : k < 8) return false;
-    return 2.0 * (double)m * (double)n * (double)k * (double)batch >= 4.0e6;
+    // (a long contraction for a batch of rows is worth it earlier: its rows' softmax can follow in the epilogue)
+    return 2.0 * (double)m * (double)n * (double)k * (double)batch >= (!form_b && m >= 8 && k >= 256 && !affine_operand ? 5.0e5 : 4.0e6);
   };
   if (as_it_lies()) {
     if (!worth(g.m.extent, g.n.extent, g.k.extent, product(gb))) return false;
@@ -846,7 +847,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     bool from_main;     // the main output's tile (already stored by the column loop's store path)
   };
   std::vector<RowNode> rownodes;
-  std::string row_code, row_decls, row_stores, final_sum, final_code;
+  std::string row_code, row_decls, row_stores, row_linear_code, final_sum, final_code;
+  struct RowStore { int tn; std::string name, off; bool linear; };
+  std::vector<RowStore> row_store_list;
+  int bn_of_tile = 0;
   std::set<int> row_written;   // nodes the row followers write
   int row_fused = 0;
   size_t scratch_bytes = 0;
@@ -861,6 +865,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     int bn_t;
     bool pair_t;
     gemm_tile_shape(g, &bn_t, &pair_t);
+    bn_of_tile = bn_t;
     bool can = !pair && !reds && !(form_b && g.accumulate) && n_syms == 1 && N <= 32 && bn_t <= 32 && !pair_t && outs[0].unit_n;
     if (can) {
       int na = -1;
@@ -1110,7 +1115,11 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
         Indices at = canon;
         if (na >= 0) { at[(size_t)na].kind = Index::Fixed; at[(size_t)na].fixed = 0; at[(size_t)na].sym.clear(); }
         const std::string off = em.offset(at, T.dims);
-        if (na >= 0) {
+        OutMap rm;
+        const int tb = prec_bytes(T.prec);
+        if (na >= 0 && N % 8 != 0 && (tb == 2 || tb == 4) && regular(fo.set->tn, canon, &rm) && rm.m_stride == N) {
+          row_store_list.push_back({fo.set->tn, name, off, true});
+        } else if (na >= 0) {
           int64_t stride = 1;
           for (size_t a = (size_t)na + 1; a < T.dims.size(); ++a) stride *= T.dims[a];
           row_stores += "#pragma unroll\n    for (unsigned int b200_c = 0; b200_c < " + std::to_string(N) + "u; ++b200_c) " + T.ident + "[(" + off +
@@ -1150,6 +1159,24 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     }
     if (all) out_maps = maps;
     else for (auto& o : outs) o.tma = -1;
+  }
+
+  // outputs whose rows follow one another in memory and fit one chunk, but are no multiple of 16 bytes
+  std::set<int> linear_rows;
+  for (auto& o : outs)
+    if (o.unit_n && o.tma < 0 && o.m_stride == N && N <= 32 && N % 8 != 0 && !reds && !pair && bn_of_tile >= N && prec_bytes(P.tn(o.tn).prec) <= 4 && prec_bytes(P.tn(o.tn).prec) >= 2)
+      linear_rows.insert(o.tn);
+  for (auto& rs : row_store_list)
+    if (rs.linear) linear_rows.insert(rs.tn);
+  for (auto& rs : row_store_list) {
+    if (rs.linear) {
+      const std::string T = Emitter::ctype(P.tn(rs.tn).prec);
+      row_linear_code += "  {\n    " + T + " b200_v[" + std::to_string(N) + "];\n#pragma unroll\n    for (int b200_c = 0; b200_c < " + std::to_string(N) +
+                         "; ++b200_c) b200_v[b200_c] = " + Emitter::store_wrap(P.tn(rs.tn).prec, rs.name + "[b200_c]") + ";\n    " + T +
+                         "* const b200_p = b200_row_ok ? " + P.tn(rs.tn).ident + " + (" + rs.off + ") : (" + T + "*)0;\n"
+                         "    b200_store_rows<" + std::to_string(N) + ">(b200_stage, (" + T + "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, 0), "
+                         "__popc(__ballot_sync(0xffffffffu, b200_row_ok)), b200_lane, b200_v);\n  }\n";
+    }
   }
 
   std::ostringstream fn;
@@ -1265,6 +1292,17 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   fn << "__device__ __forceinline__ void b200_red_add_v4(unsigned long long addr, uint4 q) {\n"
         "  asm volatile(\"red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\" ::\"l\"(addr), \"f\"(__uint_as_float(q.x)), \"f\"(__uint_as_float(q.y)),\n"
         "               \"f\"(__uint_as_float(q.z)), \"f\"(__uint_as_float(q.w)) : \"memory\");\n}\n";
+  // Rows of N elements that follow one another in memory (the logits of a classifier: 10 or 27 columns): the
+  // warp's 32 rows are one stretch, so they pass through the staging tile as one and leave with whole-warp
+  // accesses -- each lane storing its own row would touch 32 lines per instruction, N times.
+  if (!linear_rows.empty())
+    fn << "template <int N, typename T>\n__device__ __forceinline__ void b200_store_rows(uint4* stage, T* first, unsigned int live, unsigned int lane, const T* v) {\n"
+          "  T* const sm = (T*)stage;\n  __syncwarp();\n#pragma unroll\n  for (int j = 0; j < N; ++j) sm[lane * N + j] = v[j];\n  __syncwarp();\n"
+          "  const unsigned int n = live * N, V = 16u / sizeof(T);\n"
+          "  if (((unsigned long long)first & 15ull) == 0ull) {\n"
+          "    for (unsigned int i = lane; i < n / V; i += 32u) ((uint4*)first)[i] = stage[i];\n"
+          "    for (unsigned int i = n / V * V + lane; i < n; i += 32u) first[i] = sm[i];\n"
+          "  } else {\n    for (unsigned int i = lane; i < n; i += 32u) first[i] = sm[i];\n  }\n  __syncwarp();\n}\n";
   fn << "#define B200_STAGE_KEY(row, G) ((G) >= 8 ? ((row) & 7u) : (((row) / (8u / ((G) >= 8 ? 8u : (G)))) % (G)))\n";
   // developer trace: the first epilogue thread of CTA 0 adds up the clock cycles it spends in
   // each phase of the epilogue (slot = phase that just ended)
@@ -1397,7 +1435,12 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     const int ebytes = prec_bytes(t.prec);
     const bool vec = o.unit_n && (ebytes == 4 || ebytes == 2);
     const std::string T = Emitter::ctype(t.prec);
-    if (o.unit_n) {
+    if (linear_rows.count(o.tn)) {
+      fn << "  {\n    " << T << " b200_v[" << N << "];\n#pragma unroll\n    for (int b200_c = 0; b200_c < " << N << "; ++b200_c) b200_v[b200_c] = "
+         << Emitter::store_wrap(t.prec, o.arr + "[b200_c]") << ";\n    " << T << "* const b200_p = b200_row_ok ? (" << t.ident << " + (" << o.row_off << ")) : (" << T
+         << "*)0;\n    b200_store_rows<" << N << ">(b200_stage, (" << T << "*)__shfl_sync(0xffffffffu, (unsigned long long)b200_p, 0), "
+         << "__popc(__ballot_sync(0xffffffffu, b200_row_ok)), b200_lane, b200_v);\n  }\n";
+    } else if (o.unit_n) {
       fn << "  {\n    " << T << "* b200_p = b200_row_ok ? (" << t.ident << " + (" << o.row_off << ") + b200_n0) : (" << T << "*)0;\n";
       if (vec) {
         const std::string V = ebytes == 4 ? "4" : "8";  // elements per 16 bytes
@@ -1463,6 +1506,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     }
   }
   if (!row_stores.empty()) fn << "  if (b200_row_ok) {\n" << row_stores << "  }\n";
+  fn << row_linear_code;
   fn << final_code;
   fn << "  B200_TRE(15);\n}\n";
 
