@@ -428,7 +428,7 @@ struct Builder {
       else if (ext != extent) return CoopInfo{};
       ci.scopes.push_back({sc->scope_id, op});
     }
-    if (extent < 64) return CoopInfo{};
+    if (extent < 32) return CoopInfo{};
     ci.sym = "*";
     // few outputs and a long reduction: a whole block per output element
     ci.width = (par_total <= 256 && extent >= 4096) ? 1024 : 32;
@@ -1174,12 +1174,15 @@ struct Builder {
     Emitter em(code.prog);
     std::set<int> written;
     std::string text;
+    int64_t most = 1;                 // threads the widest stage could use
+    bool ordered = false;             // some stage depends on another
     std::set<int> fresh_w, fresh_r;   // written / read since the last barrier
     auto barrier_for = [&](const std::set<int>& used, const std::set<int>& writes) {
       bool need = false;
       for (int n : used) need = need || fresh_w.count(n);
       for (int n : writes) need = need || fresh_r.count(n);
       if (need) {
+        ordered = true;
         text += "  __syncthreads();\n";
         fresh_w.clear();
         fresh_r.clear();
@@ -1201,8 +1204,9 @@ struct Builder {
         barrier_for({t.id}, {t.id});
         em.used_nodes.insert(t.id);
         written.insert(t.id);
-        text += "  for (unsigned int b200_z = threadIdx.x; b200_z < " + std::to_string(t.num_elems()) +
-                "u; b200_z += blockDim.x) " + t.ident + "[b200_z] = " + em.storage_zero(t.prec) + ";\n";
+        most = std::max<int64_t>(most, t.num_elems());
+        text += "  for (unsigned int b200_z = B200_FIRST; b200_z < " + std::to_string(t.num_elems()) +
+                "u; b200_z += B200_STEP) " + t.ident + "[b200_z] = " + em.storage_zero(t.prec) + ";\n";
       } else {
         const Piece& pc = pieces[i];
         barrier_for(pc.used, pc.written);
@@ -1234,7 +1238,9 @@ struct Builder {
         int64_t share = 1;   // lanes per sum
         if (pc.sum)
           while (share < 32 && share * 2 * st.total <= 1024 && share * 4 <= ser_total) share *= 2;
+        most = std::max<int64_t>(most, st.total * std::max(1, st.coop));
         if (share > 1) {
+          ordered = true;
           const std::string S = std::to_string(share) + "u";
           text += "  {\n  const unsigned int b200_s = threadIdx.x % " + S + ", b200_gq = threadIdx.x / " + S + ";\n  const bool b200_on = b200_gq < " +
                   std::to_string(st.total) + "u;\n  const unsigned int b200_g = b200_on ? b200_gq : 0u;\n" + pc.decomp + "    " + pc.self_type + " b200_self = " +
@@ -1261,17 +1267,27 @@ struct Builder {
           text += "  {\n";
           if (st.coop) {
             text += "  const unsigned int b200_t = threadIdx.x & 31u;\n";
-            text += "  for (unsigned int b200_g = threadIdx.x >> 5; b200_g < " + std::to_string(st.total) + "u; b200_g += blockDim.x >> 5) {\n";
+            text += "  for (unsigned int b200_g = B200_FIRST >> 5; b200_g < " + std::to_string(st.total) + "u; b200_g += B200_STEP >> 5) {\n";
           } else {
-            text += "  for (unsigned int b200_g = threadIdx.x; b200_g < " + std::to_string(st.total) + "u; b200_g += blockDim.x) {\n";
+            text += "  for (unsigned int b200_g = B200_FIRST; b200_g < " + std::to_string(st.total) + "u; b200_g += B200_STEP) {\n";
           }
           text += pc.decomp + pc.body_text + "  }\n  }\n";
         }
       }
     }
+    // Stages that do not depend on one another (the updates of several parameters, the margins of a padded
+    // image) need no single block: every stage is spread over the whole grid.
+    const bool wide = !ordered && most > 1024;
+    {
+      auto put = [&](const std::string& what, const std::string& by) {
+        for (size_t q = 0; (q = text.find(what, q)) != std::string::npos; q += by.size()) text.replace(q, what.size(), by);
+      };
+      put("B200_FIRST", wide ? "(blockIdx.x * 256u + threadIdx.x)" : "threadIdx.x");
+      put("B200_STEP", wide ? "(gridDim.x * 256u)" : "blockDim.x");
+    }
     // which nodes move into shared memory: the smallest first
     std::vector<int> small;
-    if (!opt.bounds)
+    if (!opt.bounds && !wide)
       for (int n : em.used_nodes) {
         const Tnode& t = code.prog.tn(n);
         if (t.mode != Mode::Virtual && t.prec != Prec::Uint4x32 && t.bytes() <= 12288 && !moving.count(n)) small.push_back(n);
@@ -1319,10 +1335,14 @@ struct Builder {
       }
     }
     moved_to_shared.clear();
-    k_src << "extern \"C\" __global__ void __launch_bounds__(1024) " << f.kernel << "(" << ps << ") {\n" << kGridEntry << decls << statics << load << land
+    if (wide) {
+      f.block = 256;
+      f.grid_override = (int)std::min<int64_t>((most + 255) / 256, 148 * 8);
+    }
+    k_src << "extern \"C\" __global__ void __launch_bounds__(" << f.block << ") " << f.kernel << "(" << ps << ") {\n" << kGridEntry << decls << statics << load << land
           << (load.empty() ? "" : "  __syncthreads();\n") << text << (store.empty() ? "" : "  __syncthreads();\n") << store << "}\n\n";
     src << k_src.str();
-    f.note = "fused " + std::to_string(idx.size()) + " small stages in one block";
+    f.note = "fused " + std::to_string(idx.size()) + (wide ? " small stages over one grid" : " small stages in one block");
     return f;
   }
   std::set<int> moved_to_shared;
@@ -1545,9 +1565,11 @@ struct Builder {
       }
       stages.push_back(st);
     }
-    if (R < 64 || R % 32 != 0) return false;
-    const int EPL = (int)(R / 32);
-    if (EPL != 2 && EPL != 4 && EPL != 8 && EPL != 16) return false;
+    if (R < 32 || R > 1024) return false;
+    const int EPL = (int)((R + 31) / 32);
+    const bool dealt = R % 128 == 0 && EPL <= 16, pairwise = R == 64;
+    const bool strided = !dealt && !pairwise;   // one element per lane and step, the last step perhaps partly filled
+    const bool tail = strided && R % 32 != 0;
 
     // ---- classify every access
     struct RowNode { Indices idcs; Prec prec; bool loaded = false, produced = false; int writer = -1; };
@@ -1636,6 +1658,7 @@ struct Builder {
       written_nodes.insert(set.tn);
       if (!ok) return false;
     }
+    if ((int64_t)rownodes.size() * EPL > 160) return false;   // the rows have to fit the registers
     // a node read at other positions by a LATER plain load after being written here was refused above;
     // a row node that is both loaded and produced was refused as well
 
@@ -1662,18 +1685,22 @@ struct Builder {
     // Which elements of a row a lane owns.  Four at a time, dealt round the warp (element
     // (k * 32 + lane) * 4 + j in register 4 k + j) when the lane's share is a multiple of four: every
     // access of the warp then covers one contiguous stretch of the row.  A share of two elements stays
-    // consecutive (lane * 2 + e).
-    const bool dealt = EPL % 4 == 0;
-    const std::string own = dealt ? "(((b200_e >> 2) * 32u + b200_t) * 4u + (b200_e & 3u))" : "(b200_t0 + b200_e)";
+    // consecutive (lane * 2 + e).  Rows of any other length go one element per lane and step (element e * 32 +
+    // lane in register e), the lanes beyond the row's end idle in the last step.
+    const std::string own = dealt ? "(((b200_e >> 2) * 32u + b200_t) * 4u + (b200_e & 3u))" : strided ? "(b200_e * 32u + b200_t)" : "(b200_t0 + b200_e)";
+    const std::string Rs = std::to_string(R);
     auto row_ptr = [&](int tn, const RowNode& rn) {
       const Tnode& t = code.prog.tn(tn);
       Indices at = rn.idcs;
       Index zero;
       at.push_back(zero);
-      return t.ident + " + (" + em.offset(at, t.dims) + ")" + (dealt ? "" : " + b200_t0");
+      return t.ident + " + (" + em.offset(at, t.dims) + ")" + (pairwise ? " + b200_t0" : "");
     };
     auto ld = [&](int tn, const RowNode& rn) {
       const std::string n = std::to_string(EPL);
+      if (strided)
+        return "#pragma unroll\n    for (unsigned int b200_e = 0; b200_e < " + n + "u; ++b200_e) " + reg(tn) + "[b200_e] = " + (tail ? own + " < " + Rs + "u ? " : std::string()) +
+               Emitter::load_wrap(rn.prec, "(" + row_ptr(tn, rn) + ")[" + own + "]") + (tail ? " : 0.0f" : "") + ";\n";
       max_bytes = std::max(max_bytes, dealt ? 4 * prec_bytes(rn.prec) : std::min(16, EPL * prec_bytes(rn.prec)));
       const std::string lane = dealt ? "b200_t, " : "";
       if (rn.prec == Prec::Single) return std::string("    b200_ld_row") + (dealt ? "v<" : "<") + n + ">(" + row_ptr(tn, rn) + ", " + lane + reg(tn) + ");\n";
@@ -1681,6 +1708,9 @@ struct Builder {
     };
     auto stv = [&](int tn, const RowNode& rn) {
       const std::string n = std::to_string(EPL);
+      if (strided)
+        return "#pragma unroll\n    for (unsigned int b200_e = 0; b200_e < " + n + "u; ++b200_e)" + (tail ? " if (" + own + " < " + Rs + "u)" : std::string()) + " (" + row_ptr(tn, rn) + ")[" + own +
+               "] = " + Emitter::store_wrap(rn.prec, reg(tn) + "[b200_e]") + ";\n";
       max_bytes = std::max(max_bytes, dealt ? 4 * prec_bytes(rn.prec) : std::min(16, EPL * prec_bytes(rn.prec)));
       const std::string lane = dealt ? "b200_t, " : "";
       if (rn.prec == Prec::Single) return std::string("    b200_st_row") + (dealt ? "v<" : "<") + n + ">(" + row_ptr(tn, rn) + ", " + lane + reg(tn) + ");\n";
@@ -1743,7 +1773,8 @@ struct Builder {
             const double neutral = op == "add" ? 0.0 : (op == "max" ? -INFINITY : INFINITY);
             text += "      " + std::string(Emitter::ctype(p)) + " " + name + " = " + em.constant(neutral, p) + ";\n";
             text += "#pragma unroll\n      for (unsigned int b200_e = 0; b200_e < " + std::to_string(EPL) + "u; ++b200_e) {\n"
-                    "        const unsigned int " + b->index + " = " + own + ";\n" + em.stmt(*b->body, 8) + "      }\n";
+                    "        const unsigned int " + b->index + " = " + own + ";\n" + (tail ? "        if (" + b->index + " < " + Rs + "u) {\n" : std::string()) +
+                    em.stmt(*b->body, 8) + (tail ? "        }\n" : "") + "      }\n";
             text += "      " + name + " = b200_warp_" + (op == "add" ? std::string("sum") : op) + "(" + name + ");\n";
             em.scope_subst[e.scope_id] = name;
             ++si;
@@ -1795,7 +1826,7 @@ struct Builder {
         have.insert(set.tn);
       }
     }
-    f.min_align = max_bytes;
+    f.min_align = strided ? 0 : max_bytes;
     std::string statics = static_prologue(text, em, 2);
     std::ostringstream k_src;
     k_src << "extern \"C\" __global__ void __launch_bounds__(" << f.block << ") " << f.kernel << "(";
@@ -1823,7 +1854,7 @@ struct Builder {
     // SMs (three of 256 threads at this kernel's register use), each warp striding over the rows
     if (any_invariant && rows >= 2 * 148 * 3 * 8) f.grid_override = 148 * 3;
     f.note = "row-fused " + std::to_string(run.size()) + " stages, one warp per row, rows in registers (" + std::to_string(EPL) +
-             " elements per lane" + (dealt ? ", dealt four at a time" : "") + ")";
+             " elements per lane" + (dealt ? ", dealt four at a time" : strided ? ", one per step" : "") + ")";
     *out = f;
     return true;
   }

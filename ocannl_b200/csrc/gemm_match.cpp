@@ -995,7 +995,8 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
         final_sum = code;
         row_decls += "  float b200_part = 0.0f;\n";
         // per-warp partial, ticket, ordered combine by the last warp
-        code = "  {\n    b200_part = b200_warp_sum(b200_part);\n"
+        // (a warp adds up all of its tiles first: one slot per warp of the grid, not per tile)
+        code = "  b200_es.part += b200_part;\n  if (!b200_nx_ok) {\n    b200_part = b200_warp_sum(b200_es.part);\n"
                 "    float* b200_slots = (float*)b200_partials;\n"
                 "    unsigned int* b200_ticket = (unsigned int*)(b200_partials + 4ull * b200_nslots);\n"
                 "    unsigned int b200_last = 0u;\n"
@@ -1003,7 +1004,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
                 "      b200_last = atomicAdd(b200_ticket, 1u) == b200_nslots - 1u ? 1u : 0u;\n    }\n"
                 "    b200_last = __shfl_sync(0xffffffffu, b200_last, 0);\n"
                 "    if (b200_last) {\n      __threadfence();\n      float b200_total = 0.0f;\n"
-                "      for (unsigned int b200_i = b200_lane; b200_i < b200_nslots; b200_i += 32u) b200_total += ((volatile float*)b200_slots)[b200_i];\n"
+                "#pragma unroll 8\n      for (unsigned int b200_i = b200_lane; b200_i < b200_nslots; b200_i += 32u) b200_total += __ldcg(b200_slots + b200_i);\n"
                 "      b200_total = b200_warp_sum(b200_total);\n      if (b200_lane == 0u) {\n";
         em.scope_subst[gscope->scope_id] = "b200_total";
         Emitter::Res v = em.scalar(T.prec, *fo.set->value);

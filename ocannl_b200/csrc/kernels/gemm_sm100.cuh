@@ -313,6 +313,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     b200_es.lph = 0u;
     b200_es.abort_flag = abort_flag;
     b200_es.status = status;
+    b200_es.part = 0.0f;
     B200_EPI_PROLOGUE
     unsigned int acc = 0, acc_phase = 0;
     // (batch, row, first column) of the part of a unit's tile that this thread works on
@@ -337,9 +338,8 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       unsigned int tile, b200_b0, b200_b1, mt, nt;
       b200_coords(unit, tile, b200_b0, b200_b1, mt, nt);
       const unsigned int b200_m = mt * B200_BM + cta_rank * B200_CTA_M + quarter * 32u + lane;
-      // one scratch slot per (tile, CTA, epilogue warp) for epilogues that end in a grid-wide sum
-      const unsigned int b200_slot = (tile * (1u + B200_CTA_PAIR) + cta_rank) * B200_EPI_WARPS + ew;
-      const unsigned int b200_nslots = total_tiles * (1u + B200_CTA_PAIR) * B200_EPI_WARPS;
+      // one scratch slot per epilogue warp of the grid for epilogues that end in a grid-wide sum
+      const unsigned int b200_slot = blockIdx.x * B200_EPI_WARPS + ew, b200_nslots = gridDim.x * B200_EPI_WARPS;
       // this warp's share of the next tile, for the prefetch at the end of this one
       bool b200_nx_ok = false;
       unsigned int b200_nx_b0 = 0, b200_nx_b1 = 0, b200_nx_m = 0, b200_nx_n0 = 0;

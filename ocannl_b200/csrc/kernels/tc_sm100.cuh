@@ -257,6 +257,7 @@ struct b200_epi_state {
   unsigned int lph;                    // parity of the next completion to wait for
   volatile unsigned int* abort_flag;   // the CTA's abort flag and the device status word, for the bounded wait
   unsigned int* status;
+  float part;                          // this warp's share of a grid-wide sum over the tiles it has worked on
 };
 
 #endif  // B200_TC_SM100_CUH
