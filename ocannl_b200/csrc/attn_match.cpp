@@ -280,8 +280,8 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   };
   const int64_t S = extent_of(n[0], s_sym), T = extent_of(n[0], t_sym), E = r1.loop.extent();
   // Tiles of 128 queries on the tensor cores for whole tiles of keys; every other number of keys up to 256
-  // (and every head dimension that is a multiple of 16, and short sequences) goes to the kernel that keeps
-  // score rows in registers.
+  // (and every head dimension that is a multiple of 16, and short sequences) goes to the kernel that gives
+  // 16 queries to a warp.
   const bool rows_kernel = !(E == 64 && (T == 64 || T == 128 || T == 256) && S >= 64);
   if (rows_kernel && (T > 256 || E % 16 != 0 || E > 128)) return false;
   if (SC.dims.back() != T) return false;
@@ -811,8 +811,16 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   a.rows_kernel = rows_kernel;
   a.masked = masked;
   a.out_type = Emitter::ctype(O.prec);
-  // (sequences of a few positions: no idle warps)
-  a.warps = (int)std::min<int64_t>(8, (S + 15) / 16);
+  // (sequences of a few positions: no idle warps; long rows of wide heads: as many score rows as fit beside the keys
+  // and values in 227 KB)
+  const int64_t key_rows = (T + 15) / 16 * 16, kv_bytes = 2 * key_rows * (E + 8) * 2;
+  if (rows_kernel) {
+    a.warps = (int)std::min<int64_t>({8, (S + 15) / 16, (227 * 1024 - kv_bytes) / (64 * key_rows)});
+    // few heads: the queries of one over several blocks, while two blocks in the place of one still find an SM each
+    // (5 x 4 heads of 100 queries: 14.6 us as 20 blocks, 12.7 as 80; 20 heads of 149: 24.9 and 17.5)
+    while (a.warps > 2 && 2 * B0 * B1 * ((S + 16 * a.warps - 1) / (16 * a.warps)) <= 148) a.warps = (a.warps + 1) / 2;
+    st.smem_bytes = (int)(kv_bytes + a.warps * 64 * key_rows);
+  }
   st.block = rows_kernel ? 32 * a.warps : 256;
   st.min_align = rows_kernel ? 0 : 16;
   a.q_tn = oq.tn; a.k_tn = ok_.tn; a.v_tn = ov.tn;
@@ -851,7 +859,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   st.note = "fused attention: scores, softmax and weights . values in one tcgen05 kernel (" + std::to_string(T) + " keys, " +
             std::to_string(kept_rows) + " of the 3 row nodes written)";
   if (rows_kernel)
-    st.note = "fused attention, rows in registers: " + std::to_string(T) + " keys, head dimension " + std::to_string(E) + ", " + std::to_string(kept_rows) +
+    st.note = "fused attention, a warp per 16 rows: " + std::to_string(T) + " keys, head dimension " + std::to_string(E) + ", " + std::to_string(kept_rows) +
               " of the 3 row nodes written";
   *out = st;
   *n_absorbed = 6;
@@ -867,7 +875,6 @@ std::string attn_translation_unit(const Program&, Stage& st, const std::string& 
       << "\n#define B200_MASKED " << (a.masked ? 1 : 0) << "\n#define B200_KEEP_SCORES " << (a.scores.keep ? 1 : 0) << "\n#define B200_KEEP_EXP "
       << (a.exps.keep ? 1 : 0) << "\n#define B200_KEEP_W " << (a.weights.keep ? 1 : 0) << "\n#define B200_ATTN_PARAMS " << st.epi_params
       << "\n#define B200_ATTN_ARGS " << st.epi_args << "\n" << kAttnRowsSource << "\n" << a.code << "\n";
-    st.smem_bytes = (int)(2 * ((a.T + 15) / 16 * 16) * (a.E + 8) * 2);
     return o.str();
   }
   const unsigned int fmt = a.in_prec == Prec::Bfloat16 ? 1u : 0u;

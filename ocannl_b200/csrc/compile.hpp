@@ -91,7 +91,7 @@ struct AttnPlan {
     int64_t off = 0, row = 0, b0 = 0, b1 = 0;   // element offset and strides of (query position, outer batch, inner batch)
   };
   RowNode scores, exps, weights;
-  // short rows: whole score rows in registers, one warp per 16 queries (kernels/attn_rows.cuh)
+  // short rows: one warp per 16 queries (kernels/attn_rows.cuh)
   bool rows_kernel = false;
   bool masked = false;         // the score is a constant wherever the first condition is zero
   std::string out_type;        // storage type of the output

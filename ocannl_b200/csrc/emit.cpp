@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstdio>
 #include <cstring>
 
@@ -338,6 +339,15 @@ std::string Emitter::binop(Prec prec, const std::string& op, const std::string& 
         char r[32];
         snprintf(r, sizeof r, "0x1p%+df", -e2);
         const std::string q = "(" + a + " * " + r + ")";
+        return lowp(prec) ? std::string(round_fn(prec)) + q + ")" : q;
+      }
+    }
+    {
+      // any other literal of ordinary size: multiplied by its reciprocal and corrected once
+      char* end = nullptr;
+      const double v = std::fabs(strtod(b.c_str(), &end));
+      if (end && end != b.c_str() && end[0] == 'f' && !end[1] && v >= 0x1p-60 && v <= 0x1p+60) {
+        const std::string q = "b200_div_literal(" + a + ", " + b + ")";
         return lowp(prec) ? std::string(round_fn(prec)) + q + ")" : q;
       }
     }

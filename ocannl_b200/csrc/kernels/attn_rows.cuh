@@ -1,21 +1,24 @@
 // Fused attention stage for short rows: the chain of attn_sm100.cuh (scores, softmax, weights . values) for
 // any number of keys up to 256 and any head dimension that is a multiple of 16.
 //
-// A warp takes 16 queries of one (batch, head) and keeps their whole score rows in registers, in the
-// accumulator layout of mma.m16n8k16: thread (g, c) = (lane / 4, lane % 4) holds columns 8 n + 2 c and + 1 of
-// rows g and g + 8 for every key tile n.  Row maximum and sum are two shuffles within four lanes; the
-// weights, rounded to the node's 16-bit format, are at once the A fragments of the second product, whose B
-// fragments come transposed out of shared memory (ldmatrix.trans).  Keys and values of the (batch, head) lie
-// in shared memory, rows padded by 16 bytes so that the eight rows of an ldmatrix fall into different banks.
-// What bounds it: the softmax arithmetic, about 25 instructions per score; with 16 rows per warp there is
-// neither a tensor-memory round trip nor a block-wide barrier between its passes, and a sequence of 100
-// positions is 7 warps' work where the tile kernels pad it to 128 x 128.  (Before, such rows took four
-// launches: scores, softmax, a gathered copy of the weights, weights . values.)
+// A warp takes 16 queries of one (batch, head), in the accumulator layout of mma.m16n8k16: thread (g, c) =
+// (lane / 4, lane % 4) holds columns 8 n + 2 c and + 1 of rows g and g + 8 for every key tile n.  Scores, then
+// exponentials, lie in shared memory, four per thread and tile, each read back by the thread that wrote it (no
+// barrier); row maximum and sum are two shuffles within four lanes; the weights, rounded to the node's 16-bit
+// format, are at once the A fragments of the second product, whose B fragments come transposed out of shared
+// memory (ldmatrix.trans).  Keys and values of the (batch, head) lie in shared memory too, rows padded by 16
+// bytes so that the eight rows of an ldmatrix fall into different banks.
+// What bounds it: latency, of the loads and of three short loops per warp (scores; exponentials; weights and
+// their product); neither a tensor-memory round trip nor a block-wide barrier stands between them, and a
+// sequence of 100 positions is 7 warps' work where the tile kernels pad it to 128 x 128.  The loops run over 16
+// keys at a time and are not unrolled further than twice: score rows held in registers instead meant straight
+// code of up to 150 KB, which was fetched from memory more slowly than it ran (66 heads of 192 queries and keys: 23 us,
+// now 17 us, 6 of it the launch).
 //
-// Key tiles in which no query of the warp has a mask bit set are not multiplied, and their scores are one
+// 16 keys for which no query of the warp has a mask bit set are not multiplied, and their scores are one
 // constant per row: exponential and weight are evaluated once for all of them, and when that weight is zero
-// (it is, unless a row is masked throughout) the tile adds nothing to the output either.  A causal mask
-// halves the work this way.
+// (it is, unless a row is masked throughout) they add nothing to the output either.  A causal mask halves the
+// work this way.
 //
 // The translation unit defines B200_AR_NAME, B200_T, B200_E, B200_HALF (1: half, 0: bfloat16), B200_WARPS,
 // B200_OUT_T (storage type of the output), B200_NCOND, B200_MASKED (1: the score is a constant where mask 0 is
@@ -38,7 +41,7 @@ struct b200_ar_ptrs {   // addresses of this row in the nodes the routine keeps 
 #define B200_NT ((B200_T + 15) / 16 * 2)          // key tiles of 8, an even number
 #define B200_TP (B200_NT * 8)
 #define B200_LD (B200_E + 8)                      // elements per padded row in shared memory
-#define B200_CW ((B200_T + 31) / 32)              // mask words per row
+#define B200_NP (B200_NT / 2)                     // the loops' steps, 16 keys each
 
 __device__ __forceinline__ float b200_ar_score(const b200_attn_row& row, unsigned int b200_t, float b200_acc, unsigned int cb0, unsigned int cb1 B200_ATTN_PARAMS);
 __device__ __forceinline__ float b200_ar_masked_score();
@@ -98,28 +101,31 @@ __device__ __forceinline__ void b200_ar_put16(unsigned long long p, unsigned int
 }
 
 // softmax passes behind the row maximum, on the score fragments `x`; `skip`: bit n set when tile n is masked throughout
+// the rows of one (batch, head) on their way into shared memory, one group of copies
+__device__ __forceinline__ void b200_ar_fetch(unsigned short* to, const unsigned short* from, long long row) {
+  constexpr unsigned int P = B200_E / 8;   // 16-byte pieces per row
+  const unsigned int at = (unsigned int)__cvta_generic_to_shared(to);
+  for (unsigned int i = threadIdx.x; i < B200_TP * P; i += 32u * B200_WARPS) {
+    const unsigned int t = i / P, piece = i % P;
+    const bool in = t < B200_T;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"(at + 2u * (t * B200_LD + 8u * piece)), "l"(__cvta_generic_to_global(from + (in ? (long long)t * row + 8u * piece : 0ll))), "r"(in ? 16u : 0u) : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// all of the block's warps, wherever they are in the kernel
+__device__ __forceinline__ void b200_ar_barrier() { asm volatile("bar.sync 0;" ::: "memory"); }
+
+// the weights of one key tile of the thread's two rows, as rounded pairs
 template <bool FAST>
-__device__ __forceinline__ void b200_ar_weights(const b200_attn_row* row, const b200_ar_ptrs* p, unsigned int c, float (*x)[4], unsigned int skip,
-                                                const float* sum, const b200_divisor* dv, const unsigned int* wm, unsigned int (*w)[2] B200_ATTN_PARAMS) {
+__device__ __forceinline__ void b200_ar_weight4(const b200_attn_row* row, unsigned int t, const float4& x, const float* sum, const b200_divisor* dv,
+                                                unsigned int* w B200_ATTN_PARAMS) {
+  const float v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-  for (unsigned int n = 0; n < B200_NT; ++n) {
-    const unsigned int t = 8u * n + 2u * c;
-    if (B200_MASKED && ((skip >> n) & 1u)) {
-      w[n][0] = wm[0];
-      w[n][1] = wm[1];
-    } else {
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float a = t < B200_T ? b200_ar_weight<FAST>(row[r], t, x[n][2 * r], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
-        const float b = t + 1u < B200_T ? b200_ar_weight<FAST>(row[r], t + 1u, x[n][2 * r + 1], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
-        w[n][r] = b200_ar_pack(a, b);
-      }
-    }
-    // (a masked tile that ends beyond the row keeps zeros there: the values beyond T are zero rows, so its weights do not matter)
-#if B200_KEEP_W
-    b200_ar_put16(p[0].w, t, w[n][0]);
-    b200_ar_put16(p[1].w, t, w[n][1]);
-#endif
+  for (int r = 0; r < 2; ++r) {
+    const float a = t < B200_T ? b200_ar_weight<FAST>(row[r], t, v[2 * r], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
+    const float b = t + 1u < B200_T ? b200_ar_weight<FAST>(row[r], t + 1u, v[2 * r + 1], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
+    w[r] = b200_ar_pack(a, b);
   }
 }
 
@@ -135,23 +141,10 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
   const unsigned int tile = blockIdx.x % shape.tiles, bh = blockIdx.x / shape.tiles;
   const unsigned int b0 = bh / shape.B1, b1 = bh - b0 * shape.B1;
 
-  // keys and values into shared memory, 16 bytes at a time; rows beyond T are zero
-  {
-    const unsigned short* const kb = b200_kp + (long long)b0 * shape.k_b0 + (long long)b1 * shape.k_b1;
-    const unsigned short* const vb = b200_vp + (long long)b0 * shape.v_b0 + (long long)b1 * shape.v_b1;
-    constexpr unsigned int P = B200_E / 8;   // 16-byte pieces per row
-#pragma unroll 4
-    for (unsigned int i = threadIdx.x; i < B200_TP * P; i += 32u * B200_WARPS) {
-      const unsigned int t = i / P, piece = i % P;
-      uint4 kq = make_uint4(0u, 0u, 0u, 0u), vq = kq;
-      if (t < B200_T) {
-        kq = *(const uint4*)(kb + (long long)t * shape.k_row + 8u * piece);
-        vq = *(const uint4*)(vb + (long long)t * shape.v_row + 8u * piece);
-      }
-      *(uint4*)(ks + t * B200_LD + 8u * piece) = kq;
-      *(uint4*)(vs + t * B200_LD + 8u * piece) = vq;
-    }
-  }
+  // keys and values into shared memory, 16 bytes at a time, all of them under way at once (through registers
+  // they came in several round trips to memory, a third of the kernel's time with few warps); rows beyond T zero
+  b200_ar_fetch(ks, b200_kp + (long long)b0 * shape.k_b0 + (long long)b1 * shape.k_b1, shape.k_row);
+  b200_ar_fetch(vs, b200_vp + (long long)b0 * shape.v_b0 + (long long)b1 * shape.v_b1, shape.v_row);
   const unsigned int s0 = (tile * B200_WARPS + warp) * 16u;
   b200_attn_row row[2];
 #pragma unroll
@@ -175,85 +168,92 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
       }
   }
   // mask bits: word k of a row covers keys 32 k .. 32 k + 31
-  unsigned int cw[2][B200_NCOND > 0 ? B200_NCOND : 1][B200_CW];
+  const unsigned int* cp[2][B200_NCOND > 0 ? B200_NCOND : 1];
 #if B200_NCOND > 0
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const unsigned int* cp[B200_NCOND];
-    b200_ar_cond_rows(row[r], cp B200_ATTN_ARGS);
-#pragma unroll
-    for (int i = 0; i < B200_NCOND; ++i)
-#pragma unroll
-      for (int k = 0; k < B200_CW; ++k) cw[r][i][k] = cp[i] ? cp[i][k] : 0u;
-  }
+  b200_ar_cond_rows(row[0], cp[0] B200_ATTN_ARGS);
+  b200_ar_cond_rows(row[1], cp[1] B200_ATTN_ARGS);
 #endif
-  __syncthreads();
-  if (s0 >= shape.S) return;   // (no barrier follows)
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  b200_ar_barrier();
+  if (s0 >= shape.S) {   // no queries for this warp: it only brought its part of the keys and values
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    b200_ar_barrier();
+    return;
+  }
   b200_ar_ptrs p[2];
   b200_ar_rows(row[0], p[0] B200_ATTN_ARGS);
   b200_ar_rows(row[1], p[1] B200_ATTN_ARGS);
 
-  // tiles without a mask bit in any of the warp's rows
+  // bit j: no row of the warp has a mask bit among keys 16 j .. 16 j + 15
   unsigned int skip = 0u;
 #if B200_MASKED
   {
-    unsigned int any = 0u;   // bit n: some row of this thread has a bit in tile n
+    unsigned int any = 0u;
 #pragma unroll
-    for (int k = 0; k < B200_CW; ++k) {
-      const unsigned int m = cw[0][0][k] | cw[1][0][k];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (4 * k + q < B200_NT && ((m >> (8 * q)) & 0xFFu)) any |= 1u << (4 * k + q);
+    for (unsigned int k = 0; k < (B200_NP + 1) / 2; ++k) {
+      const unsigned int m = (cp[0][0] ? cp[0][0][k] : 0u) | (cp[1][0] ? cp[1][0][k] : 0u);
+      any |= (m & 0xFFFFu ? 1u << (2u * k) : 0u) | (m >> 16 ? 2u << (2u * k) : 0u);
     }
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) any |= __shfl_xor_sync(0xffffffffu, any, o);
-    skip = ~any;
+    skip = ~any & ((1u << B200_NP) - 1u);
   }
 #endif
+  // this thread's scores: float4 n * 32 holds key tile n of rows g (x, y) and g + 8 (z, w)
+  float4* const xs = (float4*)(vs + B200_TP * B200_LD) + warp * (B200_NT * 32u) + lane;
 
   // ---- scores and row maximum
-  float x[B200_NT][4];
   float mx[2] = {b200_ar_max_init(), b200_ar_max_init()};
   const unsigned int k_at = (unsigned int)__cvta_generic_to_shared(ks), v_at = (unsigned int)__cvta_generic_to_shared(vs);
+#pragma unroll 2
+  for (unsigned int j = 0; j < B200_NP; ++j) {
+    if (B200_MASKED && ((skip >> j) & 1u)) {
+#if B200_KEEP_SCORES
 #pragma unroll
-  for (unsigned int n = 0; n < B200_NT; ++n) {
-    const bool off = B200_MASKED && ((skip >> n) & 1u);
-    if (!off) {
-      float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      // an x4 load: keys 8 n .. 8 n + 7, head dimensions 32 k2 .. 32 k2 + 31 (two k steps); an odd last step loads 16 twice
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (unsigned int k2 = 0; k2 < (B200_E + 31) / 32; ++k2) {
+        for (int r = 0; r < 2; ++r) b200_ar_put(p[r].scores, 16u * j + 8u * h + 2u * c, b200_ar_masked_score(), b200_ar_masked_score());
+#endif
+      continue;
+    }
+    unsigned int cw[2][2] = {{0u, 0u}, {0u, 0u}};
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < B200_NCOND; ++i) cw[r][i] = cp[r][i] ? cp[r][i][j >> 1] >> (16u * (j & 1u)) : 0u;
+    float d[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+    // an x4 load: eight keys, head dimensions 32 k2 .. 32 k2 + 31 (two k steps); an odd last step loads 16 twice
+#pragma unroll
+    for (unsigned int k2 = 0; k2 < (B200_E + 31) / 32; ++k2)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
         unsigned int b[4];
         const unsigned int col = 32u * k2 + 8u * (lane >> 3);
-        b200_ldsm4(b, k_at + 2u * ((8u * n + (lane & 7u)) * B200_LD + (col < B200_E ? col : col - 16u)));
-        b200_ar_mma(d, qa[2 * k2], b[0], b[1]);
-        if (2 * k2 + 1 < B200_E / 16) b200_ar_mma(d, qa[2 * k2 + 1 < B200_E / 16 ? 2 * k2 + 1 : 0], b[2], b[3]);
+        b200_ldsm4(b, k_at + 2u * ((16u * j + 8u * h + (lane & 7u)) * B200_LD + (col < B200_E ? col : col - 16u)));
+        b200_ar_mma(d[h], qa[2 * k2], b[0], b[1]);
+        if (2 * k2 + 1 < B200_E / 16) b200_ar_mma(d[h], qa[2 * k2 + 1 < B200_E / 16 ? 2 * k2 + 1 : 0], b[2], b[3]);
       }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float x[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = i >> 1;
-        const unsigned int t = 8u * n + 2u * c + (i & 1);
-        const unsigned int cb0 = B200_NCOND > 0 ? (cw[r][0][n / 4] >> (t & 31u)) & 1u : 0u;
-        const unsigned int cb1 = B200_NCOND > 1 ? (cw[r][B200_NCOND > 1 ? 1 : 0][n / 4] >> (t & 31u)) & 1u : 0u;
-        x[n][i] = t < B200_T ? b200_ar_score(row[r], t, d[i], cb0, cb1 B200_ATTN_ARGS) : b200_ar_max_init();
-        mx[r] = fmaxf(mx[r], x[n][i]);
+        const unsigned int in = 8u * h + 2u * c + (i & 1), t = 16u * j + in;
+        x[i] = t < B200_T ? b200_ar_score(row[r], t, d[h][i], (cw[r][0] >> in) & 1u, (cw[r][1] >> in) & 1u B200_ATTN_ARGS) : b200_ar_max_init();
+        mx[r] = fmaxf(mx[r], x[i]);
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[n][i] = b200_ar_masked_score();
-      if (8u * n < B200_T) {
-        mx[0] = fmaxf(mx[0], b200_ar_masked_score());
-        mx[1] = fmaxf(mx[1], b200_ar_masked_score());
-      }
-    }
+      xs[32u * (2u * j + h)] = make_float4(x[0], x[1], x[2], x[3]);
 #if B200_KEEP_SCORES
-    b200_ar_put(p[0].scores, 8u * n + 2u * c, x[n][0], x[n][1]);
-    b200_ar_put(p[1].scores, 8u * n + 2u * c, x[n][2], x[n][3]);
+      b200_ar_put(p[0].scores, 16u * j + 8u * h + 2u * c, x[0], x[1]);
+      b200_ar_put(p[1].scores, 16u * j + 8u * h + 2u * c, x[2], x[3]);
 #endif
+    }
   }
   float sum[2] = {0.0f, 0.0f}, em[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
+    if (B200_MASKED && skip) mx[r] = fmaxf(mx[r], b200_ar_masked_score());
     mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
     mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
     mx[r] = b200_ar_row_max(row[r], mx[r] B200_ATTN_ARGS);
@@ -261,24 +261,34 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
     em[r] = B200_MASKED ? b200_ar_exp(row[r], 0u, b200_ar_masked_score(), mx[r] B200_ATTN_ARGS) : 0.0f;
   }
   // ---- exponentials and row sum
-#pragma unroll
-  for (unsigned int n = 0; n < B200_NT; ++n) {
-    if (B200_MASKED && ((skip >> n) & 1u)) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[n][i] = em[i >> 1];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[n][i] = b200_ar_exp(row[i >> 1], 8u * n + 2u * c + (i & 1), x[n][i], mx[i >> 1] B200_ATTN_ARGS);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (8u * n + 7u >= B200_T && 8u * n + 2u * c + (i & 1) >= B200_T) x[n][i] = 0.0f;
-      sum[i >> 1] += x[n][i];
-    }
-#if B200_KEEP_EXP
-    b200_ar_put(p[0].exps, 8u * n + 2u * c, x[n][0], x[n][1]);
-    b200_ar_put(p[1].exps, 8u * n + 2u * c, x[n][2], x[n][3]);
+#pragma unroll 2
+  for (unsigned int j = 0; j < B200_NP; ++j) {
+    const bool off = B200_MASKED && ((skip >> j) & 1u);
+#if !B200_KEEP_EXP
+    if (off && em[0] == 0.0f && em[1] == 0.0f) continue;
 #endif
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned int t = 16u * j + 8u * h + 2u * c;
+      float x[4] = {em[0], em[0], em[1], em[1]};
+      if (!off) {
+        const float4 v = xs[32u * (2u * j + h)];
+        x[0] = b200_ar_exp(row[0], t, v.x, mx[0] B200_ATTN_ARGS);
+        x[1] = b200_ar_exp(row[0], t + 1u, v.y, mx[0] B200_ATTN_ARGS);
+        x[2] = b200_ar_exp(row[1], t, v.z, mx[1] B200_ATTN_ARGS);
+        x[3] = b200_ar_exp(row[1], t + 1u, v.w, mx[1] B200_ATTN_ARGS);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (t + (i & 1) >= B200_T) x[i] = 0.0f;
+        sum[i >> 1] += x[i];
+      }
+      if (!off) xs[32u * (2u * j + h)] = make_float4(x[0], x[1], x[2], x[3]);
+#if B200_KEEP_EXP
+      b200_ar_put(p[0].exps, t, x[0], x[1]);
+      b200_ar_put(p[1].exps, t, x[2], x[3]);
+#endif
+    }
   }
   b200_divisor dv[2];
   unsigned int wm[2];
@@ -293,26 +303,46 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
     wz[r] = B200_MASKED ? b200_ar_weight<false>(row[r], 0u, em[r], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
     wm[r] = b200_ar_pack(wz[r], wz[r]);
   }
-  // ---- weights: the A fragments of the second product
-  unsigned int w[B200_NT][2];
-  if (__all_sync(0xffffffffu, dv[0].fast && dv[1].fast)) b200_ar_weights<true>(row, p, c, x, skip, sum, dv, wm, w B200_ATTN_ARGS);
-  else b200_ar_weights<false>(row, p, c, x, skip, sum, dv, wm, w B200_ATTN_ARGS);
-  // masked tiles that weigh nothing in any row of the warp are left out of the product
-  const unsigned int leave = __any_sync(0xffffffffu, wz[0] != 0.0f || wz[1] != 0.0f) ? 0u : skip;
+  // ---- weights, the A fragments of the second product, and the product; masked keys that weigh nothing in any
+  // row of the warp are left out of it
+  const bool fast = __all_sync(0xffffffffu, dv[0].fast && dv[1].fast);
+  const bool leave = !__any_sync(0xffffffffu, wz[0] != 0.0f || wz[1] != 0.0f);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  b200_ar_barrier();
   float o[B200_E / 8][4];
 #pragma unroll
   for (unsigned int e = 0; e < B200_E / 8; ++e)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[e][i] = 0.0f;
+#pragma unroll 2
+  for (unsigned int j = 0; j < B200_NP; ++j) {
+    const bool off = B200_MASKED && ((skip >> j) & 1u);
+#if !B200_KEEP_W
+    if (off && leave) continue;
+#endif
+    // (masked keys that end beyond the row: the values beyond T are zero rows, so the weights there do not matter)
+    unsigned int a[4] = {wm[0], wm[1], wm[0], wm[1]};
+    if (!off) {
 #pragma unroll
-  for (unsigned int k = 0; k < B200_NT / 2; ++k) {
-    if (((leave >> (2u * k)) & 3u) == 3u) continue;
-    const unsigned int a[4] = {w[2 * k][0], w[2 * k][1], w[2 * k + 1][0], w[2 * k + 1][1]};
+      for (int h = 0; h < 2; ++h) {
+        const unsigned int t = 16u * j + 8u * h + 2u * c;
+        const float4 x = xs[32u * (2u * j + h)];
+        if (fast) b200_ar_weight4<true>(row, t, x, sum, dv, a + 2 * h B200_ATTN_ARGS);
+        else b200_ar_weight4<false>(row, t, x, sum, dv, a + 2 * h B200_ATTN_ARGS);
+      }
+    }
+#if B200_KEEP_W
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) b200_ar_put16(p[r].w, 16u * j + 8u * h + 2u * c, a[2 * h + r]);
+    if (off && leave) continue;
+#endif
 #pragma unroll
     for (unsigned int e = 0; e < B200_E / 8; e += 2) {
-      // keys 16 k .. 16 k + 15, head dimensions 8 e .. 8 e + 15
+      // keys 16 j .. 16 j + 15, head dimensions 8 e .. 8 e + 15
       unsigned int b[4];
-      b200_ldsm4t(b, v_at + 2u * ((16u * k + (lane & 15u)) * B200_LD + 8u * e + 8u * (lane >> 4)));
+      b200_ldsm4t(b, v_at + 2u * ((16u * j + (lane & 15u)) * B200_LD + 8u * e + 8u * (lane >> 4)));
       b200_ar_mma(o[e], a, b[0], b[1]);
       b200_ar_mma(o[e + 1], a, b[2], b[3]);
     }

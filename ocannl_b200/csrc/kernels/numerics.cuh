@@ -400,6 +400,16 @@ __device__ __forceinline__ float b200_div_by(float a, const b200_divisor& d) {
   const float q = fmaf(rem, d.r, q0);
   return fabsf(q0) == B200_INF ? q0 : q;   // an infinite numerator (or an overflow) stays infinite
 }
+// The same for a divisor known when the routine is compiled, a literal within [2^-60, 2^60]: its reciprocal
+// folds, and three operations without a branch remain of the division's twenty with their out-of-line part
+// (a score divided by the square root of an odd head size is evaluated for every pair of positions).  A zero,
+// infinite or undefined numerator leaves no remainder to correct by, and the first estimate is the answer.
+__device__ __forceinline__ float b200_div_literal(float a, float b) {
+  const float r = 1.0f / b;
+  const float q0 = a * r;
+  const float rem = fmaf(-q0, b, a);
+  return fabsf(rem) > 0.0f ? fmaf(rem, r, q0) : q0;
+}
 
 // ---- range-checked node accesses (routines compiled with bounds=1).  The proxy stands where the
 //      node's pointer stood: node[i] with i outside the node records (code 2, node id, index) in the
