@@ -16,6 +16,7 @@
 using namespace b200;
 
 static const size_t kRing = 512;
+static const size_t kDirectStages = 4;   // routines of so few kernels are launched without a graph
 
 CUdeviceptr b200_dev::address(int pool_id, size_t offset, size_t bytes) {
   std::lock_guard<std::mutex> g(mu);
@@ -167,10 +168,12 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
   for (auto& st : c->code.stages)
     for (auto& a : st.args) statics_by_value |= a.kind == KArg::StaticValues;
   if (statics_by_value) static_values.assign(P.statics.size(), 0u);
-  // One kernel and nothing else: launched on its own even when graphs are on.  A graph of one node adds about
-  // 1.5 us between two runs (and waits for the previous one at a granularity of 2 us); from two kernels on
-  // it saves as much in launch calls.
-  direct = c->code.stages.size() == 1 && c->code.stages[0].kind != Stage::Memset && scratch_zero.empty();
+  // A few kernels and nothing else: launched one by one even when graphs are on.  A graph adds about 1.5 us
+  // between two runs (and waits for the previous one at a granularity of 2 us), and the launch calls, 2 us each,
+  // pass while the kernels before them run.  Two kernels: 16.6 -> 15.2 us, 8.4 -> 6.7; four: 14.9 -> 13.5,
+  // 16.5 -> 16.2; with five it is as often slower (18.7 -> 20.7).
+  direct = c->code.stages.size() <= kDirectStages && scratch_zero.empty();
+  for (auto& st : c->code.stages) direct &= st.kind != Stage::Memset;
   if (!P.statics.empty() && !statics_by_value) {
     cu_check(cu().cuMemAlloc_(&statics_dev, 256 + 4 * P.statics.size()), "cuMemAlloc(statics)");
     void* hp = nullptr;
