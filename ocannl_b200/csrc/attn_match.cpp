@@ -638,17 +638,19 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     // rows beyond the last query compute on whatever the registers hold (nothing of it is stored)
     // unless the expression reads memory itself: no branch per element
     const std::string guard1 = em.direct_reads > reads_before ? "row.ok ? (float)(" + r.expr + ") : 0.f" : "(float)(" + r.expr + ")";
-    if (rows_kernel) {
-      // where(mask, score, constant): the score of a masked position is known without its product
-      std::string masked_value = "0.0f";
+    // where(mask, score, constant): the score of a masked position is known without its product
+    std::string masked_value = "0.0f";
+    {
       if (v1->kind == Scalar::Tern && v1->op == "where" && n_cond == 1 && v1->args[0].s->kind == Scalar::Get && v1->args[0].s->tn == cond_tns[0] &&
           v1->args[2].s->kind == Scalar::Const) {
         masked = true;
         masked_value = em.constant(v1->args[2].s->cval, Prec::Single);
       }
+    }
+    fn << "__device__ __forceinline__ float " << (rows_kernel ? "b200_ar_" : "b200_attn_") << "masked_score() { return " << masked_value << "; }\n";
+    if (rows_kernel) {
       fn << "__device__ __forceinline__ float b200_ar_score(const b200_attn_row& row, unsigned int b200_t, float b200_acc, unsigned int cb0, unsigned int cb1 B200_ATTN_PARAMS) {\n"
          << syms << "  return " << guard1 << ";\n}\n"
-         << "__device__ __forceinline__ float b200_ar_masked_score() { return " << masked_value << "; }\n"
          << "__device__ __forceinline__ void b200_ar_cond_rows(const b200_attn_row& row, const unsigned int** p B200_ATTN_PARAMS) {\n"
          << syms << cond_rows << "}\n";
     } else {
@@ -691,7 +693,16 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     const int reads_before = em.direct_reads;
     Emitter::Res r = em.scalar(Prec::Single, *v3);
     if (!r.defs.empty()) return false;
-    const std::string guard3 = em.direct_reads > reads_before ? "row.ok ? (float)(" + r.expr + ") : 0.f" : "(float)(" + r.expr + ")";
+    const bool reads3 = em.direct_reads > reads_before;
+    // (an expression that differs from key to key has no one value for the masked ones)
+    if (r.expr.find("b200_t") != std::string::npos) masked = false;
+    if (!rows_kernel) {
+      em.forwarded[s1.tn] = {scores_idcs, "x"};
+      Emitter::Res one = em.scalar(Prec::Single, *v3);
+      fn << "__device__ __forceinline__ float b200_attn_exp_one(const b200_attn_row& row, float x, float mx B200_ATTN_PARAMS) {\n"
+         << syms << "  const unsigned int b200_t = 0u; (void)b200_t;\n  return " << (reads3 ? "row.ok ? (float)(" + one.expr + ") : 0.f" : "(float)(" + one.expr + ")") << ";\n}\n";
+    }
+    const std::string guard3 = reads3 ? "row.ok ? (float)(" + r.expr + ") : 0.f" : "(float)(" + r.expr + ")";
     if (rows_kernel)
       fn << "__device__ __forceinline__ float b200_ar_exp(const b200_attn_row& row, unsigned int b200_t, float x, float mx B200_ATTN_PARAMS) {\n"
          << syms << "  return " << guard3 << ";\n}\n";
@@ -733,11 +744,19 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
     Emitter::Res r = em.scalar(W.prec, *v5);
     if (!r.defs.empty()) return false;
     const bool guarded = em.direct_reads > reads_before;
+    if (r.expr.find("b200_t") != std::string::npos) masked = false;
     auto loop = [&](const std::string& expr) {
       return "#pragma unroll\n  for (int b200_j = 0; b200_j < 32; ++b200_j) {\n    const unsigned int b200_t = t0 + (unsigned int)b200_j; (void)b200_t;\n"
              "    b200_a[b200_j] = " + (guarded ? "row.ok ? (float)(" + expr + ") : 0.f" : "(float)(" + expr + ")") + ";\n  }\n";
     };
     const char* pack = W.prec == Prec::Bfloat16 ? "b200_pack_bf" : "b200_pack_hf";
+    if (!rows_kernel) {
+      em.forwarded[s3.tn] = {exp_idcs, "e"};
+      Emitter::Res one = em.scalar(W.prec, *v5);
+      fn << "__device__ __forceinline__ unsigned int b200_attn_weight_one(const b200_attn_row& row, float e, float sum B200_ATTN_PARAMS) {\n"
+         << syms << "  const unsigned int b200_t = 0u; (void)b200_t;\n  const float b200_w = "
+         << (guarded ? "row.ok ? (float)(" + one.expr + ") : 0.f" : "(float)(" + one.expr + ")") << ";\n  return " << pack << "(b200_w, b200_w);\n}\n";
+    }
     if (rows_kernel) {
       auto guarded_expr = [&](const std::string& e) { return guarded ? "row.ok ? (float)(" + e + ") : 0.f" : "(float)(" + e + ")"; };
       fn << "__device__ __forceinline__ float b200_ar_divisor(const b200_attn_row& row, float sum B200_ATTN_PARAMS) {\n" << syms << "  return "
@@ -886,6 +905,7 @@ std::string attn_translation_unit(const Program&, Stage& st, const std::string& 
   o << "#define B200_ATTN_NAME " << kernel_name << "\n#define B200_T " << a.T << "\n#define B200_E " << a.E << "\n#define B200_IDESC1 "
     << idesc1 << "u\n#define B200_IDESC2 " << idesc2 << "u\n#define B200_HALF " << (a.in_prec == Prec::Half ? 1 : 0)
     << "\n#define B200_OUT_BYTES " << a.out_bytes << "\n#define B200_ATTN_NCOND " << a.n_cond << "\n#define B200_ATTN_NTILES " << a.n_tiles
+    << "\n#define B200_MASKED " << (a.masked ? 1 : 0)
     << "\n#define B200_KEEP_SCORES " << (a.scores.keep ? 1 : 0) << "\n#define B200_KEEP_EXP " << (a.exps.keep ? 1 : 0)
     << "\n#define B200_KEEP_W " << (a.weights.keep ? 1 : 0) << "\n#define B200_ATTN_PARAMS " << st.epi_params << "\n#define B200_ATTN_ARGS "
     << st.epi_args << "\n";

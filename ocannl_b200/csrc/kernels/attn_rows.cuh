@@ -138,7 +138,9 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, c = lane & 3u;
-  const unsigned int tile = blockIdx.x % shape.tiles, bh = blockIdx.x / shape.tiles;
+  // (last tiles first: under a causal mask they look at the most keys)
+  const unsigned int heads = shape.B0 * shape.B1;
+  const unsigned int tile = shape.tiles - 1u - blockIdx.x / heads, bh = blockIdx.x % heads;
   const unsigned int b0 = bh / shape.B1, b1 = bh - b0 * shape.B1;
 
   // keys and values into shared memory, 16 bytes at a time, all of them under way at once (through registers

@@ -24,3 +24,22 @@ def test_row_attention(device, b, h, s, t, e, mode, mask, prec):
     got, info = run_device(device, ir, inputs)
     assert any(st["kind"] == "row attention" for st in info["stages"]), info
     compare(ir, got, want, rtol=2e-2, atol=2e-2 if prec == "bfloat16" else 4e-3)
+
+
+@pytest.mark.parametrize("t", [64, 128, 256])
+@pytest.mark.parametrize("mode,prec", [("ctx", "bfloat16"), ("local", "half")])
+def test_masked_chunks(device, t, mode, prec):
+    """Whole tiles of keys: chunks of 32 keys that are masked for all queries of a warp, rows masked throughout
+    alone and 32 together, a single key left in a chunk."""
+    s = t + 3
+    ir = W.attention(2, 2, s, t, prec=prec, row_mode=mode)
+    inputs = W.attention_inputs(2, 2, s, t, prec=prec)
+    mask = np.tril(np.ones((s, t)))
+    mask[5] = 0.0
+    mask[32:64] = 0.0
+    mask[70:, t - 33] = 1.0
+    inputs["mask"] = mask.reshape(inputs["mask"].shape).astype(inputs["mask"].dtype)
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert any(st["kind"] == "attention" for st in info["stages"]), info
+    compare(ir, got, want, rtol=2e-2, atol=2e-2 if prec == "bfloat16" else 4e-3)
