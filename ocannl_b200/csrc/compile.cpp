@@ -776,6 +776,45 @@ struct Builder {
     return true;
   }
 
+  // The part of its node that a stage overwrites without reading any of it, an interval per axis (empty: not known).
+  using Box = std::vector<std::pair<int64_t, int64_t>>;
+  Box written_box(const Piece& pc) {
+    if (!pc.any_body || pc.any_body->kind != Stmt::Set || pc.any_body->vec_len > 0 || pc.sum) return {};
+    const Stmt& set = *pc.any_body;
+    bool reads = false;
+    walk_scalar(*set.value, [&](const Scalar& e) {
+      if ((e.kind == Scalar::Get || e.kind == Scalar::GetDyn) && e.tn == set.tn) reads = true;
+    }, [](const Stmt&) {});
+    if (reads) return {};
+    Box box;
+    for (auto& ix : set.idcs) {
+      int64_t lo = ix.kind == Index::Iter ? 0 : ix.fixed, hi = lo;
+      auto add = [&](int64_t k, const std::string& sym) {
+        for (auto* loops : {&pc.par, &pc.ser})
+          for (auto& d : *loops)
+            if (d.sym == sym) {
+              const int64_t a = k * d.from, b = k * (d.from + d.extent() - 1);
+              lo += std::min(a, b);
+              hi += std::max(a, b);
+              return true;
+            }
+        return false;
+      };
+      bool known = ix.kind != Index::SubAxis;
+      if (ix.kind == Index::Iter) known = add(1, ix.sym);
+      if (ix.kind == Index::Affine)
+        for (auto& t : ix.terms) known = known && add(t.first, t.second);
+      if (!known) return {};
+      box.push_back({lo, hi});
+    }
+    return box;
+  }
+  static bool apart(const Box& a, const Box& b) {
+    for (size_t i = 0; i < a.size() && i < b.size(); ++i)
+      if (a[i].second < b[i].first || b[i].second < a[i].first) return true;
+    return false;
+  }
+
   // `lhs_zero`: the node the body assigns is known to be all zero when the stage starts.
   // Returns true when the stage made an earlier zero_out of that node unnecessary.
   bool generic_stage(const std::vector<LoopDim>& nest, const StmtP& body, bool lhs_zero = false) {
@@ -1177,20 +1216,30 @@ struct Builder {
     int64_t most = 1;                 // threads the widest stage could use
     bool ordered = false;             // some stage depends on another
     std::set<int> fresh_w, fresh_r;   // written / read since the last barrier
-    auto barrier_for = [&](const std::set<int>& used, const std::set<int>& writes) {
+    // (stages that overwrite different parts of one node, the margins of a padded image, do not depend on one another)
+    std::map<int, std::vector<Box>> fresh_boxes;   // node -> the parts overwritten since the last barrier, where all are known
+    auto barrier_for = [&](const std::set<int>& used, const std::set<int>& writes, int boxed = -1, const Box& box = {}) {
       bool need = false;
-      for (int n : used) need = need || fresh_w.count(n);
-      for (int n : writes) need = need || fresh_r.count(n);
+      auto clear_of_all = [&](int n) {
+        if (n != boxed || box.empty() || fresh_boxes[n].empty()) return false;
+        for (auto& b : fresh_boxes[n])
+          if (b.empty() || !apart(b, box)) return false;
+        return true;
+      };
+      for (int n : used) need = need || (fresh_w.count(n) && !clear_of_all(n));
+      for (int n : writes) need = need || (fresh_r.count(n) && !(fresh_w.count(n) && clear_of_all(n)));
       if (need) {
         ordered = true;
         text += "  __syncthreads();\n";
         fresh_w.clear();
         fresh_r.clear();
+        fresh_boxes.clear();
       } else if (!text.empty()) {
         text += "  // __syncthreads() left out: neither stage writes what the other touches\n";
       }
       fresh_r.insert(used.begin(), used.end());
       fresh_w.insert(writes.begin(), writes.end());
+      for (int n : used) fresh_boxes[n].push_back(n == boxed ? box : Box());
     };
     std::set<int> first_cleared;   // nodes whose first use here overwrites them
     std::set<int> moving;          // nodes read at a static index: a slice of something larger
@@ -1209,7 +1258,8 @@ struct Builder {
                 "u; b200_z += B200_STEP) " + t.ident + "[b200_z] = " + em.storage_zero(t.prec) + ";\n";
       } else {
         const Piece& pc = pieces[i];
-        barrier_for(pc.used, pc.written);
+        const Box box = written_box(pc);
+        barrier_for(pc.used, pc.written, box.empty() ? -1 : pc.any_body->tn, box);
         if (pc.any_body && pc.any_body->kind == Stmt::Set && !em.used_nodes.count(pc.any_body->tn) && !pc.sum && covers_node(*pc.any_body, pc.par)) {
           bool reads = false;
           walk_scalar(*pc.any_body->value, [&](const Scalar& e) {

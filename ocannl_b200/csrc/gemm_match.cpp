@@ -1428,6 +1428,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
              << "u % b200_group) * (B200_STAGING_BYTES / 16)), (int)b200_n0, (int)(b200_m - b200_lane), (int)b200_b1, (int)b200_b0);\n";
         fn << "        b200_tma_commit();\n      }\n      b200_es.nst = 1u;\n      B200_TRE(14);\n    }\n";
       }
+      // what follows through the staging tile without a map (rows that leave as one stretch): the copies have read it
+      bool staged_later = !row_linear_code.empty();
+      for (auto& o : outs) staged_later = staged_later || o.tma < 0;
+      if (staged_later) fn << "    if (b200_lane == 0) b200_tma_store_read_wait<0>();\n    __syncwarp();\n";
       fn << "  }\n";
     }
   }

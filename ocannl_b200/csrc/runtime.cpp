@@ -397,7 +397,14 @@ void b200_routine::enqueue_stages(bool capturing) {
     const Placed& p = placed[i];
     pdl = p.waits.empty();
     if (!streams[(size_t)p.branch]) {
-      cu_check(cu().cuStreamCreate_(&streams[(size_t)p.branch], CU_STREAM_NON_BLOCKING), "cuStreamCreate(branch)");
+      {
+        std::lock_guard<std::mutex> lock(dev->fork_mu);
+        if (!dev->fork_pool.empty()) {
+          streams[(size_t)p.branch] = dev->fork_pool.back();
+          dev->fork_pool.pop_back();
+        }
+      }
+      if (!streams[(size_t)p.branch]) cu_check(cu().cuStreamCreate_(&streams[(size_t)p.branch], CU_STREAM_NON_BLOCKING), "cuStreamCreate(branch)");
       cu_check(cu().cuStreamWaitEvent_(streams[(size_t)p.branch], done[-1], 0), "cuStreamWaitEvent(branch)");
       pdl = false;
     }
@@ -542,10 +549,14 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       graph_merge_epoch = dev->merge_epoch;
       CUgraph g = nullptr;
       cu_check(cu().cuStreamBeginCapture_(dev->stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL), "cuStreamBeginCapture");
-      auto release_branches = [&] {
+      auto release_branches = [&](bool intact) {
         for (auto e : fork_events) cu().cuEventDestroy_(e);
-        for (size_t b = 1; b < fork_streams.size(); ++b)
-          if (fork_streams[b]) cu().cuStreamDestroy_(fork_streams[b]);
+        std::lock_guard<std::mutex> lock(dev->fork_mu);
+        for (size_t b = 1; b < fork_streams.size(); ++b) {
+          if (!fork_streams[b]) continue;
+          if (intact && dev->fork_pool.size() + 1 < (size_t)kBranches) dev->fork_pool.push_back(fork_streams[b]);
+          else cu().cuStreamDestroy_(fork_streams[b]);
+        }
         fork_events.clear();
         fork_streams.clear();
       };
@@ -554,11 +565,11 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       } catch (...) {
         cu().cuStreamEndCapture_(dev->stream, &g);
         if (g) cu().cuGraphDestroy_(g);
-        release_branches();
+        release_branches(false);
         throw;
       }
       const CUresult ended = cu().cuStreamEndCapture_(dev->stream, &g);
-      release_branches();
+      release_branches(ended == CUDA_SUCCESS);
       cu_check(ended, "cuStreamEndCapture");
       CUresult r = cu().cuGraphInstantiateWithFlags_(&graph, g, 0);
       cu().cuGraphDestroy_(g);

@@ -31,6 +31,10 @@ struct b200_dev {
   int sm_count = 0, cc_major = 0, cc_minor = 0;
   std::mutex mu;
   std::map<int, Pool> pools;
+  // streams for the branches of a capture, kept between captures (a stream costs some 150 us to make): at most one
+  // capture's worth, each used by one capture at a time
+  std::mutex fork_mu;
+  std::vector<CUstream> fork_pool;
   size_t used = 0;
   volatile unsigned int* status_host = nullptr;  // written by kernels whose bounded waits expire
   CUdeviceptr status_dev = 0;

@@ -87,3 +87,14 @@ def test_convolution_gradients_by_windows(device, cfg, prec):
         w, g = (W.load(prec, a[name]) if a[name].dtype == np.uint16 else a[name] for a in (want, got))
         scale = float(np.abs(w).max())
         np.testing.assert_allclose(g, w, rtol=2e-2 if prec != "single" else 1e-4, atol=(2e-2 if prec != "single" else 1e-5) * scale, err_msg=name)
+
+
+@pytest.mark.parametrize("classes", [4, 8, 10, 16])
+def test_classifier_widths(device, classes):
+    """Logits that leave through a tensor map (rows of whole 16 bytes) and rows behind them that leave as one
+    stretch share a staging tile; rows enough that tiles follow one another."""
+    ir = W.mlp_forward(rows=4098, dims=(64, 64, 256, classes), wprec="bfloat16")
+    x, onehot = W.mlp_inputs(rows=4098, in_dim=64, classes=classes)
+    inputs = dict(W.mlp_params(dims=(64, 64, 256, classes)), x=x, labels=onehot)
+    got, _ = run_device(device, ir, inputs)
+    compare(ir, got, run_oracle(ir, inputs), rtol=2e-2, atol=2e-2)
