@@ -310,6 +310,7 @@ struct Piece {
   bool pairs = false;
   int64_t ser_work = 1;
   std::vector<int> staged;   // small read-only nodes the kernel first copies into shared memory
+  std::string whole;         // the kernel's body where it is not the grid-stride loop over the stage's iterations
   // a sum kept in `b200_self` over the serial loops (`t[p] := t[p] + term`): its parts, so that several
   // lanes may share one sum
   bool sum = false;
@@ -815,6 +816,159 @@ struct Builder {
     return false;
   }
 
+  // A single-precision sum of products whose one factor is a small table (the kernel of a convolution, at most
+  // 40 KB) and whose other factor is looked up at moving positions.  The table lies in shared memory with its
+  // outputs next to one another; a thread sums T outputs at P neighbouring positions, so that T table entries and
+  // P looked-up values, T / 4 + P loads, serve T P multiplications.  Sums run in the order of the loops.
+  // On the tensor cores the same sum would need three products of two-part operands, and a copy of every
+  // window in memory: 64 images of 32 x 32 x 3, 32 outputs of 3 x 3: 14.6 us, 6 us here.
+  // T P is as large as leaves 12 warps per SM; below four outputs per thread the plain kernel is as good.
+  bool table_stage(const std::vector<LoopDim>& nest, const StmtP& body) {
+    if (opt.bounds || body->kind != Stmt::Set || body->vec_len > 0 || nest.size() < 2) return false;
+    const Tnode& out = code.prog.tn(body->tn);
+    if (out.prec != Prec::Single) return false;
+    for (auto& d : nest)
+      if (d.extent() <= 0 || !parallel_safe(d.sym, *body)) return false;
+    // the one local sum of the assigned value
+    const Scalar* scope = nullptr;
+    int scopes = 0;
+    bool plain = true;
+    walk_scalar(*body->value, [&](const Scalar& e) {
+      if (e.kind == Scalar::LocalScope) { scope = &e; ++scopes; }
+      if (e.kind == Scalar::GetDyn || e.kind == Scalar::GetMerge || (e.kind == Scalar::Get && e.tn == body->tn)) plain = false;
+    }, [](const Stmt&) {});
+    if (scopes != 1 || !plain || code.prog.tn(scope->tn).prec != Prec::Single) return false;
+    const Stmt* at = scope->body.get();
+    if (!at || at->kind != Stmt::Seq || at->items.size() != 2) return false;
+    const Stmt* init = at->items[0].get();
+    if (init->kind != Stmt::SetLocal || init->scope_id != scope->scope_id || init->value->kind != Scalar::Const) return false;
+    std::vector<LoopDim> red;
+    for (at = at->items[1].get(); at->kind == Stmt::For; at = at->body.get()) {
+      LoopDim d;
+      d.sym = at->index; d.from = at->from; d.to = at->to;
+      if (d.extent() <= 0) return false;
+      red.push_back(d);
+      if (!at->body) return false;
+    }
+    if (red.empty() || at->kind != Stmt::SetLocal || at->scope_id != scope->scope_id) return false;
+    const Scalar& step = *at->value;
+    if (step.kind != Scalar::Tern || step.op != "fma" || step.args[2].s->kind != Scalar::GetLocal || step.args[2].s->scope_id != scope->scope_id) return false;
+    const LoopDim& c = nest.back();
+    auto uses_sym = [](const Scalar& e, const std::string& sym) {
+      for (auto& ix : e.idcs)
+        if (ix.uses(sym)) return true;
+      return false;
+    };
+    const Scalar* W = step.args[0].s.get();
+    const Scalar* X = step.args[1].s.get();
+    for (auto* e : {W, X})
+      if (e->kind != Scalar::Get || code.prog.tn(e->tn).prec != Prec::Single || e->tn == body->tn) return false;
+    if (!uses_sym(*W, c.sym)) std::swap(W, X);
+    if (!uses_sym(*W, c.sym) || uses_sym(*X, c.sym)) return false;
+    for (size_t i = 0; i + 1 < nest.size(); ++i)
+      if (uses_sym(*W, nest[i].sym)) return false;
+    bool moving = false;
+    for (auto& ix : X->idcs) moving = moving || ix.kind == Index::Affine;
+    for (auto& ix : W->idcs)
+      if (ix.kind == Index::SubAxis) return false;
+    for (auto& ix : X->idcs)
+      if (ix.kind == Index::SubAxis) return false;
+    if (!moving) return false;
+    int64_t K = 1, outputs = 1;
+    for (auto& d : red) K *= d.extent();
+    for (auto& d : nest) outputs *= d.extent();
+    const LoopDim& w = nest[nest.size() - 2];
+    const int64_t C = c.extent();
+    int T = 0, P = 0;
+    for (auto tp : {std::pair<int, int>{16, 4}, {16, 2}, {8, 4}, {8, 2}, {16, 1}, {8, 1}, {4, 2}, {4, 1}}) {
+      const int64_t padded = (C + tp.first - 1) / tp.first * tp.first;
+      // (no more than a fifth of the sums for columns that do not exist)
+      if (w.extent() % tp.second || padded * 4 > C * 5 || padded * K * 4 > 40960) continue;
+      if (outputs / C * (padded / tp.first) / tp.second < 148 * 384) continue;
+      T = tp.first;
+      P = tp.second;
+      break;
+    }
+    if (!T || outputs >= (1ll << 31)) return false;
+    const int64_t Cp = (C + T - 1) / T * T, G = Cp / T, threads = outputs / C * G / P;
+
+    Emitter em(code.prog);
+    Emitter::Res wr = em.scalar(Prec::Single, *W), xr = em.scalar(Prec::Single, *X);
+    em.scope_subst[scope->scope_id] = "b200_acc[b200_p][b200_q]";
+    Emitter::Res vr = em.scalar(Prec::Single, *body->value);
+    if (!wr.defs.empty() || !xr.defs.empty() || !vr.defs.empty()) return false;
+    em.used_nodes.insert(body->tn);
+    auto u = [](int64_t v) { return std::to_string(v) + "u"; };
+    auto plus = [&](const LoopDim& d) { return d.from ? " + " + u(d.from) : std::string(); };
+    std::ostringstream o;
+    o << "  __shared__ __align__(16) float b200_table[" << K * Cp << "];\n"
+      << "  for (unsigned int b200_i = threadIdx.x; b200_i < " << u(K * Cp) << "; b200_i += blockDim.x) {\n    const unsigned int b200_c = b200_i % " << u(Cp)
+      << ", " << c.sym << " = b200_c" << plus(c) << ";\n    unsigned int b200_k = b200_i / " << u(Cp) << ";\n";
+    for (size_t i = red.size(); i-- > 0;) {
+      o << "    const unsigned int " << red[i].sym << " = " << (i ? "b200_k % " + u(red[i].extent()) : std::string("b200_k")) << plus(red[i]) << ";\n";
+      if (i) o << "    b200_k /= " << u(red[i].extent()) << ";\n";
+    }
+    o << "    b200_table[b200_i] = b200_c < " << u(C) << " ? " << wr.expr << " : 0.0f;\n  }\n  __syncthreads();\n"
+      << "  for (unsigned int b200_g = blockIdx.x * blockDim.x + threadIdx.x; b200_g < " << u(threads) << "; b200_g += gridDim.x * blockDim.x) {\n"
+      << "    const unsigned int b200_c0 = b200_g % " << u(G) << " * " << u(T) << ";\n    unsigned int b200_r = b200_g / " << u(G) << ";\n";
+    o << "    const unsigned int b200_w0 = b200_r % " << u(w.extent() / P) << " * " << u(P) << plus(w) << ";\n    b200_r /= " << u(w.extent() / P) << ";\n";
+    for (size_t i = nest.size() - 2; i-- > 0;) {
+      o << "    const unsigned int " << nest[i].sym << " = " << (i ? "b200_r % " + u(nest[i].extent()) : std::string("b200_r")) << plus(nest[i]) << ";\n";
+      if (i) o << "    b200_r /= " << u(nest[i].extent()) << ";\n";
+    }
+    o << "    float b200_acc[" << P << "][" << T << "];\n#pragma unroll\n    for (int b200_p = 0; b200_p < " << P << "; ++b200_p)\n#pragma unroll\n      for (int b200_q = 0; b200_q < "
+      << T << "; ++b200_q) b200_acc[b200_p][b200_q] = " << em.constant(init->value->cval, Prec::Single) << ";\n";
+    // the innermost loops without jumps, up to 32 steps
+    std::vector<bool> flat(red.size(), false);
+    int64_t steps = 1;
+    for (size_t i = red.size(); i-- > 0 && steps * red[i].extent() <= 32;) {
+      steps *= red[i].extent();
+      flat[i] = true;
+    }
+    std::string k = "0u";
+    for (size_t i = 0; i < red.size(); ++i) {
+      o << (flat[i] ? "#pragma unroll\n" : i + 1 == red.size() ? "#pragma unroll 8\n" : "#pragma unroll 1\n") << "    for (unsigned int " << red[i].sym << " = " << u(red[i].from) << "; " << red[i].sym << " <= " << u(red[i].to)
+        << "; ++" << red[i].sym << ") {\n";
+      k = "(" + k + " * " + u(red[i].extent()) + " + " + red[i].sym + (red[i].from ? " - " + u(red[i].from) : std::string()) + ")";
+    }
+    o << "      float b200_w[" << T << "];\n#pragma unroll\n      for (int b200_q = 0; b200_q < " << T << "; b200_q += 4) {\n        const float4 b200_v = *(const float4*)(b200_table + "
+      << k << " * " << u(Cp) << " + b200_c0 + b200_q);\n        b200_w[b200_q] = b200_v.x; b200_w[b200_q + 1] = b200_v.y; b200_w[b200_q + 2] = b200_v.z; b200_w[b200_q + 3] = b200_v.w;\n      }\n"
+      << "#pragma unroll\n      for (int b200_p = 0; b200_p < " << P << "; ++b200_p) {\n        const unsigned int " << w.sym << " = b200_w0 + b200_p;\n        const float b200_x = " << xr.expr
+      << ";\n#pragma unroll\n        for (int b200_q = 0; b200_q < " << T << "; ++b200_q) b200_acc[b200_p][b200_q] = fmaf(b200_w[b200_q], b200_x, b200_acc[b200_p][b200_q]);\n      }\n";
+    for (size_t i = 0; i < red.size(); ++i) o << "    }\n";
+    o << "#pragma unroll\n    for (int b200_p = 0; b200_p < " << P << "; ++b200_p) {\n      const unsigned int " << w.sym << " = b200_w0 + b200_p;\n      float b200_v[" << T
+      << "];\n#pragma unroll\n      for (int b200_q = 0; b200_q < " << T << "; ++b200_q) {\n        b200_v[b200_q] = 0.0f;\n        if (" << (Cp == C ? std::string("true") : "b200_c0 + b200_q < " + u(C)) << ") {\n          const unsigned int " << c.sym << " = b200_c0 + b200_q"
+      << plus(c) << ";\n          b200_v[b200_q] = " << vr.expr << ";\n        }\n      }\n";
+    Indices first = body->idcs;
+    const std::string off = em.offset(first, out.dims);
+    const bool unit = !first.empty() && first.back().kind == Index::Iter && first.back().sym == c.sym && C % 4 == 0;
+    o << "#pragma unroll\n      for (int b200_q = 0; b200_q < " << T << "; b200_q += " << (unit ? 4 : 1) << ") {\n        const unsigned int " << c.sym << " = b200_c0 + b200_q" << plus(c)
+      << ";\n        float* const b200_to = " << out.ident << " + (" << off << ");\n";
+    if (unit)
+      o << "        if (b200_c0 + b200_q >= " << u(C) << ") break;\n        if (((unsigned long long)b200_to & 15ull) == 0ull) *(float4*)b200_to = make_float4(b200_v[b200_q], b200_v[b200_q + 1], b200_v[b200_q + 2], b200_v[b200_q + 3]);\n"
+        << "        else { b200_to[0] = b200_v[b200_q]; b200_to[1] = b200_v[b200_q + 1]; b200_to[2] = b200_v[b200_q + 2]; b200_to[3] = b200_v[b200_q + 3]; }\n";
+    else
+      o << "        if (b200_c0 + b200_q < " << u(C) << ") *b200_to = b200_v[b200_q];\n";
+    o << "      }\n    }\n  }\n";
+
+    Stage st;
+    st.kind = Stage::Generic;
+    st.kernel = kernel_name();
+    st.par = nest;
+    st.total = threads;
+    st.block = 256;
+    st.grid_override = (int)std::min<int64_t>((threads + 255) / 256, 148 * 4);
+    st.note = "table of " + std::to_string(K) + " x " + std::to_string(C) + " in shared memory, " + std::to_string(T) + " outputs at " + std::to_string(P) + " positions per thread";
+    st.writes = {body->tn};
+    Piece pc;
+    pc.whole = o.str();
+    pc.used = em.used_nodes;
+    pc.written = {body->tn};
+    pieces[code.stages.size()] = pc;
+    code.stages.push_back(st);
+    return true;
+  }
+
   // `lhs_zero`: the node the body assigns is known to be all zero when the stage starts.
   // Returns true when the stage made an earlier zero_out of that node unnecessary.
   bool generic_stage(const std::vector<LoopDim>& nest, const StmtP& body, bool lhs_zero = false) {
@@ -1132,11 +1286,15 @@ struct Builder {
     Emitter em(code.prog);
     em.used_nodes = pc.used;
     em.uses_merge = pc.uses_merge;
-    std::string statics = static_prologue(pc.body_text + pc.decomp, em, 2);
+    std::string statics = static_prologue(pc.body_text + pc.decomp + pc.whole, em, 2);
     std::ostringstream k_src;
     k_src << "extern \"C\" __global__ void __launch_bounds__(" << st.block << ") " << st.kernel << "(";
     emit_params(k_src, st, em, pc.written);
     k_src << ") {\n" << kGridEntry << statics;
+    if (!pc.whole.empty()) {
+      src << k_src.str() << pc.whole << "}\n\n";
+      return;
+    }
     for (int tn : pc.staged) {
       const Tnode& t = code.prog.tn(tn);
       const std::string sm = "b200_sm_" + t.ident;
@@ -2498,6 +2656,15 @@ struct Builder {
       elems *= d.extent();
     }
     if (first.empty() || second.empty() || red.empty() || elems * 4 > (1ll << 30) || elems >= (1ll << 31)) return false;
+    // a few hundred multiplications per gathered row do not pay for the gathering (see the convolutions' windows in
+    // match_gemm): 8 outputs of 3 x 3 on one channel, 262144 positions: 9 us as scattered additions, 49 us as this
+    {
+      int64_t e[3] = {1, 1, 1};
+      for (auto& d : first) e[0] *= d.extent();
+      for (auto& d : second) e[1] *= d.extent();
+      for (auto& d : red) e[2] *= d.extent();
+      if (e[0] * e[1] * e[2] / std::max({e[0], e[1], e[2]}) < 256) return false;
+    }
     const std::string t_ident = code.prog.tn(set.tn).ident;
     const std::vector<int64_t> t_dims = code.prog.tn(set.tn).dims;
     const int64_t t_elems = code.prog.tn(set.tn).num_elems();
@@ -2914,6 +3081,7 @@ struct Builder {
           return;
         }
       }
+      if (gemm_at(i) && table_stage(nest, body)) return;
       if (gemm_at(i) && body->kind == Stmt::Set) {
         Stage g;
         int n_fused = 0;

@@ -382,6 +382,14 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     // ---- gather what the maps cannot express.  m, n, k and the batch become one axis each, the
     // loops concatenated outer to inner; an operand that already lies that way stays where it is.
     if (!worth(product(all_m), product(all_n), product(all_k), product(all_b))) return false;
+    // A convolution's windows cost as much to gather, padded and in two parts, as some hundred multiplications
+    // each: not worth it for a few outputs over a few inputs (8 outputs of 3 x 3 on 1 to 3 channels, forward and
+    // backward: 36 - 48 us without, 52 - 62 us with; 32 outputs on one channel, or 8 on 8: 70 and 51 without, 66
+    // and 44 with).
+    if (affine_operand) {
+      const int64_t pm = product(all_m), pn = product(all_n), pk = product(all_k);
+      if (pm * pn * pk / std::max({pm, pn, pk}) < 256) return false;
+    }
     if (all_m.empty() || all_n.empty() || all_k.empty()) return false;
     auto concat = [&](const std::vector<Dim>& v) {
       Dim d;

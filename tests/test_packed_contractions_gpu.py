@@ -98,3 +98,17 @@ def test_classifier_widths(device, classes):
     inputs = dict(W.mlp_params(dims=(64, 64, 256, classes)), x=x, labels=onehot)
     got, _ = run_device(device, ir, inputs)
     compare(ir, got, run_oracle(ir, inputs), rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("size,cin,cout,kernel,stride", [(33, 2, 10, 3, 1), (32, 3, 32, 3, 1), (34, 1, 20, 5, 2), (28, 1, 8, 5, 1), (32, 2, 64, 3, 1)])
+def test_small_table(device, size, cin, cout, kernel, stride):
+    """Single-precision convolutions whose kernel is a table in shared memory: widths that leave columns over,
+    odd numbers of positions, the order of the sum (the same bits as the loops give)."""
+    ir = W.conv2d_update(batch=80, size=size, cin=cin, cout=cout, kernel=kernel, stride=stride, prec="single")
+    rng = np.random.default_rng(3)
+    inputs = {t.ident: rng.standard_normal(t.dims).astype(np.float32) for t in ir.params() if t.ident in ("x", "target", "kernel", "bias")}
+    got, info = run_device(device, ir, inputs)
+    assert any("table of" in s.get("note", "") for s in info["stages"]), info
+    plain, _ = run_device(device, ir, inputs, options="gemm=0")
+    assert np.array_equal(got["y"], plain["y"])
+    compare(ir, got, run_oracle(ir, inputs), rtol=1e-3, atol=1e-3, only=["y"])
