@@ -1235,11 +1235,11 @@ struct Builder {
       // than what leaving it out costs: its own launch, and a second one for the block's other half (8 us,
       // 16000 cycles, with the stage's own time on many SMs).  Each of a thread's iterations takes the
       // latency of its loads or, with many warps, their issue, about six instructions per warp and
-      // scheduler.  (The 37 x 10 logits over 1024 hidden units took 25 us of one block.)
+      // scheduler, twice that for pairs.  (The 37 x 10 logits over 1024 hidden units took 25 us of one block.)
       const double threads = (double)st.total * std::max(1, st.coop);
       const double rounds = std::ceil(threads / 1024.0), warps = std::ceil(std::min(threads, 1024.0) / 32.0);
       const double iters = rounds * (double)ser_work * iterations(*body) / std::max(1, st.coop);
-      if (iters * std::max(30.0, 6.0 * warps / 4.0) > 16000.0) pc.fusable = false;
+      if (iters * std::max(30.0, (pairs ? 12.0 : 6.0) * warps / 4.0) > 16000.0) pc.fusable = false;
     }
     if (opt.enable_fuse && !scatter && st.coop == 0 && st.total > 0 && !st.par.empty() && st.par[0].from == 0 && !(pairs && st.par.size() == 1)) {
       pc.body = body;
