@@ -338,7 +338,8 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // each for m, n and k, unit stride along k or along m / n
   // Single-precision operands of the shapes the tensor cores are also used for, but which are small or
   // narrow in some direction, keep their precision (tf32 pairs); so do those that have to be gathered.
-  const bool pairs_of_tf32 = A.prec == Prec::Single && (opt.exact_single || product(all_m) < 32 || product(all_n) < 8 || product(all_k) < 16);
+  const bool pairs_of_tf32 = A.prec == Prec::Single && (opt.exact_single || product(all_m) < 32 || product(all_n) < 8 || product(all_k) < 16 ||
+                                                           2.0 * (double)product(all_m) * (double)product(all_n) * (double)product(all_k) * (double)product(all_b) < 4.0e6);
   auto as_it_lies = [&] {
     if (pairs_of_tf32) return false;
     if (gm.size() != 1 || gn.size() != 1 || gk.size() != 1 || gb.size() > 2) return false;
@@ -373,8 +374,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (batch > 1 && (m < 16 || n < 8)) return false;
     if (m == 1 && n == 1) return false;
     if (form_b ? ((m <= 16 && !affine_operand) || n < 8 || k < 4) : k < 8) return false;
-    // (a long contraction for a batch of rows is worth it earlier: its rows' softmax can follow in the epilogue)
-    return 2.0 * (double)m * (double)n * (double)k * (double)batch >= (!form_b && m >= 8 && k >= 256 && !affine_operand ? 5.0e5 : 4.0e6);
+    // (a long contraction for a batch of rows is worth it earlier: its rows' softmax can follow in the epilogue;
+    // not in single precision, where it would take a copy of the operands in two parts)
+    return 2.0 * (double)m * (double)n * (double)k * (double)batch >=
+           (!form_b && m >= 8 && k >= 256 && !affine_operand && A.prec != Prec::Single ? 5.0e5 : 4.0e6);
   };
   if (as_it_lies()) {
     if (!worth(g.m.extent, g.n.extent, g.k.extent, product(gb))) return false;
