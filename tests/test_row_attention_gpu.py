@@ -1,4 +1,4 @@
-"""The attention chain with short or odd rows in one kernel (score rows in registers): key counts at the
+"""The attention chain with short or odd rows in one kernel: key counts at the
 edges of its tiles of 8 and 16, head dimensions of one to eight k steps, fewer queries than a warp takes,
 with and without a mask, a row masked throughout, nodes kept or routine-local."""
 import numpy as np
