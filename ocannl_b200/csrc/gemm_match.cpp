@@ -393,6 +393,10 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
       const int64_t pm = product(all_m), pn = product(all_n), pk = product(all_k);
       if (pm * pn * pk / std::max({pm, pn, pk}) < 256) return false;
     }
+    // Single precision in two parts: the weights, read, split and written, are worth it for 32 rows or more
+    // (10 rows of 496-2032-200-14: 54 us with, 34 us by a warp per output; 31 rows of 400-2000-300-10: 56 us with, 31
+    // without; 37 of 784-1024-1024-10, in plain tf32 there: 33 us, 47 without).
+    if (A.prec == Prec::Single && !form_b && !affine_operand && product(all_m) < 32) return false;
     if (all_m.empty() || all_n.empty() || all_k.empty()) return false;
     auto concat = [&](const std::vector<Dim>& v) {
       Dim d;
