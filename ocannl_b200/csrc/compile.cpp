@@ -2803,8 +2803,9 @@ struct Builder {
   }
 
   // A routine of one kernel takes its static indices as a kernel argument instead of through the device
-  // table: such a routine is always launched directly (see b200_routine::launch), where the table would cost a
-  // copy ahead of the kernel every time an index moves -- the next minibatch of a training step.
+  // table: such a routine is never captured in a graph (`direct` in b200_routine::link follows from the argument),
+  // and the table would cost a copy ahead of the kernel every time an index moves -- the next minibatch of a
+  // training step.
   void statics_by_value() {
     if (code.stages.size() != 1 || code.stages[0].kind != Stage::Generic || opt.bounds) return;
     for (auto& a : code.stages[0].args)

@@ -174,6 +174,10 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
   // 16.5 -> 16.2; with five it is as often slower (18.7 -> 20.7).
   direct = c->code.stages.size() <= kDirectStages && scratch_zero.empty();
   for (auto& st : c->code.stages) direct &= st.kind != Stage::Memset;
+  // Static indices that are a kernel argument would be captured with their values of the first run: such a routine
+  // is launched directly whatever else it queues (a node of its scratch that starts at zero is a clear ahead of its
+  // kernel: 200 points through 2-16-16-1).
+  direct = direct || statics_by_value;
   if (!P.statics.empty() && !statics_by_value) {
     cu_check(cu().cuMemAlloc_(&statics_dev, 256 + 4 * P.statics.size()), "cuMemAlloc(statics)");
     void* hp = nullptr;

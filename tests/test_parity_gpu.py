@@ -194,6 +194,24 @@ def test_moons_training_steps(device, graph, options):
     assert abs(float(got["scalar_loss"][0])) > 0
 
 
+@pytest.mark.parametrize("batch,hid", [(200, 16), (240, 16), (100, 24)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_moons_steps_with_cleared_nodes_in_memory(device, graph, batch, hid):
+    """The same step, still one kernel, at sizes where nodes that start at zero find no room in the block's
+    shared memory: every run clears them first.  With graph replay on as without, each run takes its own
+    minibatch and its own point of the learning-rate schedule.  A sum of n products in another order moves by
+    about sqrt(n) 2^-24 of its terms' size, n = the batch at most, doubled by each of the four steps behind it."""
+    ir = W.moons_train_step(n_batches=1024 // batch, batch=batch, hid=hid)
+    x, y = W.moons_inputs(batch=batch)
+    inputs = dict(W.moons_params(hid=hid), moons_flat=x, moons_classes=y)
+    statics = [{"i1": b, "i2": s} for s, b in ((0, 0), (1000, 3), (2000, 1), (4079, 2))]
+    want = run_oracle(ir, inputs, statics)
+    got, info = run_device(device, ir, inputs, statics, graph=graph)
+    assert len(info["stages"]) == 1, info
+    rtol = 16 * np.sqrt(batch) * 2.0 ** -24
+    compare(ir, got, want, rtol=rtol, atol=rtol)
+
+
 def test_moons_static_index_errors(device):
     from ocannl_b200 import backend as bk
     ir = W.moons_train_step()
