@@ -95,8 +95,9 @@ int b200_set_async_uploads(b200_dev* dev, int on);
  *      lib/nn_blocks.ml:222-236) as one kernel; coop: cooperative reductions; fuse: several stages per
  *      launch; pairs: two neighbouring elements per thread with packed 16-bit arithmetic; splitk:
  *      few-tile fp32 accumulations split over K (atomic adds, order not fixed); tf32: contractions of
- *      single-precision operands on the tensor cores as tf32 (10-bit mantissas, fp32 sums; with
- *      tf32=0 they stay on the exact generic kernels); bounds: a range-checked build of the generated
+ *      single-precision operands on the tensor cores as tf32 (10-bit mantissas, fp32 sums; convolutions
+ *      and small, narrow or unaligned products as two such parts an operand, which keeps single
+ *      precision; with tf32=0 all stay on the exact generic kernels); bounds: a range-checked build of the generated
  *      kernels (generic kernels only): an access outside a node is skipped and the next wait returns
  *      B200_E_DEVICE naming the node id and the element. */
 int b200_compile(const char* name, const char* b200ir, size_t len, const char* options, b200_code** out);

@@ -337,8 +337,13 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // ---- what the tensor maps can express: 16-byte aligned bases and strides, 32-bit extents, one axis
   // each for m, n and k, unit stride along k or along m / n
   // Single-precision operands of the shapes the tensor cores are also used for, but which are small or
-  // narrow in some direction, keep their precision (tf32 pairs); so do those that have to be gathered.
-  const bool pairs_of_tf32 = A.prec == Prec::Single && (opt.exact_single || product(all_m) < 32 || product(all_n) < 8 || product(all_k) < 16 ||
+  // narrow in some direction, keep their precision (tf32 pairs); so do those that have to be gathered, and all
+  // convolutions: whether a patch happens to lie on a tensor map depends on the kernel's height, and plain tf32
+  // (2^-11 an operand) would come and go with it.
+  bool affine_operand = false;
+  for (auto* op : {x, y})
+    for (auto& ix : op->idcs) affine_operand = affine_operand || ix.kind == Index::Affine;
+  const bool pairs_of_tf32 = A.prec == Prec::Single && (opt.exact_single || affine_operand || product(all_m) < 32 || product(all_n) < 8 || product(all_k) < 16 ||
                                                            2.0 * (double)product(all_m) * (double)product(all_n) * (double)product(all_k) * (double)product(all_b) < 4.0e6);
   auto as_it_lies = [&] {
     if (pairs_of_tf32) return false;
@@ -358,7 +363,6 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
     if (!ok16(g.a_kmajor ? g.m.sa : g.k.sa) || !ok16(g.b_kmajor ? g.n.sb : g.k.sb)) return false;
     for (auto& b : g.batch)
       if ((b.sa && !ok16(b.sa)) || (b.sb && !ok16(b.sb))) return false;
-    // neighbouring convolution patches overlap; only a gathered copy has them one after the other
     return true;
   };
   // Worth a tensor-core launch?  From a few million operations on, whatever the shape: a tile that is mostly
@@ -366,9 +370,6 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // outputs plus about 3 us, where the loop-nest kernels take a warp or a serial loop per output
   // (303 x 5 x 1608: 21 us).  Accumulations into few rows stay with the kernel that keeps them in registers,
   // unless an operand has to be looked up element by element (a convolution's patches).
-  bool affine_operand = false;
-  for (auto* op : {x, y})
-    for (auto& ix : op->idcs) affine_operand = affine_operand || ix.kind == Index::Affine;
   auto worth = [&](int64_t m, int64_t n, int64_t k, int64_t batch) {
     // (products of single rows or columns, one per batch index, are reductions: a layer norm's sum of squares)
     if (batch > 1 && (m < 16 || n < 8)) return false;

@@ -72,6 +72,36 @@ def test_convolution_patches(device, cin, cout, kernel, stride, prec):
     compare(r, got, want, only=["y"], **tol)
 
 
+def convolution(batch, size, cin, cout, kh, kw, stride, prec):
+    """relu of a `valid` convolution with kh x kw kernels, as the reference lowers it."""
+    oh_, ow_ = (size - kh) // stride + 1, (size - kw) // stride + 1
+    r = Routine("conv_%d_%d_%d_%dx%d_%d" % (size, cin, cout, kh, kw, stride))
+    x = r.tn("x", prec, [batch, size, size, cin], read_only=True)
+    w = r.tn("kernel", prec, [cout, kh, kw, cin], read_only=True)
+    y = r.tn("y", prec, [batch, oh_, ow_, cout])
+    ib, oh, ow, co, i, j, ci = r.syms(7)
+    at = lambda: x[ib, Affine(((stride, oh), (1, i))), Affine(((stride, ow), (1, j))), ci]
+    acc = W.reduce_scope(r, "acc", "single", [(i, kh), (j, kw), (ci, cin)], lambda: (w[co, i, j, ci], at()), orig=(ib, oh, ow, co))
+    r.body = Seq([loops([(ib, batch), (oh, oh_), (ow, ow_), (co, cout)], Set(y, (ib, oh, ow, co), un("relu", acc)))])
+    return r
+
+
+@pytest.mark.parametrize("cin,cout,kh,kw,stride", [(64, 256, 1, 1, 1), (64, 256, 1, 1, 2), (64, 128, 1, 5, 1), (32, 64, 3, 3, 1)])
+@pytest.mark.parametrize("prec", ["bfloat16", "single"])
+def test_patches_that_lie_on_a_tensor_map(device, cin, cout, kh, kw, stride, prec):
+    """Kernels one row high have patches that a tensor map can describe where they lie, overlapping ones among
+    them (1 x 5); higher ones do not.  16-bit patches are read there, without a copy; single precision keeps its
+    precision whatever the kernel."""
+    ir = convolution(8, 40, cin, cout, kh, kw, stride, prec)
+    inputs = _inputs(ir, kh * kw * cin)
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    kinds = [s["kind"] for s in info["stages"]]
+    assert kinds == (["gemm"] if prec == "bfloat16" and kh == 1 else ["generic", "gemm"]), info
+    tol = dict(rtol=1e-5, atol=2e-6) if prec == "single" else dict(rtol=2e-2, atol=2e-3)
+    compare(ir, got, want, only=["y"], **tol)
+
+
 @pytest.mark.parametrize("cfg", [dict(batch=8, size=16, cin=8, cout=16), dict(batch=5, size=23, cin=3, cout=33, kernel=5),
                                  dict(batch=40, size=17, cin=8, cout=20, stride=2)])
 @pytest.mark.parametrize("prec", ["bfloat16", "single"])
