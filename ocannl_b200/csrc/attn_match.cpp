@@ -504,6 +504,7 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
 
   // ---- generated code
   Emitter em(P);
+  em.straight_division = true;
   em.large_models = opt.large_models;
   std::ostringstream fn;
   const std::string syms =

@@ -347,7 +347,7 @@ std::string Emitter::binop(Prec prec, const std::string& op, const std::string& 
       char* end = nullptr;
       const double v = std::fabs(strtod(b.c_str(), &end));
       if (end && end != b.c_str() && end[0] == 'f' && !end[1] && v >= 0x1p-60 && v <= 0x1p+60) {
-        const std::string q = "b200_div_literal(" + a + ", " + b + ")";
+        const std::string q = (straight_division ? "b200_div_literal_straight(" : "b200_div_literal(") + a + ", " + b + ")";
         return lowp(prec) ? std::string(round_fn(prec)) + q + ")" : q;
       }
     }

@@ -59,6 +59,7 @@ struct Emitter {
   // when set, the emitted text of every single-precision divisor is appended here (a caller that
   // wants to prepare row-invariant divisors emits once to see them)
   std::vector<std::string>* divisor_probe = nullptr;
+  bool straight_division = false;   // divisions by a literal without a branch (see b200_div_literal_straight)
   // nodes read through another name (a copy staged in shared memory)
   std::map<int, std::string> node_alias;
   // nodes whose loads may use the read-only data path

@@ -68,6 +68,30 @@ def test_operator_table(device, prec, options):
     compare(ir, got, want, rtol=rtol, atol=atol, only=rest)
 
 
+@pytest.mark.parametrize("literal", [0.001, 0.1, 1e-5, 3.0, 7.0, -0.3, 10.0, 500.0, 5.656854152679443, 1.9999998807907104, 1e15, 1e-15])
+@pytest.mark.parametrize("options", [None, "pairs=0"])
+def test_division_by_a_literal_bits(device, options, literal):
+    """A single-precision division by a constant is the IEEE quotient over every numerator: ordinary ones, those
+    whose quotient overflows, lies near or below the normal range or is zero, infinities and NaN."""
+    n = 1 << 20
+    r = R.Routine("divide_by_literal")
+    x = r.tn("x", "single", [n], read_only=True)
+    y = r.tn("y", "single", [n])
+    i = r.sym()
+    r.body = R.For(i, 0, n - 1, R.Set(y, (i,), x[i] / literal))
+    g = np.random.default_rng(17)
+    v = g.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32).view(np.float32)      # every exponent alike
+    v[: n // 2] = (g.uniform(1.0, 2.0, n // 2) * g.choice([-1.0, 1.0], n // 2)).astype(np.float32)
+    big = np.finfo(np.float32).max
+    v[:12] = [0.0, -0.0, np.inf, -np.inf, np.nan, big, -big, 1e-45, -1e-45, 2.0 ** -126, 3e38, np.nextafter(np.float32(literal), np.float32(2))]
+    with np.errstate(all="ignore"):
+        want = v / np.float32(literal)
+    got, _ = run_device(device, r, {"x": v}, options=options)
+    got = got["y"].reshape(-1)
+    same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
+    assert same.all(), (int((~same).sum()), v[~same][:4], got[~same][:4], want[~same][:4])
+
+
 @pytest.mark.parametrize("shape", [(1000, 10), (8192, 27), (300, 1000)])
 @pytest.mark.parametrize("options", [None, "fuse=0 coop=0"])
 def test_argmax_bit_exact(device, shape, options):
