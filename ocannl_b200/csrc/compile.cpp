@@ -2563,9 +2563,7 @@ struct Builder {
     for (size_t a = 1; a < inner.size(); ++a) o << "        }\n";
     o << "      }\n";
     if (op.split) {
-      o << "      b200_u32 w[4];\n#pragma unroll\n      for (int e = 0; e < 4; ++e) {\n        const float hi = b200_tf32(v[e]);\n"
-        << "        w[e] = __float_as_uint(sg == 1" << S << " ? b200_tf32(v[e] - hi) : hi);\n      }\n"
-        << "      " << dst << "[i] = make_uint4(w[0], w[1], w[2], w[3]);\n";
+      o << "      " << dst << "[i] = b200_tf32_parts(v, sg == 1" << S << ");\n";
     } else if (eb == 4) {
       o << "      " << dst << "[i] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));\n";
     } else {

@@ -149,11 +149,36 @@ __device__ __forceinline__ float b200_tanh_fast(float x) {
   return y;
 }
 
-// the nearest tf32 value (the low 13 bits of the result are zero)
+// the nearest tf32 value of a finite one, halves away from zero (the low 13 bits of the result are zero); what lies
+// beyond the largest tf32 value by half a place or more becomes infinite
 __device__ __forceinline__ float b200_tf32(float f) {
-  b200_u32 u;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(f));
-  return __uint_as_float(u & 0xFFFFE000u);
+  return __uint_as_float((__float_as_uint(f) + 0x1000u) & 0xFFFFE000u);
+}
+// A single-precision value as two tf32 parts: hi + lo = f to 2^-22 (below 2^-114, where the parts of a part fall
+// below the normal range, to 2^-136), and products are formed as hi hi + hi lo + lo hi.
+// Both parts of a finite value that would round up to infinity are truncated instead.  An infinity or NaN is the lo
+// part, behind a hi part of one with its sign: whatever the other factor is -- finite, zero, infinite, undefined --
+// its hi part meets the lo part, and the sum of the three products is what the single product would be.
+__device__ __forceinline__ float b200_tf32_extreme(float f, bool lo) {
+  const float a = fabsf(f);
+  if (a < 0x1.ffep+127f) return lo ? b200_tf32(f - b200_tf32(f)) : b200_tf32(f);
+  const float hi = a < B200_INF ? __uint_as_float(__float_as_uint(f) & 0xFFFFE000u) : copysignf(1.0f, f);
+  return !lo ? hi : a < B200_INF ? __uint_as_float(__float_as_uint(f - hi) & 0xFFFFE000u) : f == f ? f : B200_NAN;
+}
+// four values' hi or lo parts; extreme ones are seen to together, behind one branch
+__device__ __forceinline__ uint4 b200_tf32_parts(const float* v, bool lo) {
+  float w[4];
+  bool plain = true;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    plain = plain && fabsf(v[e]) < 0x1.ffep+127f;
+    w[e] = b200_tf32(v[e] - (lo ? b200_tf32(v[e]) : 0.0f));
+  }
+  if (!plain) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = b200_tf32_extreme(v[e], lo);
+  }
+  return make_uint4(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), __float_as_uint(w[3]));
 }
 __device__ __forceinline__ b200_u32 b200_bits32(float f) { return __float_as_uint(f); }
 __device__ __forceinline__ b200_u32 b200_bits32(b200_u32 u) { return u; }

@@ -119,6 +119,35 @@ def test_convolution_gradients_by_windows(device, cfg, prec):
         np.testing.assert_allclose(g, w, rtol=2e-2 if prec != "single" else 1e-4, atol=(2e-2 if prec != "single" else 1e-5) * scale, err_msg=name)
 
 
+def test_extreme_values_in_two_parts(device):
+    """A two-part product keeps what single precision has: an infinite operand times a finite one is infinite,
+    infinity times zero and anything with a NaN is NaN, infinities of either sign in one sum are NaN, and
+    values next to the largest float multiply like any other."""
+    m, n, k = 130, 77, 333
+    ir = _mm(1, m, n, k, "single", False, False, act=False)
+    inputs = _inputs(ir, k)
+    x, w = inputs["x"].reshape(m, k), inputs["w"].reshape(n, k)
+    big = np.finfo(np.float32).max
+    x[0, 5], x[1, 332], x[2, 7], x[3, 0] = np.inf, -np.inf, np.nan, np.inf
+    x[3, 1] = -np.inf                                # of both signs in one row
+    w[4, 5] = 0.0                                    # meets the first infinity
+    w[6, 9] = np.inf                                 # an infinity on the other side, and one that meets an infinity
+    x[8, 9] = -np.inf
+    x[9, :], x[10, :], x[11, :] = 0.0, 0.0, 0.0
+    x[9, 3], x[10, 3], x[11, 3] = big, np.nextafter(big, np.float32(0)), -big * np.float32(1 - 2.0 ** -12)
+    w[:, 3] = np.random.default_rng(2).uniform(0.1, 0.9, n).astype(np.float32)
+    w[12, 3], w[13, 3] = 1.0, 1e-34
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert info["stages"][-1]["kind"] == "gemm" and "tf32 pairs" in info["stages"][0]["note"], info
+    g, w_ = got["y"].reshape(m, n).astype(np.float64), want["y"].reshape(m, n).astype(np.float64)
+    assert np.array_equal(np.isnan(g), np.isnan(w_)), np.argwhere(np.isnan(g) != np.isnan(w_))[:4]
+    inf = np.isinf(w_) | np.isinf(g)
+    assert np.array_equal(g[inf], w_[inf]), (np.argwhere(inf & (g != w_))[:4], g[inf & (g != w_)][:4], w_[inf & (g != w_)][:4])
+    fin = np.isfinite(w_)
+    assert (np.abs(g[fin] - w_[fin]) <= 2e-6 + 1e-5 * np.abs(w_[fin])).all()
+
+
 @pytest.mark.parametrize("classes", [4, 8, 10, 16])
 def test_classifier_widths(device, classes):
     """Logits that leave through a tensor map (rows of whole 16 bytes) and rows behind them that leave as one
