@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <thread>
@@ -455,6 +456,12 @@ int b200_compile(const char* name, const char* ir, size_t len, const char* optio
         else if (k == "tf32") opt.enable_tf32 = on;
         else if (k == "large_models") opt.large_models = on;
         else if (k == "bounds") opt.bounds = on;
+        else if (k == "gather_mb") {
+          char* end = nullptr;
+          opt.gather_mb = strtoll(v.c_str(), &end, 10);
+          if (v.empty() || *end || opt.gather_mb < 0 || opt.gather_mb > (1ll << 20))
+            throw Error(B200_E_INVALID, "compile option gather_mb takes a number of megabytes up to 1048576, got '" + v + "'");
+        }
         else throw Error(B200_E_INVALID, "unknown compile option '" + k + "'");
       }
     }

@@ -2452,6 +2452,7 @@ struct Builder {
       }
       (&op == &g.gemm.packs[0] && g.gemm.pack_a ? g.gemm.a_slot : g.gemm.b_slot) = slot;
     }
+    g.copies = g.gemm.pack_a || g.gemm.pack_b;
     if (todo.empty()) return;
     Stage st;
     st.kind = Stage::Generic;
@@ -2653,7 +2654,7 @@ struct Builder {
       (ix == last_in_x ? second : first).push_back(d);
       elems *= d.extent();
     }
-    if (first.empty() || second.empty() || red.empty() || elems * 4 > (1ll << 30) || elems >= (1ll << 31)) return false;
+    if (first.empty() || second.empty() || red.empty() || elems * 4 > (std::min<int64_t>(opt.gather_mb, 1024) << 20) || elems >= (1ll << 31)) return false;
     // a few hundred multiplications per gathered row do not pay for the gathering (see the convolutions' windows in
     // match_gemm): 8 outputs of 3 x 3 on one channel, 262144 positions: 9 us as scattered additions, 49 us as this
     {
@@ -2729,6 +2730,7 @@ struct Builder {
     }
     kept_stmts.push_back(product);
     pack_stage(g);
+    g.copies = true;
     g.kernel = kernel_name();
     g.gemm_source = gemm_translation_unit(code.prog, g, g.kernel, opt);
     code.stages.push_back(g);

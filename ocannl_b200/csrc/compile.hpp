@@ -140,6 +140,7 @@ struct Stage {
   std::vector<int> origins;      // indices of the routine's top-level statements this stage runs
   std::vector<int> writes;       // nodes the stage writes
   std::vector<int> pack_writes;  // slots of packed operands the stage fills
+  bool copies = false;           // a contraction with gathered operands or a window node: its statement also has a form without scratch
 };
 
 // A loop nest that follows a contraction and may be folded into its epilogue.
@@ -171,6 +172,9 @@ struct CompileOptions {
   bool enable_tf32 = true;   // single-precision operands of a contraction go through the tensor cores as tf32
   bool exact_single = false; // (planner only) single-precision operands keep their precision: as tf32 pairs
   bool large_models = false;
+  // What a contraction may copy into the routine's scratch, in MB: each gathered operand, each node of windows of an
+  // input gradient (at most 1024 of those).  Contractions that would take more run on the generic kernels.
+  int64_t gather_mb = 2048;
   // Range-checked build: every access a generated kernel makes to a node is checked against the node's
   // size; an access outside it is skipped and reported through the device status word.  Implies the
   // generic kernels (no tensor-core stages, no pair or register-row forms).
@@ -178,7 +182,8 @@ struct CompileOptions {
   // Top-level statements (by index) that must not use the forms with alignment demands: the pair
   // form of generic stages (8-byte accesses) / the TMA-fed contraction kernel (16-byte operand
   // bases).  Filled when a routine is linked to buffers at element-size-aligned offsets, as
-  // `Raise_backend.allocate_delta` hands them out (arrayjit/lib/backends.ml:529-614).
+  // `Raise_backend.allocate_delta` hands them out (arrayjit/lib/backends.ml:529-614), or when the device
+  // has no room for the copies a contraction wants.
   std::set<int> no_pairs_at, no_gemm_at;
 };
 

@@ -457,7 +457,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
         const int64_t unit = 16 / eb, parts = split ? 2 : 1;
         const int64_t mn_extent = of_a ? g.m.extent : g.n.extent;
         op.ld = kmajor ? (op.seg * parts + unit - 1) / unit * unit : (mn_extent + unit - 1) / unit * unit;
-        if (op.bytes() > (2ll << 30)) return false;   // the copy would cost more memory than it is worth
+        if (op.bytes() > (opt.gather_mb << 20)) return false;   // the copy would cost more memory than it is worth
         s_mn = kmajor ? op.ld : 1;
         s_k = kmajor ? 1 : op.ld;
         s_b = (kmajor ? mn_extent : op.seg * parts) * op.ld;

@@ -98,6 +98,35 @@ static bool misaligned_stages(const b200_code* c, const std::map<int, CUdevicept
   return any;
 }
 
+// Lays out the scratch slab of `code`: routine-local nodes, partial results of reductions, packed operands.
+void b200_routine::place_scratch(std::map<int, size_t>* local_off) {
+  const Program& P = code->code.prog;
+  size_t off = 0;
+  local_off->clear();
+  scratch_zero.clear();
+  for (int id : code->code.local_nodes) {
+    const Tnode& t = P.tn(id);
+    (*local_off)[id] = off;
+    if (t.zero_init) scratch_zero.push_back({off, (size_t)t.bytes()});
+    off += ((size_t)t.bytes() + 255) & ~(size_t)255;
+  }
+  // neighbouring zero ranges become one memset (the padding between nodes may be cleared too)
+  std::vector<std::pair<size_t, size_t>> merged;
+  for (auto& z : scratch_zero) {
+    if (!merged.empty() && merged.back().first + merged.back().second + 256 >= z.first)
+      merged.back().second = z.first + z.second - merged.back().first;
+    else
+      merged.push_back(z);
+  }
+  scratch_zero.swap(merged);
+  reduce_base = off;
+  off += code->code.reduce_scratch_bytes;
+  off = (off + 255) & ~(size_t)255;
+  pack_base = off;
+  off += code->code.pack_scratch_bytes;
+  scratch_bytes = off;
+}
+
 void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n) {
   dev = d;
   requested = c;
@@ -116,49 +145,32 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
                                       ", not a multiple of its element size");
     param_ptr[t.id] = d->address(it->second->pool_id, it->second->offset, (size_t)t.bytes());
   }
-  {
-    std::set<int> no_pairs_at = c->opt.no_pairs_at, no_gemm_at = c->opt.no_gemm_at;
+  std::set<int> no_pairs_at = c->opt.no_pairs_at, no_gemm_at = c->opt.no_gemm_at;
+  std::map<int, size_t> local_off;
+  for (;;) {
     b200_code* use = c;
+    if (no_pairs_at != c->opt.no_pairs_at || no_gemm_at != c->opt.no_gemm_at) use = c->variant(no_pairs_at, no_gemm_at);
     for (int round = 0; round < 4 && misaligned_stages(use, param_ptr, &no_pairs_at, &no_gemm_at); ++round)
       use = c->variant(no_pairs_at, no_gemm_at);
-    c = use;
+    code = use;
+    place_scratch(&local_off);
+    if (!scratch_bytes) break;
+    const CUresult r = cu().cuMemAlloc_(&scratch, scratch_bytes);
+    if (r == CUDA_SUCCESS) break;
+    scratch = 0;
+    // No room: the contractions whose operands (or windows) are copied into scratch also run without, on the
+    // generic kernels -- slower, but the routine links.
+    const size_t had = no_gemm_at.size();
+    if (r == CUDA_ERROR_OUT_OF_MEMORY)
+      for (auto& st : code->code.stages)
+        if (st.copies) no_gemm_at.insert(st.origins.begin(), st.origins.end());
+    if (no_gemm_at.size() == had) cu_check(r, "cuMemAlloc(scratch)");
   }
-  code = c;
+  c = code;
   const Program& P = c->code.prog;
-
-  // routine-local nodes live in a scratch slab owned by the routine
-  size_t off = 0;
-  std::map<int, size_t> local_off;
-  for (int id : c->code.local_nodes) {
-    const Tnode& t = P.tn(id);
-    local_off[id] = off;
-    if (t.zero_init) scratch_zero.push_back({off, (size_t)t.bytes()});
-    off += ((size_t)t.bytes() + 255) & ~(size_t)255;
-  }
-  // neighbouring zero ranges become one memset (the padding between nodes may be cleared too)
-  {
-    std::vector<std::pair<size_t, size_t>> merged;
-    for (auto& z : scratch_zero) {
-      if (!merged.empty() && merged.back().first + merged.back().second + 256 >= z.first)
-        merged.back().second = z.first + z.second - merged.back().first;
-      else
-        merged.push_back(z);
-    }
-    scratch_zero.swap(merged);
-  }
-  const size_t reduce_off = off;
-  reduce_base = off;
-  off += c->code.reduce_scratch_bytes;
-  off = (off + 255) & ~(size_t)255;
-  pack_base = off;
-  off += c->code.pack_scratch_bytes;
-  scratch_bytes = off;
-  if (scratch_bytes) {
-    cu_check(cu().cuMemAlloc_(&scratch, scratch_bytes), "cuMemAlloc(scratch)");
-    // the tickets of grid-wide reductions start at zero (each kernel resets its own afterwards)
-    if (c->code.reduce_scratch_bytes)
-      cu_check(cu().cuMemsetD8Async_(scratch + reduce_off, 0, c->code.reduce_scratch_bytes, d->stream), "cuMemsetD8Async(reduce scratch)");
-  }
+  // the tickets of grid-wide reductions start at zero (each kernel resets its own afterwards)
+  if (c->code.reduce_scratch_bytes)
+    cu_check(cu().cuMemsetD8Async_(scratch + reduce_base, 0, c->code.reduce_scratch_bytes, d->stream), "cuMemsetD8Async(reduce scratch)");
 
   for (auto& t : P.tnodes) {
     if (t.mode == Mode::Local) node_ptr[t.id] = scratch + local_off[t.id];
@@ -212,7 +224,7 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
       } else if (a.kind == KArg::Statics) {
         arg_values[i].push_back(statics_dev);
       } else if (a.kind == KArg::Scratch) {
-        arg_values[i].push_back(scratch + reduce_off + (size_t)a.tn);
+        arg_values[i].push_back(scratch + reduce_base + (size_t)a.tn);
       } else if (a.kind == KArg::StaticValues) {
         arg_values[i].push_back(0);   // (the launch passes static_values)
       } else if (a.kind == KArg::Pack) {

@@ -174,6 +174,7 @@ struct b200_routine {
   std::set<int> pools_used;   // pools of the bound nodes (what a launch has to wait for, uploads-wise)
   b200_code* requested = nullptr;  // the code `link` was given; `code` may be a variant of it
   void link(b200_dev* d, b200_code* c, const b200_binding* b, int n);
+  void place_scratch(std::map<int, size_t>* local_off);
   void launch(const int64_t* static_idx, int n_static);
   void enqueue_stages(bool capturing = false);
   void set_graph(bool on);

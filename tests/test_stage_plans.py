@@ -178,3 +178,20 @@ def test_attention_stage_writes_a_local_node_that_a_later_statement_reads():
     st = _plan(ir)
     notes = [x["note"] for x in st if x["kind"] == "attention"]
     assert notes and "1 of the 3 row nodes written" in notes[0], [x["note"] for x in st]
+
+
+def test_copies_of_operands_stay_within_the_stated_size():
+    """`gather_mb`: contractions whose gathered operands, or windows of an input gradient, would take more
+    scratch are planned on the generic kernels."""
+    ir = lambda: W.conv2d_update(batch=32, size=32, cin=16, cout=16, kernel=5)    # windows of 105 MB in two parts, 52 MB of gradient
+    def copies(options):
+        notes = [s["note"] or "" for s in _plan(ir(), options)]
+        return sum("gathers operands" in n for n in notes), sum("gathers the windows" in n for n in notes)
+    gathered, windows = copies(None)
+    assert gathered >= 2 and windows == 1
+    assert copies("gather_mb=2048") == (gathered, windows)
+    assert copies("gather_mb=64") == (1, 1)          # the gradient of the input only
+    assert copies("gather_mb=16") == (0, 0)
+    for bad in ("gather_mb=", "gather_mb=-1", "gather_mb=x", "gather_mb=1e3"):
+        with pytest.raises(bk.B200Error):
+            bk.Code(ir(), bad)
