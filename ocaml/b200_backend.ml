@@ -294,6 +294,11 @@ module Fresh () : Backend_impl.Lowered_backend = struct
              | "" -> None
              | v -> Some (k ^ "=" ^ if String.(v = "true" || v = "1") then "1" else "0"))
        in
+       let set =
+         match Utils.get_global_arg ~default:"" ~arg_name:"b200_gather_mb" with
+         | "" -> set
+         | mb -> ("gather_mb=" ^ mb) :: set
+       in
        let set = if Utils.settings.large_models then "large_models=1" :: set else set in
        if List.is_empty set then None else Some (String.concat ~sep:" " set))
 
