@@ -1338,8 +1338,8 @@ struct Builder {
   // Nodes small enough live in shared memory for the length of the block: read once at its start, written
   // back at its end, and routine-local ones that no other stage touches never reach memory at all.  A stage
   // then waits some 30 cycles for what the one before it wrote instead of some 300.  The barrier
-  // between two stages is left out when neither writes what the other touches; a sum with few outputs
-  // (a gradient over the batch) is shared by as many lanes of a warp as there are.  (The 25 stages of the
+  // between two stages is left out when neither writes what the other touches; a long sum with few outputs
+  // (a gradient over the batch) is shared by up to four lanes of a warp.  (The 25 stages of the
   // 2-16-16-1 training step: 11.6 us through memory.)
   std::map<int, std::set<size_t>> node_stages;   // node -> stages that touch it, by index into code.stages
   void note_node_stages() {
@@ -1358,6 +1358,29 @@ struct Builder {
         for (int n : {st.attn.q_tn, st.attn.k_tn, st.attn.v_tn}) node_stages[n].insert(i);
       for (int n : st.writes) node_stages[n].insert(i);
     }
+  }
+
+  // Short innermost loops of a known number of steps are unrolled 32 times: one block has too few warps to hide
+  // the latency of a load per step, and how far the compiler unrolls by itself changes with the size of the kernel
+  // around the loop (64 points through 2-64-64-1: 26.7 us or 30.7; 150 through 2-40-40-1: 41.0, 33.1 so).
+  static std::string unrolled(const std::string& text) {
+    std::vector<std::string> lines;
+    std::istringstream in(text);
+    for (std::string line; std::getline(in, line);) lines.push_back(line);
+    std::string out;
+    for (size_t i = 0; i < lines.size(); ++i) {
+      const size_t at = lines[i].find_first_not_of(' ');
+      if (at != std::string::npos && lines[i].compare(at, 4, "for ") == 0 && lines[i].back() == '{' &&
+          (lines[i].find(" <= ") != std::string::npos || lines[i].find("b200_k < ") != std::string::npos)) {
+        size_t j = i + 1;
+        while (j < lines.size() && lines[j].find("for (") == std::string::npos && lines[j].find_first_not_of(' ') != std::string::npos &&
+               lines[j][lines[j].find_first_not_of(' ')] != '}')
+          ++j;
+        if (j < lines.size() && j - i <= 9 && lines[j].find("for (") == std::string::npos) out += "#pragma unroll 32\n";
+      }
+      out += lines[i] + "\n";
+    }
+    return out;
   }
 
   Stage emit_fused(const std::vector<size_t>& idx) {
@@ -1443,28 +1466,38 @@ struct Builder {
           });
         int64_t ser_total = 1;
         for (auto& d : pc.ser) ser_total *= d.extent();
-        int64_t share = 1;   // lanes per sum
+        // Lanes per sum: two or four, 16 steps each at least.  Neighbouring lanes keep neighbouring outputs, so that a
+        // step reads stretches of a row.  (Training steps of points x hidden units, us.  No sharing, up to 4 lanes, up
+        // to 32: 200 x 16 23.1, 18.5, 23.0; 100 x 100 35.0, 30.7, 30.9; 8 x 128 16.8, 17.2, 19.4; 64 x 64 26.7, 28.7, 34.9;
+        // with two steps a lane 12 x 112 takes 22.0 instead of 18.8.)
+        int64_t share = 1;
         if (pc.sum)
-          while (share < 32 && share * 2 * st.total <= 1024 && share * 4 <= ser_total) share *= 2;
+          while (share < 4 && share * 2 * st.total <= 1024 && share * 32 <= ser_total) share *= 2;
         most = std::max<int64_t>(most, st.total * std::max(1, st.coop));
         if (share > 1) {
           ordered = true;
-          const std::string S = std::to_string(share) + "u";
-          text += "  {\n  const unsigned int b200_s = threadIdx.x % " + S + ", b200_gq = threadIdx.x / " + S + ";\n  const bool b200_on = b200_gq < " +
+          const std::string S = std::to_string(share) + "u", O = std::to_string(32 / share) + "u";
+          text += "  {\n  const unsigned int b200_s = threadIdx.x % 32u / " + O + ", b200_gq = threadIdx.x / 32u * " + O + " + threadIdx.x % " + O + ";\n  const bool b200_on = b200_gq < " +
                   std::to_string(st.total) + "u;\n  const unsigned int b200_g = b200_on ? b200_gq : 0u;\n" + pc.decomp + "    " + pc.self_type + " b200_self = " +
-                  pc.zero + ";\n    if (b200_on) {\n      if (b200_s == 0u) b200_self = " + pc.self_init + ";\n      for (unsigned int b200_l = b200_s; b200_l < " +
-                  std::to_string(ser_total) + "u; b200_l += " + S + ") {\n";
-          std::string rem = "b200_l";
+                  pc.zero + ";\n    if (b200_on) {\n      if (b200_s == 0u) b200_self = " + pc.self_init + ";\n";
+          std::string term, rem = "b200_l";
           for (size_t q = pc.ser.size(); q-- > 0;) {
             const LoopDim& d = pc.ser[q];
             const std::string ext = std::to_string(d.extent()) + "u";
-            text += "        const unsigned int " + d.sym + " = " + (q == 0 ? rem : rem + " % " + ext) + (d.from ? " + " + std::to_string(d.from) + "u" : std::string()) + ";\n";
+            term += "        const unsigned int " + d.sym + " = " + (q == 0 ? rem : rem + " % " + ext) + (d.from ? " + " + std::to_string(d.from) + "u" : std::string()) + ";\n";
             if (q) {
-              text += "        const unsigned int b200_lq" + std::to_string(q) + " = " + rem + " / " + ext + ";\n";
+              term += "        const unsigned int b200_lq" + std::to_string(q) + " = " + rem + " / " + ext + ";\n";
               rem = "b200_lq" + std::to_string(q);
             }
           }
-          text += pc.inner + "      }\n    }\n#pragma unroll\n    for (unsigned int b200_o = 1u; b200_o < " + S + "; b200_o <<= 1) ";
+          term += pc.inner;
+          // (a number of steps that is the same for every lane, and known: the loads of many steps are under way together)
+          text += "      for (unsigned int b200_k = 0; b200_k < " + std::to_string(ser_total / share) + "u; ++b200_k) {\n        const unsigned int b200_l = b200_k * " + S +
+                  " + b200_s;\n" + term + "      }\n";
+          if (ser_total % share)
+            text += "      if (b200_s < " + std::to_string(ser_total % share) + "u) {\n        const unsigned int b200_l = " + std::to_string(ser_total / share * share) +
+                    "u + b200_s;\n" + term + "      }\n";
+          text += "    }\n#pragma unroll\n    for (unsigned int b200_o = " + O + "; b200_o < 32u; b200_o <<= 1) ";
           if (pc.pairs)
             text += "{\n      const b200_f2 b200_w = {__shfl_xor_sync(0xffffffffu, b200_self.x, b200_o), __shfl_xor_sync(0xffffffffu, b200_self.y, b200_o)};\n"
                     "      b200_self = b200_f2{b200_self.x + b200_w.x, b200_self.y + b200_w.y};\n    }\n";
@@ -1486,6 +1519,7 @@ struct Builder {
     // Stages that do not depend on one another (the updates of several parameters, the margins of a padded
     // image) need no single block: every stage is spread over the whole grid.
     const bool wide = !ordered && most > 1024;
+    if (!wide) text = unrolled(text);
     {
       auto put = [&](const std::string& what, const std::string& by) {
         for (size_t q = 0; (q = text.find(what, q)) != std::string::npos; q += by.size()) text.replace(q, what.size(), by);

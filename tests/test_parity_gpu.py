@@ -212,6 +212,21 @@ def test_moons_steps_with_cleared_nodes_in_memory(device, graph, batch, hid):
     compare(ir, got, want, rtol=rtol, atol=rtol)
 
 
+@pytest.mark.parametrize("batch,hid", [(63, 9), (64, 64), (67, 9), (150, 40), (131, 33)])
+def test_moons_sums_shared_by_lanes(device, batch, hid):
+    """Sums over the batch inside the block of small stages: too short to be shared by lanes, shared by two or
+    four, with and without points left over; odd widths.  Tolerance as above."""
+    ir = W.moons_train_step(n_batches=1024 // batch, batch=batch, hid=hid)
+    x, y = W.moons_inputs(batch=batch)
+    inputs = dict(W.moons_params(hid=hid), moons_flat=x, moons_classes=y)
+    statics = [{"i1": 0, "i2": 0}, {"i1": 3, "i2": 1}]
+    want = run_oracle(ir, inputs, statics)
+    got, info = run_device(device, ir, inputs, statics)
+    assert any("small stages in one block" in s["note"] for s in info["stages"]), info
+    rtol = 16 * np.sqrt(batch) * 2.0 ** -24
+    compare(ir, got, want, rtol=rtol, atol=rtol)
+
+
 def test_moons_static_index_errors(device):
     from ocannl_b200 import backend as bk
     ir = W.moons_train_step()
