@@ -137,6 +137,21 @@ def merge_add(n: int, prec: str = "single") -> Routine:
     return r
 
 
+def merge_add_chain(n: int, kernels: int) -> Routine:
+    """`merge_add` followed by statements over other lengths that each keep a kernel of their own under `fuse=0`:
+    c_k := a[0] + k, twice as long as the one before it."""
+    r = merge_add(n)
+    r.name = "merge_add_%d_chain_%d" % (n, kernels)
+    a = r.tnodes[0]
+    body = [r.body]
+    for k in range(1, kernels):
+        c = r.tn("c%d" % k, "single", [2 << k])
+        i = r.sym()
+        body.append(For(i, 0, (2 << k) - 1, Set(c, (i,), a[0] + float(k))))
+    r.body = Seq(body)
+    return r
+
+
 # ------------------------------------------------------------------ the reference's printed known answers
 def range_of_shape(dims) -> np.ndarray:
     """`TDSL.range_of_shape`: 0, 1, 2, ... in row-major order."""

@@ -175,9 +175,9 @@ def test_local_shared_inside_a_loop_body(device):
 
 
 # ------------------------------------------------------------------ merge buffer, copies, stream order
-def _linked_merge_add(device, n, graph):
-    ir = R.merge_add(n)
-    code = bk.Code(ir)
+def _linked_merge_add(device, n, graph, kernels=1):
+    ir = R.merge_add(n) if kernels == 1 else R.merge_add_chain(n, kernels)
+    code = bk.Code(ir, None if kernels == 1 else "fuse=0")
     rt = bk.Context(device).link(code)
     if graph:
         rt.use_graph(True)
@@ -200,28 +200,36 @@ def test_merge_buffer_known_answer(device, graph):
     _free(device, rt, code)
 
 
-def test_graph_replay_follows_a_merge_buffer_that_grew(device):
+@pytest.mark.parametrize("kernels", [1, 6])
+def test_graph_replay_follows_a_merge_buffer_that_grew(device, kernels):
     """A captured graph holds the merge buffer's address; when a larger copy makes the buffer grow
-    (a new slab), the next run must read the new one."""
-    small_ir, small_code, small = _linked_merge_add(device, 2, True)
-    big_ir, big_code, big = _linked_merge_add(device, 1 << 16, True)
-    src = device.alloc_pool(4 << 16)
+    (a new slab), the next run must read the new one.  Six kernels are captured; one is launched as it is
+    and reads the address at each launch."""
+    n_big = 1 << (16 + kernels)                   # (larger than what any other test here has left behind)
+    small_ir, small_code, small = _linked_merge_add(device, 2, True, kernels)
+    big_ir, big_code, big = _linked_merge_add(device, n_big, True, kernels)
+    assert small.kernels_per_run() == kernels
+    graphs = device.get_debug_info()["graph_launches"]
+    src = device.alloc_pool(4 * n_big)
     device.from_host(src, 0, np.float32([3, 4]))
     small.context.from_host("a", np.float32([1, 2]))
     device.merge_copy(device, src, 0, 8)
-    small.run()                                   # captures with the small merge slab
+    small.run()
     assert list(small.context.to_host("a")) == [4.0, 6.0]
+    small.run()                                   # holds a graph with the small merge slab by now
+    assert (device.get_debug_info()["graph_launches"] > graphs) == (kernels > 4)
+    assert list(small.context.to_host("a")) == [7.0, 10.0]
     before = device.pool_address(0)
-    ones = np.ones(1 << 16, np.float32)
+    ones = np.ones(n_big, np.float32)
     device.from_host(src, 0, ones * 5)
     big.context.from_host("a", ones)
-    device.merge_copy(device, src, 0, 4 << 16)    # grows pool 0: new slab
+    device.merge_copy(device, src, 0, 4 * n_big)   # grows pool 0: new slab
     big.run()
     assert np.array_equal(big.context.to_host("a"), ones * 6)
     assert device.pool_address(0) != before
     device.merge_copy(device, src, 0, 8)          # [5 5] into the grown buffer
     small.run()                                   # replay: must not read the freed slab
-    assert list(small.context.to_host("a")) == [9.0, 11.0]
+    assert list(small.context.to_host("a")) == [12.0, 15.0]
     device.free_pool(src)
     _free(device, small, small_code)
     _free(device, big, big_code)
