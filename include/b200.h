@@ -128,6 +128,9 @@ int b200_routine_info(b200_routine* r, char* json, size_t cap);   /* like b200_c
  * of the routine, in declaration order; a negative or out-of-range value is B200_E_USER
  * (cuda: arrayjit/lib/cuda_backend.ml:1015-1030). */
 int b200_launch(b200_routine* r, const int64_t* static_idx, int n_static);
+/* Replays the routine's launches as one captured graph from its second run on (the first is launched
+ * directly).  Routines of up to four kernels that clear no node, and those whose only kernel takes the
+ * static indices as an argument, are launched directly all the same: a graph would only add its own time. */
 int b200_routine_use_graph(b200_routine* r, int enable);
 int b200_routine_launch_count(b200_routine* r, int64_t* kernels_per_run);
 /* Per-stage device timing (CUDA events around every stage of the next runs; disables graph

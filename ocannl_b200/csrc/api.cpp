@@ -745,7 +745,7 @@ int b200_routine_overlap_allreduce(b200_routine* r, b200_comm* comm, int n, cons
       if (b.done) cu().cuEventDestroy_(b.done);
     }
     r->buckets.clear();
-    r->overlap_warm = false;
+    r->warm = false;
     if (r->overlap_comm) r->overlap_comm->routines.erase(r);
     r->overlap_comm = n > 0 ? comm : nullptr;
     if (n > 0) comm->routines.insert(r);

@@ -549,11 +549,12 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
       }
     }
   }
-  // The first run with collectives attached is queued directly: NCCL sets up the connections a
-  // collective needs the first time it runs (allocations, exchanges with the peers), which must
-  // not happen inside a stream capture.  Later runs capture and replay.
-  const bool capture_ok = buckets.empty() || overlap_warm;
-  if (!buckets.empty()) overlap_warm = true;
+  // The first run is queued directly; later runs capture and replay.  With collectives attached it has to be: NCCL sets
+  // up the connections a collective needs the first time it runs (allocations, exchanges with the peers), which must
+  // not happen inside a stream capture.  And making a graph takes as long as several runs (17 stages on four branches:
+  // 0.55 ms, of which 0.47 instantiate it, for runs of 0.15 ms), which a routine that runs once need not wait for.
+  const bool capture_ok = warm;
+  warm = true;
   if (want_graph && !direct && !profiling && capture_ok) {
     if (graph && reads_merge && graph_merge_epoch != dev->merge_epoch) {
       // the merge buffer moved since the capture (`b200_merge_copy` grew pool 0): the graph holds

@@ -155,7 +155,7 @@ struct b200_routine {
 
   b200_comm* overlap_comm = nullptr;
   std::vector<OverlapBucket> buckets;
-  bool overlap_warm = false;      // the attached collectives have run once outside a capture
+  bool warm = false;              // the routine, and the collectives attached to it, have run once outside a capture
   void enqueue_bucket(OverlapBucket& b);
   // Where the next stage is queued: the device's stream, or -- while a graph is being captured -- the branch
   // the stage belongs to; and whether its launch may start before the one ahead of it in that stream ends.

@@ -214,9 +214,10 @@ def test_graph_replay_follows_a_merge_buffer_that_grew(device, kernels):
     device.from_host(src, 0, np.float32([3, 4]))
     small.context.from_host("a", np.float32([1, 2]))
     device.merge_copy(device, src, 0, 8)
-    small.run()
+    small.run()                                   # the first run is launched directly
+    assert device.get_debug_info()["graph_launches"] == graphs
     assert list(small.context.to_host("a")) == [4.0, 6.0]
-    small.run()                                   # holds a graph with the small merge slab by now
+    small.run()                                   # captures with the small merge slab
     assert (device.get_debug_info()["graph_launches"] > graphs) == (kernels > 4)
     assert list(small.context.to_host("a")) == [7.0, 10.0]
     before = device.pool_address(0)
