@@ -195,3 +195,12 @@ def test_copies_of_operands_stay_within_the_stated_size():
     for bad in ("gather_mb=", "gather_mb=-1", "gather_mb=x", "gather_mb=1e3"):
         with pytest.raises(bk.B200Error):
             bk.Code(ir(), bad)
+
+
+def test_units_compiled_side_by_side_report_a_failure(monkeypatch):
+    """The kernels of a routine are compiled on several threads; a failure on any of them is the call's."""
+    monkeypatch.setenv("B200_NVRTC_FLAGS", "--no-such-option")
+    with pytest.raises(bk.B200Error, match="NVRTC failed to compile"):
+        bk.Code(W.mlp_forward(rows=96))
+    monkeypatch.delenv("B200_NVRTC_FLAGS")
+    assert len(_plan(W.mlp_forward(rows=96))) >= 3
