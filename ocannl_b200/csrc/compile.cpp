@@ -2511,7 +2511,7 @@ struct Builder {
       const int64_t first = total;
       total += op.rows() * op.ld * prec_bytes(op.prec) / 16;
       body << "    " << (i ? "else " : "") << "if (b200_g < " << total << "ull) {\n" << pack_body(op, dst, first) << "    }\n";
-      what += (i ? ", " : "") + code.prog.tn(op.tn).ident;
+      what += (i ? ", " : "") + code.prog.tn(op.tn).label;
     }
     st.total = total;
     st.note = "gathers operands of the next contraction into padded rows" + std::string(g.gemm.tf32_pairs ? " (tf32 pairs)" : "") + ": " + what;
@@ -2529,8 +2529,8 @@ struct Builder {
     const bool narrow = first + op.rows() * groups < (1ll << 31) && code.prog.tn(op.tn).num_elems() < (1ll << 31);
     const std::string IT = narrow ? "unsigned int" : "unsigned long long", S = narrow ? "u" : "ull";
     auto num = [&](int64_t v) { return std::to_string(v) + S; };
-    o << "      const " << IT << " i = (" << IT << ")(b200_g - " << first << "ull);\n"
-      << "      const " << IT << " grp = i % " << num(groups) << ", row = i / " << num(groups) << ";\n";
+    o << "      const " << IT << " b200_i = (" << IT << ")(b200_g - " << first << "ull);\n"
+      << "      const " << IT << " b200_grp = b200_i % " << num(groups) << ", b200_row = b200_i / " << num(groups) << ";\n";
     // `at`: adds the position `var` along the axes to the variable `acc`
     int tmp = 0;
     auto at = [&](const std::vector<PackOp::Axis>& axes, std::string var, const std::string& acc, const std::string& pad) {
@@ -2539,7 +2539,7 @@ struct Builder {
         if (a == 0) {
           t += pad + acc + " += (" + var + ") * " + num(axes[a].stride) + ";\n";
         } else {
-          const std::string q = "q" + std::to_string(tmp++);
+          const std::string q = "b200_q" + std::to_string(tmp++);
           t += pad + acc + " += ((" + var + ") % " + num(axes[a].extent) + ") * " + num(axes[a].stride) + ";\n" + pad + "const " + IT + " " + q + " = (" + var +
                ") / " + num(axes[a].extent) + ";\n";
           var = q;
@@ -2555,55 +2555,55 @@ struct Builder {
     const int64_t K = extent(op.k), MN = extent(op.mn);
     const std::vector<PackOp::Axis>& inner = op.kmajor ? op.k : op.mn;
     const int64_t outer_rows = op.kmajor ? MN : op.seg * (op.split ? 2 : 1);
-    o << "      " << IT << " base = " << num(op.off) << ";\n";
-    if (!op.batch.empty()) o << "      const " << IT << " bt = row / " << num(outer_rows) << ", rr = row % " << num(outer_rows) << ";\n" << at(op.batch, "bt", "base", "      ");
-    else o << "      const " << IT << " rr = row;\n";
+    o << "      " << IT << " b200_base = " << num(op.off) << ";\n";
+    if (!op.batch.empty()) o << "      const " << IT << " b200_bt = b200_row / " << num(outer_rows) << ", b200_rr = b200_row % " << num(outer_rows) << ";\n" << at(op.batch, "b200_bt", "b200_base", "      ");
+    else o << "      const " << IT << " b200_rr = b200_row;\n";
     const int64_t inner_real = op.kmajor ? K : MN;
     std::string seg_of, in0;
     if (op.kmajor) {
-      o << at(op.mn, "rr", "base", "      ");
+      o << at(op.mn, "b200_rr", "b200_base", "      ");
       if (op.split) {
-        o << "      const " << IT << " sg = (grp * " << V << S << ") / " << num(op.seg) << ", j0 = grp * " << V << S << " - sg * " << num(op.seg) << ";\n";
+        o << "      const " << IT << " b200_sg = (b200_grp * " << V << S << ") / " << num(op.seg) << ", b200_j0 = b200_grp * " << V << S << " - b200_sg * " << num(op.seg) << ";\n";
       } else {
-        o << "      const " << IT << " j0 = grp * " << V << S << ";\n";
+        o << "      const " << IT << " b200_j0 = b200_grp * " << V << S << ";\n";
       }
-      o << "      const bool row_ok = true;\n";
+      o << "      const bool b200_row_ok = true;\n";
     } else {
-      if (op.split) o << "      const " << IT << " sg = rr / " << num(op.seg) << ", kk = rr % " << num(op.seg) << ";\n";
-      else o << "      const " << IT << " kk = rr;\n";
-      o << "      const bool row_ok = kk < " << num(K) << ";\n" << at(op.k, "kk", "base", "      ") << "      const " << IT << " j0 = grp * " << V << S << ";\n";
+      if (op.split) o << "      const " << IT << " b200_sg = b200_rr / " << num(op.seg) << ", b200_kk = b200_rr % " << num(op.seg) << ";\n";
+      else o << "      const " << IT << " b200_kk = b200_rr;\n";
+      o << "      const bool b200_row_ok = b200_kk < " << num(K) << ";\n" << at(op.k, "b200_kk", "b200_base", "      ") << "      const " << IT << " b200_j0 = b200_grp * " << V << S << ";\n";
     }
     const std::string T = Emitter::ctype(op.prec);
     // the group's elements: the first position is taken apart with divisions, the others by counting on
-    o << "      " << T << " v[" << V << "];\n      " << IT << " p = base;\n";
-    std::string rest = "j0";
+    o << "      " << T << " b200_v[" << V << "];\n      " << IT << " b200_p = b200_base;\n";
+    std::string rest = "b200_j0";
     for (size_t a = inner.size(); a-- > 0;) {
-      const std::string c = "c" + std::to_string(a);
+      const std::string c = "b200_c" + std::to_string(a);
       if (a == 0) {
-        o << "      p += (" << rest << ") * " << num(inner[a].stride) << ";\n";
+        o << "      b200_p += (" << rest << ") * " << num(inner[a].stride) << ";\n";
       } else {
-        o << "      " << IT << " " << c << " = (" << rest << ") % " << num(inner[a].extent) << ";\n      p += " << c << " * " << num(inner[a].stride) << ";\n"
-          << "      const " << IT << " r" << a << " = (" << rest << ") / " << num(inner[a].extent) << ";\n";
-        rest = "r" + std::to_string(a);
+        o << "      " << IT << " " << c << " = (" << rest << ") % " << num(inner[a].extent) << ";\n      b200_p += " << c << " * " << num(inner[a].stride) << ";\n"
+          << "      const " << IT << " b200_r" << a << " = (" << rest << ") / " << num(inner[a].extent) << ";\n";
+        rest = "b200_r" + std::to_string(a);
       }
     }
-    o << "#pragma unroll\n      for (unsigned int e = 0; e < " << V << "u; ++e) {\n"
-      << "        v[e] = row_ok && j0 + e < " << num(inner_real) << " ? " << src_name << "[p] : (" << T << ")0;\n        p += " << num(inner.back().stride) << ";\n";
+    o << "#pragma unroll\n      for (unsigned int b200_e = 0; b200_e < " << V << "u; ++b200_e) {\n"
+      << "        b200_v[b200_e] = b200_row_ok && b200_j0 + b200_e < " << num(inner_real) << " ? " << src_name << "[b200_p] : (" << T << ")0;\n        b200_p += " << num(inner.back().stride) << ";\n";
     for (size_t a = inner.size(); a-- > 1;) {
-      const std::string c = "c" + std::to_string(a);
+      const std::string c = "b200_c" + std::to_string(a);
       // carry: this axis starts over, the one outside moves on (strides are unsigned and wrap around)
-      o << "        if (++" << c << " == " << num(inner[a].extent) << ") {\n        " << c << " = 0;\n        p += " << num(inner[a - 1].stride) << " - "
+      o << "        if (++" << c << " == " << num(inner[a].extent) << ") {\n        " << c << " = 0;\n        b200_p += " << num(inner[a - 1].stride) << " - "
         << num(inner[a].extent * inner[a].stride) << ";\n";
     }
     for (size_t a = 1; a < inner.size(); ++a) o << "        }\n";
     o << "      }\n";
     if (op.split) {
-      o << "      " << dst << "[i] = b200_tf32_parts(v, sg == 1" << S << ");\n";
+      o << "      " << dst << "[b200_i] = b200_tf32_parts(b200_v, b200_sg == 1" << S << ");\n";
     } else if (eb == 4) {
-      o << "      " << dst << "[i] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));\n";
+      o << "      " << dst << "[b200_i] = make_uint4(__float_as_uint(b200_v[0]), __float_as_uint(b200_v[1]), __float_as_uint(b200_v[2]), __float_as_uint(b200_v[3]));\n";
     } else {
-      o << "      " << dst << "[i] = make_uint4((b200_u32)v[0] | ((b200_u32)v[1] << 16), (b200_u32)v[2] | ((b200_u32)v[3] << 16), "
-        << "(b200_u32)v[4] | ((b200_u32)v[5] << 16), (b200_u32)v[6] | ((b200_u32)v[7] << 16));\n";
+      o << "      " << dst << "[b200_i] = make_uint4((b200_u32)b200_v[0] | ((b200_u32)b200_v[1] << 16), (b200_u32)b200_v[2] | ((b200_u32)b200_v[3] << 16), "
+        << "(b200_u32)b200_v[4] | ((b200_u32)b200_v[5] << 16), (b200_u32)b200_v[6] | ((b200_u32)b200_v[7] << 16));\n";
     }
     return o.str();
   }
@@ -2780,14 +2780,14 @@ struct Builder {
     std::string rem = "b200_g";
     std::vector<std::string> pos(t_dims.size());
     for (size_t a = t_dims.size(); a-- > 0;) {
-      pos[a] = "p" + std::to_string(a);
+      pos[a] = "b200_p" + std::to_string(a);
       b << "    const unsigned int " << pos[a] << " = " << (a == 0 ? rem : rem + " % " + std::to_string(t_dims[a]) + "u") << ";\n";
       if (a) {
-        b << "    const unsigned int r" << a << " = " << rem << " / " << t_dims[a] << "u;\n";
-        rem = "r" + std::to_string(a);
+        b << "    const unsigned int b200_r" << a << " = " << rem << " / " << t_dims[a] << "u;\n";
+        rem = "b200_r" + std::to_string(a);
       }
     }
-    b << "    float sum = 0.0f;\n";
+    b << "    float b200_sum = 0.0f;\n";
     std::string pad = "    ", close;
     for (size_t a = 0; a < set.idcs.size(); ++a) {
       const Index& ix = set.idcs[a];
@@ -2803,20 +2803,20 @@ struct Builder {
           b << "#pragma unroll\n" << pad << "for (unsigned int " << k.second << " = 0; " << k.second << " < " << extent[k.second] << "u; ++" << k.second << ") {\n";
           pad += "  ";
           close = pad.substr(2) + "}\n" + close;
-          b << pad << "const unsigned int d" << a << " = " << pos[a] << " - " << ix.fixed << "u - " << k.second << " * " << k.first << "u;\n";
+          b << pad << "const unsigned int b200_d" << a << " = " << pos[a] << " - " << ix.fixed << "u - " << k.second << " * " << k.first << "u;\n";
         } else {
-          b << pad << "const unsigned int d" << a << " = " << pos[a] << " - " << ix.fixed << "u;\n";
+          b << pad << "const unsigned int b200_d" << a << " = " << pos[a] << " - " << ix.fixed << "u;\n";
         }
         // (a difference below zero wraps around and fails the comparison)
-        b << pad << "const unsigned int " << o.second << " = d" << a << (o.first > 1 ? " / " + std::to_string(o.first) + "u" : std::string()) << ";\n"
-          << pad << "if (" << o.second << " < " << extent[o.second] << "u" << (o.first > 1 ? " && d" + std::to_string(a) + " % " + std::to_string(o.first) + "u == 0u" : std::string()) << ") {\n";
+        b << pad << "const unsigned int " << o.second << " = b200_d" << a << (o.first > 1 ? " / " + std::to_string(o.first) + "u" : std::string()) << ";\n"
+          << pad << "if (" << o.second << " < " << extent[o.second] << "u" << (o.first > 1 ? " && b200_d" + std::to_string(a) + " % " + std::to_string(o.first) + "u == 0u" : std::string()) << ") {\n";
       }
       close = pad + "}\n" + close;
       pad += "  ";
     }
     Emitter em(code.prog);
-    b << pad << "sum += " << P.ident << "[" << em.offset(at, P.dims) << "];\n" << close
-      << "    " << t_ident << "[b200_g] = " << (was_zero ? "sum" : t_ident + "[b200_g] + sum") << ";\n";
+    b << pad << "b200_sum += " << P.ident << "[" << em.offset(at, P.dims) << "];\n" << close
+      << "    " << t_ident << "[b200_g] = " << (was_zero ? "b200_sum" : t_ident + "[b200_g] + b200_sum") << ";\n";
     src << "extern \"C\" __global__ void __launch_bounds__(256) " << st.kernel << "(float* " << t_ident << ", const float* __restrict__ " << P.ident << ") {\n" << kGridEntry
         << "  for (unsigned int b200_g = blockIdx.x * 256u + threadIdx.x; b200_g < " << t_elems << "u; b200_g += gridDim.x * 256u) {\n"
         << b.str() << "  }\n}\n\n";
@@ -3169,9 +3169,31 @@ struct Builder {
 
 }  // namespace
 
+// Kernel pointers carry the nodes' own names, and generated code keeps to names that begin with b200_.  The
+// hand-written kernels around a generated epilogue, and the functions of the attention stages, use shorter ones: a node
+// called like one of them (a bias `acc`, a row sum `sum`) gets its number as a suffix.
+static void avoid_kernel_names(Program& prog) {
+  static const std::set<std::string> taken = [] {
+    std::set<std::string> words;
+    for (const char* text : {kTcSource, kGemmSource, kAttnSource, kAttnRowsSource}) {
+      std::string word;
+      for (const char* c = text; ; ++c) {
+        if (*c && (isalnum((unsigned char)*c) || *c == '_')) { word += *c; continue; }
+        if (!word.empty()) words.insert(word);
+        word.clear();
+        if (!*c) break;
+      }
+    }
+    return words;
+  }();
+  for (auto& t : prog.tnodes)
+    if (taken.count(t.ident)) t.ident += "_n" + std::to_string(t.id);
+}
+
 Code compile_program(Program prog, const CompileOptions& opt) {
   Code code;
   code.prog = std::move(prog);
+  if (opt.enable_gemm || opt.enable_attn) avoid_kernel_names(code.prog);
   Builder b{code, opt};
   b.run();
   return code;

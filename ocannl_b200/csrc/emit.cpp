@@ -501,7 +501,7 @@ Emitter::Res Emitter::scalar(Prec prec, const Scalar& e) {
             return r;
           }
         }
-        if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: read of virtual node '" + t.ident + "'");
+        if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: read of virtual node '" + t.label + "'");
         used_nodes.insert(e.tn);
         for (auto& lt : load_tiles)
           if (lt.tn == e.tn && same_indices(lt.idcs, e.idcs)) {
@@ -674,7 +674,7 @@ std::string Emitter::stmt(const Stmt& s, int ind) {
     }
     case Stmt::Set: {
       const Tnode& t = P.tn(s.tn);
-      if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: write to virtual node '" + t.ident + "'");
+      if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: write to virtual node '" + t.label + "'");
       if (s.vec_len > 0) {
         // C_syntax (arrayjit/lib/c_syntax.ml:548-592): one evaluation of the argument, then one
         // store per element; a Fixed last index advances, any other gets "+ i" on the offset
@@ -824,7 +824,7 @@ std::string Emitter::pair_scalar(Prec prec, const Scalar& e, std::string& code) 
       const Tnode& t = P.tn(e.tn);
       auto f = forwarded.find(e.tn);
       if (f != forwarded.end() && same_indices(f->second.first, e.idcs)) return pair_convert(t.prec, prec, f->second.second, code);
-      if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: read of virtual node '" + t.ident + "'");
+      if (t.mode == Mode::Virtual) throw Error(-3, "b200ir: read of virtual node '" + t.label + "'");
       used_nodes.insert(e.tn);
       for (auto& lt : load_tiles)
         if (lt.tn == e.tn && same_indices(lt.idcs, e.idcs)) return pair_convert(t.prec, prec, lt.expr, code);

@@ -76,7 +76,7 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
   const Program& P = r->code->code.prog;
   auto ptr = [&](int tn) {
     auto it = r->node_ptr.find(tn);
-    if (it == r->node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(tn).ident + "' has no buffer binding");
+    if (it == r->node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(tn).label + "' has no buffer binding");
     return it->second;
   };
   const int eb = prec_bytes(g.in_prec);
@@ -211,7 +211,7 @@ AttnLaunch* attn_prepare(b200_routine* r, int si) {
   const Program& P = r->code->code.prog;
   auto ptr = [&](int tn) {
     auto it = r->node_ptr.find(tn);
-    if (it == r->node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(tn).ident + "' has no buffer binding");
+    if (it == r->node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(tn).label + "' has no buffer binding");
     return it->second;
   };
   const int eb = prec_bytes(a.in_prec);

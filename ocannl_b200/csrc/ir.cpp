@@ -265,7 +265,7 @@ Program parse_program(const char* text, size_t len) {
         const Sx& t = sec.l[k];
         Tnode tn;
         tn.id = (int)to_int(t.at(1));
-        tn.ident = t.at(2).a;
+        tn.ident = tn.label = t.at(2).a;
         tn.prec = prec_of_string(t.at(3).a);
         for (auto& d : t.at(4).l) {
           int64_t v = to_int(d);

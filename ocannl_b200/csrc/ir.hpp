@@ -33,7 +33,8 @@ enum class Mode { Virtual, Local, Ctx, Global };
 
 struct Tnode {
   int id = 0;
-  std::string ident;
+  std::string ident;   // the name of its pointer in the kernels
+  std::string label;   // the routine's own name for it, for messages
   Prec prec = Prec::Single;
   std::vector<int64_t> dims;
   Mode mode = Mode::Ctx;

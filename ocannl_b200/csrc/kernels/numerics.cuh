@@ -436,9 +436,9 @@ __device__ __forceinline__ float b200_div_literal(float a, float b) {
   if (m >= 0x1p-60f && m <= 0x1p+60f) return fmaf(fmaf(-q0, b, a), r, q0);
   return a == 0.0f ? q0 : a / b;
 }
-// ... without a branch, for the attention kernels, whose loops over keys are unrolled and divide every score by
-// the square root of the head size (64 sequences of 256, 8 heads of 32, six layers: 1110 us with the branch above, 1044 us
-// with a test of the remainder, 946 us so).  Where no remainder can be formed (infinite and undefined numerators, quotients
+// ... without a branch, for the attention kernels, which divide every score by the square root of the head size (64
+// sequences of 256, 8 heads of 32, six layers: 1110 us with the branch above, 1044 us with a test of the remainder, 946 us
+// so).  Where no remainder can be formed (infinite and undefined numerators, quotients
 // that overflow) the estimate is the answer.  The last place may differ for numerators below 2^-60 and for
 // quotients within two units of the largest float, and the zero of a negative zero is positive.
 __device__ __forceinline__ float b200_div_literal_straight(float a, float b) {

@@ -141,7 +141,7 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
     auto it = bind.find(t.id);
     if (it == bind.end()) continue;  // checked per stage below: only nodes a stage uses are required
     if (it->second->offset % (uint64_t)prec_bytes(t.prec) != 0)
-      throw Error(B200_E_INVALID, "link: node '" + t.ident + "' is bound at offset " + std::to_string(it->second->offset) +
+      throw Error(B200_E_INVALID, "link: node '" + t.label + "' is bound at offset " + std::to_string(it->second->offset) +
                                       ", not a multiple of its element size");
     param_ptr[t.id] = d->address(it->second->pool_id, it->second->offset, (size_t)t.bytes());
   }
@@ -208,16 +208,16 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
     const Stage& st = c->code.stages[i];
     if (st.kind == Stage::Memset) {
       if (!node_ptr.count(st.memset_tn))
-        throw Error(B200_E_USER, "link: node '" + P.tn(st.memset_tn).ident + "' has no buffer binding");
+        throw Error(B200_E_USER, "link: node '" + P.tn(st.memset_tn).label + "' has no buffer binding");
       continue;
     }
     for (auto& a : st.args) {
       if (a.kind == KArg::Node) {
         auto it = node_ptr.find(a.tn);
-        if (it == node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(a.tn).ident + "' has no buffer binding");
+        if (it == node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(a.tn).label + "' has no buffer binding");
         if (st.min_align > 1 && (it->second % (CUdeviceptr)st.min_align) != 0)
           throw Error(B200_E_INVALID, "link: internal error: stage '" + st.kernel + "' kept a form that needs " +
-                                          std::to_string(st.min_align) + "-byte alignment for node '" + P.tn(a.tn).ident + "'");
+                                          std::to_string(st.min_align) + "-byte alignment for node '" + P.tn(a.tn).label + "'");
         arg_values[i].push_back(it->second);
       } else if (a.kind == KArg::Status) {
         arg_values[i].push_back(dev->status_dev);
