@@ -473,14 +473,21 @@ int b200_compile(const char* name, const char* ir, size_t len, const char* optio
   });
 }
 
-// The units of a routine -- its generic kernels, and one per contraction or attention stage -- compiled side by side:
-// a decoder of six layers has 45, half a second of one core each (22.0 -> 3.5 s on eight cores).
+// The units of a routine -- its generic kernels, and one per contraction or attention stage.  Those that no routine
+// before had are compiled side by side: a decoder of six layers has 45, half a second of one core each (22.0 -> 3.5 s on
+// eight cores).
 static std::vector<const std::string*> compile_units(const std::vector<std::pair<const std::string*, const std::string*>>& units) {
   std::vector<const std::string*> out(units.size(), nullptr);
+  std::vector<size_t> todo;
+  for (size_t i = 0; i < units.size(); ++i) {
+    out[i] = compiled_cubin(*units[i].first);
+    if (!out[i]) todo.push_back(i);
+  }
   std::vector<std::exception_ptr> failed(units.size());
   std::atomic<size_t> next{0};
   auto work = [&] {
-    for (size_t i; (i = next++) < units.size();) {
+    for (size_t q; (q = next++) < todo.size();) {
+      const size_t i = todo[q];
       try {
         out[i] = &compile_cubin(*units[i].first, *units[i].second);
       } catch (...) {
@@ -492,7 +499,7 @@ static std::vector<const std::string*> compile_units(const std::vector<std::pair
   others.reserve(8);
   const size_t cores = std::max(1u, std::thread::hardware_concurrency());
   try {
-    for (size_t t = 1; t < std::min<size_t>({units.size(), cores, 8}); ++t) others.emplace_back(work);
+    for (size_t t = 1; t < std::min<size_t>({todo.size(), cores, 8}); ++t) others.emplace_back(work);
   } catch (const std::system_error&) {
     // (no more threads to be had: the others, or this one alone, do the work)
   }

@@ -93,16 +93,20 @@ void cu_check(CUresult r, const char* what) {
   throw Error((int)r, std::string(what) + ": " + (msg ? msg : "CUDA error") + " (CUresult " + std::to_string((int)r) + ")");
 }
 
+static std::mutex cubins_mu;
+static std::map<std::string, std::string> cubins;   // by source; the extra flags are part of what is compiled
+static std::string cubin_key(const std::string& source) { return source + "\n// flags: " + env("B200_NVRTC_FLAGS"); }
+static const std::string* find_cubin(const std::string& key) {
+  std::lock_guard<std::mutex> g(cubins_mu);
+  auto it = cubins.find(key);
+  return it != cubins.end() ? &it->second : nullptr;
+}
+
+const std::string* compiled_cubin(const std::string& source) { return find_cubin(cubin_key(source)); }
+
 const std::string& compile_cubin(const std::string& source, const std::string& name, std::string* log_out) {
-  static std::mutex mu;
-  static std::map<std::string, std::string> cache;
-  // the extra flags are part of what is compiled
-  const std::string key = source + "\n// flags: " + env("B200_NVRTC_FLAGS");
-  {
-    std::lock_guard<std::mutex> g(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-  }
+  const std::string key = cubin_key(source);
+  if (const std::string* have = find_cubin(key)) return *have;
   NvrtcApi& n = nvrtc();
   if (!n.loaded) throw Error(-2, "NVRTC is not available: " + n.why);
   nvrtcProgram prog;
@@ -136,8 +140,8 @@ const std::string& compile_cubin(const std::string& source, const std::string& n
   std::string cubin(cs, '\0');
   n.nvrtcGetCUBIN_(prog, &cubin[0]);
   n.nvrtcDestroyProgram_(&prog);
-  std::lock_guard<std::mutex> g(mu);
-  return cache.emplace(key, std::move(cubin)).first->second;
+  std::lock_guard<std::mutex> g(cubins_mu);
+  return cubins.emplace(key, std::move(cubin)).first->second;
 }
 
 }  // namespace b200

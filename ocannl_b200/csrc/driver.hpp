@@ -62,5 +62,7 @@ void cu_check(CUresult r, const char* what);  // throws Error(positive code)
 // Compiles one translation unit to sm_100a machine code (cached by source text).
 // Throws Error(-2) when NVRTC is unavailable and Error(positive) with the log on failure.
 const std::string& compile_cubin(const std::string& source, const std::string& name, std::string* log = nullptr);
+// ... or null where this source has not been compiled yet.
+const std::string* compiled_cubin(const std::string& source);
 
 }  // namespace b200
