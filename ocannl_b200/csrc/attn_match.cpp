@@ -281,7 +281,11 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   const int64_t S = extent_of(n[0], s_sym), T = extent_of(n[0], t_sym), E = r1.loop.extent();
   // Tiles of 128 queries on the tensor cores for whole tiles of keys; every other number of keys up to 256
   // (and every head dimension that is a multiple of 16, and short sequences) goes to the kernel that gives
-  // 16 queries to a warp.
+  // 16 queries to a warp.  The line lies where the tile kernel's layouts end (its chunks of keys, its 16-byte rows), not
+  // where it stops being faster.  Square causal attention, nodes local, us (tiles / rows / separate stages), at 512 heads:
+  // 64 keys 11.9 / - / 17.8, 65 - / 12.1 / 29, 128 16.9 / - / 38, 129 - / 42.5 / 76, 255 - / 90 / 184, 256 41.1 / - / 128;
+  // at 16 heads: 64 5.7 / - / 7.8, 127 - / 11.2 / 10.9, 200 - / 14.2 / 12.3, 255 - / 16.2 / 16.1, 256 10.8 / - / 12.0.
+  // So a full batch of 129 to 255 keys would gain from tiles padded to whole chunks.
   const bool rows_kernel = !(E == 64 && (T == 64 || T == 128 || T == 256) && S >= 64);
   if (rows_kernel && (T > 256 || E % 16 != 0 || E > 128)) return false;
   if (SC.dims.back() != T) return false;

@@ -9,11 +9,12 @@
 //        [zero_out t;] for f.., k.. { t[f..] := fma(x[..], y[..], t[f..]) }
 // A loop symbol is a batch axis when both operands carry it, an M (N) axis when only the
 // first (second) operand carries it, and a K axis when it is reduced.  Operands are bf16 or
-// half pairs, or single-precision pairs that the tensor cores read as tf32 (`tf32=0` keeps those
-// on the exact generic path).  Anything else —
-// affine or static indices in the operands, mixed operand precisions, an accumulator that
-// is not fp32 (the cc backend would round every step, arrayjit/lib/cc_backend.ml:169-186),
-// strides the tensor maps cannot express — is left to the generic loop-nest kernels.
+// half pairs, or single-precision pairs that the tensor cores read as tf32, plainly or in two parts
+// (`tf32=0` keeps those on the exact generic path).  Operands that the tensor maps cannot describe where
+// they lie (strides that are no multiple of 16 bytes, several loops along an axis, affine indices) are
+// gathered into padded rows first (PackOp).  Anything else -- static indices in the operands, mixed
+// operand precisions, an accumulator that is not fp32 (the cc backend would round every step,
+// arrayjit/lib/cc_backend.ml:169-186) -- is left to the generic loop-nest kernels.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

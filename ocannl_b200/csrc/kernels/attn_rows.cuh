@@ -100,7 +100,6 @@ __device__ __forceinline__ void b200_ar_put16(unsigned long long p, unsigned int
   }
 }
 
-// softmax passes behind the row maximum, on the score fragments `x`; `skip`: bit n set when tile n is masked throughout
 // the rows of one (batch, head) on their way into shared memory, one group of copies
 __device__ __forceinline__ void b200_ar_fetch(unsigned short* to, const unsigned short* from, long long row) {
   constexpr unsigned int P = B200_E / 8;   // 16-byte pieces per row

@@ -64,11 +64,9 @@ __device__ __forceinline__ bool b200_wait(unsigned int bar, unsigned int parity,
 }
 
 // One thread of a converged warp, chosen by the hardware.  The roles that issue tcgen05.mma and TMA
-// copies enter through this instead of `lane == 0`: the compiler then knows that exactly one thread
-// runs the region and keeps descriptors and addresses in uniform registers.  Behind a comparison of
-// the lane index it moves every operand of every instruction there first; a 128 x 16 x 16 MMA was
-// issued every 67 cycles that way, every 44 behind the election (128 x 128: 65 either way, 128 x 256:
-// 130, the tensor pipe's own rate).
+// copies enter through this instead of `lane == 0`, which costs issue time: a 128 x 16 x 16 MMA was issued
+// every 67 cycles behind the comparison and every 44 behind the election (128 x 128: 65 either way,
+// 128 x 256: 130, the tensor pipe's own rate).
 __device__ __forceinline__ bool b200_elect() {
   unsigned int p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
