@@ -160,8 +160,9 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit." B200_CG ".sync.aligned;" ::: "memory");
   }
-  // set-up above touched no global memory; from here on the grids before this one must be complete
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // Set-up touches no global memory and is over, block-wide barrier included, before the grids ahead of this one
+  // end; the threads that read or write global memory (the producer, the epilogue) then wait for those grids
+  // themselves, right ahead of their first access.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   b200_cluster_sync();   // the peer's barriers are initialised before anything is signalled on them
@@ -182,6 +183,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     if (b200_elect()) {
       unsigned int slot = 0, phase = 0;
       bool live = true;
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
         const unsigned int tile = unit % total_tiles, split = unit / total_tiles;
         const unsigned int kb0 = split * k_blocks / B200_SPLITK, kb1 = (split + 1u) * k_blocks / B200_SPLITK;
@@ -315,6 +317,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     b200_es.status = status;
     b200_es.part = 0.0f;
     B200_EPI_PROLOGUE
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     unsigned int acc = 0, acc_phase = 0;
     // (batch, row, first column) of the part of a unit's tile that this thread works on
     auto b200_coords = [&](unsigned int u, unsigned int& tile, unsigned int& b0, unsigned int& b1, unsigned int& mt, unsigned int& nt) {
