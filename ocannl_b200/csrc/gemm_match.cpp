@@ -1724,7 +1724,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   st.tile_n = bn;
   st.tile_k = bk;
   st.cta_pair = pair ? 1 : 0;
-  st.box_m = 128;
+  st.box_m = g.a_kmajor && g.m.extent < 128 ? (int)((g.m.extent + 7) / 8 * 8) : 128;   // (B200_A_ROWS of the kernel)
   st.box_n = pair ? bn / 2 : bn;
   st.smem_bytes = stages * stage_bytes + 1024 + 512 + epi_warps * (staging * staging_tiles + load_tile);
   st.epi_chunk = chunk;

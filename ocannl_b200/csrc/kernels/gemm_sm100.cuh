@@ -67,6 +67,18 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 #define B200_CTA_M 128
 #define B200_CTA_N (B200_BN / (1 + B200_CTA_PAIR))
 #define B200_A_TILE_BYTES (B200_CTA_M * B200_BK * B200_ELEM_BYTES)
+// Rows of A that are staged.  A contraction of fewer than 128 rows copies those alone, in whole swizzle groups of
+// eight (k-major) or chunks of 128 bytes (m-major): what the copies fill with zeros beyond M also passes through
+// the 64 bytes a clock that an SM takes in, which bound 37 rows of 784-1024-1024 (2.8 us for 13 k blocks of
+// 128 x 16 tiles).  The rest of the tile stays as it is: it only reaches accumulator rows that nobody reads.
+#if B200_M >= B200_CTA_M
+#define B200_A_ROWS B200_CTA_M
+#elif B200_A_KMAJOR
+#define B200_A_ROWS ((B200_M + 7) / 8 * 8)
+#else
+#define B200_A_ROWS ((B200_M + B200_ROW_ELEMS - 1) / B200_ROW_ELEMS * B200_ROW_ELEMS)
+#endif
+#define B200_STAGE_COPY_BYTES ((B200_A_ROWS * B200_BK * B200_ELEM_BYTES + B200_B_TILE_BYTES) * (1 + B200_PAIRS))
 #define B200_B_TILE_BYTES (B200_CTA_N * B200_BK * B200_ELEM_BYTES)
 // B200_PAIRS: single-precision operands as tf32 pairs, x = hi + lo, stored by the gathering kernel as two
 // segments of B200_SEG positions along k.  A ring slot then holds both parts of both operands, and each
@@ -208,7 +220,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           if (!b200_wait(bar_empty + 8u * slot, phase ^ 1u, abort_flag, status, 1u)) { live = false; break; }
           // both CTAs' copies complete on the leader's barrier; the leader announces the bytes of both
           const unsigned int full = b200_map_to_cta(bar_full + 8u * slot, 0u);   // (the barrier itself when not paired)
-          if (cta_rank == 0u) b200_mbar_expect_tx(bar_full + 8u * slot, B200_STAGE_BYTES * (1 + B200_CTA_PAIR));
+          if (cta_rank == 0u) b200_mbar_expect_tx(bar_full + 8u * slot, B200_STAGE_COPY_BYTES * (1 + B200_CTA_PAIR));
           const unsigned int sa = tiles_at + slot * B200_STAGE_BYTES;
           const unsigned int sb = sa + B200_B_AT;
 #pragma unroll
@@ -219,7 +231,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           b200_tma_load_4d(pa, &map_a, full, k0, m0, (int)(b1 * B200_A_B1), (int)(b0 * B200_A_B0));
 #else
 #pragma unroll
-          for (int c = 0; c < B200_CTA_M / B200_ROW_ELEMS; ++c)
+          for (int c = 0; c < (int)B200_A_ROWS / B200_ROW_ELEMS; ++c)
             b200_tma_load_4d(pa + c * (B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES), &map_a, full, m0 + c * B200_ROW_ELEMS, k0,
                              (int)(b1 * B200_A_B1), (int)(b0 * B200_A_B0));
 #endif
