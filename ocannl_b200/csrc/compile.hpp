@@ -130,6 +130,7 @@ struct Stage {
   int tile_m = 0, tile_n = 0, tile_k = 0;
   int min_align = 0;             // >0: every node the stage touches must be bound at a multiple of this many bytes
   int cta_pair = 0;              // 1: two CTAs of a cluster share one tile_m x tile_n tile (cta_group::2)
+  int cluster_k = 1;             // > 1: that many CTAs of a cluster share the k blocks of a tile
   int box_m = 0, box_n = 0;      // rows of A / B one CTA stages per k block (the TMA boxes)
   int smem_bytes = 0;            // dynamic shared memory of the contraction kernel
   int epi_out_bytes = 4;         // widest element the epilogue stores through the staging tile (2 or 4)

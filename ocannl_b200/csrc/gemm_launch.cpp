@@ -159,6 +159,8 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
     int active = 0;
     if (cu().cuOccupancyMaxActiveClusters_(&active, r->fns[si], &cfg) == CUDA_SUCCESS && active > 0 && active < clusters) clusters = active;
     L->grid = 2u * (unsigned)(tiles < (unsigned long long)clusters ? tiles : (unsigned long long)clusters);
+  } else if (st.cluster_k > 1) {
+    L->grid = (unsigned)st.cluster_k * (unsigned)tiles;   // a cluster takes one tile
   } else {
     L->grid = (unsigned)(tiles < (unsigned long long)r->dev->sm_count ? tiles : (unsigned long long)r->dev->sm_count);
   }
@@ -179,7 +181,7 @@ void gemm_enqueue(b200_routine* r, int si) {
   for (auto& m : L->in_maps) args.push_back(&m);
   for (auto& m : L->out_maps) args.push_back(&m);
   launch_kernel(r, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(contraction)",
-                st.cta_pair ? 2u : 1u);
+                st.cta_pair ? 2u : (unsigned)st.cluster_k);
 }
 
 void gemm_release(GemmLaunch* g) { delete g; }

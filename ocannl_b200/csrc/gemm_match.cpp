@@ -103,7 +103,12 @@ void walk_stmt_simple(const Stmt& s, const std::function<void(const Scalar&)>& f
 
 }  // namespace
 
-static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out);
+struct TileShape {
+  int bn = 256;        // columns
+  bool pair = false;   // two CTAs share a tile of 256 rows
+  int cluster = 1;     // > 1: that many CTAs share the k blocks of a tile of 128 rows
+};
+static TileShape gemm_tile_shape(const GemmPlan& g);
 static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, const Stmt& set, bool zeroed_before,
                             const CompileOptions& opt, const std::vector<Follower>& followers, int* n_fused, Stage* out,
                             bool pair);
@@ -879,11 +884,9 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
       for (auto& sy : dn.syms) is_n = is_n || sy.first == d.sym;
       if (!is_n) row_loops.push_back(d);
     }
-    int bn_t;
-    bool pair_t;
-    gemm_tile_shape(g, &bn_t, &pair_t);
-    bn_of_tile = bn_t;
-    bool can = !pair && !reds && !(form_b && g.accumulate) && n_syms == 1 && N <= 32 && bn_t <= 32 && !pair_t && outs[0].unit_n;
+    const TileShape tile = gemm_tile_shape(g);
+    bn_of_tile = tile.bn;
+    bool can = !pair && !reds && !(form_b && g.accumulate) && n_syms == 1 && N <= 32 && tile.bn <= 32 && !tile.pair && outs[0].unit_n;
     if (can) {
       int na = -1;
       for (size_t a = 0; a < set.idcs.size(); ++a)
@@ -1380,7 +1383,7 @@ static bool match_gemm_mode(const Program& P, const std::vector<LoopDim>& nest, 
   // the accumulator chunk is consumed: start fetching the next one while this one is stored
   // ... or, after the tile's last chunk, the operand tiles of the first chunk of this warp's NEXT
   // tile: their latency then hides behind this chunk's stores and the wait for the next accumulator
-  fn << "  B200_TRE(13);\n  if (b200_has_next) {\n#if !B200_FLUSH\n    b200_tmem_ld_chunk(b200_next_taddr, b200_r);\n#endif\n"
+  fn << "  B200_TRE(13);\n  if (b200_has_next) {\n#if !B200_FLUSH && B200_CLUSTER_K == 1\n    b200_tmem_ld_chunk(b200_next_taddr, b200_r);\n#endif\n"
      << "    b200_epilogue_load(b200_t, b200_b0, b200_b1, b200_m, b200_row_ok, b200_n0 + B200_EPI_CHUNK, b200_N, b200_es" << args << ");\n"
      << "  } else if (b200_nx_ok) {\n"
      << "    b200_epilogue_load(b200_t, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_row_ok, b200_nx_n0, b200_N, b200_es" << args << ");\n  }\n  B200_TRE(10);\n";
@@ -1571,6 +1574,11 @@ static double gemm_kb_us(int bn, bool pair, bool tf32_pairs) {
   return tf32_pairs ? 2.5 * v : v;   // three products per k block, twice the operand bytes
 }
 
+// Columns that one of the four epilogue warps of a CTA finishes when a cluster shares the k blocks: the CTA's rows are
+// one or two groups of 32, the warps that are left over share the columns, in chunks of 16 (a tile of up to 32 columns is
+// one chunk: assignments over whole rows may follow)
+static int gemm_cluster_cols(int bn, int cluster) { return bn <= 32 ? bn : (bn / cluster + 15) / 16 * 16; }
+
 // Tile shape of a contraction: columns per tile, and whether two CTAs share a 256-row tile.
 //
 // Measured times follow   2.3 us + e + l + (waves - 1) (max(l, e) + 0.25 us)   within 10 %, with l the main
@@ -1580,7 +1588,7 @@ static double gemm_kb_us(int bn, bool pair, bool tf32_pairs) {
 // therefore take the widest pairs; one of few tiles takes the shape that spreads it over the SMs
 // (1024^3: 64 columns 5.9 us, 256 columns 10.2 us; 500 x 1024 x 256: 32 columns 3.4 us, 128 columns
 // 4.9 us).  148 SMs are assumed (compilation knows no device).
-static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
+static TileShape gemm_tile_shape(const GemmPlan& g) {
   const int eb = prec_bytes(g.in_prec);
   const int row_elems = 128 / eb;
   int bn0;
@@ -1592,8 +1600,8 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
   for (auto& b : g.batch) batch *= b.extent;
   const double k_blocks = (double)((g.k.extent + row_elems - 1) / row_elems);
   double best = 1e300;
-  int best_bn = bn0;
-  bool best_pair = false;
+  TileShape shape;
+  shape.bn = bn0;
   const bool flush = g.tf32_pairs;   // running sums in registers: at most 64 columns per epilogue thread
   std::vector<int> widths = {bn0};
   // (an output row of up to 32 columns stays in one tile: assignments over whole rows may follow it)
@@ -1616,13 +1624,36 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
       const double t = 2.3 + (pair ? 0.5 : 0.0) + epi + loop + (waves - 1.0) * (std::max(loop, epi) + 0.25);
       if (t < best - 1e-9) {
         best = t;
-        best_bn = bn;
-        best_pair = pair != 0;
+        shape.bn = bn;
+        shape.pair = pair != 0;
       }
     }
   }
-  *bn_out = best_bn;
-  *pair_out = best_pair;
+  // Few tiles and a long K: a cluster shares the k blocks (kernels/gemm_sm100.cuh).  Accumulations that may be cut into
+  // work units of their own, and products in two parts, whose sums are in registers, are left alone; so are problems
+  // whose clusters would not all be resident at once (a second round costs more than the walk along k: 500 x 1024 over
+  // K = 1024, 17.5 us for two layers and the logits, 28 with 256 CTAs).
+  if (flush || g.may_split) return shape;
+  for (int cluster = 4; cluster >= 2; cluster /= 2) {
+    if (k_blocks < 2.0 * cluster) continue;
+    for (int bn : {16, 32, 64, 128}) {
+      if (bn > bn0 && !(bn0 > 32 && bn - bn0 < 32)) continue;
+      if (bn < bn0 && bn0 <= 32) continue;
+      if (!g.b_kmajor && bn % row_elems != 0) continue;
+      const long long tiles = batch * ((g.m.extent + 127) / 128) * ((g.n.extent + bn - 1) / bn);
+      if (tiles * cluster > 128) continue;
+      const double loop = std::ceil(k_blocks / cluster) * gemm_kb_us(bn, false, false);
+      const double epi = 0.25 + 3.4 * gemm_cluster_cols(bn, cluster) / 256.0;
+      const double t = 2.3 + epi + loop + 0.15 + 0.0165 * bn;   // (the exchange of the partials)
+      if (t < best - 0.2) {   // (where it hardly matters, without)
+        best = t;
+        shape.bn = bn;
+        shape.pair = false;
+        shape.cluster = cluster;
+      }
+    }
+  }
+  return shape;
 }
 
 // Work units per tile.  An accumulation into an fp32 node with few output tiles and a long K (the
@@ -1630,9 +1661,9 @@ static void gemm_tile_shape(const GemmPlan& g, int* bn_out, bool* pair_out) {
 // every tile to several workers, each over a slice of K; their partial tiles meet in the output
 // through vector reductions in global memory.  148 SMs are assumed (the compile step knows no device).
 static int gemm_split_k(const GemmPlan& g) {
-  int bn;
-  bool pair;
-  gemm_tile_shape(g, &bn, &pair);
+  const TileShape tile = gemm_tile_shape(g);
+  const int bn = tile.bn;
+  const bool pair = tile.pair;
   const int bm = pair ? 256 : 128;
   long long tiles = ((g.m.extent + bm - 1) / bm) * ((g.n.extent + bn - 1) / bn);
   for (auto& b : g.batch) tiles *= b.extent;
@@ -1646,9 +1677,9 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   GemmPlan& g = st.gemm;
   const int eb = prec_bytes(g.in_prec);
   const int row_elems = 128 / eb;
-  int bn;
-  bool pair;
-  gemm_tile_shape(g, &bn, &pair);
+  const TileShape tile = gemm_tile_shape(g);
+  const int bn = tile.bn, cluster = tile.cluster;
+  const bool pair = tile.pair;
   const int bm = pair ? 256 : 128, bk = row_elems;
   const int umma_k = 32 / eb;
   const int stage_bytes = (128 + (pair ? bn / 2 : bn)) * bk * eb * (g.tf32_pairs ? 2 : 1);   // per CTA
@@ -1662,14 +1693,21 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   if (st.row_followers > 0) chunk = bn;   // the whole row in one chunk
   const bool light = false;  // 16 warps measured slower: the register cap (96) makes the epilogue spill
   int epi_warps = light ? 16 : (bn >= 64 && bn % 64 == 0 ? 8 : 4);
+  const int warp_cols = cluster > 1 ? gemm_cluster_cols(bn, cluster) : 0;
+  int x_bytes = 0;   // partials of the other CTAs of a cluster
+  if (cluster > 1) {
+    epi_warps = 4;
+    if (warp_cols % 32 != 0) chunk = 16;
+    x_bytes = 4 * 32 * bn * 4;
+  }
   const int staging = 32 * chunk * st.epi_out_bytes;   // one staging tile
   const int load_tile = st.in_maps.empty() ? 0 : 32 * chunk * st.in_maps[0].elem_bytes;   // a row operand's chunk, per warp
   // outputs that leave as TMA stores alternate between two tiles per warp (the copy engine reads one
   // while the warp fills the other) when that leaves the ring at least four slots
   int staging_tiles = 1;
-  if (!st.out_maps.empty() && (227 * 1024 - 1024 - 512 - epi_warps * (staging * 2 + load_tile)) / stage_bytes >= 4) staging_tiles = 2;
+  if (!st.out_maps.empty() && (227 * 1024 - 1024 - 512 - x_bytes - epi_warps * (staging * 2 + load_tile)) / stage_bytes >= 4) staging_tiles = 2;
   // 227 KB per CTA: ring + alignment slack + barriers + the staging tiles of the epilogue warps
-  int stages = (227 * 1024 - 1024 - 512 - epi_warps * (staging * staging_tiles + load_tile)) / stage_bytes;
+  int stages = (227 * 1024 - 1024 - 512 - x_bytes - epi_warps * (staging * staging_tiles + load_tile)) / stage_bytes;
   if (stages > 8) stages = 8;
   if (stages < 2) stages = 2;
   int tmem_cols = 32;
@@ -1689,6 +1727,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
     << (g.a_kmajor ? 1 : 0) << "\n#define B200_B_KMAJOR " << (g.b_kmajor ? 1 : 0) << "\n#define B200_IDESC " << idesc
     << "u\n#define B200_TMEM_COLS " << tmem_cols << "\n#define B200_RASTER " << raster << "\n#define B200_CTA_PAIR "
     << (pair ? 1 : 0) << "\n#define B200_SPLITK " << g.split_k << "\n#define B200_FLUSH " << (g.tf32_pairs ? 1 : 0) << "\n";
+  if (cluster > 1) o << "#define B200_CLUSTER_K " << cluster << "\n#define B200_WARP_COLS " << warp_cols << "\n";
   if (g.tf32_pairs) o << "#define B200_PAIRS 1\n#define B200_SEG " << g.packs[0].seg << "\n";
   {
     int64_t b0 = 1, b1 = 1;
@@ -1711,7 +1750,7 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   o << "#define B200_EPILOGUE_ROW b200_epilogue_row(b200_r, b200_b0, b200_b1, b200_m, b200_m < B200_M, b200_n0, B200_N, b200_stage, b200_has_next, b200_next_taddr, b200_tiles, b200_slot, b200_nslots, b200_nx_ok, b200_nx_b0, b200_nx_b1, b200_nx_m, b200_nx_m < B200_M, b200_nx_n0, b200_es" << args << ");\n";
   o << kGemmSource << "\n";
   std::ostringstream note;
-  note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.tf32_pairs ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : "") << " stages=" << stages
+  note << "tcgen05 " << (g.in_prec == Prec::Single ? (g.tf32_pairs ? "tf32 pairs " : "tf32 ") : "") << bm << "x" << bn << "x" << bk << (pair ? " (CTA pair, cta_group::2)" : cluster > 1 ? " (k blocks over a cluster of " + std::to_string(cluster) + ")" : std::string()) << " stages=" << stages
        << " epi_warps=" << epi_warps << (g.split_k > 1 ? " split_k=" + std::to_string(g.split_k) : std::string())
        << (g.accumulate ? " beta=1" : "")
        << (st.row_followers ? " + " + std::to_string(st.row_followers) + " whole-row assignments in the epilogue" +
@@ -1724,9 +1763,10 @@ std::string gemm_translation_unit(const Program& P, Stage& st, const std::string
   st.tile_n = bn;
   st.tile_k = bk;
   st.cta_pair = pair ? 1 : 0;
+  st.cluster_k = cluster;
   st.box_m = g.a_kmajor && g.m.extent < 128 ? (int)((g.m.extent + 7) / 8 * 8) : 128;   // (B200_A_ROWS of the kernel)
   st.box_n = pair ? bn / 2 : bn;
-  st.smem_bytes = stages * stage_bytes + 1024 + 512 + epi_warps * (staging * staging_tiles + load_tile);
+  st.smem_bytes = stages * stage_bytes + 1024 + 512 + x_bytes + epi_warps * (staging * staging_tiles + load_tile);
   st.epi_chunk = chunk;
   return o.str();
 }

@@ -117,6 +117,26 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 #ifndef B200_FLUSH
 #define B200_FLUSH 0
 #endif
+// B200_CLUSTER_K > 1: few tiles, and most of the time of each is its walk along k (a k block of a 128 x 16 tile
+// brings 18 KB into the SM at some 60 bytes a clock, whatever little is multiplied with it).  A cluster of 2 or 4
+// CTAs shares a tile, each CTA taking a slice of its k blocks; every CTA then finishes 128 / B200_CLUSTER_K of the
+// tile's rows: the epilogue warps hand the rows of their tensor-memory quarter to the CTA that finishes
+// them, into its shared memory (column groups of four, a lane's row next to its neighbours': 512 bytes an
+// instruction), where its barrier counts the bytes.  The partials are added in the order of the slices.
+// The exchange is what it costs: some 16 bytes a clock leave an SM this way, 0.35 us for 16 columns, 0.75 for 32, 1.3 for
+// 64 (bulk copies out of shared memory: 0.5, 1.0, 1.6).  128 rows of 2048-2048-2048-10: 20.3 -> 17.4 us; 64 of
+// 4096-4096-256-10: 28.8 -> 19.9; 37 of 784-1024-1024-10: 15.3 -> 14.6, and 18.1 with the logits' k blocks in one CTA.
+// A cluster takes one tile: the grid has B200_CLUSTER_K CTAs for each.
+#if B200_CLUSTER_K > 1
+#define B200_X_GROUPS (4 / B200_CLUSTER_K)                 // groups of 32 rows that a CTA finishes
+#define B200_X_BYTES (4 * 32 * B200_BN * 4)                // partials on their way: CLUSTER_K x X_GROUPS x 32 rows x BN columns
+#else
+#define B200_X_BYTES 0
+#endif
+// columns of the tile that an epilogue warp works on
+#ifndef B200_WARP_COLS
+#define B200_WARP_COLS (B200_BN / (B200_EPI_WARPS / 4))
+#endif
 
 extern "C" __global__ void __launch_bounds__(B200_THREADS, 1)
 B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ b200_tmap map_b,
@@ -128,14 +148,15 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
   const unsigned int tiles_at = smem_base;
   // the epilogue warps' staging tiles follow the ring (1024-byte aligned, as the swizzled TMA stores want);
   // barriers and bookkeeping live after them
-  unsigned long long* bars = (unsigned long long*)(smem_gen + B200_STAGES * B200_STAGE_BYTES +
-                                                   B200_EPI_WARPS * (B200_STAGING_TILES * B200_STAGING_BYTES + B200_LOAD_TILE_BYTES));
+  constexpr unsigned int x_offset = B200_STAGES * B200_STAGE_BYTES + B200_EPI_WARPS * (B200_STAGING_TILES * B200_STAGING_BYTES + B200_LOAD_TILE_BYTES);
+  unsigned long long* bars = (unsigned long long*)(smem_gen + x_offset + B200_X_BYTES);
   const unsigned int bar_full = b200_smem_addr(bars);                          // [STAGES]
   const unsigned int bar_empty = bar_full + 8u * B200_STAGES;                  // [STAGES]
   const unsigned int bar_acc_full = bar_empty + 8u * B200_STAGES;              // [2]
   const unsigned int bar_acc_empty = bar_acc_full + 16u;                       // [2]
   const unsigned int bar_load = bar_acc_empty + 16u;                           // [EPI_WARPS]: row operands loaded by TMA
-  volatile unsigned int* tmem_slot = (volatile unsigned int*)(bars + 2 * B200_STAGES + 4 + B200_EPI_WARPS);
+  const unsigned int bar_x = bar_load + 8u * B200_EPI_WARPS;                   // [1]: partials of the other CTAs of a cluster
+  volatile unsigned int* tmem_slot = (volatile unsigned int*)(bars + 2 * B200_STAGES + 5 + B200_EPI_WARPS);
   volatile unsigned int* abort_flag = tmem_slot + 1;
 
   // the next kernel in the stream may be placed as soon as every CTA of this one is running
@@ -163,6 +184,10 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       b200_mbar_init(bar_acc_empty + 8u * a, B200_EPI_WARPS * (1 + B200_CTA_PAIR));
     }
     for (unsigned int w = 0; w < B200_EPI_WARPS; ++w) b200_mbar_init(bar_load + 8u * w, 1);
+    b200_mbar_init(bar_x, 1);
+#if B200_CLUSTER_K > 1
+    b200_mbar_expect_tx(bar_x, B200_X_BYTES);   // the partials of all CTAs of the cluster, this one's included
+#endif
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -181,14 +206,17 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned int tmem_base = *tmem_slot;
   const unsigned int cta_rank = b200_cta_rank();
-  // tiles are taken by CTA pairs in pair mode, by single CTAs otherwise
-  const unsigned int worker = blockIdx.x / (1 + B200_CTA_PAIR), n_workers = gridDim.x / (1 + B200_CTA_PAIR);
+  const unsigned int k_rank = b200_k_rank();
+  // tiles are taken by CTA pairs in pair mode, by clusters that share the k blocks, by single CTAs otherwise
+  constexpr unsigned int ctas_per_worker = B200_CTA_PAIR ? 2 : B200_CLUSTER_K;
+  const unsigned int worker = blockIdx.x / ctas_per_worker, n_workers = gridDim.x / ctas_per_worker;
   if (threadIdx.x == 0) B200_TR(2);   // set-up done
 
   constexpr unsigned int tiles_per_batch = B200_TILES_M * B200_TILES_N;
   constexpr unsigned int total_tiles = tiles_per_batch * B200_B0 * B200_B1;
   constexpr unsigned int k_blocks = (B200_K + B200_BK - 1) / B200_BK;
   constexpr unsigned int total_units = total_tiles * B200_SPLITK;
+  constexpr unsigned int k_slices = B200_SPLITK * B200_CLUSTER_K;   // (one of the two is 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -197,8 +225,8 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       bool live = true;
       asm volatile("griddepcontrol.wait;" ::: "memory");
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
-        const unsigned int tile = unit % total_tiles, split = unit / total_tiles;
-        const unsigned int kb0 = split * k_blocks / B200_SPLITK, kb1 = (split + 1u) * k_blocks / B200_SPLITK;
+        const unsigned int tile = unit % total_tiles, split = unit / total_tiles * B200_CLUSTER_K + k_rank;
+        const unsigned int kb0 = split * k_blocks / k_slices, kb1 = (split + 1u) * k_blocks / k_slices;
         const unsigned int bidx = tile / tiles_per_batch;
         const unsigned int t = tile - bidx * tiles_per_batch;
         // consecutive tiles walk down m first so that a wave of CTAs shares few B tiles
@@ -270,8 +298,8 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
           b200_smem_desc(tiles_at + B200_B_AT, B200_ROW_ELEMS * B200_BK * B200_ELEM_BYTES, B200_MN_GROUP_BYTES, B200_MN_SWIZZLE);
 #endif
       for (unsigned int unit = worker; live && unit < total_units; unit += n_workers) {
-        const unsigned int split = unit / total_tiles;
-        const unsigned int kb0 = split * k_blocks / B200_SPLITK, kb1 = (split + 1u) * k_blocks / B200_SPLITK;
+        const unsigned int split = unit / total_tiles * B200_CLUSTER_K + k_rank;
+        const unsigned int kb0 = split * k_blocks / k_slices, kb1 = (split + 1u) * k_blocks / k_slices;
         for (unsigned int kbf = kb0; live && kbf < kb1;) {
           // one run of k blocks into one accumulator buffer: the whole unit, or B200_FLUSH blocks of it
           const unsigned int kbe = B200_FLUSH ? min(kbf + (unsigned int)B200_FLUSH, kb1) : kb1;
@@ -313,8 +341,16 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     // ------------------------------------------------------------------ epilogue
     const unsigned int ew = warp - 2;                 // 0 .. EPI_WARPS-1
     const unsigned int quarter = warp & 3u;           // TMEM lanes this warp may read
-    const unsigned int col_half = ew >> 2;            // which part of the tile's columns this warp owns
-    const unsigned int cols_per_warp = B200_BN / (B200_EPI_WARPS / 4);
+#if B200_CLUSTER_K > 1
+    const unsigned int row_group = k_rank * B200_X_GROUPS + ew % B200_X_GROUPS;   // the 32 rows of the tile this warp finishes
+    const unsigned int col_part = ew / B200_X_GROUPS;                             // and which part of its columns
+    const bool b200_idle = col_part * B200_WARP_COLS >= B200_BN;
+#else
+    const unsigned int row_group = quarter;
+    const unsigned int col_part = ew >> 2;
+    constexpr bool b200_idle = false;
+#endif
+    constexpr unsigned int cols_per_warp = B200_WARP_COLS;
     // this warp's 4 KB staging tile (transposes a chunk so that stores cover whole row segments)
     uint4* b200_stage = (uint4*)(smem_gen + B200_STAGES * B200_STAGE_BYTES + ew * (unsigned int)(B200_STAGING_TILES * B200_STAGING_BYTES));
     b200_epi_state b200_es;
@@ -352,28 +388,33 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
     for (unsigned int unit = worker; unit < total_units; unit += n_workers) {
       unsigned int tile, b200_b0, b200_b1, mt, nt;
       b200_coords(unit, tile, b200_b0, b200_b1, mt, nt);
-      const unsigned int b200_m = mt * B200_BM + cta_rank * B200_CTA_M + quarter * 32u + lane;
-      // one scratch slot per epilogue warp of the grid for epilogues that end in a grid-wide sum
+      const unsigned int b200_m = mt * B200_BM + cta_rank * B200_CTA_M + row_group * 32u + lane;
+      // one scratch slot per epilogue warp of the grid for epilogues that end in a grid-wide sum (whose tiles are one
+      // chunk wide: of a cluster's warps, those of the first column part)
+#if B200_CLUSTER_K > 1
+      const unsigned int b200_slot = blockIdx.x * B200_X_GROUPS + ew % B200_X_GROUPS, b200_nslots = gridDim.x * B200_X_GROUPS;
+#else
       const unsigned int b200_slot = blockIdx.x * B200_EPI_WARPS + ew, b200_nslots = gridDim.x * B200_EPI_WARPS;
+#endif
       // this warp's share of the next tile, for the prefetch at the end of this one
       bool b200_nx_ok = false;
       unsigned int b200_nx_b0 = 0, b200_nx_b1 = 0, b200_nx_m = 0, b200_nx_n0 = 0;
       if (unit + n_workers < total_units) {
         unsigned int ntile, nmt, nnt;
         b200_coords(unit + n_workers, ntile, b200_nx_b0, b200_nx_b1, nmt, nnt);
-        b200_nx_m = nmt * B200_BM + cta_rank * B200_CTA_M + quarter * 32u + lane;
-        b200_nx_n0 = nnt * B200_BN + col_half * cols_per_warp;
+        b200_nx_m = nmt * B200_BM + cta_rank * B200_CTA_M + row_group * 32u + lane;
+        b200_nx_n0 = nnt * B200_BN + col_part * cols_per_warp;
         b200_nx_ok = b200_nx_n0 < B200_N;
       }
       B200_EPILOGUE_ROWS
       if (!b200_prefetched) {
-        const unsigned int b200_pn0 = nt * B200_BN + col_half * cols_per_warp;
-        if (b200_pn0 < B200_N) { B200_EPILOGUE_LOAD }
+        const unsigned int b200_pn0 = nt * B200_BN + col_part * cols_per_warp;
+        if (!b200_idle && b200_pn0 < B200_N) { B200_EPILOGUE_LOAD }
       }
-      b200_prefetched = b200_nx_ok && (nt * B200_BN + col_half * cols_per_warp < B200_N);
+      b200_prefetched = b200_nx_ok && (nt * B200_BN + col_part * cols_per_warp < B200_N);
 #if B200_FLUSH
-      constexpr int kCols = (B200_BN / (B200_EPI_WARPS / 4) + B200_EPI_CHUNK - 1) / B200_EPI_CHUNK * B200_EPI_CHUNK;
-      const unsigned int col0 = col_half * cols_per_warp;
+      constexpr int kCols = (B200_WARP_COLS + B200_EPI_CHUNK - 1) / B200_EPI_CHUNK * B200_EPI_CHUNK;
+      const unsigned int col0 = col_part * cols_per_warp;
       float b200_sum[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) b200_sum[j] = 0.0f;
@@ -410,6 +451,50 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
         const unsigned int b200_next_taddr = tmem_base;   // (a load that nothing reads)
         B200_EPILOGUE_ROW
       }
+#elif B200_CLUSTER_K > 1
+      const bool got_acc = b200_wait(bar_acc_full, 0u, abort_flag, status, 4u);
+      if (got_acc) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned int taddr = tmem_base + ((quarter * 32u) << 16);
+        // partials lie as [slice][row group][columns / 4][row]
+        const unsigned int owner = quarter / B200_X_GROUPS, bar = b200_map_to_rank(bar_x, owner);
+        const unsigned int to = b200_map_to_rank(smem_base + x_offset + ((k_rank * B200_X_GROUPS + quarter % B200_X_GROUPS) * (B200_BN / 4) * 32u + lane) * 16u, owner);
+        constexpr int step = B200_BN >= 32 ? 32 : 16;
+#pragma unroll
+        for (int c = 0; c < B200_BN; c += step) {
+          unsigned int part[step];
+          if constexpr (step == 32) b200_tmem_ld32(taddr + c, part); else b200_tmem_ld16(taddr + c, part);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int g = 0; g < step / 4; ++g) b200_st_async(to + (c / 4 + g) * 512u, bar, part[4 * g], part[4 * g + 1], part[4 * g + 2], part[4 * g + 3]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      }
+      b200_cluster_arrive_relaxed();   // nothing more goes to the other CTAs' shared memory
+      if (!got_acc || !b200_wait(bar_x, 0u, abort_flag, status, 6u)) break;
+      if (b200_idle) break;   // (a cluster takes one tile)
+      const uint4* const from = (const uint4*)(smem_gen + x_offset) + (ew % B200_X_GROUPS) * (B200_BN / 4) * 32u + lane;
+#pragma unroll 1
+      for (unsigned int c = 0; c < cols_per_warp; c += B200_EPI_CHUNK) {
+        const unsigned int col = col_part * cols_per_warp + c;
+        const unsigned int b200_n0 = nt * B200_BN + col;
+        if (b200_n0 >= B200_N) break;  // warp-uniform
+        unsigned int b200_r[B200_EPI_CHUNK];
+#pragma unroll
+        for (int g = 0; g < B200_EPI_CHUNK / 4; ++g) {
+          float4 v = *(const float4*)(from + (col / 4 + g) * 32u);
+#pragma unroll
+          for (int r = 1; r < B200_CLUSTER_K; ++r) {
+            const float4 w = *(const float4*)(from + (r * B200_X_GROUPS * (B200_BN / 4) + col / 4 + g) * 32u);
+            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+          }
+          b200_r[4 * g] = __float_as_uint(v.x); b200_r[4 * g + 1] = __float_as_uint(v.y);
+          b200_r[4 * g + 2] = __float_as_uint(v.z); b200_r[4 * g + 3] = __float_as_uint(v.w);
+        }
+        const bool b200_has_next = (c + B200_EPI_CHUNK < cols_per_warp) && (b200_n0 + B200_EPI_CHUNK < B200_N);
+        const unsigned int b200_next_taddr = tmem_base;   // (a load that nothing reads)
+        B200_EPILOGUE_ROW
+      }
 #else
       if (!b200_wait(bar_acc_full + 8u * acc, acc_phase, abort_flag, status, 4u)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -422,7 +507,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       // has consumed the current one, so the load overlaps the epilogue's stores.  (The loop is
       // deliberately not unrolled: the generated epilogue can be thousands of instructions.)
       unsigned int b200_r[B200_EPI_CHUNK];
-      const unsigned int col0 = col_half * cols_per_warp;
+      const unsigned int col0 = col_part * cols_per_warp;
       if (nt * B200_BN + col0 < B200_N) b200_tmem_ld_chunk(taddr + col0, b200_r);
 #pragma unroll 1
       for (unsigned int c = 0; c < cols_per_warp; c += B200_EPI_CHUNK) {
@@ -461,6 +546,9 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
 
   // ---------------------------------------------------------------------- teardown
   __syncwarp();
+#if B200_CLUSTER_K > 1
+  if (warp < 2) b200_cluster_arrive_relaxed();   // (the epilogue's warps have arrived after their last copies)
+#endif
   if (*abort_flag) {
     // let copies and MMAs already in flight land before the tensor memory is released
     const unsigned long long t0 = b200_now_ns();
@@ -468,7 +556,12 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  b200_cluster_sync();   // neither CTA of a pair leaves while the other may still read its memory or signal its barriers
+  // no CTA of a cluster leaves while another may still read or write its memory or signal its barriers
+#if B200_CLUSTER_K > 1
+  b200_cluster_wait();
+#else
+  b200_cluster_sync();
+#endif
   if (threadIdx.x == 0) B200_TR(12);  // all roles done
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -86,6 +86,14 @@ __device__ __forceinline__ bool b200_elect() {
 #define B200_CG "cta_group::1"
 #endif
 
+// B200_CLUSTER_K: that many CTAs of a cluster work on one tile, each over a slice of the k blocks (1: no such
+// cluster; never together with B200_CTA_PAIR).
+#ifndef B200_CLUSTER_K
+#define B200_CLUSTER_K 1
+#endif
+#define B200_CLUSTERED (B200_CTA_PAIR || B200_CLUSTER_K > 1)
+
+// rank within a CTA pair
 __device__ __forceinline__ unsigned int b200_cta_rank() {
 #if B200_CTA_PAIR
   unsigned int r;
@@ -95,12 +103,26 @@ __device__ __forceinline__ unsigned int b200_cta_rank() {
   return 0u;
 #endif
 }
+// rank among the CTAs that share a tile's k blocks
+__device__ __forceinline__ unsigned int b200_k_rank() {
+#if B200_CLUSTER_K > 1
+  unsigned int r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+#else
+  return 0u;
+#endif
+}
 // the shared::cluster address of the same shared-memory location in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned int b200_map_to_cta(unsigned int addr, unsigned int rank) {
-#if B200_CTA_PAIR
+__device__ __forceinline__ unsigned int b200_map_to_rank(unsigned int addr, unsigned int rank) {
   unsigned int r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
+}
+// ... within a pair; without pairs the address itself
+__device__ __forceinline__ unsigned int b200_map_to_cta(unsigned int addr, unsigned int rank) {
+#if B200_CTA_PAIR
+  return b200_map_to_rank(addr, rank);
 #else
   return addr;
 #endif
@@ -118,10 +140,21 @@ __device__ __forceinline__ void b200_mbar_arrive_cluster_relaxed(unsigned int cl
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void b200_cluster_sync() {
-#if B200_CTA_PAIR
+#if B200_CLUSTERED
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 #endif
+}
+// A barrier over the cluster in two halves, for threads that have nothing to order with it: nobody leaves (b200_cluster_wait)
+// before everybody has come past the arrival.
+__device__ __forceinline__ void b200_cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void b200_cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+// 16 bytes into another CTA's shared memory; its barrier counts them as they land (a plain store would have to be
+// followed by a releasing arrival, which waits for the way there and back: 0.6 us against 0.2)
+__device__ __forceinline__ void b200_st_async(unsigned int cluster_addr, unsigned int cluster_bar, unsigned int a, unsigned int b, unsigned int c, unsigned int d) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(cluster_addr), "r"(cluster_bar),
+               "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
 }
 
 __device__ __forceinline__ void b200_tma_load_4d(unsigned int dst, const b200_tmap* map, unsigned int bar, int c0, int c1,

@@ -2,7 +2,10 @@
 eight (k-major) or chunks of 64 16-bit / 32 single-precision elements (m-major): one row short of, on and past
 those edges, with an operand that varies with the row.  Tolerance: outputs of magnitude about one, sums in fp32 of
 products of 16-bit operands, rounded once (2^-9) on either side of the oracle's rounding; single-precision operands
-are read as tf32 (2^-11 each)."""
+are read as tf32 (2^-11 each).
+
+Few tiles over a long contraction: the k blocks are shared by a cluster of two or four CTAs, each of which finishes
+some of the rows; slices of unequal length, a last k block that is not whole, tiles whose columns end early."""
 import numpy as np
 import pytest
 
@@ -59,3 +62,24 @@ def test_rows_staged(device, m, batch, n, k):
 @pytest.mark.parametrize("prec", ["bfloat16", "single"])
 def test_columns_staged(device, m, prec):
     check(device, routine(1, m, 264, 512, prec, True), 512)
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 1024, 1024), (37, 264, 4096), (100, 48, 2048), (128, 136, 1032), (129, 520, 1096),
+                                   (500, 256, 1024), (500, 304, 1040), (1000, 264, 2048), (300, 72, 1160), (64, 16, 8200)])
+@pytest.mark.parametrize("prec", ["bfloat16", "half", "single"])
+@pytest.mark.parametrize("residual", [False, True])
+def test_k_blocks_over_a_cluster(device, m, n, k, prec, residual):
+    note = check(device, routine(1, m, n, k, prec, False, residual), k)
+    assert "over a cluster" in note, note
+
+
+@pytest.mark.parametrize("rows,n", [(33, 10), (37, 10), (200, 27), (1000, 32), (4096, 2)])
+def test_row_assignments_over_a_cluster(device, rows, n):
+    """The softmax and the mean loss that follow a narrow layer, each row whole in one of the cluster's CTAs."""
+    ir = W.mlp_forward(rows=rows, dims=(256, 1024, 1024, n), wprec="bfloat16")
+    x, labels = W.mlp_inputs(rows=rows, in_dim=256, classes=n)
+    inputs = dict(W.mlp_params(dims=(256, 1024, 1024, n)), x=x, labels=labels)
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert "over a cluster" in info["stages"][-1]["note"] and "grid-wide sum" in info["stages"][-1]["note"], info
+    compare(ir, got, want, rtol=2e-2, atol=2e-2)
