@@ -839,11 +839,20 @@ bool match_attention(const Program& P, const std::vector<StmtP>& flat, size_t at
   // and values in 227 KB)
   const int64_t key_rows = (T + 15) / 16 * 16, kv_bytes = 2 * key_rows * (E + 8) * 2;
   if (rows_kernel) {
-    a.warps = (int)std::min<int64_t>({8, (S + 15) / 16, (227 * 1024 - kv_bytes) / (64 * key_rows)});
+    const int64_t heads = B0 * B1;
+    // Warps that share 16 queries.  Few of these: four warps, the chain of latencies is what counts (two-layer decoders, us
+    // with 1 / 2 / 4: 5 x 4 heads of 100 positions 73.9 / 70.0 / 68.8, 2 heads of 250 71.8 / 61.5 / 57.4, 16 x 8 of 200
+    // 103.8 / 96.6 / 92.8).  Many, with long rows: two, the score rows in shared memory limit how many an SM holds (64 x 8
+    // of 200 318 / 274 / 303, 32 x 8 of 100 151.6 / 149.3 / 161.9); short rows gain nothing (64 x 8 of 60 153.6 / 156.4 / 164.1).
+    const int64_t steps = key_rows / 16, groups = heads * ((S + 15) / 16);
+    a.key_split = groups <= 3 * 148 ? (steps >= 4 ? 4 : steps >= 2 ? 2 : 1) : steps >= 6 ? 2 : 1;
+    const int64_t row_bytes = 64 * key_rows + (a.key_split > 1 ? a.key_split * (128 + 64 * E) : 0);   // per 16 queries
+    int64_t qt = std::min<int64_t>({8 / a.key_split, (S + 15) / 16, (227 * 1024 - kv_bytes) / row_bytes});
     // few heads: the queries of one over several blocks, while two blocks in the place of one still find an SM each
     // (5 x 4 heads of 100 queries: 14.6 us as 20 blocks, 12.7 as 80; 20 heads of 149: 24.9 and 17.5)
-    while (a.warps > 2 && 2 * B0 * B1 * ((S + 16 * a.warps - 1) / (16 * a.warps)) <= 148) a.warps = (a.warps + 1) / 2;
-    st.smem_bytes = (int)(kv_bytes + a.warps * 64 * key_rows);
+    while (qt > (a.key_split > 1 ? 1 : 2) && 2 * heads * ((S + 16 * qt - 1) / (16 * qt)) <= 148) qt = (qt + 1) / 2;
+    a.warps = (int)(qt * a.key_split);
+    st.smem_bytes = (int)(kv_bytes + qt * row_bytes);
   }
   st.block = rows_kernel ? 32 * a.warps : 256;
   st.min_align = rows_kernel ? 0 : 16;
@@ -895,7 +904,7 @@ std::string attn_translation_unit(const Program&, Stage& st, const std::string& 
   if (a.rows_kernel) {
     std::ostringstream o;
     o << kNumericsSource << "\n#define B200_AR_NAME " << kernel_name << "\n#define B200_T " << a.T << "\n#define B200_E " << a.E << "\n#define B200_HALF "
-      << (a.in_prec == Prec::Half ? 1 : 0) << "\n#define B200_WARPS " << a.warps << "\n#define B200_OUT_T " << a.out_type << "\n#define B200_NCOND " << a.n_cond
+      << (a.in_prec == Prec::Half ? 1 : 0) << "\n#define B200_WARPS " << a.warps << "\n#define B200_KS " << a.key_split << "\n#define B200_OUT_T " << a.out_type << "\n#define B200_NCOND " << a.n_cond
       << "\n#define B200_MASKED " << (a.masked ? 1 : 0) << "\n#define B200_KEEP_SCORES " << (a.scores.keep ? 1 : 0) << "\n#define B200_KEEP_EXP "
       << (a.exps.keep ? 1 : 0) << "\n#define B200_KEEP_W " << (a.weights.keep ? 1 : 0) << "\n#define B200_ATTN_PARAMS " << st.epi_params
       << "\n#define B200_ATTN_ARGS " << st.epi_args << "\n" << kAttnRowsSource << "\n" << a.code << "\n";

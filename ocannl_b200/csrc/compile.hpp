@@ -96,6 +96,7 @@ struct AttnPlan {
   bool masked = false;         // the score is a constant wherever the first condition is zero
   std::string out_type;        // storage type of the output
   int warps = 4;
+  int key_split = 1;           // warps that share 16 queries, each over some of the keys
   std::string code;
 };
 

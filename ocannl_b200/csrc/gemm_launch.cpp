@@ -224,7 +224,7 @@ AttnLaunch* attn_prepare(b200_routine* r, int si) {
   auto* L = new AttnLaunch();
   if (a.rows_kernel) {
     L->q = q; L->k = k; L->v = v;
-    L->rows = {(unsigned)a.S, (unsigned)a.B0, (unsigned)a.B1, (unsigned)((a.S + 16 * a.warps - 1) / (16 * a.warps)), a.q_row, a.q_b0, a.q_b1,
+    L->rows = {(unsigned)a.S, (unsigned)a.B0, (unsigned)a.B1, (unsigned)((a.S + 16 * (a.warps / a.key_split) - 1) / (16 * (a.warps / a.key_split))), a.q_row, a.q_b0, a.q_b1,
                a.k_row, a.k_b0, a.k_b1, a.v_row, a.v_b0, a.v_b1};
     L->grid = L->rows.tiles * L->rows.B0 * L->rows.B1;
     const CUresult e = cu().cuFuncSetAttribute_(r->fns[si], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, st.smem_bytes);

@@ -20,7 +20,7 @@
 // (it is, unless a row is masked throughout) they add nothing to the output either.  A causal mask halves the
 // work this way.
 //
-// The translation unit defines B200_AR_NAME, B200_T, B200_E, B200_HALF (1: half, 0: bfloat16), B200_WARPS,
+// The translation unit defines B200_AR_NAME, B200_T, B200_E, B200_HALF (1: half, 0: bfloat16), B200_WARPS, B200_KS,
 // B200_OUT_T (storage type of the output), B200_NCOND, B200_MASKED (1: the score is a constant where mask 0 is
 // zero), B200_KEEP_SCORES / _EXP / _W, B200_ATTN_PARAMS / B200_ATTN_ARGS, and the generated functions below.
 #ifndef B200_ATTN_ROWS_CUH
@@ -42,6 +42,10 @@ struct b200_ar_ptrs {   // addresses of this row in the nodes the routine keeps 
 #define B200_TP (B200_NT * 8)
 #define B200_LD (B200_E + 8)                      // elements per padded row in shared memory
 #define B200_NP (B200_NT / 2)                     // the loops' steps, 16 keys each
+// B200_KS warps share 16 queries (1, 2 or 4 of a block's B200_WARPS): each takes every B200_KS'th step of 16 keys, and
+// row maxima, sums and outputs meet in shared memory.  With few heads most SMs hold a warp or two, and a warp's
+// three loops are one chain of latencies, as long as the row.
+#define B200_QT (B200_WARPS / B200_KS)            // groups of 16 queries in a block
 
 __device__ __forceinline__ float b200_ar_score(const b200_attn_row& row, unsigned int b200_t, float b200_acc, unsigned int cb0, unsigned int cb1 B200_ATTN_PARAMS);
 __device__ __forceinline__ float b200_ar_masked_score();
@@ -112,6 +116,10 @@ __device__ __forceinline__ void b200_ar_fetch(unsigned short* to, const unsigned
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
+// the warps that share 16 queries
+__device__ __forceinline__ void b200_ar_meet(unsigned int qt) {
+  if (B200_KS > 1) asm volatile("bar.sync %0, %1;" ::"r"(1u + qt), "n"(32 * B200_KS) : "memory");
+}
 // all of the block's warps, wherever they are in the kernel
 __device__ __forceinline__ void b200_ar_barrier() { asm volatile("bar.sync 0;" ::: "memory"); }
 
@@ -146,7 +154,8 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
   // they came in several round trips to memory, a third of the kernel's time with few warps); rows beyond T zero
   b200_ar_fetch(ks, b200_kp + (long long)b0 * shape.k_b0 + (long long)b1 * shape.k_b1, shape.k_row);
   b200_ar_fetch(vs, b200_vp + (long long)b0 * shape.v_b0 + (long long)b1 * shape.v_b1, shape.v_row);
-  const unsigned int s0 = (tile * B200_WARPS + warp) * 16u;
+  const unsigned int qt = warp / B200_KS, part = warp % B200_KS;   // the queries and the share of the keys this warp looks at
+  const unsigned int s0 = (tile * B200_QT + qt) * 16u;
   b200_attn_row row[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -174,17 +183,6 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
   b200_ar_cond_rows(row[0], cp[0] B200_ATTN_ARGS);
   b200_ar_cond_rows(row[1], cp[1] B200_ATTN_ARGS);
 #endif
-  asm volatile("cp.async.wait_group 1;" ::: "memory");
-  b200_ar_barrier();
-  if (s0 >= shape.S) {   // no queries for this warp: it only brought its part of the keys and values
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    b200_ar_barrier();
-    return;
-  }
-  b200_ar_ptrs p[2];
-  b200_ar_rows(row[0], p[0] B200_ATTN_ARGS);
-  b200_ar_rows(row[1], p[1] B200_ATTN_ARGS);
-
   // bit j: no row of the warp has a mask bit among keys 16 j .. 16 j + 15
   unsigned int skip = 0u;
 #if B200_MASKED
@@ -200,14 +198,28 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
     skip = ~any & ((1u << B200_NP) - 1u);
   }
 #endif
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  b200_ar_barrier();
+  if (s0 >= shape.S) {   // no queries for this warp: it only brought its part of the keys and values
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    b200_ar_barrier();
+    return;
+  }
+  b200_ar_ptrs p[2];
+  b200_ar_rows(row[0], p[0] B200_ATTN_ARGS);
+  b200_ar_rows(row[1], p[1] B200_ATTN_ARGS);
+
   // this thread's scores: float4 n * 32 holds key tile n of rows g (x, y) and g + 8 (z, w)
-  float4* const xs = (float4*)(vs + B200_TP * B200_LD) + warp * (B200_NT * 32u) + lane;
+  float4* const xs = (float4*)(vs + B200_TP * B200_LD) + qt * (B200_NT * 32u) + lane;
+  // where the warps that share queries meet: row maxima and sums, partial outputs
+  float* const meet = (float*)(vs + B200_TP * B200_LD) + (B200_QT * B200_NT * 128u + qt * (B200_KS * (32u + 16u * B200_E)));
+  (void)meet;
 
   // ---- scores and row maximum
   float mx[2] = {b200_ar_max_init(), b200_ar_max_init()};
   const unsigned int k_at = (unsigned int)__cvta_generic_to_shared(ks), v_at = (unsigned int)__cvta_generic_to_shared(vs);
 #pragma unroll 2
-  for (unsigned int j = 0; j < B200_NP; ++j) {
+  for (unsigned int j = part; j < B200_NP; j += B200_KS) {
     if (B200_MASKED && ((skip >> j) & 1u)) {
 #if B200_KEEP_SCORES
 #pragma unroll
@@ -257,13 +269,20 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
     if (B200_MASKED && skip) mx[r] = fmaxf(mx[r], b200_ar_masked_score());
     mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
     mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+    if (B200_KS > 1 && c == 0u) meet[32u * part + g + 8u * r] = mx[r];
+  }
+  b200_ar_meet(qt);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+#pragma unroll
+    for (unsigned int i = 0; i < B200_KS && B200_KS > 1; ++i) mx[r] = fmaxf(mx[r], meet[32u * i + g + 8u * r]);
     mx[r] = b200_ar_row_max(row[r], mx[r] B200_ATTN_ARGS);
-    if (c == 0u && p[r].mx) *(float*)p[r].mx = mx[r];
+    if (part == 0u && c == 0u && p[r].mx) *(float*)p[r].mx = mx[r];
     em[r] = B200_MASKED ? b200_ar_exp(row[r], 0u, b200_ar_masked_score(), mx[r] B200_ATTN_ARGS) : 0.0f;
   }
   // ---- exponentials and row sum
 #pragma unroll 2
-  for (unsigned int j = 0; j < B200_NP; ++j) {
+  for (unsigned int j = part; j < B200_NP; j += B200_KS) {
     const bool off = B200_MASKED && ((skip >> j) & 1u);
 #if !B200_KEEP_EXP
     if (off && em[0] == 0.0f && em[1] == 0.0f) continue;
@@ -298,8 +317,16 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
   for (int r = 0; r < 2; ++r) {
     sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
     sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+    if (B200_KS > 1 && c == 0u) meet[32u * part + 16u + g + 8u * r] = sum[r];
+  }
+  b200_ar_meet(qt);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (B200_KS > 1) sum[r] = meet[16u + g + 8u * r];
+#pragma unroll
+    for (unsigned int i = 1; i < B200_KS; ++i) sum[r] += meet[32u * i + 16u + g + 8u * r];
     sum[r] = b200_ar_row_sum(row[r], sum[r] B200_ATTN_ARGS);
-    if (c == 0u && p[r].sum) *(float*)p[r].sum = sum[r];
+    if (part == 0u && c == 0u && p[r].sum) *(float*)p[r].sum = sum[r];
     dv[r] = b200_divisor_of(b200_ar_divisor(row[r], sum[r] B200_ATTN_ARGS));
     wz[r] = B200_MASKED ? b200_ar_weight<false>(row[r], 0u, em[r], sum[r], dv[r] B200_ATTN_ARGS) : 0.0f;
     wm[r] = b200_ar_pack(wz[r], wz[r]);
@@ -316,7 +343,7 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[e][i] = 0.0f;
 #pragma unroll 2
-  for (unsigned int j = 0; j < B200_NP; ++j) {
+  for (unsigned int j = part; j < B200_NP; j += B200_KS) {
     const bool off = B200_MASKED && ((skip >> j) & 1u);
 #if !B200_KEEP_W
     if (off && leave) continue;
@@ -348,17 +375,41 @@ B200_AR_NAME(const unsigned short* __restrict__ b200_qp, const unsigned short* _
       b200_ar_mma(o[e + 1], a, b[2], b[3]);
     }
   }
+  // the warps' partial outputs, as [part][tile of 8 columns][value][lane]; each warp finishes some of the tiles
+  if (B200_KS > 1) {
+    float* const mine = meet + 32u * B200_KS + part * (16u * B200_E) + lane;
 #pragma unroll
-  for (unsigned int e = 0; e < B200_E / 8; ++e)
+    for (unsigned int e = 0; e < B200_E / 8; ++e)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mine[(4u * e + i) * 32u] = o[e][i];
+    b200_ar_meet(qt);
+  }
+#pragma unroll
+  for (unsigned int e0 = 0; e0 < B200_E / 8; e0 += B200_KS) {
+    const unsigned int e = e0 + part;
+    if (e >= B200_E / 8) break;
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (B200_KS > 1) {
+        const float* const at = meet + 32u * B200_KS + (4u * e + i) * 32u + lane;
+        v[i] = at[0];
+#pragma unroll
+        for (unsigned int k = 1; k < B200_KS; ++k) v[i] += at[k * (16u * B200_E)];
+      } else {
+        v[i] = o[e0][i];
+      }
+    }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       if (!p[r].out) continue;
       const unsigned int col = 8u * e + 2u * c;
       B200_OUT_T* const d = (B200_OUT_T*)p[r].out + col;
-      const B200_OUT_T v0 = b200_ar_out(row[r], col, o[e][2 * r] B200_ATTN_ARGS), v1 = b200_ar_out(row[r], col + 1u, o[e][2 * r + 1] B200_ATTN_ARGS);
+      const B200_OUT_T v0 = b200_ar_out(row[r], col, v[2 * r] B200_ATTN_ARGS), v1 = b200_ar_out(row[r], col + 1u, v[2 * r + 1] B200_ATTN_ARGS);
       if (sizeof(B200_OUT_T) == 2 && ((unsigned long long)d & 3ull) == 0ull) *(unsigned int*)d = (unsigned int)v0 | ((unsigned int)v1 << 16);
       else { d[0] = v0; d[1] = v1; }
     }
+  }
 }
 
 #endif  // B200_ATTN_ROWS_CUH

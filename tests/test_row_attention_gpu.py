@@ -43,3 +43,21 @@ def test_masked_chunks(device, t, mode, prec):
     got, info = run_device(device, ir, inputs)
     assert any(st["kind"] == "attention" for st in info["stages"]), info
     compare(ir, got, want, rtol=2e-2, atol=2e-2 if prec == "bfloat16" else 4e-3)
+
+
+@pytest.mark.parametrize("b,h,s,t,e", [(8, 8, 97, 97, 32), (16, 8, 57, 60, 48), (15, 8, 49, 250, 16), (1, 1, 1, 64, 64), (2, 1, 15, 17, 112)])
+@pytest.mark.parametrize("mode,mask,prec", [("ctx", True, "bfloat16"), ("local", True, "half"), ("local", False, "bfloat16")])
+def test_warps_that_share_queries(device, b, h, s, t, e, mode, mask, prec):
+    """Two warps on 16 queries, one, two, four (one query alone), two of which one has a single key: shares of the keys
+    that are empty or masked throughout, output tiles that do not divide by the warps."""
+    ir = W.attention(b, h, s, t, prec=prec, mask=mask, row_mode=mode, d_head=e)
+    inputs = W.attention_inputs(b, h, s, t, prec=prec, d_head=e)
+    if not mask:
+        del inputs["mask"]
+    else:
+        inputs["mask"][s // 2] = 0.0
+    # (routine-local nodes would lie on the oracle's stack)
+    want = run_oracle(W.attention(b, h, s, t, prec=prec, mask=mask, row_mode="ctx", d_head=e), inputs)
+    got, info = run_device(device, ir, inputs)
+    assert any(st["kind"] == "row attention" for st in info["stages"]), info
+    compare(ir, got, want, rtol=2e-2, atol=2e-2 if prec == "bfloat16" else 4e-3)
