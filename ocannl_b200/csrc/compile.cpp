@@ -2299,12 +2299,20 @@ struct Builder {
             ++j;
           }
           // a trailing pointwise stage gains nothing from the warp form unless it follows a reduction
-          if (run.size() >= 2 && has_coop && rows >= 128) {
+          // Fewer than 128 rows may go to one block, whose four passes over 100 rows of 256 take 8 us longer than a warp
+          // a row in registers (decoders of two layers, 100 x 256: 93.7 -> 60.5 us; 16 x 128: 47.4 -> 39.0).  It is left to the
+          // block when that takes stages behind the rows as well (a loss) and the rows are short: a launch
+          // less then counts more (20 rows of 40: 13.7 us, 16.4 with a warp a row; 100 of 64: 18.5 and 16.4).
+          const bool block_goes_on = run.back() + 1 < code.stages.size() && fusable(run.back()) && fusable(run.back() + 1);
+          const int64_t elems = rows * std::max(code.stages[i].total / rows, code.stages[run.back()].total / rows);
+          if (run.size() >= 2 && has_coop && (rows >= 128 || (rows >= 8 && (!block_goes_on || elems >= 4096)))) {
             Stage reg_form;
-            if (emit_warp_rows_reg(run, L, &reg_form)) out.push_back(reg_form);
-            else out.push_back(emit_warp_rows(run, L));
-            i = run.back() + 1;
-            continue;
+            const bool in_registers = emit_warp_rows_reg(run, L, &reg_form);
+            if (in_registers || rows >= 128) {
+              out.push_back(in_registers ? reg_form : emit_warp_rows(run, L));
+              i = run.back() + 1;
+              continue;
+            }
           }
         }
       }
