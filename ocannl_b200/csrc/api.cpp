@@ -566,6 +566,7 @@ int b200_code_source(b200_code* code, int stage, char* buf, size_t cap, size_t* 
     const std::string* s = &code->code.source;
     if (stage >= 0) {
       if (stage >= (int)code->code.stages.size()) throw Error(B200_E_INVALID, "stage out of range");
+      while (code->code.stages[stage].in_group) --stage;
       if (code->code.stages[stage].own_module()) s = &code->code.stages[stage].gemm_source;
     }
     if (needed) *needed = s->size() + 1;
@@ -610,7 +611,7 @@ int b200_routine_launch_count(b200_routine* r, int64_t* kernels_per_run) {
   return guard([&] {
     if (!r || !kernels_per_run) throw Error(B200_E_INVALID, "null argument");
     int64_t k = 0;
-    for (auto& s : r->code->code.stages) k += s.kind != Stage::Memset;
+    for (auto& s : r->code->code.stages) k += s.launches();
     *kernels_per_run = k;
   });
 }

@@ -2229,6 +2229,79 @@ struct Builder {
     return f;
   }
 
+  // Pointwise chains that do not depend on one another -- the updates of a routine's parameters -- as one launch over
+  // their concatenated iterations; every chain begins at a multiple of a warp's 32.  The plan lists what is in it as
+  // stages: a large chain each, neighbouring small ones together.
+  void emit_pointwise_group(const std::vector<std::vector<size_t>>& parts, std::vector<Stage>* out) {
+    std::vector<size_t> all;
+    for (auto& run : parts) all.insert(all.end(), run.begin(), run.end());
+    Stage f = code.stages[all.front()];
+    merge_origins(f, all);
+    Emitter em(code.prog);
+    std::set<int> written;
+    std::string text;
+    int64_t start = 0;
+    for (auto& run : parts) {
+      const int64_t total = code.stages[run.front()].total;
+      text += std::string("    ") + (start ? "else " : "") + "if (b200_i < " + std::to_string(start + total) + "ull) {\n    if (b200_i >= " + std::to_string(start) +
+              "ull) {\n    const unsigned long long b200_g = b200_i - " + std::to_string(start) + "ull;\n";
+      for (size_t i : run) {
+        const Piece& pc = pieces[i];
+        f.min_align = std::max(f.min_align, code.stages[i].min_align);
+        em.used_nodes.insert(pc.used.begin(), pc.used.end());
+        written.insert(pc.written.begin(), pc.written.end());
+        em.uses_merge |= pc.uses_merge;
+        text += "    {\n" + pc.decomp + pc.body_text + "    }\n";
+      }
+      text += "    }\n    }\n";
+      start = (start + total + 31) / 32 * 32;
+    }
+    std::string statics = static_prologue(text, em, 2);
+    std::ostringstream k_src;
+    k_src << "extern \"C\" __global__ void __launch_bounds__(" << f.block << ") " << f.kernel << "(";
+    emit_params(k_src, f, em, written);
+    k_src << ") {\n" << kGridEntry << statics
+          << "  for (unsigned long long b200_i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_i < "
+          << start << "ull; b200_i += (unsigned long long)gridDim.x * blockDim.x) {\n"
+          << text << "  }\n}\n\n";
+    src << k_src.str();
+    std::vector<std::vector<size_t>> listed;
+    bool small_before = false;
+    for (auto& run : parts) {
+      const bool small = small_chain(run);
+      if (small && small_before) listed.back().insert(listed.back().end(), run.begin(), run.end());
+      else listed.push_back(run);
+      small_before = small;
+    }
+    f.group = (int)listed.size();
+    for (size_t k = 0; k < listed.size(); ++k) {
+      const std::vector<size_t>& run = listed[k];
+      Stage st = code.stages[run.front()];
+      std::set<int> used;
+      for (size_t i : run) used.insert(pieces[i].used.begin(), pieces[i].used.end());
+      merge_origins(st, run);
+      if (small_chain(run) && run.size() > 1) st.note = "fused " + std::to_string(run.size()) + " small stages";
+      else if (run.size() > 1) st.note = "pointwise chain of " + std::to_string(run.size()) + " stages" + (pieces[run.front()].pairs ? ", pairs" : "");
+      if (k == 0) {
+        f.note = st.note;
+        f.total = start;
+        out->push_back(f);
+      } else {
+        st.note += " (in the launch of " + f.kernel + ")";
+        st.in_group = true;
+        st.args.clear();
+        for (int n : used) st.args.push_back({KArg::Node, n});
+        out->push_back(st);
+      }
+    }
+  }
+  // a chain that one block could take with others
+  bool small_chain(const std::vector<size_t>& run) {
+    bool small = true;
+    for (size_t i : run) small = small && pieces[i].fusable && code.stages[i].total < 8192;
+    return small;
+  }
+
   // Decides which stages share a launch and writes the kernels' text.
   void emit_kernels() {
     {
@@ -2270,6 +2343,37 @@ struct Builder {
         ++j;
       }
       return run;
+    };
+    // Chains that do not depend on one another, from stage i on, where at least one is too large for a block: one launch
+    // instead of a kernel each and a block for the small ones in between.
+    auto group_from = [&](size_t i) {
+      std::vector<std::vector<size_t>> parts;
+      std::set<int> used, written;
+      bool large = false;
+      size_t j = opt.bounds ? code.stages.size() : i;
+      while (j < code.stages.size() && parts.size() < 16 && pointwise_member(j, nullptr)) {
+        std::vector<size_t> run = {j};
+        const Piece& first = pieces[j];
+        for (size_t k = j + 1; k < code.stages.size() && run.size() < 8 && pointwise_member(k, &first); ++k) {
+          run.push_back(k);
+          if (!rows_independent_prefix(run, first.par.size())) { run.pop_back(); break; }
+        }
+        bool apart_from_others = true;
+        for (size_t k : run) {
+          for (int n : pieces[k].written) apart_from_others = apart_from_others && !used.count(n) && !written.count(n);
+          for (int n : pieces[k].used) apart_from_others = apart_from_others && !written.count(n);
+        }
+        if (!apart_from_others) break;
+        for (size_t k : run) {
+          used.insert(pieces[k].used.begin(), pieces[k].used.end());
+          written.insert(pieces[k].written.begin(), pieces[k].written.end());
+        }
+        large = large || !small_chain(run);
+        parts.push_back(run);
+        j = run.back() + 1;
+      }
+      if (!large || parts.size() < 2) parts.clear();
+      return parts;
     };
     auto row_candidate = [&](size_t i) {
       auto it = pieces.find(i);
@@ -2334,6 +2438,14 @@ struct Builder {
           continue;
         }
       }
+      if (opt.enable_fuse) {
+        const std::vector<std::vector<size_t>> parts = group_from(i);
+        if (!parts.empty()) {
+          emit_pointwise_group(parts, &out);
+          i = parts.back().back() + 1;
+          continue;
+        }
+      }
       // (a long chain over thousands of elements -- the momentum update of a 300 x 100 layer -- is a kernel of
       // its own even where one block could take it: that block spent 30 us on four passes over it)
       if (opt.enable_fuse) {
@@ -2347,7 +2459,7 @@ struct Builder {
       if (fusable(i)) {
         std::vector<size_t> run;
         size_t j = i;
-        while (j < code.stages.size() && fusable(j) && (j == i || chain_from(j).size() < 3)) run.push_back(j++);
+        while (j < code.stages.size() && fusable(j) && (j == i || (chain_from(j).size() < 3 && group_from(j).empty()))) run.push_back(j++);
         int kernels = 0;
         for (size_t k : run) kernels += code.stages[k].kind != Stage::Memset;
         if (run.size() >= 2 && kernels >= 1) {

@@ -110,7 +110,10 @@ struct OutMap {
 
 struct Stage {
   enum Kind { Memset, Generic, Gemm, Attn } kind = Generic;
-  bool own_module() const { return kind == Gemm || kind == Attn; }   // compiled as a translation unit of its own
+  bool own_module() const { return (kind == Gemm && !in_group) || kind == Attn; }   // compiled as a translation unit of its own
+  bool launches() const { return kind != Memset && !in_group; }
+  int group = 1;                 // > 1: the launch also runs the group - 1 stages behind this one
+  bool in_group = false;         // one of those
   int memset_tn = -1;
   std::string kernel;            // kernel symbol in the routine's module
   std::vector<KArg> args;

@@ -184,7 +184,9 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
   // between two runs (and waits for the previous one at a granularity of 2 us), and the launch calls, 2 us each,
   // pass while the kernels before them run.  Two kernels: 16.6 -> 15.2 us, 8.4 -> 6.7; four: 14.9 -> 13.5,
   // 16.5 -> 16.2; with five it is as often slower (18.7 -> 20.7).
-  direct = c->code.stages.size() <= kDirectStages && scratch_zero.empty();
+  size_t launches = 0;
+  for (auto& st : c->code.stages) launches += !st.in_group;
+  direct = launches <= kDirectStages && scratch_zero.empty();
   for (auto& st : c->code.stages) direct &= st.kind != Stage::Memset;
   // Static indices that are a kernel argument would be captured with their values of the first run: such a routine
   // is launched directly whatever else it queues (a node of its scratch that starts at zero is a clear ahead of its
@@ -234,11 +236,14 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
         reads_merge = true;
       }
     }
+    if (st.kind == Stage::Generic && st.in_group) continue;
     if (st.kind == Stage::Generic) {
       cu_check(cu().cuModuleGetFunction_(&fns[i], module, st.kernel.c_str()), "cuModuleGetFunction");
     } else {
-      cu_check(cu().cuModuleLoadData_(&gemm_modules[i], c->gemm_cubins[i]->data()), "cuModuleLoadData(gemm)");
-      cu_check(cu().cuModuleGetFunction_(&fns[i], gemm_modules[i], st.kernel.c_str()), "cuModuleGetFunction(gemm)");
+      if (!st.in_group) {
+        cu_check(cu().cuModuleLoadData_(&gemm_modules[i], c->gemm_cubins[i]->data()), "cuModuleLoadData(gemm)");
+        cu_check(cu().cuModuleGetFunction_(&fns[i], gemm_modules[i], st.kernel.c_str()), "cuModuleGetFunction(gemm)");
+      }
       if (st.kind == Stage::Attn) attn[i] = attn_prepare(this, (int)i);
       else gemm[i] = gemm_prepare(this, (int)i);
     }
@@ -312,14 +317,16 @@ std::vector<b200_routine::Placed> b200_routine::branches() const {
   const size_t n = stages.size();
   struct Range { CUdeviceptr lo, hi; bool write; };
   std::vector<std::vector<Range>> touched(n);
+  size_t lead = 0;   // the stage whose launch stage i is part of
   for (size_t i = 0; i < n; ++i) {
     const Stage& st = stages[i];
+    if (!st.in_group) lead = i;
     auto node = [&](int tn, bool write) {
       auto it = node_ptr.find(tn);
-      if (it != node_ptr.end()) touched[i].push_back({it->second, it->second + (CUdeviceptr)P.tn(tn).bytes(), write});
+      if (it != node_ptr.end()) touched[lead].push_back({it->second, it->second + (CUdeviceptr)P.tn(tn).bytes(), write});
     };
     auto slot = [&](int s, bool write) {
-      if (s >= 0) touched[i].push_back({pack_address(s), pack_address(s) + (CUdeviceptr)code->code.pack_bytes[(size_t)s], write});
+      if (s >= 0) touched[lead].push_back({pack_address(s), pack_address(s) + (CUdeviceptr)code->code.pack_bytes[(size_t)s], write});
     };
     for (int tn : st.writes) node(tn, true);
     if (st.kind == Stage::Memset) node(st.memset_tn, true);
@@ -328,7 +335,7 @@ std::vector<b200_routine::Placed> b200_routine::branches() const {
       // a piece of the reduction scratch (partials with their ticket, packed masks): known by its first byte
       if (a.kind == KArg::Scratch) {
         const CUdeviceptr p = scratch + (CUdeviceptr)reduce_base + (CUdeviceptr)a.tn;
-        touched[i].push_back({p, p + 1, true});
+        touched[lead].push_back({p, p + 1, true});
       }
     }
     for (int s : st.pack_writes) slot(s, true);
@@ -343,6 +350,7 @@ std::vector<b200_routine::Placed> b200_routine::branches() const {
   std::vector<Placed> out(n);
   std::vector<int> last(kBranches, -1);
   for (size_t i = 0; i < n; ++i) {
+    if (stages[i].in_group) continue;
     std::vector<int> deps;   // latest first, without those implied by a later one
     for (size_t j = i; j-- > 0;) {
       if (before[i][j]) continue;
@@ -450,6 +458,7 @@ void b200_routine::enqueue_stages(bool capturing) {
   // queues stage i (a clear may take the clears that follow along, advancing i)
   auto queue_stage = [&](size_t& i) {
     const Stage& st = code->code.stages[i];
+    if (st.in_group) return;
     place(i);
     Timer timer(this, i);
     if (st.kind == Stage::Memset) {
@@ -594,7 +603,7 @@ void b200_routine::launch(const int64_t* static_idx, int n_static) {
     }
     cu_check(cu().cuGraphLaunch_(graph, dev->stream), "cuGraphLaunch");
     dev->n_graph_launches++;
-    for (auto& s : code->code.stages) dev->n_launches += s.kind != Stage::Memset;
+    for (auto& s : code->code.stages) dev->n_launches += s.launches();
     return;
   }
   enqueue_stages();
