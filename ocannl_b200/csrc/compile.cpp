@@ -491,23 +491,33 @@ struct Builder {
         const std::string at = "(b200_partials + " + std::to_string((size_t)si * G * 8) + "))";
         const std::string slot = "((" + T + "*)" + at, vslot = "((volatile " + T + "*)" + at;
         pass1 += "  {\n    " + T + " " + name + " = " + ea.constant(neutral, p) + ";\n";
-        pass1 += "    for (unsigned long long b200_l = (unsigned long long)blockIdx.x * 1024ull + threadIdx.x; b200_l < " +
-                 std::to_string(total) + "ull; b200_l += (unsigned long long)gridDim.x * 1024ull) {\n";
+        // Every thread takes the same whole number of steps and at most one more, so that the loads of eight steps are
+        // under way together (a step after the other cost their latency each: the 2 M squared differences of 64 images
+        // of 32 x 32 x 32, 10.0 us -> 8.5, most of it cold reads).
+        const bool narrow = total < (1ll << 31);
+        const std::string IT = narrow ? "unsigned int" : "unsigned long long", SUF = narrow ? "u" : "ull";
+        const int64_t stride = (int64_t)G * 1024, whole = total / stride;
+        std::string step;
         std::string rem = "b200_l";
         for (size_t i = red.size(); i-- > 0;) {
           const LoopDim& d = red[i];
-          std::string ext = std::to_string(d.extent()) + "ull";
+          std::string ext = std::to_string(d.extent()) + SUF;
           std::string val = i == 0 ? rem : "(" + rem + " % " + ext + ")";
-          pass1 += "      const unsigned int " + d.sym + " = (unsigned int)" + val +
-                   (d.from ? " + " + std::to_string(d.from) : std::string()) + ";\n";
+          step += "      const unsigned int " + d.sym + " = (unsigned int)" + val +
+                  (d.from ? " + " + std::to_string(d.from) : std::string()) + ";\n";
           if (i != 0) {
             std::string nr = "b200_q" + std::to_string(i);
-            pass1 += "      const unsigned long long " + nr + " = " + rem + " / " + ext + ";\n";
+            step += "      const " + IT + " " + nr + " = " + rem + " / " + ext + ";\n";
             rem = nr;
           }
         }
-        pass1 += ea.stmt(*inner, 6);
-        pass1 += "    }\n    " + name + " = b200_block_" + fn + "(" + name + ", b200_red);\n";
+        step += ea.stmt(*inner, 6);
+        pass1 += "    const " + IT + " b200_first = blockIdx.x * 1024u + threadIdx.x;\n#pragma unroll 8\n    for (unsigned int b200_k = 0; b200_k < " +
+                 std::to_string(whole) + "u; ++b200_k) {\n      const " + IT + " b200_l = b200_first + b200_k * " + std::to_string(stride) + SUF + ";\n" + step + "    }\n";
+        if (total % stride)
+          pass1 += "    if (b200_first < " + std::to_string(total % stride) + SUF + ") {\n      const " + IT + " b200_l = b200_first + " +
+                   std::to_string(whole * stride) + SUF + ";\n" + step + "    }\n";
+        pass1 += "    " + name + " = b200_block_" + fn + "(" + name + ", b200_red);\n";
         pass1 += "    if (threadIdx.x == 0) " + slot + "[blockIdx.x] = " + name + ";\n  }\n";
         // combine: the partials in block order
         pass2 += "  " + T + " " + name + " = " + eb.constant(neutral, p) + ";\n";
