@@ -233,8 +233,9 @@ int64_t PackOp::rows() const {
 int64_t PackOp::bytes() const { return rows() * ld * prec_bytes(prec); }
 std::string PackOp::key() const {
   std::ostringstream o;
-  o << tn << ":" << off << ":" << kmajor << ":" << ld << ":" << seg << ":" << split;
-  for (auto* v : {&batch, &mn, &k}) {
+  // (rows along m or n of values along k, or the other way round: the same copy, where a value is one part)
+  o << tn << ":" << off << ":" << (split ? 1 + kmajor : 0) << ":" << ld << ":" << (split ? seg : 0);
+  for (auto* v : {&batch, kmajor ? &mn : &k, kmajor ? &k : &mn}) {
     o << ";";
     for (auto& a : *v) o << a.extent << "," << a.stride << " ";
   }
