@@ -23,6 +23,7 @@ std::string attn_translation_unit(const Program& P, Stage& st, const std::string
 bool match_gemm(const Program& P, const std::vector<LoopDim>& nest, const Stmt& body, bool zeroed_before,
                 const CompileOptions& opt, const std::vector<Follower>& followers, int* n_fused,
                 Stage* out);  // gemm_match.cpp
+void group_contractions(Code& code, const CompileOptions& opt);
 std::string gemm_translation_unit(const Program& P, Stage& st, const std::string& kernel_name,
                                   const CompileOptions& opt);
 
@@ -3297,6 +3298,7 @@ struct Builder {
     }
     emit_kernels();
     place_packs();
+    if (opt.enable_fuse) group_contractions(code, opt);
     code.source = src.str();
     statics_by_value();
     if (opt.bounds) apply_bounds();

@@ -140,9 +140,12 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
   unsigned long long tiles = (unsigned long long)((g.m.extent + st.tile_m - 1) / st.tile_m) * (unsigned long long)((g.n.extent + st.tile_n - 1) / st.tile_n) *
                              (unsigned long long)(g.split_k > 0 ? g.split_k : 1);
   for (auto& d : g.batch) tiles *= (unsigned long long)d.extent;
-  cu_check(cu().cuFuncSetAttribute_(r->fns[si], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, st.smem_bytes),
-           "cuFuncSetAttribute(max dynamic shared memory)");
-  if (st.cta_pair) {
+  if (!st.in_group)
+    cu_check(cu().cuFuncSetAttribute_(r->fns[si], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, st.smem_bytes),
+             "cuFuncSetAttribute(max dynamic shared memory)");
+  if (st.in_group || st.group > 1) {
+    L->grid = (unsigned)tiles * (st.cta_pair ? 2u : (unsigned)st.cluster_k);   // as many as the kernel's block ranges say
+  } else if (st.cta_pair) {
     // persistent pairs: as many 2-CTA clusters as the device keeps resident at once
     int clusters = r->dev->sm_count / 2;
     CUlaunchConfig cfg;
@@ -170,17 +173,20 @@ GemmLaunch* gemm_prepare(b200_routine* r, int si) {
 
 void gemm_enqueue(b200_routine* r, int si) {
   const Stage& st = r->code->code.stages[si];
-  GemmLaunch* L = r->gemm[si];
   std::vector<void*> args;
-  args.push_back(&L->map_a);
-  args.push_back(&L->map_b);
-  args.push_back(&L->shape);
-  args.push_back(&L->status);
-  std::vector<CUdeviceptr>& vals = r->arg_values[si];
-  for (size_t a = 0; a < vals.size(); ++a) args.push_back(&vals[a]);
-  for (auto& m : L->in_maps) args.push_back(&m);
-  for (auto& m : L->out_maps) args.push_back(&m);
-  launch_kernel(r, r->fns[si], L->grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(contraction)",
+  unsigned grid = 0;
+  for (int k = si; k < si + st.group; ++k) {   // (a launch may run the contractions behind this one too)
+    GemmLaunch* L = r->gemm[k];
+    args.push_back(&L->map_a);
+    args.push_back(&L->map_b);
+    args.push_back(&L->shape);
+    args.push_back(&L->status);
+    for (auto& v : r->arg_values[k]) args.push_back(&v);
+    for (auto& m : L->in_maps) args.push_back(&m);
+    for (auto& m : L->out_maps) args.push_back(&m);
+    grid += L->grid;
+  }
+  launch_kernel(r, r->fns[si], grid, (unsigned)st.block, 1, (unsigned)st.smem_bytes, args.data(), "cuLaunchKernelEx(contraction)",
                 st.cta_pair ? 2u : (unsigned)st.cluster_k);
 }
 

@@ -138,9 +138,18 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 #define B200_WARP_COLS (B200_BN / (B200_EPI_WARPS / 4))
 #endif
 
-extern "C" __global__ void __launch_bounds__(B200_THREADS, 1)
-B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ b200_tmap map_b,
-               const b200_gemm_shape shape, unsigned int* status B200_EPI_PARAMS) {
+// Contractions that do not depend on one another and together leave SMs idle run as one launch: a kernel that calls this
+// one, compiled once for each of them as a device function, by ranges of its blocks.  B200_BLOCK / B200_GRID are then the
+// function's parameters.
+#ifndef B200_KERNEL_HEAD
+#define B200_KERNEL_HEAD extern "C" __global__ void __launch_bounds__(B200_THREADS, 1) B200_GEMM_NAME
+#define B200_TMAP_PARAM const __grid_constant__ b200_tmap
+#define B200_BLOCK_PARAMS
+#define B200_BLOCK blockIdx.x
+#define B200_GRID gridDim.x
+#endif
+
+B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_shape shape, unsigned int* status B200_BLOCK_PARAMS B200_EPI_PARAMS) {
   extern __shared__ unsigned char b200_dyn_smem[];
   // tiles need 1024-byte alignment for the 128-byte swizzle pattern
   const unsigned int smem_base = (b200_smem_addr(b200_dyn_smem) + 1023u) & ~1023u;
@@ -209,7 +218,7 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
   const unsigned int k_rank = b200_k_rank();
   // tiles are taken by CTA pairs in pair mode, by clusters that share the k blocks, by single CTAs otherwise
   constexpr unsigned int ctas_per_worker = B200_CTA_PAIR ? 2 : B200_CLUSTER_K;
-  const unsigned int worker = blockIdx.x / ctas_per_worker, n_workers = gridDim.x / ctas_per_worker;
+  const unsigned int worker = B200_BLOCK / ctas_per_worker, n_workers = B200_GRID / ctas_per_worker;
   if (threadIdx.x == 0) B200_TR(2);   // set-up done
 
   constexpr unsigned int tiles_per_batch = B200_TILES_M * B200_TILES_N;
@@ -392,9 +401,9 @@ B200_GEMM_NAME(const __grid_constant__ b200_tmap map_a, const __grid_constant__ 
       // one scratch slot per epilogue warp of the grid for epilogues that end in a grid-wide sum (whose tiles are one
       // chunk wide: of a cluster's warps, those of the first column part)
 #if B200_CLUSTER_K > 1
-      const unsigned int b200_slot = blockIdx.x * B200_X_GROUPS + ew % B200_X_GROUPS, b200_nslots = gridDim.x * B200_X_GROUPS;
+      const unsigned int b200_slot = B200_BLOCK * B200_X_GROUPS + ew % B200_X_GROUPS, b200_nslots = B200_GRID * B200_X_GROUPS;
 #else
-      const unsigned int b200_slot = blockIdx.x * B200_EPI_WARPS + ew, b200_nslots = gridDim.x * B200_EPI_WARPS;
+      const unsigned int b200_slot = B200_BLOCK * B200_EPI_WARPS + ew, b200_nslots = B200_GRID * B200_EPI_WARPS;
 #endif
       // this warp's share of the next tile, for the prefetch at the end of this one
       bool b200_nx_ok = false;
