@@ -194,6 +194,7 @@ void collect_scopes(const Stmt& s, std::set<std::pair<int, int>>& declared, std:
 struct CoopInfo {
   std::string sym;
   int width = 32;  // threads cooperating on one output element
+  int64_t extent = 0;   // terms of the reduction
   int grid_blocks = 0;  // >0: two-kernel grid-wide reduction with this many blocks in pass 1
   std::vector<std::pair<int, std::string>> scopes;  // (scope id, combine op)
 };
@@ -312,6 +313,7 @@ struct Piece {
   bool pairs = false;
   int64_t ser_work = 1;
   std::vector<int> staged;   // small read-only nodes the kernel first copies into shared memory
+  std::string alone;         // the body's text in a kernel of its own, where it differs
   std::string whole;         // the kernel's body where it is not the grid-stride loop over the stage's iterations
   // a sum kept in `b200_self` over the serial loops (`t[p] := t[p] + term`): its parts, so that several
   // lanes may share one sum
@@ -385,6 +387,8 @@ struct Builder {
   // `v := neutral; for k1 { for k2 .. { v := v (+|max|min) f(k..) } }`.  A group of threads (a
   // warp, or a whole block when there are few outputs and much to reduce) strides over the
   // flattened reduction space of one output element and combines its partial results.
+  // From here on a single output's sum is spread over many blocks.
+  static constexpr int64_t kGridSum = 32768;
   CoopInfo find_coop(const Stmt& body, int64_t par_total) {
     CoopInfo ci;
     if (!opt.enable_coop) return ci;
@@ -432,12 +436,14 @@ struct Builder {
       ci.scopes.push_back({sc->scope_id, op});
     }
     if (extent < 32) return CoopInfo{};
+    ci.extent = extent;
     ci.sym = "*";
     // few outputs and a long reduction: a whole block per output element
-    ci.width = (par_total <= 256 && extent >= 4096) ? 1024 : 32;
+    // (a single one, a loss, from 256 on: one warp took 8 us for 2130 terms)
+    ci.width = (par_total <= 256 && extent >= 4096) || (par_total == 1 && extent >= 256) ? 1024 : 32;
     // a single output fed by a very long reduction: many blocks write partial results to
     // scratch and a second, single-block kernel combines them
-    if (par_total == 1 && extent >= 32768) {
+    if (par_total == 1 && extent >= kGridSum) {
       ci.width = 1024;
       ci.grid_blocks = (int)std::min<int64_t>(296, (extent + 1023) / 1024);
     }
@@ -1184,12 +1190,17 @@ struct Builder {
         em.node_alias.clear();
       }
     }
-    std::string inner;
+    std::string inner, alone;
     int ind = 4 + 2 * (int)st.ser.size();
     if (!ci.sym.empty()) {
       st.coop = ci.width;
       if (ci.width > 32) st.block = ci.width;
-      inner = coop_body(em, *body, ci, ind);
+      // (few warps in single precision: with many, or 16-bit values to convert, there is nothing to wait for; 31 rows of
+      // 777-472-66-2, a training step, 33.9 us and 35.4, two rows of 80-1832-382-55 in half precision 14.9 and 15.7)
+      bool wide_values = true;
+      walk_scalar(*body->value, [&](const Scalar& e) { if (e.kind == Scalar::Get) wide_values = wide_values && code.prog.tn(e.tn).prec == Prec::Single; }, [](const Stmt&) {});
+      if (ci.width > 32 || (ci.extent >= 256 && st.total <= 148 * 32 && wide_values)) alone = coop_body(em, *body, ci, ind, true);
+      inner = coop_body(em, *body, ci, ind, ci.width > 32);
     } else {
       inner = em.stmt(*body, ind);
     }
@@ -1238,12 +1249,15 @@ struct Builder {
     Piece pc;
     pc.decomp = decomp;
     pc.body_text = body_text;
+    if (!alone.empty()) pc.alone = before + open + alone + close + after;
     pc.used = em.used_nodes;
     pc.written = written;
     pc.uses_merge = em.uses_merge;
     int64_t ser_work = 1;
     for (auto& d : st.ser) ser_work *= std::max<int64_t>(1, d.extent());
-    pc.fusable = opt.enable_fuse && st.total > 0 && (st.coop == 0 || st.coop == 32) &&
+    // (a single output that a whole block sums up fits the block that other small stages share)
+    const bool block_sum = st.coop == 1024 && st.total == 1;
+    pc.fusable = opt.enable_fuse && st.total > 0 && (st.coop == 0 || st.coop == 32 || block_sum) &&
                  st.total * std::max(1, st.coop) <= 16384 && ser_work <= 4096;
     if (scatter) pc.fusable = false;
     {
@@ -1255,7 +1269,11 @@ struct Builder {
       const double threads = (double)st.total * std::max(1, st.coop);
       const double rounds = std::ceil(threads / 1024.0), warps = std::ceil(std::min(threads, 1024.0) / 32.0);
       const double iters = rounds * (double)ser_work * iterations(*body) / std::max(1, st.coop);
-      if (iters * std::max(30.0, (pairs ? 12.0 : 6.0) * warps / 4.0) > 16000.0) pc.fusable = false;
+      // A warp's sums over a node that does not fit into shared memory wait for memory at every step (one row of 160-552-177-35:
+      // 23 us with the second layer in the block, 8 us without; 300 cycles a step).
+      bool far = false;
+      for (int n : em.used_nodes) far = far || (st.coop && code.prog.tn(n).bytes() > 12288);
+      if (iters * std::max(far ? 300.0 : 30.0, (pairs ? 12.0 : 6.0) * warps / 4.0) > 16000.0) pc.fusable = false;
     }
     if (opt.enable_fuse && !scatter && st.coop == 0 && st.total > 0 && !st.par.empty() && st.par[0].from == 0 && !(pairs && st.par.size() == 1)) {
       pc.body = body;
@@ -1332,7 +1350,7 @@ struct Builder {
       k_src << "  for (unsigned long long b200_g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_g < "
             << st.total << "ull; b200_g += (unsigned long long)gridDim.x * blockDim.x) {\n";
     }
-    k_src << pc.decomp << pc.body_text << "  }\n}\n\n";
+    k_src << pc.decomp << (pc.alone.empty() ? pc.body_text : pc.alone) << "  }\n}\n\n";
     src << k_src.str();
   }
 
@@ -1412,6 +1430,7 @@ struct Builder {
     std::string text;
     int64_t most = 1;                 // threads the widest stage could use
     bool ordered = false;             // some stage depends on another
+    bool block_sums = false;          // some stage sums with the whole block
     std::set<int> fresh_w, fresh_r;   // written / read since the last barrier
     // (stages that overwrite different parts of one node, the margins of a padded image, do not depend on one another)
     std::map<int, std::vector<Box>> fresh_boxes;   // node -> the parts overwritten since the last barrier, where all are known
@@ -1522,7 +1541,11 @@ struct Builder {
           text += "    if (b200_on && b200_s == 0u) {\n" + pc.after + "    }\n  }\n";
         } else {
           text += "  {\n";
-          if (st.coop) {
+          if (st.coop > 32) {
+            ordered = true;
+            block_sums = true;
+            text += "  const unsigned int b200_t = threadIdx.x;\n  {\n  const unsigned int b200_g = 0u;\n";
+          } else if (st.coop) {
             text += "  const unsigned int b200_t = threadIdx.x & 31u;\n";
             text += "  for (unsigned int b200_g = B200_FIRST >> 5; b200_g < " + std::to_string(st.total) + "u; b200_g += B200_STEP >> 5) {\n";
           } else {
@@ -1552,6 +1575,7 @@ struct Builder {
       }
     std::sort(small.begin(), small.end(), [&](int a, int b) { return code.prog.tn(a).bytes() < code.prog.tn(b).bytes() || (code.prog.tn(a).bytes() == code.prog.tn(b).bytes() && a < b); });
     std::string decls, load, land, store;
+    if (block_sums) decls = "  __shared__ double b200_red[32];\n";
     size_t bytes = 0;
     for (int n : small) {
       const Tnode& t = code.prog.tn(n);
@@ -2436,6 +2460,14 @@ struct Builder {
           }
         }
       }
+      if (opt.enable_fuse) {
+        const std::vector<std::vector<size_t>> parts = group_from(i);
+        if (!parts.empty()) {
+          emit_pointwise_group(parts, &out);
+          i = parts.back().back() + 1;
+          continue;
+        }
+      }
       if (row_candidate(i)) {
         // the longest run that stays row-independent; runs made only of small stages are left to
         // the single-block fusion below, which also takes stages of unrelated shapes
@@ -2454,14 +2486,6 @@ struct Builder {
           continue;
         }
       }
-      if (opt.enable_fuse) {
-        const std::vector<std::vector<size_t>> parts = group_from(i);
-        if (!parts.empty()) {
-          emit_pointwise_group(parts, &out);
-          i = parts.back().back() + 1;
-          continue;
-        }
-      }
       // (a long chain over thousands of elements -- the momentum update of a 300 x 100 layer -- is a kernel of
       // its own even where one block could take it: that block spent 30 us on four passes over it)
       if (opt.enable_fuse) {
@@ -2473,9 +2497,24 @@ struct Builder {
         }
       }
       if (fusable(i)) {
+        // A sum by the whole block joins the stages whose values it sums; where it comes first, only what reads it follows
+        // (the first pointwise steps of a gradient have nothing to do with the loss and are better off over a grid).
         std::vector<size_t> run;
+        std::set<int> run_writes;
+        auto depends = [&](size_t k) {
+          auto p = pieces.find(k);
+          if (p == pieces.end()) return false;
+          for (int n : p->second.used)
+            if (run_writes.count(n)) return true;
+          return false;
+        };
         size_t j = i;
-        while (j < code.stages.size() && fusable(j) && (j == i || (chain_from(j).size() < 3 && group_from(j).empty()))) run.push_back(j++);
+        while (j < code.stages.size() && fusable(j) && (j == i || (chain_from(j).size() < 3 && group_from(j).empty()))) {
+          if (j > i && (code.stages[i].coop > 32 || code.stages[j].coop > 32) && !depends(j)) break;
+          run_writes.insert(code.stages[j].writes.begin(), code.stages[j].writes.end());
+          if (code.stages[j].kind == Stage::Memset) run_writes.insert(code.stages[j].memset_tn);
+          run.push_back(j++);
+        }
         int kernels = 0;
         for (size_t k : run) kernels += code.stages[k].kind != Stage::Memset;
         if (run.size() >= 2 && kernels >= 1) {
@@ -2496,7 +2535,7 @@ struct Builder {
   // A group of threads per output element: each Local_scope reduction runs over its flattened
   // loop space strided by the group width, partial results are combined with shuffles (and
   // shared memory across warps), and thread 0 of the group evaluates and stores the rest.
-  std::string coop_body(Emitter& em, const Stmt& set, const CoopInfo& ci, int ind) {
+  std::string coop_body(Emitter& em, const Stmt& set, const CoopInfo& ci, int ind, bool unroll) {
     std::string out;
     std::string padding((size_t)ind, ' ');
     const Tnode& t = code.prog.tn(set.tn);
@@ -2522,23 +2561,35 @@ struct Builder {
         std::string lv = "b200_l" + std::to_string(e.scope_id);
         const bool narrow = total < (1ll << 31);
         const std::string IT = narrow ? "unsigned int" : "unsigned long long", SUF = narrow ? "u" : "ull";
-        out += padding + "for (" + IT + " " + lv + " = b200_t; " + lv + " < " + std::to_string(total) + SUF + "; " + lv +
-               " += " + std::to_string(ci.width) + "u) {\n";
+        std::string step;
         std::string rem = lv;
         for (size_t i = red.size(); i-- > 0;) {
           const LoopDim& d = red[i];
           std::string ext = std::to_string(d.extent()) + SUF;
           std::string val = i == 0 ? rem : "(" + rem + " % " + ext + ")";
-          out += padding + "  const unsigned int " + d.sym + " = (unsigned int)" + val +
-                 (d.from ? " + " + std::to_string(d.from) : std::string()) + ";\n";
+          step += padding + "  const unsigned int " + d.sym + " = (unsigned int)" + val +
+                  (d.from ? " + " + std::to_string(d.from) : std::string()) + ";\n";
           if (i != 0) {
             std::string nr = "b200_q" + std::to_string(e.scope_id) + "_" + std::to_string(i);
-            out += padding + "  const " + IT + " " + nr + " = " + rem + " / " + ext + ";\n";
+            step += padding + "  const " + IT + " " + nr + " = " + rem + " / " + ext + ";\n";
             rem = nr;
           }
         }
-        out += em.stmt(*inner, ind + 2);
-        out += padding + "}\n";
+        step += em.stmt(*inner, ind + 2);
+        // The lanes take the same whole number of steps, so that the loads of eight are under way together, and a shorter last
+        // one: sums by a block, and a warp's of 256 terms and more in a kernel of their own (10 rows of 496-2032-200-14 in single precision 34 -> 19 us).
+        // Not among other small stages, whose code runs once: two rows of 80-1832-382-55 took 16.6 us instead of 15.0.
+        const int64_t whole = unroll ? total / ci.width : 0, rest = unroll ? total % ci.width : 0;
+        if (!unroll)
+          out += padding + "for (" + IT + " " + lv + " = b200_t; " + lv + " < " + std::to_string(total) + SUF + "; " + lv + " += " + std::to_string(ci.width) + "u) {\n" +
+                 step + padding + "}\n";
+        if (whole > 0) {
+          out += "#pragma unroll 8\n" + padding + "for (" + IT + " " + lv + "_k = 0; " + lv + "_k < " + std::to_string(whole) + SUF + "; ++" + lv + "_k) {\n" + padding +
+                 "  const " + IT + " " + lv + " = " + lv + "_k * " + std::to_string(ci.width) + SUF + " + b200_t;\n" + step + padding + "}\n";
+        }
+        if (rest > 0)
+          out += padding + "if (b200_t < " + std::to_string(rest) + "u) {\n" + padding + "  const " + IT + " " + lv + " = " + std::to_string(whole * ci.width) + SUF +
+                 " + b200_t;\n" + step + padding + "}\n";
         const std::string fn = op == "add" ? "sum" : op;
         if (ci.width > 32) out += padding + name + " = b200_block_" + fn + "(" + name + ", b200_red);\n";
         else out += padding + name + " = b200_warp_" + fn + "(" + name + ");\n";
