@@ -171,3 +171,40 @@ def test_small_table(device, size, cin, cout, kernel, stride):
     plain, _ = run_device(device, ir, inputs, options="gemm=0")
     assert np.array_equal(got["y"], plain["y"])
     compare(ir, got, run_oracle(ir, inputs), rtol=1e-3, atol=1e-3, only=["y"])
+
+
+@pytest.mark.parametrize("m,n,k", [(333, 40, 131), (64, 65, 519), (200, 72, 30)])
+@pytest.mark.parametrize("a_mmajor", [False, True])
+@pytest.mark.parametrize("prec", ["bfloat16", "half", "single"])
+@pytest.mark.parametrize("between", [None, "reads", "overwrites"])
+def test_operand_gathered_where_it_is_made(device, m, n, k, a_mmajor, prec, between):
+    """A pointwise stage makes the operand: its elements are stored and gathered by one kernel, also when another stage reads
+    the node in between; not when what it was made from has changed by then and a copy would still have to be made."""
+    r = Routine("made_%d_%d_%d" % (m, n, k))
+    shape = [k, m] if a_mmajor else [m, k]
+    src = r.tn("src", prec, shape)
+    scale = r.tn("scale", "single", [shape[1]], read_only=True)
+    w = r.tn("w", prec, [n, k], read_only=True)
+    x, y, z = r.tn("x", prec, shape), r.tn("y", "single", [m, n]), r.tn("z", "single", shape)
+    p, q, s, t, u, v = r.syms(6)
+    body = [loops([(p, shape[0]), (q, shape[1])], Set(x, (p, q), un("tanh", src[p, q] * scale[q])))]
+    if between == "reads":
+        body.append(loops([(s, shape[0]), (t, shape[1])], Set(z, (s, t), x[s, t] + 1.0)))
+    elif between == "overwrites":
+        body.append(loops([(u, shape[0]), (v, shape[1])], Set(src, (u, v), src[u, v] * 0.5)))
+    i, j, kk = r.syms(3)
+    acc = W.reduce_scope(r, "acc", "single", [(kk, k)], lambda: (x[kk, i] if a_mmajor else x[i, kk], w[j, kk]), orig=(i, j))
+    body.append(loops([(i, m), (j, n)], Set(y, (i, j), acc)))
+    r.body = Seq(body)
+    g = np.random.default_rng(4)
+    inputs = {c.ident: W.store(c.prec, (g.standard_normal(c.dims) / (np.sqrt(k) if c.ident == "w" else 1.0)).astype(np.float32))
+              for c in (src, scale, w)}
+    want = run_oracle(r, inputs)
+    got, info = run_device(device, r, inputs)
+    notes = [s["note"] or "" for s in info["stages"]]
+    if 2 * m * n * k >= 4e6:
+        assert any("gathers operands" in c for c in notes), notes
+        lies = prec != "single" and (m if a_mmajor else k) % 8 == 0      # on a tensor map as it is
+        assert any("where it is made" in c for c in notes) == (between != "overwrites" and not lies), notes
+    tol = dict(rtol=1e-5, atol=4e-6) if prec == "single" else dict(rtol=2e-2, atol=4e-3)
+    compare(r, got, want, only=["x", "y", "z"] if between == "reads" else ["x", "y"], **tol)
