@@ -115,6 +115,7 @@ struct Stage {
   bool launches() const { return kind != Memset && !in_group; }
   int group = 1;                 // > 1: the launch also runs the group - 1 stages behind this one
   bool in_group = false;         // one of those
+  bool clears = false;           // a kernel (or part of one) that does nothing but clear nodes: listed as a clear
   int memset_tn = -1;
   std::string kernel;            // kernel symbol in the routine's module
   std::vector<KArg> args;
