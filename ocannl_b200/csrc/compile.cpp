@@ -720,10 +720,13 @@ struct Builder {
     auto sum_of = [&](const std::string& a, const std::string& b) {
       return pairs ? "b200_f2{" + a + ".x + " + b + ".x, " + a + ".y + " + b + ".y}" : a + " + " + b;
     };
+    // Values of the tiled loop that are combined at a time, between two barriers: as many as 40 KB of partials hold.  (One at
+    // a time, ten outputs over 500 rows spent most of their 10 us there, ten times two barriers and a chain of 16 sums.)
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(e0, 40960 / (BY * Q * CW * (pairs ? 8 : prec_bytes(t.prec)))));
     std::ostringstream k;
     k << "extern \"C\" __global__ void __launch_bounds__(" << 32 * BY << ") " << st.kernel << "(";
     emit_params(k, st, em, written);
-    k << ") {\n" << kGridEntry << statics << "  __shared__ " << T << " b200_part[" << BY << "][" << Q * CW + 1 << "];\n"
+    k << ") {\n" << kGridEntry << statics << "  __shared__ " << T << " b200_part[" << BY << "][" << per * Q * CW + 1 << "];\n"
       << "  const unsigned int b200_c = threadIdx.x % " << CWS << "u, b200_sub = threadIdx.y * " << XR << "u + threadIdx.x / " << CWS << "u;\n"
       << "  for (unsigned int b200_u = blockIdx.x; b200_u < " << groups * Z << "u; b200_u += gridDim.x) {\n"
       << "    const unsigned int b200_g0 = (b200_u % " << groups << "u) * " << Q * CW << "u, b200_z = b200_u / " << groups << "u;\n"
@@ -739,10 +742,10 @@ struct Builder {
       << (tiled ? o_sym : std::string("b200_one")) << ") {\n"
       << "            " << T << " b200_acc = b200_accs[b200_q][" << (tiled ? o_sym : std::string("0")) << "];\n            " << step << "\n            b200_accs[b200_q]["
       << (tiled ? o_sym : std::string("0")) << "] = b200_acc;\n          }\n        }\n      }\n";
-    // combine: lane groups by shuffles, then the BY rows through shared memory, one tiled value at a time
-    k << "#pragma unroll\n    for (unsigned int " << (tiled ? o_sym : std::string("b200_one")) << " = 0; " << (tiled ? o_sym : std::string("b200_one")) << " < " << E0 << "u; ++"
-      << (tiled ? o_sym : std::string("b200_one")) << ") {\n#pragma unroll\n      for (int b200_q = 0; b200_q < " << QS << "; ++b200_q) {\n        " << T
-      << " b200_acc = b200_accs[b200_q][" << (tiled ? o_sym : std::string("0")) << "];\n";
+    // combine: lane groups by shuffles, then the BY rows through shared memory, `per` values of the tiled loop at a time
+    k << "#pragma unroll\n    for (unsigned int b200_o0 = 0; b200_o0 < " << E0 << "u; b200_o0 += " << per << "u) {\n"
+      << "#pragma unroll\n      for (unsigned int b200_oo = 0; b200_oo < " << per << "u; ++b200_oo) {\n        if (b200_o0 + b200_oo >= " << E0 << "u) break;\n"
+      << "#pragma unroll\n      for (int b200_q = 0; b200_q < " << QS << "; ++b200_q) {\n        " << T << " b200_acc = b200_accs[b200_q][b200_o0 + b200_oo];\n";
     if (XR > 1) {
       k << "#pragma unroll\n        for (unsigned int b200_s = " << CWS << "u; b200_s < 32u; b200_s <<= 1) {\n";
       if (pairs)
@@ -751,9 +754,10 @@ struct Builder {
         k << "          const " << T << " b200_w = __shfl_xor_sync(0xffffffffu, b200_acc, b200_s);\n";
       k << "          b200_acc = " << sum_of("b200_acc", "b200_w") << ";\n        }\n";
     }
-    k << "        if (threadIdx.x < " << CWS << "u) b200_part[threadIdx.y][b200_q * " << CWS << " + b200_c] = b200_acc;\n      }\n      __syncthreads();\n"
-      << "      for (unsigned int b200_i = threadIdx.y * 32u + threadIdx.x; b200_i < " << Q * CW << "u; b200_i += " << 32 * BY << "u) {\n"
-      << "        const unsigned int b200_g = b200_g0 + b200_i;\n        if (b200_g < " << outputs << "u) {\n" << decomp
+    k << "        if (threadIdx.x < " << CWS << "u) b200_part[threadIdx.y][(b200_oo * " << QS << " + b200_q) * " << CWS << " + b200_c] = b200_acc;\n      }\n      }\n      __syncthreads();\n"
+      << "      for (unsigned int b200_i = threadIdx.y * 32u + threadIdx.x; b200_i < " << per * Q * CW << "u; b200_i += " << 32 * BY << "u) {\n"
+      << "        const unsigned int b200_g = b200_g0 + b200_i % " << Q * CW << "u, " << (tiled ? o_sym : std::string("b200_one")) << " = b200_o0 + b200_i / " << Q * CW
+      << "u;\n        if (b200_g < " << outputs << "u && " << (tiled ? o_sym : std::string("b200_one")) << " < " << E0 << "u) {\n" << decomp
       << "          " << T << " b200_s = b200_part[0][b200_i];\n#pragma unroll\n          for (int b200_y = 1; b200_y < " << BY << "; ++b200_y) b200_s = "
       << sum_of("b200_s", "b200_part[b200_y][b200_i]") << ";\n";
     if (pairs) {
