@@ -51,6 +51,42 @@ void walk_scalar(const Scalar& e, const std::function<void(const Scalar&)>& fs,
   for (auto& a : e.args) walk_scalar(*a.s, fs, ft);
 }
 
+// Nodes whose values are compared, gate something or are truncated, and those that they are computed from: a change in the
+// last bits of such a value may change a result by a whole step.  (A position read by a value, `GetDyn`, is one too.)
+std::set<int> find_deciding(const Program& P) {
+  static const std::set<std::string> first = {"relu_gate", "sat01_gate", "where", "trunc", "not"},
+                                     both = {"lt", "eq", "ne", "or", "and", "mod"};
+  std::set<int> found;
+  std::map<int, std::set<int>> made_from;
+  walk_stmt(*P.body, [](const Scalar&) {}, [&](const Stmt& st) {
+    if (st.kind != Stmt::Set) return;
+    std::set<int> all;
+    bool open = is_int_prec(P.tn(st.tn).prec);   // values of scopes are followed to the whole assignment
+    auto reads = [&](const Scalar& e, std::set<int>& into) {
+      walk_scalar(e, [&](const Scalar& x) {
+        if (x.kind == Scalar::Get || x.kind == Scalar::GetDyn || x.kind == Scalar::GetMerge) into.insert(x.tn);
+        if (x.kind == Scalar::GetLocal) open = open || &into == &found;
+      }, [](const Stmt&) {});
+    };
+    reads(*st.value, all);
+    walk_scalar(*st.value, [&](const Scalar& x) {
+      if (x.kind == Scalar::GetDyn || (x.kind == Scalar::LocalScope && is_int_prec(P.tn(x.tn).prec))) open = true;
+      for (size_t a = 0; a < x.args.size(); ++a)
+        if (both.count(x.op) || (a == 0 && first.count(x.op))) reads(*x.args[a].s, found);
+    }, [](const Stmt&) {});
+    if (open) found.insert(all.begin(), all.end());
+    made_from[st.tn].insert(all.begin(), all.end());
+  });
+  std::vector<int> todo(found.begin(), found.end());
+  while (!todo.empty()) {
+    const int n = todo.back();
+    todo.pop_back();
+    for (int m : made_from[n])
+      if (found.insert(m).second) todo.push_back(m);
+  }
+  return found;
+}
+
 // Is loop symbol `s` safe to run in parallel over `body`?  Sufficient condition: every
 // node written in the body is written only at positions that carry `s` as a plain iterator
 // on one fixed axis, and every read of such a node carries `s` on that same axis — so
@@ -3530,6 +3566,7 @@ Code compile_program(Program prog, const CompileOptions& opt) {
   Code code;
   code.prog = std::move(prog);
   if (opt.enable_gemm || opt.enable_attn) avoid_kernel_names(code.prog);
+  code.prog.deciding = find_deciding(code.prog);
   Builder b{code, opt};
   b.run();
   return code;

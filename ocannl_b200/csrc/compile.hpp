@@ -62,6 +62,7 @@ struct GemmPlan {
   bool accumulate = false;           // beta = 1: add to the existing output (form B without zero_out)
   Prec in_prec = Prec::Bfloat16;     // operand precision (bf16 / half; single runs as tf32)
   bool may_split = false;            // an fp32 accumulation whose K may be cut into work units (see split_k)
+  bool decides = false;              // a value of the result on the other side of a threshold changes what follows by a step
   int siblings = 1;                  // contractions of one launch, this one included (group_contractions)
   int split_k = 1;                   // >1: that many work units per tile, each over a slice of K, added with vector reds
   std::string epilogue;              // generated device code, see codegen

@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -122,6 +123,7 @@ struct Program {
   std::vector<StaticSym> statics;
   int merge_node = -1;
   StmtP body;
+  std::set<int> deciding;  // nodes that decide comparisons, gates or truncations (filled by the compile step)
   const Tnode& tn(int id) const {
     auto it = tn_index.find(id);
     if (it == tn_index.end()) throw Error(-3, "b200ir: unknown tensor node id " + std::to_string(id));

@@ -1,0 +1,41 @@
+"""Which contractions share their k blocks over a cluster (another order of the sums): none whose result a gate or a comparison
+reads, directly or through what is made of it; the others of the same routine as before.  Plans only, no GPU."""
+import pytest
+
+from ocannl_b200 import backend as bk
+from ocannl_b200 import workloads as W
+from ocannl_b200.low_level import Routine, Seq, Set, binop, loops, un, where
+
+
+def _clusters(ir):
+    code = bk.Code(ir)
+    try:
+        return ["over a cluster" in (s["note"] or "") for s in code.info()["stages"] if s["kind"] == "gemm"]
+    finally:
+        code.free()
+
+
+@pytest.mark.parametrize("prec", ["single", "bfloat16"])
+def test_training_steps_keep_the_order_of_gated_sums(prec):
+    forward = _clusters(W.mlp_forward(rows=200, dims=(784, 1024, 1024, 10), wprec=prec))
+    assert forward[1:] == [True, True]
+    step = _clusters(W.mlp_train_update(rows=200, dims=(784, 1024, 1024, 10), wprec=prec))
+    assert step[:2] == [False, False] and step[2]      # hidden layers: gated; logits: nothing compares them
+
+
+@pytest.mark.parametrize("use,clustered", [("none", True), ("relu", True), ("gate", False), ("lt", False), ("where", False), ("behind", False), ("value of where", True)])
+def test_what_counts_as_a_decision(use, clustered):
+    m, n, k = 64, 64, 1024
+    r = Routine("decide_" + use.replace(" ", "_"))
+    a, b = r.tn("a", "bfloat16", [m, k], read_only=True), r.tn("b", "bfloat16", [n, k], read_only=True)
+    c, d, e = r.tn("c", "single", [m, n]), r.tn("d", "single", [m, n]), r.tn("e", "single", [m, n])
+    i, j, p, q, s, u, v = r.syms(7)
+    body = [loops([(i, m), (j, n)], Set(c, (i, j), W.reduce_scope(r, "acc", "single", [(p, k)], lambda: (a[i, p], b[j, p]))))]
+    value = {"none": lambda: c[q, s] * 2.0, "relu": lambda: un("relu", c[q, s]), "gate": lambda: binop("relu_gate", c[q, s], d[q, s]),
+             "lt": lambda: binop("lt", c[q, s], d[q, s]), "where": lambda: where(c[q, s], d[q, s], e[q, s]),
+             "behind": lambda: un("exp", c[q, s]), "value of where": lambda: where(d[q, s], c[q, s], 0.0)}[use]
+    body.append(loops([(q, m), (s, n)], Set(e, (q, s), value())))
+    if use == "behind":
+        body.append(loops([(u, m), (v, n)], Set(d, (u, v), binop("relu_gate", e[u, v], d[u, v]))))
+    r.body = Seq(body)
+    assert _clusters(r) == [clustered]
