@@ -27,6 +27,8 @@
 //   B200_A_KMAJOR/B_KMAJOR    1: k is the contiguous axis of the operand, 0: m/n is
 //   B200_IDESC                tcgen05 instruction descriptor (formats, majors, M, N)
 //   B200_TMEM_COLS            power of two >= 2*B200_BN (and >= 32)
+//   B200_CLUSTER_K            > 1: CTAs that share the k blocks of a tile (undefined: one); B200_WARP_COLS: columns a warp finishes
+//   B200_BLOCK / B200_GRID    the kernel's block index and block count (a device function of a launch group: its share)
 //   B200_EPI_PARAMS           extra kernel parameters (node pointers) of the epilogue
 //   B200_EPILOGUE_ROW(...)    statement block evaluated per (row, 32-column chunk), see below
 #ifndef B200_GEMM_SM100_CUH
