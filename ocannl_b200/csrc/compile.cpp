@@ -2942,6 +2942,8 @@ struct Builder {
       const Tnode& t = code.prog.tn(op.tn);
       const Stmt& set = *pieces[maker].any_body;
       o << "        " << T << " b200_m = (" << T << ")0;\n        if (b200_row_ok && b200_j0 + b200_e < " << num(inner_real) << ") {\n          " << IT << " b200_w = b200_p;\n";
+      for (auto& d : code.stages[maker].ser)   // (loops of one iteration that the node does not carry)
+        o << "          const unsigned int " << d.sym << " = " << d.from << "u;\n";
       for (size_t a = t.dims.size(); a-- > 0;) {
         if (set.idcs[a].kind == Index::Iter) o << "          const unsigned int " << set.idcs[a].sym << " = (unsigned int)(" << (a ? "b200_w % " + num(t.dims[a]) : std::string("b200_w")) << ");\n";
         if (a) o << "          b200_w /= " << num(t.dims[a]) << ";\n";

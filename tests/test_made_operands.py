@@ -1,0 +1,70 @@
+"""Which pointwise stages may make a contraction's operand where it is gathered, and that every form of such a stage
+compiles: the gathering kernel gives the maker its loops and nothing else.  Plans and compilation, which need no GPU, and
+one run of each form."""
+import numpy as np
+import pytest
+
+from ocannl_b200 import backend as bk
+from ocannl_b200 import workloads as W
+from ocannl_b200.low_level import Routine, Seq, Set, loops, un
+from tests.parity import compare, run_device, run_oracle
+
+
+def _stages(ir, options=None):
+    code = bk.Code(ir, options)      # (compiles every kernel of the routine)
+    try:
+        return code.info()["stages"]
+    finally:
+        code.free()
+
+
+def _made(stages):
+    return any("where it is made" in (s["note"] or "") for s in stages)
+
+
+def _contraction(r, x, body, m, n, k):
+    """`body`, which makes x, and y := x w^T behind it."""
+    w, y = r.tn("w", x.prec, [n, k], read_only=True), r.tn("y", "single", [m, n])
+    i, j, kk = r.syms(3)
+    acc = W.reduce_scope(r, "acc", "single", [(kk, k)], lambda: (x[i, kk], w[j, kk]), orig=(i, j))
+    r.body = Seq([body, loops([(i, m), (j, n)], Set(y, (i, j), acc))])
+    return r
+
+
+M, N, K = 333, 40, 333      # (rows of 666 or 1332 bytes: not on a tensor map)
+
+
+@pytest.mark.parametrize("prec", ["bfloat16", "half", "single"])
+@pytest.mark.parametrize("outer", [True, False])
+@pytest.mark.parametrize("read", ["value", "twice", "not"])
+def test_loops_of_one_iteration(built_lib, prec, outer, read):
+    """A loop of one iteration that the written node does not carry: a batch or a channel of one."""
+    r = Routine("unit_loop_%s" % read)
+    src, one = r.tn("src", prec, [1, M, K], read_only=True), r.tn("one", "single", [1, K], read_only=True)
+    x = r.tn("x", prec, [M, K])
+    p, q, e = r.syms(3)
+    value = {"value": lambda: un("tanh", src[e, p, q]), "twice": lambda: src[e, p, q] * one[e, q], "not": lambda: un("tanh", src[0, p, q])}[read]
+    nest = [(e, 1), (p, M), (q, K)] if outer else [(p, M), (e, 1), (q, K)]
+    stages = _stages(_contraction(r, x, loops(nest, Set(x, (p, q), value())), M, N, K))
+    assert stages[-1]["kind"] == "gemm" and _made(stages), stages
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["bfloat16", "single"])
+def test_loops_of_one_iteration_on_the_device(device, prec):
+    """Tolerances of the contractions of gathered operands: 2e-2 for 16-bit operands, 1e-5 where they travel in two parts."""
+    r = Routine("unit_loop")
+    src, one = r.tn("src", prec, [1, M, K], read_only=True), r.tn("one", "single", [1, K], read_only=True)
+    x = r.tn("x", prec, [M, K])
+    p, q, e = r.syms(3)
+    _check(device, _contraction(r, x, loops([(p, M), (e, 1), (q, K)], Set(x, (p, q), src[e, p, q] * one[e, q])), M, N, K), prec)
+
+
+def _check(device, ir, prec, statics=({},)):
+    g = np.random.default_rng(6)
+    inputs = {t.ident: W.store(t.prec, (g.standard_normal(t.dims) / (np.sqrt(K) if t.ident == "w" else 1.0)).astype(np.float32))
+              for t in ir.params() if t.read_only}
+    want = run_oracle(ir, inputs, statics=statics)
+    got, _ = run_device(device, ir, inputs, statics=statics)
+    tol = dict(rtol=1e-5, atol=4e-6) if prec == "single" else dict(rtol=2e-2, atol=4e-3)
+    compare(ir, got, want, only=["x", "y"], **tol)
