@@ -2837,14 +2837,17 @@ struct Builder {
       return -1;
     bool plain = true;
     std::set<int> reads;
+    auto position = [&](const Index& ix) {   // the gathering kernel has no static indices
+      for (auto& sy : code.prog.statics)
+        if (ix.uses(sy.sym)) plain = false;
+    };
     walk_scalar(*pc.any_body->value, [&](const Scalar& e) {
       if (e.kind == Scalar::LocalScope || e.kind == Scalar::GetLocal || e.kind == Scalar::GetMerge) plain = false;
+      if (e.kind == Scalar::EmbedIdx) position(e.idx);
       if (e.kind == Scalar::Get || e.kind == Scalar::GetDyn) {
         if (e.tn == op.tn) plain = false;
         reads.insert(e.tn);
-        for (auto& ix : e.idcs)
-          for (auto& sy : code.prog.statics)
-            if (ix.uses(sy.sym)) plain = false;
+        for (auto& ix : e.idcs) position(ix);
       }
     }, [](const Stmt&) {});
     for (size_t i = (size_t)j + 1; i < code.stages.size(); ++i) {
