@@ -2832,6 +2832,7 @@ struct Builder {
     }
     if (j < 0 || code.stages[(size_t)j].kind != Stage::Generic || !pieces.count((size_t)j)) return -1;
     const Piece& pc = pieces[(size_t)j];
+    if (code.stages[(size_t)j].total <= 0) return -1;   // (a loop of no iterations: nothing is assigned)
     if (!pc.any_body || pc.any_body->kind != Stmt::Set || pc.any_body->tn != op.tn || pc.coop != 0 || pc.ser_work != 1 || pc.uses_merge || pc.sum ||
         !pc.whole.empty() || !pc.staged.empty() || pc.written.size() != 1 || !covers_node(*pc.any_body, pc.par))
       return -1;

@@ -96,3 +96,11 @@ def _check(device, ir, prec, statics=({},)):
     scale = max(1.0, float(np.abs(W.load(prec, want["x"])).max()) / 4.0)     # (the absolute part is that of operands of unit variance)
     tol = dict(rtol=1e-5, atol=4e-6 * scale) if prec == "single" else dict(rtol=2e-2, atol=4e-3 * scale)
     compare(ir, got, want, only=["x", "y"], **tol)
+
+
+def test_loop_without_iterations(built_lib):
+    r = Routine("empty_loop")
+    src, x = r.tn("src", "bfloat16", [M, K], read_only=True), r.tn("x", "bfloat16", [M, K])
+    p, q, e = r.syms(3)
+    stages = _stages(_contraction(r, x, loops([(p, M), (e, 0), (q, K)], Set(x, (p, q), un("tanh", src[p, q]))), M, N, K))
+    assert not _made(stages), stages
