@@ -2753,7 +2753,7 @@ struct Builder {
     int folded = -1;
     size_t at_stage = code.stages.size();
     Emitter::Res made;
-    for (size_t i = 0; i < todo.size() && folded < 0; ++i) {
+    for (size_t i = 0; opt.enable_fuse && i < todo.size() && folded < 0; ++i) {
       const int j = pointwise_maker(*todo[i]);
       bool fits = j >= 0;
       for (auto* op : todo)

@@ -104,3 +104,13 @@ def test_loop_without_iterations(built_lib):
     p, q, e = r.syms(3)
     stages = _stages(_contraction(r, x, loops([(p, M), (e, 0), (q, K)], Set(x, (p, q), un("tanh", src[p, q]))), M, N, K))
     assert not _made(stages), stages
+
+
+def test_a_launch_for_every_statement(built_lib):
+    """Without fusion the maker keeps a launch of its own."""
+    r = Routine("unfused")
+    src, x = r.tn("src", "bfloat16", [M, K], read_only=True), r.tn("x", "bfloat16", [M, K])
+    p, q = r.syms(2)
+    ir = _contraction(r, x, loops([(p, M), (q, K)], Set(x, (p, q), un("tanh", src[p, q]))), M, N, K)
+    assert _made(_stages(ir)) and not _made(_stages(ir, "fuse=0"))
+    assert len(_stages(ir, "fuse=0")) == len(_stages(ir)) + 1
