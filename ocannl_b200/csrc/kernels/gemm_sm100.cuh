@@ -209,8 +209,8 @@ B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_s
     asm volatile("tcgen05.relinquish_alloc_permit." B200_CG ".sync.aligned;" ::: "memory");
   }
   // Set-up touches no global memory and is over, block-wide barrier included, before the grids ahead of this one
-  // end; the threads that read or write global memory (the producer, the epilogue) then wait for those grids
-  // themselves, right ahead of their first access.
+  // end; every role then waits for those grids itself: the producer and the epilogue right ahead of their first access
+  // to global memory, the MMA issuer ahead of its first wait for operands, whose limit would count those grids' time.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   b200_cluster_sync();   // the peer's barriers are initialised before anything is signalled on them
@@ -294,6 +294,7 @@ B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_s
     if (cta_rank == 0u && b200_elect()) {
       unsigned int slot = 0, phase = 0, acc = 0, acc_phase = 0;
       bool live = true;
+      asm volatile("griddepcontrol.wait;" ::: "memory");   // (the limit of the waits below is for this kernel's own work)
       // operand descriptors of ring slot 0.  k-major: rows of 128 bytes, 8-row groups 1024 bytes
       // apart.  m/n-major: 64-element (128-byte) chunks of m/n, k rows 128 bytes apart, 8-row groups
       // 1024 bytes apart, chunks one box apart.
