@@ -1028,6 +1028,97 @@ struct Builder {
     return true;
   }
 
+  // Accumulations at few moving positions, by position.  `t[.., c * o + k, ..] := t[same] + term`: a thread takes one
+  // position of t and walks the loops in their order, without the innermost symbol of every moving axis: the position
+  // gives that one.  Every position so gets its terms one after the other in the order of the loops, as when a thread
+  // walks all of them by itself, and the sums have the same bits from run to run, which atomic adds would not give.
+  struct Solved {
+    size_t within = 0;   // the serial loop that fixes the symbol
+    std::string text;    // leaves out the iterations that do not reach the position, declares the symbol
+  };
+  bool positions_of(Stage& st, const Stmt& set, std::vector<Solved>* solved, Indices* at) {
+    if (opt.bounds) return false;   // (an access outside the node has to be seen)
+    const Tnode& t = code.prog.tn(set.tn);
+    const int64_t limit = 1 << 28;  // keeps the arithmetic on positions in 32 bits
+    std::map<std::string, int> axes;   // serial symbol -> axes it is on
+    auto terms = [&](const Index& ix) {
+      std::vector<std::pair<int64_t, std::string>> v = ix.terms;
+      if (ix.kind == Index::Iter) v = {{1, ix.sym}};
+      if (ix.kind != Index::Iter && ix.kind != Index::Affine) v.clear();
+      return v;
+    };
+    auto serial = [&](const std::string& s) {
+      for (size_t i = 0; i < st.ser.size(); ++i)
+        if (st.ser[i].sym == s) return (int)i;
+      return -1;
+    };
+    for (auto& ix : set.idcs)
+      for (auto& d : st.ser) axes[d.sym] += ix.uses(d.sym);
+    std::vector<LoopDim> par;
+    std::set<std::string> given;
+    *at = set.idcs;
+    for (size_t a = 0; a < set.idcs.size(); ++a) {
+      const auto on = terms(set.idcs[a]);
+      int last = -1, outer = -1;      // the symbol that the position gives; the innermost of the others
+      int64_t c = 0, most = std::abs(set.idcs[a].fixed) + t.dims[a];
+      std::set<std::string> seen;
+      for (auto& v : on) {
+        if (!seen.insert(v.second).second) return false;
+        const int i = serial(v.second);
+        if (i < 0) {
+          for (auto& d : st.par)
+            if (d.sym == v.second) par.push_back(d);
+          continue;
+        }
+        if (st.ser[(size_t)i].from < 0 || std::abs(v.first) > limit || st.ser[(size_t)i].to > limit) return false;
+        most += std::abs(v.first) * st.ser[(size_t)i].to;
+        if (i > last) { last = i; c = v.first; }
+      }
+      if (last < 0) continue;
+      if (axes[st.ser[(size_t)last].sym] != 1 || c == 0 || most > limit) return false;
+      for (auto& v : on) {
+        const int i = serial(v.second);
+        if (i != last) outer = std::max(outer, i);
+      }
+      if (outer < 0 || on.size() != seen.size()) return false;
+      const LoopDim& e = st.ser[(size_t)last];
+      const std::string pos = "b200_at" + std::to_string(a), n = "b200_n" + std::to_string(a);
+      const std::string pad(6 + 2 * (size_t)outer, ' '), v_at = c == 1 ? n : "(" + n + " / " + std::to_string(c) + ")";
+      std::string text = pad + "const int " + n + " = (int)" + pos + " - (" + std::to_string(set.idcs[a].fixed);
+      for (auto& v : on)
+        if (v.second != e.sym) text += " + " + std::to_string(v.first) + " * (int)" + v.second;
+      text += ");\n" + pad + "if (" + (c == 1 || c == -1 ? std::string() : n + " % " + std::to_string(c) + " != 0 || ") + v_at + " < " + std::to_string(e.from) +
+              " || " + v_at + " > " + std::to_string(e.to) + ") continue;\n" + pad + "const unsigned int " + e.sym + " = (unsigned int)" + v_at + ";\n";
+      solved->push_back({(size_t)outer, text});
+      given.insert(e.sym);
+      (*at)[a] = Index();
+      (*at)[a].kind = Index::Iter;
+      (*at)[a].sym = pos;
+      par.push_back({pos, 0, t.dims[a] - 1});
+    }
+    if (given.empty()) return false;
+    // the loops that remain, and where among them each symbol is fixed
+    std::vector<LoopDim> ser;
+    std::vector<size_t> place(st.ser.size(), 0);
+    for (size_t i = 0; i < st.ser.size(); ++i) {
+      place[i] = ser.size();
+      if (!given.count(st.ser[i].sym)) ser.push_back(st.ser[i]);
+    }
+    for (auto& v : *solved) {
+      if (given.count(st.ser[v.within].sym)) return false;   // (fixed by a symbol that a position gives itself)
+      v.within = place[v.within];
+    }
+    int64_t total = 1;
+    for (auto& d : par) {
+      total *= d.extent();
+      if (total > (1 << 20)) return false;
+    }
+    st.par = par;
+    st.ser = ser;
+    st.total = total;
+    return true;
+  }
+
   // `lhs_zero`: the node the body assigns is known to be all zero when the stage starts.
   // Returns true when the stage made an earlier zero_out of that node unnecessary.
   bool generic_stage(const std::vector<LoopDim>& nest, const StmtP& body, bool lhs_zero = false) {
@@ -1051,7 +1142,10 @@ struct Builder {
     // moves with loops that therefore cannot run in parallel (the input gradient of a
     // convolution).  Those loops are spread over threads all the same: a thread sums over the
     // loops that do not move the position and adds its partial sum with one atomic add.
-    bool scatter = false;
+    // Few of them, and each thread would walk far: a thread per position instead (positions_of).
+    bool scatter = false, by_position = false;
+    std::vector<Solved> solved;
+    Indices at;
     if (opt.enable_coop && !st.ser.empty() && st.total > 0 && body->kind == Stmt::Set && body->vec_len == 0 &&
         accumulates_into_self(*body)) {
       const Tnode& t = code.prog.tn(body->tn);
@@ -1064,20 +1158,22 @@ struct Builder {
       }
       int64_t total = 1;
       for (auto& d : spread) total *= d.extent();
-      // (Also for few positions where a thread would otherwise walk a long way by itself: the input gradient of 19 images
-      // of 9 x 9 under 38 kernels of 3 x 3, stride 2, was 19 threads of 5472 steps each, 221 us.)
       int64_t walk = 1;
       for (auto& d : st.ser) walk *= d.extent();
-      if ((t.prec == Prec::Single || t.prec == Prec::Double) && t.mode != Mode::Virtual && spread.size() > st.par.size() &&
-          (total >= 4096 || walk >= 256)) {
-        scatter = true;
-        st.par = spread;
-        st.ser = kept;
-        st.total = total;
+      if ((t.prec == Prec::Single || t.prec == Prec::Double) && t.mode != Mode::Virtual && spread.size() > st.par.size()) {
+        if (total >= 4096) {
+          scatter = true;
+          st.par = spread;
+          st.ser = kept;
+          st.total = total;
+        } else if (walk >= 256) {
+          by_position = positions_of(st, *body, &solved, &at);
+        }
       }
     }
+    const bool moving = scatter || by_position;
 
-    if (!scatter && !st.ser.empty() && st.total > 0 && opt.enable_coop && ser_split_stage(st, *body)) return false;
+    if (!moving && !st.ser.empty() && st.total > 0 && opt.enable_coop && ser_split_stage(st, *body)) return false;
 
     CoopInfo ci;
     if (st.ser.empty() && st.total > 0) ci = find_coop(*body, st.total);
@@ -1095,7 +1191,7 @@ struct Builder {
     // axis of the written node, and everything in it is fp32, bf16 or half, a thread takes TWO
     // neighbouring iterations of that loop: 4- and 8-byte accesses, packed 16-bit arithmetic.
     bool pairs = false;
-    if (pairs_here() && !scatter && ci.sym.empty() && body->kind == Stmt::Set && body->vec_len == 0 && !st.par.empty() && st.total > 0) {
+    if (pairs_here() && !moving && ci.sym.empty() && body->kind == Stmt::Set && body->vec_len == 0 && !st.par.empty() && st.total > 0) {
       const Stmt& set = *body;
       const Tnode& t = code.prog.tn(set.tn);
       const LoopDim& p = st.par.back();
@@ -1124,6 +1220,15 @@ struct Builder {
       em.used_nodes.insert(set.tn);
       before = std::string("    ") + Emitter::ctype(t.prec) + " b200_self = 0;\n";
       after = "    atomicAdd(&" + t.ident + "[" + em.offset(set.idcs, t.dims) + "], b200_self);\n";
+      em.forwarded[set.tn] = {set.idcs, "b200_self"};
+      em.set_redirect[set.tn] = {set.idcs, "b200_self"};
+    } else if (by_position) {
+      const Stmt& set = *body;
+      const Tnode& t = code.prog.tn(set.tn);
+      em.used_nodes.insert(set.tn);
+      const std::string lv = t.ident + "[" + em.offset(at, t.dims) + "]";
+      before = std::string("    ") + Emitter::ctype(t.prec) + " b200_self = " + lv + ";\n";
+      after = "    " + lv + " = b200_self;\n";
       em.forwarded[set.tn] = {set.idcs, "b200_self"};
       em.set_redirect[set.tn] = {set.idcs, "b200_self"};
     } else if (ci.sym.empty() && (pairs || !st.ser.empty()) && body->kind == Stmt::Set && body->vec_len == 0) {
@@ -1189,7 +1294,7 @@ struct Builder {
     // shared memory once per block; the strided reads then hit shared-memory banks instead of L1
     // sectors.  Such a stage keeps its own kernel (few blocks, each looping over many elements).
     std::vector<int> staged;
-    if (opt.enable_coop && !scatter && !pairs && ci.sym.empty() && body->kind == Stmt::Set && st.total > 0) {
+    if (opt.enable_coop && !moving && !pairs && ci.sym.empty() && body->kind == Stmt::Set && st.total > 0) {
       int64_t work = st.total;
       for (auto& d : st.ser) work *= std::max<int64_t>(1, d.extent());
       std::set<std::string> inner_syms;
@@ -1248,10 +1353,13 @@ struct Builder {
     // serial loops wrap the body in their original order
     std::string open, close;
     int k = 4;
-    for (auto& d : st.ser) {
+    for (size_t i = 0; i < st.ser.size(); ++i) {
+      const LoopDim& d = st.ser[i];
       open += std::string((size_t)k, ' ') + "for (unsigned int " + d.sym + " = " + std::to_string(d.from) + "; " + d.sym +
               " <= " + std::to_string(d.to) + "; ++" + d.sym + ") {\n";
       k += 2;
+      for (auto& v : solved)
+        if (v.within == i) open += v.text;
     }
     for (size_t i = st.ser.size(); i-- > 0;) {
       k -= 2;
@@ -1300,7 +1408,7 @@ struct Builder {
     const bool block_sum = st.coop == 1024 && st.total == 1;
     pc.fusable = opt.enable_fuse && st.total > 0 && (st.coop == 0 || st.coop == 32 || block_sum) &&
                  st.total * std::max(1, st.coop) <= 16384 && ser_work <= 4096;
-    if (scatter) pc.fusable = false;
+    if (moving) pc.fusable = false;
     {
       // A stage shares the single block of small stages only while that block gets through it in less
       // than what leaving it out costs: its own launch, and a second one for the block's other half (8 us,
@@ -1316,13 +1424,13 @@ struct Builder {
       for (int n : em.used_nodes) far = far || (st.coop && code.prog.tn(n).bytes() > 12288);
       if (iters * std::max(far ? 300.0 : 30.0, (pairs ? 12.0 : 6.0) * warps / 4.0) > 16000.0) pc.fusable = false;
     }
-    if (opt.enable_fuse && !scatter && st.coop == 0 && st.total > 0 && !st.par.empty() && st.par[0].from == 0 && !(pairs && st.par.size() == 1)) {
+    if (opt.enable_fuse && !moving && st.coop == 0 && st.total > 0 && !st.par.empty() && st.par[0].from == 0 && !(pairs && st.par.size() == 1)) {
       pc.body = body;
       pc.row_sym = st.par[0].sym;
       pc.rows = st.par[0].extent();
       pc.per_row = st.total / pc.rows * ser_work;
     }
-    if (!scatter) pc.any_body = body;
+    if (!moving) pc.any_body = body;
     if (!self_type.empty() && ser_work > 1 && (code.prog.tn(body->tn).prec == Prec::Single || code.prog.tn(body->tn).prec == Prec::Double) &&
         accumulates_into_self(*body)) {
       pc.sum = true;
@@ -1348,7 +1456,7 @@ struct Builder {
     std::ostringstream note;
     note << "par=" << st.par.size() << " ser=" << st.ser.size()
          << (st.coop > 32 ? " block-per-element" : st.coop ? " warp-per-element" : "") << (pairs ? " pairs" : "")
-         << (scatter ? " scatter accumulation (atomic adds)" : "") << (staged.empty() ? "" : " small table staged in shared memory");
+         << (scatter ? " scatter accumulation (atomic adds)" : by_position ? " accumulation by position" : "") << (staged.empty() ? "" : " small table staged in shared memory");
     st.note = note.str();
     pieces[code.stages.size()] = pc;
     st.writes.assign(written.begin(), written.end());
