@@ -52,7 +52,9 @@ void walk_scalar(const Scalar& e, const std::function<void(const Scalar&)>& fs,
 }
 
 // Nodes whose values are compared, gate something or are truncated, and those that they are computed from: a change in the
-// last bits of such a value may change a result by a whole step.  (A position read by a value, `GetDyn`, is one too.)
+// last bits of such a value may change a result by a whole step.  (A position read by a value, `GetDyn`, is one too.)  A sum
+// that is decided on by the assignment that holds it counts as that assignment's node.  What another routine does with a
+// node is not known here: a forward pass compiled by itself may add in another order than the step that gates its values.
 std::set<int> find_deciding(const Program& P) {
   static const std::set<std::string> first = {"relu_gate", "sat01_gate", "where", "trunc", "not"},
                                      both = {"lt", "eq", "ne", "or", "and", "mod"};
@@ -62,19 +64,24 @@ std::set<int> find_deciding(const Program& P) {
     if (st.kind != Stmt::Set) return;
     std::set<int> all;
     bool open = is_int_prec(P.tn(st.tn).prec);   // values of scopes are followed to the whole assignment
+    bool own = open;                             // a sum of this assignment decides something
     auto reads = [&](const Scalar& e, std::set<int>& into) {
       walk_scalar(e, [&](const Scalar& x) {
         if (x.kind == Scalar::Get || x.kind == Scalar::GetDyn || x.kind == Scalar::GetMerge) into.insert(x.tn);
         if (x.kind == Scalar::GetLocal) open = open || &into == &found;
+        if (x.kind == Scalar::GetLocal || x.kind == Scalar::LocalScope) own = own || &into == &found;
       }, [](const Stmt&) {});
     };
     reads(*st.value, all);
     walk_scalar(*st.value, [&](const Scalar& x) {
-      if (x.kind == Scalar::GetDyn || (x.kind == Scalar::LocalScope && is_int_prec(P.tn(x.tn).prec))) open = true;
+      const bool truncated = x.kind == Scalar::LocalScope && is_int_prec(P.tn(x.tn).prec);
+      if (x.kind == Scalar::GetDyn || truncated) open = true;
+      own = own || truncated;
       for (size_t a = 0; a < x.args.size(); ++a)
         if (both.count(x.op) || (a == 0 && first.count(x.op))) reads(*x.args[a].s, found);
     }, [](const Stmt&) {});
     if (open) found.insert(all.begin(), all.end());
+    if (own) found.insert(st.tn);
     made_from[st.tn].insert(all.begin(), all.end());
   });
   std::vector<int> todo(found.begin(), found.end());

@@ -39,3 +39,21 @@ def test_what_counts_as_a_decision(use, clustered):
         body.append(loops([(u, m), (v, n)], Set(d, (u, v), binop("relu_gate", e[u, v], d[u, v]))))
     r.body = Seq(body)
     assert _clusters(r) == [clustered]
+
+
+@pytest.mark.parametrize("use,clustered", [("relu", True), ("gate", False), ("gate of product", False), ("lt", False), ("where", False), ("trunc", False), ("not", False),
+                                           ("value of gate", True), ("value of where", True)])
+@pytest.mark.parametrize("prec", ["single", "bfloat16"])
+def test_decisions_on_the_sum_itself(use, clustered, prec):
+    """The sum is gated, compared or truncated by the assignment that holds it."""
+    m, n, k = 64, 64, 1024
+    r = Routine("decide_at_once_" + use.replace(" ", "_"))
+    a, b = r.tn("a", "bfloat16", [m, k], read_only=True), r.tn("b", "bfloat16", [n, k], read_only=True)
+    c, d, e = r.tn("c", prec, [m, n]), r.tn("d", "single", [m, n], read_only=True), r.tn("e", "single", [m, n], read_only=True)
+    i, j, p = r.syms(3)
+    s = W.reduce_scope(r, "acc", "single", [(p, k)], lambda: (a[i, p], b[j, p]))
+    value = {"relu": lambda: un("relu", s), "gate": lambda: binop("relu_gate", s, d[i, j]), "gate of product": lambda: binop("relu_gate", s * e[i, j], d[i, j]),
+             "lt": lambda: binop("lt", s, d[i, j]), "where": lambda: where(binop("lt", s, d[i, j]), d[i, j], e[i, j]), "trunc": lambda: un("trunc", s), "not": lambda: un("not", s),
+             "value of gate": lambda: binop("relu_gate", d[i, j], s), "value of where": lambda: where(d[i, j], s, 0.0)}[use]
+    r.body = Seq([loops([(i, m), (j, n)], Set(c, (i, j), value()))])
+    assert _clusters(r) == [clustered]
