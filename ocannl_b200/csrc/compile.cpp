@@ -2432,6 +2432,7 @@ struct Builder {
     std::vector<size_t> all;
     for (auto& run : parts) all.insert(all.end(), run.begin(), run.end());
     Stage f = code.stages[all.front()];
+    f.min_align = 0;
     merge_origins(f, all);
     Emitter em(code.prog);
     std::set<int> written;
@@ -2441,14 +2442,19 @@ struct Builder {
       const int64_t total = code.stages[run.front()].total;
       text += std::string("    ") + (start ? "else " : "") + "if (b200_i < " + std::to_string(start + total) + "ull) {\n    if (b200_i >= " + std::to_string(start) +
               "ull) {\n    const unsigned long long b200_g = b200_i - " + std::to_string(start) + "ull;\n";
+      // (a parameter off its boundary takes its own chain's pairs away, not those of the others in the launch)
+      Stage::AlignNeed need{0, {}, {}};
       for (size_t i : run) {
         const Piece& pc = pieces[i];
-        f.min_align = std::max(f.min_align, code.stages[i].min_align);
+        need.bytes = std::max(need.bytes, code.stages[i].min_align);
+        need.nodes.insert(need.nodes.end(), pc.used.begin(), pc.used.end());
+        need.origins.insert(need.origins.end(), code.stages[i].origins.begin(), code.stages[i].origins.end());
         em.used_nodes.insert(pc.used.begin(), pc.used.end());
         written.insert(pc.written.begin(), pc.written.end());
         em.uses_merge |= pc.uses_merge;
         text += "    {\n" + pc.decomp + pc.body_text + "    }\n";
       }
+      if (need.bytes > 1) f.needs.push_back(need);
       text += "    }\n    }\n";
       start = (start + total + 31) / 32 * 32;
     }
@@ -2485,6 +2491,7 @@ struct Builder {
       } else {
         st.note += " (in the launch of " + f.kernel + ")";
         st.in_group = true;
+        st.min_align = 0;
         st.args.clear();
         for (int n : used) st.args.push_back({KArg::Node, n});
         out->push_back(st);

@@ -136,6 +136,11 @@ struct Stage {
   int epi_chunk = 32;                // columns per epilogue step (the inner box of the output maps)
   int tile_m = 0, tile_n = 0, tile_k = 0;
   int min_align = 0;             // >0: every node the stage touches must be bound at a multiple of this many bytes
+  struct AlignNeed {
+    int bytes;
+    std::vector<int> nodes, origins;
+  };
+  std::vector<AlignNeed> needs;  // chains that share a launch: what each of them asks of its own nodes
   int cta_pair = 0;              // 1: two CTAs of a cluster share one tile_m x tile_n tile (cta_group::2)
   int cluster_k = 1;             // > 1: that many CTAs of a cluster share the k blocks of a tile
   int box_m = 0, box_n = 0;      // rows of A / B one CTA stages per k block (the TMA boxes)

@@ -72,12 +72,19 @@ static bool misaligned_stages(const b200_code* c, const std::map<int, CUdevicept
     return it == param_ptr.end() ? 0 : it->second;   // routine-local nodes sit at 256-byte multiples
   };
   for (auto& st : c->code.stages) {
-    if (st.kind == Stage::Generic && st.min_align > 1) {
+    if (st.kind == Stage::Generic) {
       bool bad = false;
-      for (auto& a : st.args)
-        if (a.kind == KArg::Node && (at(a.tn) % (CUdeviceptr)st.min_align) != 0) bad = true;
+      if (st.min_align > 1)
+        for (auto& a : st.args)
+          if (a.kind == KArg::Node && (at(a.tn) % (CUdeviceptr)st.min_align) != 0) bad = true;
       if (bad)
         for (int o : st.origins) any |= no_pairs_at->insert(o).second;
+      for (auto& need : st.needs) {
+        bad = false;
+        for (int n : need.nodes) bad = bad || (at(n) % (CUdeviceptr)need.bytes) != 0;
+        if (bad)
+          for (int o : need.origins) any |= no_pairs_at->insert(o).second;
+      }
     } else if (st.kind == Stage::Gemm) {
       const int eb = prec_bytes(st.gemm.in_prec);
       const CUdeviceptr a = at(st.gemm.a_tn) + (CUdeviceptr)(st.gemm.a_off * eb), b = at(st.gemm.b_tn) + (CUdeviceptr)(st.gemm.b_off * eb);
@@ -217,9 +224,12 @@ void b200_routine::link(b200_dev* d, b200_code* c, const b200_binding* b, int n)
       if (a.kind == KArg::Node) {
         auto it = node_ptr.find(a.tn);
         if (it == node_ptr.end()) throw Error(B200_E_USER, "link: node '" + P.tn(a.tn).label + "' has no buffer binding");
-        if (st.min_align > 1 && (it->second % (CUdeviceptr)st.min_align) != 0)
+        int want = st.min_align;
+        for (auto& need : st.needs)
+          if (std::count(need.nodes.begin(), need.nodes.end(), a.tn)) want = std::max(want, need.bytes);
+        if (want > 1 && (it->second % (CUdeviceptr)want) != 0)
           throw Error(B200_E_INVALID, "link: internal error: stage '" + st.kernel + "' kept a form that needs " +
-                                          std::to_string(st.min_align) + "-byte alignment for node '" + P.tn(a.tn).label + "'");
+                                          std::to_string(want) + "-byte alignment for node '" + P.tn(a.tn).label + "'");
         arg_values[i].push_back(it->second);
       } else if (a.kind == KArg::Status) {
         arg_values[i].push_back(dev->status_dev);

@@ -5,8 +5,9 @@ n 2^-24 of itself; in trees of 1024 threads over 300 blocks far less, 1e-5 is al
 import numpy as np
 import pytest
 
+from ocannl_b200 import backend as bk
 from ocannl_b200 import workloads as W
-from ocannl_b200.low_level import Routine, Seq, Set, loops
+from ocannl_b200.low_level import PREC_BYTES, Routine, Seq, Set, loops
 from tests.parity import compare, run_device, run_oracle
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +55,44 @@ def test_sum_over_a_grid(device, shape, op):
     exact = np.square(inputs["x"].astype(np.float64))
     want = exact.sum() if op == "add" else exact.max()
     assert abs(float(got["y"][0]) - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("off", ["b1", "b2_grad", "w2"])
+@pytest.mark.parametrize("kwargs", [dict(), dict(momentum=0.9, weight_decay=1e-4, nesterov=True)])
+def test_a_parameter_off_its_boundary(device, off, kwargs):
+    """A parameter (or its gradient) an element off the boundary of its pairs: its own update goes element by element, the
+    updates that share the launch keep their pairs, and the same bits; its own differ by a rounding of the format at most."""
+    ir = W.mlp_sgd(dims=(512, 256, 256, 64), wprec="bfloat16", **kwargs)
+    g = np.random.default_rng(5)
+    inputs = {t.ident: W.store(t.prec, np.float32([0.05]) if t.ident == "learning_rate" else g.standard_normal(t.dims).astype(np.float32)) for t in ir.params()}
+    code = bk.Code(ir)
+    outs, pairs = [], []
+    for shift in (0, 1):
+        places, total = {}, 0
+        for t in ir.params():
+            total = (total + 255) // 256 * 256
+            places[t.ident] = total + (shift * PREC_BYTES[t.prec] if t.ident == off else 0)
+            total += t.size_in_bytes + 256
+        pool = device.alloc_pool(total)
+        rt = bk.Context(device, {t.ident: (pool, places[t.ident], t) for t in ir.params()}).link(code)
+        for k, v in inputs.items():
+            rt.context.from_host(k, v)
+        rt.run()
+        device.await_()
+        outs.append({t.ident: rt.context.to_host(t.ident) for t in ir.params()})
+        stages = rt.info()["stages"]
+        assert rt.kernels_per_run() == 1 and len(stages) > 1, stages
+        pairs.append({s["kernel"]: "pairs" in (s["note"] or "") for s in stages if "small" not in (s["note"] or "")})
+        rt.free()
+        device.free_pool(pool)
+    code.free()
+    own = off.split("_")[0]
+    for t in ir.params():
+        a, b = outs[0][t.ident], outs[1][t.ident]
+        if t.ident.split("_")[0] != own:
+            assert np.array_equal(a, b), t.ident
+        else:
+            np.testing.assert_allclose(W.load(t.prec, b), W.load(t.prec, a), rtol=2.0 ** -7, atol=1e-6, err_msg=t.ident)
+    lost = [k for k in pairs[0] if not pairs[1].get(k)]
+    listed = off == "w2" or not kwargs      # (small chains of several stages are listed together, without their form)
+    assert all(pairs[0].values()) and len(lost) == (1 if listed else 0), pairs
