@@ -2663,10 +2663,11 @@ struct Builder {
       // node on some branch (2706 rows through 141-82-270-5, a training step: 65 us with five of them, 53 so; 8192 of 784-1024-1024-10 143.1 and 133.4).
       if (opt.enable_fuse && code.stages[i].kind == Stage::Memset) {
         std::vector<size_t> run;
+        std::set<int> cleared;   // (a second clear of the same node has to wait for the first: one block would do both)
         size_t j = i;
         for (; j < code.stages.size() && code.stages[j].kind == Stage::Memset; ++j) {
           const Tnode& t = code.prog.tn(code.stages[j].memset_tn);
-          if (prec_bytes(t.prec) > 8 || t.prec == Prec::Uint4x32 || t.num_elems() >= (1ll << 31)) break;
+          if (prec_bytes(t.prec) > 8 || t.prec == Prec::Uint4x32 || t.num_elems() >= (1ll << 31) || !cleared.insert(t.id).second) break;
           run.push_back(j);
         }
         // (those that stages behind them join share a launch with these anyway)

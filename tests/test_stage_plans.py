@@ -2,6 +2,7 @@
 so the plan (which stages exist, what each one is) can be read back from `b200_code_info`."""
 from ocannl_b200 import backend as bk
 from ocannl_b200 import workloads as W
+from ocannl_b200.low_level import Routine, Seq, ZeroOut
 import pytest
 
 
@@ -204,3 +205,16 @@ def test_units_compiled_side_by_side_report_a_failure(monkeypatch):
         bk.Code(W.mlp_forward(rows=96))
     monkeypatch.delenv("B200_NVRTC_FLAGS")
     assert len(_plan(W.mlp_forward(rows=96))) >= 3
+
+
+def test_clears_of_one_node_share_no_launch(built_lib):
+    r = Routine("cleared_twice")
+    a, b = r.tn("a", "single", [1 << 20]), r.tn("b", "single", [1 << 20])
+    r.body = Seq([ZeroOut(a), ZeroOut(b), ZeroOut(b), ZeroOut(a)])
+    notes = [s["note"] for s in _plan(r)]
+    assert [("in the launch of" in n) for n in notes] == [False, True, False, True], notes
+    code = bk.Code(r)
+    try:
+        assert "\n  __syncthreads();" not in code.source().split("__global__", 1)[1]     # spread over a grid, not one block
+    finally:
+        code.free()
