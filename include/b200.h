@@ -129,12 +129,14 @@ int b200_routine_info(b200_routine* r, char* json, size_t cap);   /* like b200_c
  * (cuda: arrayjit/lib/cuda_backend.ml:1015-1030). */
 int b200_launch(b200_routine* r, const int64_t* static_idx, int n_static);
 /* Replays the routine's launches as one captured graph from its second run on (the first is launched
- * directly).  Routines of up to four kernels that clear no node, and those whose only kernel takes the
- * static indices as an argument, are launched directly all the same: a graph would only add its own time. */
+ * directly).  Routines of up to four launches, all of them kernels (a lone clear of a node is none; clears that
+ * share a launch are one), and those whose only kernel takes the static indices as an argument, are launched
+ * directly all the same: a graph would only add its own time. */
 int b200_routine_use_graph(b200_routine* r, int enable);
 int b200_routine_launch_count(b200_routine* r, int64_t* kernels_per_run);
-/* Per-stage device timing (CUDA events around every stage of the next runs; disables graph
- * replay while on).  No counterpart in the reference, which has no profiler hooks. */
+/* Per-stage device timing (CUDA events around every launch of the next runs; disables graph
+ * replay while on).  A stage that runs in the launch of another (its note says of which) has 0 runs: its
+ * time is part of that stage's.  No counterpart in the reference, which has no profiler hooks. */
 int b200_routine_profile(b200_routine* r, int enable);
 int b200_routine_stage_time(b200_routine* r, int stage, float* total_ms, int* runs);
 int b200_routine_free(b200_routine* r);

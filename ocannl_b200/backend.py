@@ -431,7 +431,8 @@ class Routine:
         check(lib().b200_routine_profile(self.h, ctypes.c_int(int(on))))
 
     def stage_times(self):
-        """[(total_ms, runs)] per stage, over the runs made while profiling was on."""
+        """[(total_ms, runs)] per stage, over the runs made while profiling was on; 0 runs for a stage in the launch
+        of another, whose time includes it."""
         out = []
         for i in range(len(self.info()["stages"])):
             ms, n = ctypes.c_float(0), ctypes.c_int(0)
