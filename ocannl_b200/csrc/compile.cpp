@@ -1039,9 +1039,18 @@ struct Builder {
   // position of t and walks the loops in their order, without the innermost symbol of every moving axis: the position
   // gives that one.  Every position so gets its terms one after the other in the order of the loops, as when a thread
   // walks all of them by itself, and the sums have the same bits from run to run, which atomic adds would not give.
+  // The loop that fixes the given symbol covers the iterations that reach the position and no others: threads of a warp, whose
+  // positions differ, then walk side by side (with a test in each iteration instead they took turns).
+  // A chain of dependent additions with its loads in between bounds it: 16 steps unrolled, blocks of one warp, on as many
+  // SMs as there are.  Convolution steps, one thread / atomic adds / by position, us: 1 image of 8 x 8 under 50 kernels of
+  // 5 x 5 590 / 15 / 34, 3 of 16 x 16 x 3 under 56 of 3 x 3, stride 2, 645 / 31 / 33, 19 of 9 x 9 under 38, stride 2,
+  // 695 / 10.4 / 10.4, 1 of 8 x 8 x 32 under 16 20.7 / 16.6 / 16.6.  (First case with 8 steps unrolled 43, with
+  // blocks of 256 threads 52.)
   struct Solved {
-    size_t within = 0;   // the serial loop that fixes the symbol
-    std::string text;    // leaves out the iterations that do not reach the position, declares the symbol
+    size_t within = 0;        // the serial loop that fixes the symbol
+    std::string ahead;        // ahead of that loop: what is left of the position
+    std::string from, to;     // the iterations of that loop
+    std::string text;         // in the loop: declares the symbol
   };
   bool positions_of(Stage& st, const Stmt& set, std::vector<Solved>* solved, Indices* at) {
     if (opt.bounds) return false;   // (an access outside the node has to be seen)
@@ -1090,13 +1099,32 @@ struct Builder {
       if (outer < 0 || on.size() != seen.size()) return false;
       const LoopDim& e = st.ser[(size_t)last];
       const std::string pos = "b200_at" + std::to_string(a), n = "b200_n" + std::to_string(a);
-      const std::string pad(6 + 2 * (size_t)outer, ' '), v_at = c == 1 ? n : "(" + n + " / " + std::to_string(c) + ")";
-      std::string text = pad + "const int " + n + " = (int)" + pos + " - (" + std::to_string(set.idcs[a].fixed);
-      for (auto& v : on)
-        if (v.second != e.sym) text += " + " + std::to_string(v.first) + " * (int)" + v.second;
-      text += ");\n" + pad + "if (" + (c == 1 || c == -1 ? std::string() : n + " % " + std::to_string(c) + " != 0 || ") + v_at + " < " + std::to_string(e.from) +
-              " || " + v_at + " > " + std::to_string(e.to) + ") continue;\n" + pad + "const unsigned int " + e.sym + " = (unsigned int)" + v_at + ";\n";
-      solved->push_back({(size_t)outer, text});
+      Solved v;
+      v.within = (size_t)outer;
+      int64_t co = 0;
+      v.ahead = "const int " + n + " = (int)" + pos + " - (" + std::to_string(set.idcs[a].fixed);
+      for (auto& x : on)
+        if (x.second == st.ser[(size_t)outer].sym) co = x.first;
+        else if (x.second != e.sym) v.ahead += " + " + std::to_string(x.first) + " * (int)" + x.second;
+      v.ahead += ");\n";
+      if (co == 0) return false;
+      // c * symbol = n - co * loop, with the symbol between its ends: the loop lies between two quotients
+      auto less = [&](int64_t by) { return by ? n + " - " + std::to_string(by) : n; };
+      std::string low = less(c > 0 ? c * e.to : c * e.from), high = less(c > 0 ? c * e.from : c * e.to);
+      if (co < 0) {
+        const std::string was = low;
+        low = "-(" + high + ")";
+        high = "-(" + was + ")";
+      }
+      const std::string by = std::to_string(std::abs(co));
+      v.from = by == "1" ? low : "-b200_floor_div(-(" + low + "), " + by + ")";
+      v.to = by == "1" ? high : "b200_floor_div(" + high + ", " + by + ")";
+      const std::string m = "b200_m" + std::to_string(a);
+      const std::string pad(6 + 2 * (size_t)outer, ' ');
+      v.text = pad + "const int " + m + " = " + n + " - " + std::to_string(co) + " * (int)" + st.ser[(size_t)outer].sym + ";\n";
+      if (std::abs(c) != 1) v.text += pad + "if (" + m + " % " + std::to_string(c) + " != 0) continue;\n";
+      v.text += pad + "const unsigned int " + e.sym + " = (unsigned int)(" + m + (c == 1 ? "" : " / " + std::to_string(c)) + ");\n";
+      solved->push_back(v);
       given.insert(e.sym);
       (*at)[a] = Index();
       (*at)[a].kind = Index::Iter;
@@ -1179,6 +1207,7 @@ struct Builder {
       }
     }
     const bool moving = scatter || by_position;
+    if (by_position) st.block = 32;
 
     if (!moving && !st.ser.empty() && st.total > 0 && opt.enable_coop && ser_split_stage(st, *body)) return false;
 
@@ -1362,8 +1391,22 @@ struct Builder {
     int k = 4;
     for (size_t i = 0; i < st.ser.size(); ++i) {
       const LoopDim& d = st.ser[i];
-      open += std::string((size_t)k, ' ') + "for (unsigned int " + d.sym + " = " + std::to_string(d.from) + "; " + d.sym +
-              " <= " + std::to_string(d.to) + "; ++" + d.sym + ") {\n";
+      const std::string pad((size_t)k, ' ');
+      std::string from, to;
+      for (auto& v : solved)
+        if (v.within == i) {
+          open += pad + v.ahead;
+          from = "max(" + (from.empty() ? std::to_string(d.from) : from) + ", " + v.from + ")";
+          to = "min(" + (to.empty() ? std::to_string(d.to) : to) + ", " + v.to + ")";
+        }
+      if (!from.empty()) {
+        const std::string last = "b200_last" + std::to_string(i);
+        open += pad + "const int " + last + " = " + to + ";\n" + pad + "for (unsigned int " + d.sym + " = (unsigned int)" + from + "; (int)" + d.sym + " <= " + last + "; ++" + d.sym + ") {\n";
+      } else {
+        // (by position: the terms are added one after the other, but the loads of sixteen of them are under way together)
+        if (by_position && i + 1 == st.ser.size()) open += "#pragma unroll 16\n";
+        open += pad + "for (unsigned int " + d.sym + " = " + std::to_string(d.from) + "; " + d.sym + " <= " + std::to_string(d.to) + "; ++" + d.sym + ") {\n";
+      }
       k += 2;
       for (auto& v : solved)
         if (v.within == i) open += v.text;

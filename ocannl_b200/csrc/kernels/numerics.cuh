@@ -448,6 +448,9 @@ __device__ __forceinline__ float b200_div_literal_straight(float a, float b) {
   return q == q ? q : q0;
 }
 
+// a / b rounded down, b > 0
+__device__ __forceinline__ int b200_floor_div(int a, int b) { return a >= 0 ? a / b : -((b - 1 - a) / b); }
+
 // ---- range-checked node accesses (routines compiled with bounds=1).  The proxy stands where the
 //      node's pointer stood: node[i] with i outside the node records (code 2, node id, index) in the
 //      device status word and lands on a sink instead of memory the node does not own.
