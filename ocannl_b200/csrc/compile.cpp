@@ -2468,9 +2468,14 @@ struct Builder {
     return f;
   }
 
-  // Pointwise chains that do not depend on one another -- the updates of a routine's parameters -- as one launch over
-  // their concatenated iterations; every chain begins at a multiple of a warp's 32.  The plan lists what is in it as
-  // stages: a large chain each, neighbouring small ones together.
+  // Pointwise chains that do not depend on one another -- the updates of a routine's parameters -- as one launch.  Small ones
+  // over their concatenated iterations, every chain beginning at a multiple of a warp's 32.  Where a chain has more
+  // than a few rounds of a launch's threads, each has a range of the blocks instead, as many as its own launch would have, and
+  // the loop that it would have there: one that tells the chains apart in its body is not unrolled.  (Updates of
+  // n-n-n-10, us, a launch each / concatenated / ranges: n = 1024 in bf16 9.9 / 5.3 / 5.5, 1448 10.4 / 5.5 / 6.6, 1023 11.7 /
+  // 6.2 / 7.4; 2048 14.0 / 9.3 / 7.7, 2047 18.6 / 19.0 / 14.8, 2895 35.6 / 42.2 / 35.1, 4096 47.8 / 53.1 / 48.5; with
+  // momentum 4096 131.8 / 132.1 / 128.4.  Working sets next to the size of L2 may be better off one by one: 2895 in single
+  // precision 36.7 / 49.1 / 44.0.)  The plan lists what is in it as stages: a large chain each, neighbouring small ones together.
   void emit_pointwise_group(const std::vector<std::vector<size_t>>& parts, std::vector<Stage>* out) {
     std::vector<size_t> all;
     for (auto& run : parts) all.insert(all.end(), run.begin(), run.end());
@@ -2480,11 +2485,18 @@ struct Builder {
     Emitter em(code.prog);
     std::set<int> written;
     std::string text;
-    int64_t start = 0;
+    int64_t most = 0, threads = 0, first = 0;   // iterations of a chain, of all of them; blocks
+    for (auto& run : parts) most = std::max(most, code.stages[run.front()].total);
+    const bool ranges = most > 3 << 19;
     for (auto& run : parts) {
-      const int64_t total = code.stages[run.front()].total;
-      text += std::string("    ") + (start ? "else " : "") + "if (b200_i < " + std::to_string(start + total) + "ull) {\n    if (b200_i >= " + std::to_string(start) +
-              "ull) {\n    const unsigned long long b200_g = b200_i - " + std::to_string(start) + "ull;\n";
+      const int64_t total = code.stages[run.front()].total, blocks = std::min<int64_t>((total + f.block - 1) / f.block, 148 * 16);
+      text += std::string("    ") + (first ? "else " : "");
+      if (ranges)
+        text += "if (blockIdx.x < " + std::to_string(first + blocks) + "u) {\n    for (unsigned long long b200_g = (unsigned long long)(blockIdx.x - " + std::to_string(first) +
+                "u) * blockDim.x + threadIdx.x; b200_g < " + std::to_string(total) + "ull; b200_g += " + std::to_string(blocks) + "ull * blockDim.x) {\n";
+      else
+        text += "if (b200_i < " + std::to_string(threads + total) + "ull) {\n    if (b200_i >= " + std::to_string(threads) + "ull) {\n    const unsigned long long b200_g = b200_i - " +
+                std::to_string(threads) + "ull;\n";
       // (a parameter off its boundary takes its own chain's pairs away, not those of the others in the launch)
       Stage::AlignNeed need{0, {}, {}};
       for (size_t i : run) {
@@ -2499,16 +2511,19 @@ struct Builder {
       }
       if (need.bytes > 1) f.needs.push_back(need);
       text += "    }\n    }\n";
-      start = (start + total + 31) / 32 * 32;
+      threads = (threads + total + 31) / 32 * 32;
+      first += blocks;
     }
+    if (ranges) f.grid_override = (int)first;
     std::string statics = static_prologue(text, em, 2);
     std::ostringstream k_src;
     k_src << "extern \"C\" __global__ void __launch_bounds__(" << f.block << ") " << f.kernel << "(";
     emit_params(k_src, f, em, written);
-    k_src << ") {\n" << kGridEntry << statics
-          << "  for (unsigned long long b200_i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_i < "
-          << start << "ull; b200_i += (unsigned long long)gridDim.x * blockDim.x) {\n"
-          << text << "  }\n}\n\n";
+    k_src << ") {\n" << kGridEntry << statics;
+    if (!ranges)
+      k_src << "  for (unsigned long long b200_i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; b200_i < " << threads
+            << "ull; b200_i += (unsigned long long)gridDim.x * blockDim.x) {\n";
+    k_src << text << (ranges ? "}\n\n" : "  }\n}\n\n");
     src << k_src.str();
     std::vector<std::vector<size_t>> listed;
     bool small_before = false;
@@ -2529,7 +2544,7 @@ struct Builder {
       else if (run.size() > 1) st.note = "pointwise chain of " + std::to_string(run.size()) + " stages" + (pieces[run.front()].pairs ? ", pairs" : "");
       if (k == 0) {
         f.note = st.note;
-        f.total = start;
+        f.total = threads;
         out->push_back(f);
       } else {
         st.note += " (in the launch of " + f.kernel + ")";

@@ -40,6 +40,20 @@ def test_updates_in_one_launch(device, dims, prec, kwargs):
             assert np.all(np.abs(w - d) <= u * np.abs(w) * 2 + u * 0.05 * delta), t.ident
 
 
+@pytest.mark.parametrize("dims", [(1773, 887, 1773, 3), (2049, 1025, 3, 2)])
+def test_large_updates_take_ranges_of_the_blocks(device, dims):
+    """One chain just below and just above the size from which each has blocks of its own, odd lengths, beside small ones; the
+    arithmetic of test_updates_in_one_launch in single precision."""
+    ir = W.mlp_sgd(dims=dims, wprec="single", momentum=0.9)
+    g = np.random.default_rng(7)
+    inputs = {t.ident: np.float32([0.05]) if t.ident == "learning_rate" else g.standard_normal(t.dims).astype(np.float32) for t in ir.params()}
+    want = run_oracle(ir, inputs)
+    got, info = run_device(device, ir, inputs)
+    assert any("in the launch of" in (s["note"] or "") for s in info["stages"]), info
+    for t in ir.params():
+        np.testing.assert_allclose(got[t.ident], want[t.ident], rtol=1e-6, atol=1e-6, err_msg=t.ident)
+
+
 @pytest.mark.parametrize("shape", [(1, 32768), (3, 10923), (7, 4683), (296, 1024), (297, 1024), (1, 303103), (5, 606209), (64, 41, 259)])
 @pytest.mark.parametrize("op", ["add", "max"])
 def test_sum_over_a_grid(device, shape, op):
