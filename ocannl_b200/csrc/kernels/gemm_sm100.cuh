@@ -209,8 +209,10 @@ B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_s
     asm volatile("tcgen05.relinquish_alloc_permit." B200_CG ".sync.aligned;" ::: "memory");
   }
   // Set-up touches no global memory and is over, block-wide barrier included, before the grids ahead of this one
-  // end; every role then waits for those grids itself: the producer and the epilogue right ahead of their first access
-  // to global memory, the MMA issuer ahead of its first wait for operands, whose limit would count those grids' time.
+  // end; the threads that read or write global memory (the producer, the epilogue) then wait for those grids
+  // themselves, right ahead of their first access, and no limited wait begins before that.  The MMA issuer goes
+  // straight to its first operands, however long those grids take: should operands never come, it is the epilogue
+  // that finds out, and ends this wait too.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   b200_cluster_sync();   // the peer's barriers are initialised before anything is signalled on them
@@ -294,7 +296,6 @@ B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_s
     if (cta_rank == 0u && b200_elect()) {
       unsigned int slot = 0, phase = 0, acc = 0, acc_phase = 0;
       bool live = true;
-      asm volatile("griddepcontrol.wait;" ::: "memory");   // (the limit of the waits below is for this kernel's own work)
       // operand descriptors of ring slot 0.  k-major: rows of 128 bytes, 8-row groups 1024 bytes
       // apart.  m/n-major: 64-element (128-byte) chunks of m/n, k rows 128 bytes apart, 8-row groups
       // 1024 bytes apart, chunks one box apart.
@@ -319,7 +320,7 @@ B200_KERNEL_HEAD(B200_TMAP_PARAM map_a, B200_TMAP_PARAM map_b, const b200_gemm_s
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const unsigned int d_tmem = tmem_base + acc * B200_BN;
           for (unsigned int kb = kbf; kb < kbe; ++kb) {
-            if (!b200_wait(bar_full + 8u * slot, phase, abort_flag, status, 3u)) { live = false; break; }
+            if (!b200_wait_aborted(bar_full + 8u * slot, phase, abort_flag)) { live = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (unit == worker && kb == kb0) B200_TR(5);   // first operands landed
             // descriptors of this slot: the start-address field (bits 0-13, address >> 4) moves, the rest is fixed

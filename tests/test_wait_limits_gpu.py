@@ -1,5 +1,5 @@
 """The limit of a contraction's waits counts its own work, not that of the kernels ahead of it, beside which it is already
-set up: every role that waits with a limit first waits for those kernels."""
+set up: a role whose waits have a limit first waits for those kernels, and the one that does not ends with the others."""
 import re
 
 import numpy as np
@@ -26,7 +26,7 @@ def _behind(steps):
 
 @pytest.mark.parametrize("ir", [_behind(64), W.mlp_forward(rows=37), W.mlp_forward(rows=8192), W.mlp_train_update(rows=8192), W.einsum_gelu(1, 300, 300, 304, "single", "single")],
                          ids=["plain", "clusters", "pairs", "split k", "two parts"])
-def test_roles_wait_for_the_kernels_ahead(built_lib, ir):
+def test_limits_begin_behind_the_kernels_ahead(built_lib, ir):
     code = bk.Code(ir)
     try:
         sources = [code.source(i) for i, s in enumerate(code.info()["stages"]) if s["kind"] == "gemm"]
@@ -36,8 +36,11 @@ def test_roles_wait_for_the_kernels_ahead(built_lib, ir):
     for text in sources:
         roles = re.split(r"// -+ (TMA producer|MMA issuer[^\n]*|epilogue|teardown)\n", text[text.index("B200_KERNEL_HEAD(B200_TMAP_PARAM"):])
         assert [x.split()[0] for x in roles[1::2]] == ["TMA", "MMA", "epilogue", "teardown"], roles[1::2]
-        for role in roles[2:-1:2]:
+        producer, issuer, epilogue = roles[2:-1:2]
+        for role in (producer, epilogue):
             assert "griddepcontrol.wait" in role[:role.index("b200_wait(")], role[:400]
+        # the issuer: accumulators, which are free at first, and operands, whose wait the epilogue's limit ends
+        assert re.findall(r"b200_wait(\w*)\((\w+)", issuer) == [("", "bar_acc_empty"), ("_aborted", "bar_full")], issuer
 
 
 @pytest.mark.gpu
