@@ -2719,13 +2719,15 @@ struct Builder {
       }
       // Clears in a row are one kernel, which nothing before them holds up: in a captured graph every clear of its own was a
       // node on some branch (2706 rows through 141-82-270-5, a training step: 65 us with five of them, 53 so; 8192 of 784-1024-1024-10 143.1 and 133.4).
+      // Not the largest: the driver's clear has the higher bandwidth (two nodes each, us, by the driver / as a kernel: 2^23 floats
+      // 12.4 / 10.5, 2^24 21.0 / 22.0, 2^26 76 / 90; 2^24 values of 16 bits 12.5 / 11.3, 2^25 22.3 / 23.0; 2^24 bytes 8.3 / 7.8, 2^25 12.5 / 14.0).
       if (opt.enable_fuse && code.stages[i].kind == Stage::Memset) {
         std::vector<size_t> run;
         std::set<int> cleared;   // (a second clear of the same node has to wait for the first: one block would do both)
         size_t j = i;
         for (; j < code.stages.size() && code.stages[j].kind == Stage::Memset; ++j) {
           const Tnode& t = code.prog.tn(code.stages[j].memset_tn);
-          if (prec_bytes(t.prec) > 8 || t.prec == Prec::Uint4x32 || t.num_elems() >= (1ll << 31) || !cleared.insert(t.id).second) break;
+          if (prec_bytes(t.prec) > 8 || t.prec == Prec::Uint4x32 || t.num_elems() > (1 << 24) || t.bytes() > (1 << 25) || !cleared.insert(t.id).second) break;
           run.push_back(j);
         }
         // (those that stages behind them join share a launch with these anyway)

@@ -218,3 +218,11 @@ def test_clears_of_one_node_share_no_launch(built_lib):
         assert "\n  __syncthreads();" not in code.source().split("__global__", 1)[1]     # spread over a grid, not one block
     finally:
         code.free()
+
+
+@pytest.mark.parametrize("prec,largest", [("single", 1 << 23), ("double", 1 << 22), ("bfloat16", 1 << 24), ("byte", 1 << 24)])
+def test_the_largest_clears_are_the_drivers(built_lib, prec, largest):
+    for elems, shared in ((largest, 1), (largest + 1, 0)):
+        r = Routine("clears_of_%d" % elems)
+        r.body = Seq([ZeroOut(r.tn("a", prec, [elems])), ZeroOut(r.tn("b", prec, [elems]))])
+        assert sum("in the launch of" in s["note"] for s in _plan(r)) == shared
