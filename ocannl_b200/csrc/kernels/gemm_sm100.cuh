@@ -126,8 +126,8 @@ __device__ __forceinline__ void b200_tmem_ld_chunk(unsigned int taddr, unsigned 
 // them, into its shared memory (column groups of four, a lane's row next to its neighbours': 512 bytes an
 // instruction), where its barrier counts the bytes.  The partials are added in the order of the slices.
 // The exchange is what it costs: some 16 bytes a clock leave an SM this way, 0.35 us for 16 columns, 0.75 for 32, 1.3 for
-// 64 (bulk copies out of shared memory: 0.5, 1.0, 1.6).  128 rows of 2048-2048-2048-10: 20.3 -> 17.4 us; 64 of
-// 4096-4096-256-10: 28.8 -> 19.9; 37 of 784-1024-1024-10: 15.3 -> 14.6, and 18.1 with the logits' k blocks in one CTA.
+// 64 (bulk copies out of shared memory: 0.5, 1.0, 1.6).  Runs back to back without
+// and with clusters: 128 rows of 2048-2048-2048-10 24.3 -> 17.8 us; 64 of 4096-4096-256-10 27.5 -> 18.1; 37 of 784-1024-1024-10 16.8 -> 14.9.
 // A cluster takes one tile: the grid has B200_CLUSTER_K CTAs for each.
 #if B200_CLUSTER_K > 1
 #define B200_X_GROUPS (4 / B200_CLUSTER_K)                 // groups of 32 rows that a CTA finishes
