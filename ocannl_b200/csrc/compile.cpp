@@ -60,15 +60,20 @@ std::set<int> find_deciding(const Program& P) {
                                      both = {"lt", "eq", "ne", "or", "and", "mod"};
   std::set<int> found;
   std::map<int, std::set<int>> made_from;
+  auto local = [](int scope_id) { return -1 - scope_id; };   // scalar locals stand beside the nodes
   walk_stmt(*P.body, [](const Scalar&) {}, [&](const Stmt& st) {
-    if (st.kind != Stmt::Set) return;
+    if (st.kind != Stmt::Set && st.kind != Stmt::SetLocal) return;
+    const int target = st.kind == Stmt::Set ? st.tn : local(st.scope_id);
     std::set<int> all;
     bool open = is_int_prec(P.tn(st.tn).prec);   // values of scopes are followed to the whole assignment
     bool own = open;                             // a sum of this assignment decides something
     auto reads = [&](const Scalar& e, std::set<int>& into) {
       walk_scalar(e, [&](const Scalar& x) {
         if (x.kind == Scalar::Get || x.kind == Scalar::GetDyn || x.kind == Scalar::GetMerge) into.insert(x.tn);
-        if (x.kind == Scalar::GetLocal) open = open || &into == &found;
+        if (x.kind == Scalar::GetLocal) {
+          into.insert(local(x.scope_id));
+          open = open || &into == &found;
+        }
         if (x.kind == Scalar::GetLocal || x.kind == Scalar::LocalScope) own = own || &into == &found;
       }, [](const Stmt&) {});
     };
@@ -81,8 +86,8 @@ std::set<int> find_deciding(const Program& P) {
         if (both.count(x.op) || (a == 0 && first.count(x.op))) reads(*x.args[a].s, found);
     }, [](const Stmt&) {});
     if (open) found.insert(all.begin(), all.end());
-    if (own) found.insert(st.tn);
-    made_from[st.tn].insert(all.begin(), all.end());
+    if (own) found.insert(target);
+    made_from[target].insert(all.begin(), all.end());
   });
   std::vector<int> todo(found.begin(), found.end());
   while (!todo.empty()) {

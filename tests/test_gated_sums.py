@@ -1,10 +1,10 @@
 """Which contractions share their k blocks over a cluster (another order of the sums): none whose result a gate or a comparison
-reads, directly or through what is made of it; the others of the same routine as before.  Plans only, no GPU."""
+reads, directly, through what is made of it or through a local; the others of the same routine as before.  Plans only, no GPU."""
 import pytest
 
 from ocannl_b200 import backend as bk
 from ocannl_b200 import workloads as W
-from ocannl_b200.low_level import Routine, Seq, Set, binop, loops, un, where
+from ocannl_b200.low_level import DeclareLocal, GetLocal, Routine, Seq, Set, SetLocal, binop, loops, un, where
 
 
 def _clusters(ir):
@@ -56,4 +56,26 @@ def test_decisions_on_the_sum_itself(use, clustered, prec):
              "lt": lambda: binop("lt", s, d[i, j]), "where": lambda: where(binop("lt", s, d[i, j]), d[i, j], e[i, j]), "trunc": lambda: un("trunc", s), "not": lambda: un("not", s),
              "value of gate": lambda: binop("relu_gate", d[i, j], s), "value of where": lambda: where(d[i, j], s, 0.0)}[use]
     r.body = Seq([loops([(i, m), (j, n)], Set(c, (i, j), value()))])
+    assert _clusters(r) == [clustered]
+
+
+@pytest.mark.parametrize("use,clustered", [("plain", True), ("gate", False), ("behind", False), ("two locals", False)])
+def test_decisions_on_a_local(use, clustered):
+    """The sum's node is read into a local of the loop body, and the local decides."""
+    m, n, k = 64, 64, 1024
+    r = Routine("decide_local_" + use.replace(" ", "_"))
+    a, b = r.tn("a", "bfloat16", [m, k], read_only=True), r.tn("b", "bfloat16", [n, k], read_only=True)
+    c, d, e, f = r.tn("c", "single", [m, n]), r.tn("d", "single", [m, n], read_only=True), r.tn("e", "single", [m, n]), r.tn("f", "single", [m, n])
+    v, w = r.scope(r.tn("v", "single", [1], mode="virtual")), r.scope(r.tn("w", "single", [1], mode="virtual"))
+    i, j, p, q, s, x, y = r.syms(7)
+    body = [loops([(i, m), (j, n)], Set(c, (i, j), W.reduce_scope(r, "acc", "single", [(p, k)], lambda: (a[i, p], b[j, p]))))]
+    inner = [DeclareLocal(v, False), SetLocal(v, c[q, s] * 2.0)]
+    if use == "two locals":
+        inner += [DeclareLocal(w, False), SetLocal(w, GetLocal(v) + 1.0)]
+    got = GetLocal(w if use == "two locals" else v)
+    inner.append(Set(e, (q, s), got * d[q, s] if use in ("plain", "behind") else binop("relu_gate", got, d[q, s])))
+    body.append(loops([(q, m), (s, n)], Seq(inner)))
+    if use == "behind":
+        body.append(loops([(x, m), (y, n)], Set(f, (x, y), binop("relu_gate", e[x, y], d[x, y]))))
+    r.body = Seq(body)
     assert _clusters(r) == [clustered]
